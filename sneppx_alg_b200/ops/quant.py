@@ -10,6 +10,7 @@ import torch
 
 from . import _lib
 from ._lib import c_int, c_ll, ptr, stream
+from .gemm import _static
 
 E4M3_MAX = 448.0
 
@@ -207,7 +208,7 @@ def gemm_dequant(x, qweight, scales, mode="fp8", bias=None):
         b = bias.float().contiguous() if bias is not None else None
         _lib.call("sx_gemm_dequant", ptr(x2), c_ll(x2.stride(0)), ptr(qweight), ptr(scales.contiguous()), ptr(b),
                   ptr(out), c_ll(out.stride(0)), c_int(x2.shape[0]), c_int(N), c_int(K),
-                  c_int(0 if mode == "fp8" else 1), ptr(_lib.status_word(x.device)), stream())
+                  c_int(0 if mode == "fp8" else 1), c_int(int(_static.on and scales.is_contiguous())), ptr(_lib.status_word(x.device)), stream())
         return out.view(*x.shape[:-1], N)
     w = dequant_fp8(qweight.view(torch.float8_e4m3fn) if qweight.dtype == torch.uint8 else qweight, scales, "128x128",
                     torch.float32) if mode == "fp8" else dequant_int4(qweight, scales, torch.float32)

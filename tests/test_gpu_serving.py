@@ -114,6 +114,33 @@ def test_dequant_gemm(mode, M, N, K):
     assert _rel(y, ref) < 1.5e-2
 
 
+@pytest.mark.parametrize("mode", ["fp8", "int4"])
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64, 65, 128, 129])
+@pytest.mark.parametrize("N,K", [(128, 128), (200, 384), (4096, 4224), (1000, 3968)])
+def test_dequant_gemm_tiles(mode, M, N, K):
+    """Edges of the row tiles (16 / 32 / 64 / 128), ragged N, one and odd numbers of 128-wide k-blocks (an int4 stage holds two), K split
+    over clusters. Products of bf16 inputs with unscaled weight values are exact and summed in 32 bits, so against 64 bits only the
+    rounding of the bf16 output remains (8 significant bits: at most 2^-8 relative), plus 2^-20 of the sum of magnitudes for the 32-bit
+    sums."""
+    torch.manual_seed(M + N)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    if mode == "fp8":
+        q, s = quant.quant_fp8_128x128(w)
+        wd = q.double() * s.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+        q = q.view(torch.uint8)
+    else:
+        q, s = quant.quant_int4(w)
+        wd = torch.stack([q & 15, q >> 4], -1).view(N, K).double() - 8
+        wd = wd * s.double().repeat_interleave(128, 1)
+    bias = torch.randn(N, device="cuda")
+    y = quant.gemm_dequant(x, q, s, mode, bias)
+    ops.check_status()
+    ref = x.double() @ wd.t() + bias.double()
+    bound = ref.abs() * 2.0 ** -8 + (x.double().abs() @ wd.abs().t() + bias.abs().double()) * 2.0 ** -20
+    assert bool(((y.double() - ref).abs() <= bound).all())
+
+
 def test_paged_engine_matches_cached_generation_gpu():
     from sneppx_alg_b200.models import ModelConfig, build_model
     from sneppx_alg_b200.serving.generation import generate
