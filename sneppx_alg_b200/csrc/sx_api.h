@@ -382,6 +382,22 @@ int sx_ssd_gate(const SxSsdArgs* args, const float* o, cudaStream_t stream); // 
 int sx_ssd_step(const SxSsdArgs* args, cudaStream_t stream);       // one token per sequence, from u to y
 int sx_ssd_scan_ok(int P, int N);
 int sx_ssd_scan(const SxSsdArgs* args, cudaStream_t stream);       // prompt form on tensor cores (bf16): operands -> state, y
+// One token per sequence through a Mamba-2 layer (mamba_step.cu). Rows b < B; table [B, 3]: addresses of the sequence's fp32 states
+// [layers, H, P, N], of its convolution inputs [layers, taps - 1, C] (oldest first) and of where the shifted ones go.
+typedef struct SxMambaStepArgs {
+  const void* x; const void* res_in; void* res_out;      // [B, d]; res_in null: first layer (res_out null as well)
+  const void* norm_w; void* hn;                          // [d], [B, d]
+  const void* in_w; void* zx; long long zx_ld;           // [zx_ld, d], [B, zx_ld] = z | x | B | C | dt
+  const void* conv_w; const void* conv_b;                // [C, taps], [C]
+  const float* dt_bias; const float* a_log; const float* D;   // [H]
+  const void* gate_norm_w; void* g; void* gn;            // [H P], [B, H P] twice
+  const void* out_w; void* out;                          // [d, H P], [B, d]
+  const long long* table;
+  int B, d, H, P, N, G, taps, layer;
+  float eps, gate_eps;
+  int* status;
+} SxMambaStepArgs;
+int sx_mamba2_step(const SxMambaStepArgs* args, cudaStream_t stream);
 // Operands of window attention over tokens and averaged blocks, from projected rows u = q [H d] | k [G d] | v [G dv]: bias,
 // rotation of the first `rot` entries of query and key heads, rotation of whole value heads, cache append.
 typedef struct SxWinPrepArgs {

@@ -129,6 +129,16 @@ class SxSsdArgs(C.Structure):
     ]
 
 
+class SxMambaStepArgs(C.Structure):
+    _fields_ = [
+        ("x", c_void_p), ("res_in", c_void_p), ("res_out", c_void_p), ("norm_w", c_void_p), ("hn", c_void_p), ("in_w", c_void_p),
+        ("zx", c_void_p), ("zx_ld", c_ll), ("conv_w", c_void_p), ("conv_b", c_void_p), ("dt_bias", c_void_p), ("a_log", c_void_p),
+        ("D", c_void_p), ("gate_norm_w", c_void_p), ("g", c_void_p), ("gn", c_void_p), ("out_w", c_void_p), ("out", c_void_p),
+        ("table", c_void_p), ("B", c_int), ("d", c_int), ("H", c_int), ("P", c_int), ("N", c_int), ("G", c_int), ("taps", c_int),
+        ("layer", c_int), ("eps", c_float), ("gate_eps", c_float), ("status", c_void_p),
+    ]
+
+
 class SxWinPrepArgs(C.Structure):
     _fields_ = [
         ("u", c_void_p), ("u_ld", c_ll), ("bias", c_void_p), ("freq", c_void_p), ("vfreq", c_void_p), ("temp", c_void_p),

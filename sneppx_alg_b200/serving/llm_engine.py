@@ -22,6 +22,7 @@ from ..ops import paged
 from .generation import apply_repetition_penalty, sample_from_logits
 from .hybrid_runner import HybridRunner
 from .kv_cache import PagedKVCache
+from .mamba_states import SequenceStates, decode_step
 
 
 @dataclass
@@ -336,14 +337,15 @@ class StatefulRunner:
     """Runs any model that follows the generation contract ``forward(input_ids, past_key_values, use_cache) ->
     {"logits", "past_key_values"}`` with a per-layer state of tensors batched along dim 0 (``Mamba2ForCausalLM``: a
     list of {"conv", "ssm"} dicts). Prefill runs one sequence; decode stacks the states of all running sequences,
-    advances them together by one token, and splits them again."""
+    advances them together by one token, and splits them again. A bf16 ``Mamba2ForCausalLM`` on a GPU steps its states where
+    they lie instead (``mamba_states.decode_step``)."""
 
     def __init__(self, model):
         self.model = model
-        self.states = {}
+        self.states = SequenceStates()
 
     def release(self, seq_id):
-        self.states.pop(seq_id, None)
+        dict.pop(self.states, seq_id, None)
 
     @torch.no_grad()
     def prefill(self, seq_id: int, tokens: List[int], start: int):
@@ -361,6 +363,9 @@ class StatefulRunner:
 
     @torch.no_grad()
     def decode(self, seq_ids: List[int], last_tokens: List[int]):
+        logits = decode_step(self.model, self.states, seq_ids, last_tokens)
+        if logits is not None:
+            return logits
         dev = next(self.model.parameters()).device
         batched = self._stack([self.states[s] for s in seq_ids])
         ids = torch.tensor(last_tokens, dtype=torch.long, device=dev).unsqueeze(1)

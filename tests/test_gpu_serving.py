@@ -165,3 +165,58 @@ def test_paged_engine_matches_cached_generation_gpu():
     eng2 = LLMEngine(model, num_blocks=256, block_size=16)
     assert len(eng2.generate(prompts[:2], SamplingParams(max_new_tokens=4))[0]) == 4
     ops.check_status()
+
+
+@pytest.mark.parametrize("hidden,headdim,state,groups,taps,layers,batch", [
+    (256, 64, 128, 1, 4, 3, 5), (320, 64, 128, 2, 4, 2, 1), (128, 32, 64, 4, 2, 1, 17), (192, 24, 40, 2, 3, 2, 3), (256, 128, 256, 1, 4, 2, 128),
+    (128, 16, 136, 16, 4, 2, 2), (64, 72, 8, 1, 2, 2, 4)])
+def test_mamba2_decode_step(hidden, headdim, state, groups, taps, layers, batch):
+    """The in-place decode step against the same weights in 32 bits on the CPU: logits and states over steps with a changing batch, state
+    rows and columns that do not fill a warp, two to four taps. A handed-out state is not written by later steps, a sequence twice in a
+    batch goes through the model's forward. Bound: every activation of a layer is rounded to bf16 (2^-9) about eight times, errors of the
+    layers add up; measured 0.003 to 0.012."""
+    import copy
+    from sneppx_alg_b200.models import ModelConfig, build_model
+    from sneppx_alg_b200.serving.llm_engine import StatefulRunner
+    from sneppx_alg_b200.serving.mamba_states import _Block
+    torch.manual_seed(hidden + state)
+    inner = 9 * 72 if headdim == 72 else 2 * hidden
+    cfg = ModelConfig(architecture="mamba2", hidden_size=hidden if headdim != 72 else 324 * 2, num_hidden_layers=layers, vocab_size=1000,
+                      ssm_state_size=state, ssm_expand=2 if headdim != 72 else 1, ssm_head_dim=headdim, ssm_ngroups=groups,
+                      ssm_conv_kernel=taps, rms_norm_eps=1e-5, tie_word_embeddings=True)
+    assert inner % headdim == 0
+    model = build_model(cfg, dtype=torch.bfloat16, device="cuda").eval()
+    with torch.no_grad():
+        for n, p in model.named_parameters():
+            if "conv_bias" in n or n.endswith(".D"):
+                p.copy_(torch.randn_like(p.float()))
+    plain = copy.deepcopy(model).float().cpu()
+    run, ref = StatefulRunner(model), StatefulRunner(plain)
+    g = torch.Generator().manual_seed(1)
+    for sid in range(batch):
+        # the same states on both sides
+        st = [{"conv": torch.randn(1, taps - 1, plain.layers[0].mixer.conv_dim, generator=g).bfloat16(),
+               "ssm": 0.3 * torch.randn(1, plain.layers[0].mixer.nheads, headdim, state, generator=g)} for _ in range(layers)]
+        run.states[sid] = [{k: v.cuda() for k, v in d.items()} for d in st]
+        ref.states[sid] = [{k: v.float() for k, v in d.items()} for d in st]
+
+    def close(a, b):
+        return (a.cpu().float() - b).norm().item() <= 0.03 * b.norm().item()
+
+    kept = None
+    for step in range(4):
+        ids = list(range(batch)) if step != 1 else list(range(batch - 1, -1, -2))
+        tokens = [(37 * step + 11 * i) % 1000 for i in ids]
+        a, b = run.decode(ids, tokens), ref.decode(ids, tokens)
+        ops.check_status()
+        assert a.shape == (len(ids), 1000) and a.dtype == torch.float32 and close(a, b)
+        assert all(isinstance(run.states.entry(i), _Block) for i in ids)
+        if step == 1:
+            kept = run.states[ids[0]]
+            before = [{k: v.clone() for k, v in d.items()} for d in kept]
+    for sid in range(batch):
+        for x, y in zip(run.states[sid], ref.states[sid]):
+            assert close(x["ssm"], y["ssm"]) and close(x["conv"], y["conv"])
+    assert all(torch.equal(x[k], y[k]) for x, y in zip(kept, before) for k in x)
+    a, b = run.decode([0, 0], [3, 3]), ref.decode([0, 0], [3, 3])
+    assert close(a, b) and isinstance(run.states.entry(0), list)

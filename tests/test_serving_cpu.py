@@ -149,3 +149,33 @@ def test_prefix_cache_gives_blocks_back_under_pressure():
     assert rid in eng.failed and rid in done and not eng.has_work()
     # and the engine still serves afterwards
     assert eng.generate(ref_prompts[:1], SamplingParams(max_new_tokens=6))[0] == refs[0]
+
+
+def test_recurrent_states_leave_their_block_when_read():
+    """Every way of reading a sequence's states gives the ordinary per-layer dicts with the values of the buffer that is current, and
+    the sequence keeps what was handed out."""
+    import copy
+    import pickle
+    import torch
+    from sneppx_alg_b200.serving.mamba_states import SequenceStates, _Block
+
+    def fresh():
+        s, b = SequenceStates(), _Block(torch.arange(2 * 3 * 4 * 8.).view(2, 3, 4, 8), torch.arange(2 * 2 * 3 * 5.).view(2, 2, 3, 5))
+        b.cur = 1
+        dict.__setitem__(s, 7, b)
+        s[8] = [{"conv": None, "ssm": None}]
+        return s, b
+
+    reads = [lambda s: s[7], lambda s: s.get(7), lambda s: list(s.values())[0], lambda s: dict(s.items())[7], lambda s: dict(s)[7],
+             lambda s: {**s}[7], lambda s: s.copy()[7], lambda s: (s | {})[7], lambda s: copy.copy(s)[7],
+             lambda s: pickle.loads(pickle.dumps(s))[7], lambda s: s.setdefault(7), lambda s: s.pop(7)]
+    for read in reads:
+        s, b = fresh()
+        got = read(s)
+        assert type(got) is list and len(got) == 2
+        for i, layer in enumerate(got):
+            assert torch.equal(layer["ssm"], b.ssm[i:i + 1]) and torch.equal(layer["conv"], b.conv[1, i:i + 1])
+        assert not any(isinstance(s.entry(k), _Block) for k in s.keys())
+    s, b = fresh()
+    assert s.entry(7) is b and 7 in s and len(s) == 2 and s.get(9) is None
+    assert s != {} and SequenceStates() == {}
