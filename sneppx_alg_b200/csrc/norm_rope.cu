@@ -11,14 +11,88 @@
 
 namespace sx {
 
+// Sum over the block with one barrier: every thread adds the warps' partial sums. `red`: 32 floats, not reused before the next barrier.
+__device__ __forceinline__ float row_sum(float v, float* red) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum(lane < nw ? red[lane] : 0.f);
+}
+
 // y = rmsnorm(x + res_in) * w ; res_out = x + res_in ; rstd saved for backward.
-__global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                          const __nv_bfloat16* __restrict__ res_in,
-                                                          const __nv_bfloat16* __restrict__ w,
-                                                          __nv_bfloat16* __restrict__ y,
-                                                          __nv_bfloat16* __restrict__ res_out,
-                                                          float* __restrict__ rstd, int d, float eps) {
+// Bound: memory. A row stays in the registers of one CTA between the sum and the output (V vectors of 8 a thread), so it is read once and
+// all of its loads are in flight together; rows are spread over CTAs and overlap. Two vectors a thread keep CTAs small enough that
+// several share an SM. [4096, 4096] with residual: 31 us with a cold L2 full of dirty lines (read + write once: 20 us at copy
+// bandwidth), 37 us when a second pass
+// read the row again.
+template <int V>
+__global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in,
+                                                           const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                                                           __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd, int d, float eps) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a dependent launch may start its prologue
+  __shared__ float red[32];
+  const long long row = blockIdx.x;
+  const int nvec = d >> 3, t = threadIdx.x;
+  bf16x8 a[V], b[V], wv[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int i = t + k * blockDim.x;
+    if (i < nvec) {
+      a[k] = ld8(x + row * d + i * 8);
+      if (res_in) b[k] = ld8(res_in + row * d + i * 8);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < V; ++k)
+    if (t + k * blockDim.x < nvec) wv[k] = ld8(w + (t + k * blockDim.x) * 8);
+  float f[V][8], ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int i = t + k * blockDim.x;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[k][j] = 0.f;
+    if (i >= nvec) continue;
+    unpack8(a[k], f[k]);
+    float h[8];
+    if (res_in) {
+      unpack8(b[k], h);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[k][j] += h[j];
+      // round through bf16 so that the statistics match what backward will re-read
+      const bf16x8 hp = pack8(f[k]);
+      unpack8(hp, h);
+      if (res_out) {
+        st8(res_out + row * d + i * 8, hp);
+        unpack8(hp, f[k]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) h[j] = f[k][j];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += h[j] * h[j];
+  }
+  ss = row_sum(ss, red);
+  const float r = rsqrtf(ss / d + eps);
+  if (t == 0 && rstd) rstd[row] = r;
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    const int i = t + k * blockDim.x;
+    if (i >= nvec) continue;
+    float g[8];
+    unpack8(wv[k], g);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g[j] = f[k][j] * r * g[j];
+    st8(y + row * d + i * 8, pack8(g));
+  }
+}
+// Rows longer than 8192: two passes.
+__global__ void __launch_bounds__(256) rmsnorm_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in,
+                                                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                                                               __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd, int d,
+                                                               float eps) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float red[33];
   const long long row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * d;
@@ -32,7 +106,6 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
       unpack8(ld8(res_in + row * d + i * 8), g);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] += g[j];
-      // round through bf16 so that the statistics match what backward will re-read
       bf16x8 hp = pack8(f);
       unpack8(hp, f);
       if (res_out) st8(res_out + row * d + i * 8, hp);
@@ -60,84 +133,114 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
 }
 
 // dx = rstd * (w*dy) - h * rstd^3 * mean(w*dy*h) (+ dres) ; dw partial sums per CTA.
-// Each CTA walks rows blockIdx.x, blockIdx.x + gridDim.x, ... and keeps its dw partials in
-// registers (thread t owns column vectors t, t + blockDim, ...; at most MAXV of them).
-template <int MAXV>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                          const __nv_bfloat16* __restrict__ h,
-                                                          const __nv_bfloat16* __restrict__ w,
-                                                          const float* __restrict__ rstd,
-                                                          const __nv_bfloat16* __restrict__ dres,
-                                                          __nv_bfloat16* __restrict__ dx,
+// Each CTA walks rows blockIdx.x, blockIdx.x + gridDim.x, ... and keeps its dw partials in registers (thread t owns column vectors
+// t, t + blockDim, ...; at most V of them). Bound: memory; the loads of the next row are issued before the sum of this one, otherwise
+// a CTA has one row in flight and the barrier's latency between rows. [4096, 4096] with dres: 46 us (20 us at copy bandwidth) with the
+// reduction of the partials, 75 us before; [8192, 5120]: 122 and 263 us.
+template <int V>
+__global__ void __launch_bounds__(512) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
+                                                          const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
+                                                          const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                                                           float* __restrict__ dw_partial, int T, int d) {
-  __shared__ float red[33];
-  const int nvec = d >> 3;
-  float acc[MAXV][8];
-  float wv[MAXV][8];
+  __shared__ float red[2][32];
+  const int nvec = d >> 3, t = threadIdx.x;
+  float acc[V][8];
+  bf16x8 wv[V], gv[V], hv[V], ev[V], gn[V], hn[V], en[V];
+  float rn = 0.f;
 #pragma unroll
-  for (int k = 0; k < MAXV; ++k) {
-    const int i = threadIdx.x + k * blockDim.x;
+  for (int k = 0; k < V; ++k) {
+    const int i = t + k * blockDim.x;
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[k][j] = 0.f;
-    if (i < nvec) unpack8(ld8(w + i * 8), wv[k]);
+    if (i < nvec) wv[k] = ld8(w + i * 8);
   }
-  for (long long row = blockIdx.x; row < T; row += gridDim.x) {
-    const float r = rstd[row];
-    float dot = 0.f;
-    float g[MAXV][8], hv[MAXV][8];
+  auto fetch = [&](long long row) {
+    rn = rstd[row];
 #pragma unroll
-    for (int k = 0; k < MAXV; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
+    for (int k = 0; k < V; ++k) {
+      const int i = t + k * blockDim.x;
       if (i < nvec) {
-        unpack8(ld8(dy + row * d + i * 8), g[k]);
-        unpack8(ld8(h + row * d + i * 8), hv[k]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          acc[k][j] += g[k][j] * hv[k][j] * r;
-          g[k][j] *= wv[k][j];
-          dot += g[k][j] * hv[k][j];
-        }
+        gn[k] = ld8(dy + row * d + i * 8);
+        hn[k] = ld8(h + row * d + i * 8);
+        if (dres) en[k] = ld8(dres + row * d + i * 8);
       }
     }
-    dot = block_sum(dot, red);
+  };
+  if ((int)blockIdx.x < T) fetch(blockIdx.x);
+  int buf = 0;
+  for (long long row = blockIdx.x; row < T; row += gridDim.x, buf ^= 1) {
+    const float r = rn;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      gv[k] = gn[k];
+      hv[k] = hn[k];
+      ev[k] = en[k];
+    }
+    if (row + gridDim.x < T) fetch(row + gridDim.x);
+    float dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      if (t + k * blockDim.x >= nvec) continue;
+      float g[8], hh[8], ww[8];
+      unpack8(gv[k], g);
+      unpack8(hv[k], hh);
+      unpack8(wv[k], ww);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        acc[k][j] += g[j] * hh[j] * r;
+        dot += g[j] * ww[j] * hh[j];
+      }
+    }
+    dot = row_sum(dot, red[buf]);      // two buffers: the next row's partial sums do not meet slow readers of this one's
     const float c = dot * r * r * r / d;
 #pragma unroll
-    for (int k = 0; k < MAXV; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
-      if (i < nvec) {
-        float o[8];
+    for (int k = 0; k < V; ++k) {
+      const int i = t + k * blockDim.x;
+      if (i >= nvec) continue;
+      float g[8], hh[8], ww[8];
+      unpack8(gv[k], g);
+      unpack8(hv[k], hh);
+      unpack8(wv[k], ww);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = g[k][j] * r - hv[k][j] * c;
-        if (dres) {
-          float e[8];
-          unpack8(ld8(dres + row * d + i * 8), e);
+      for (int j = 0; j < 8; ++j) g[j] = g[j] * ww[j] * r - hh[j] * c;
+      if (dres) {
+        unpack8(ev[k], hh);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += e[j];
-        }
-        st8(dx + row * d + i * 8, pack8(o));
+        for (int j = 0; j < 8; ++j) g[j] += hh[j];
       }
+      st8(dx + row * d + i * 8, pack8(g));
     }
   }
 #pragma unroll
-  for (int k = 0; k < MAXV; ++k) {
-    const int i = threadIdx.x + k * blockDim.x;
+  for (int k = 0; k < V; ++k) {
+    const int i = t + k * blockDim.x;
     if (i < nvec) {
-      float* o = dw_partial + (long long)blockIdx.x * d + i * 8;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = acc[k][j];
+      float4* o = reinterpret_cast<float4*>(dw_partial + (long long)blockIdx.x * d + i * 8);
+      o[0] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+      o[1] = make_float4(acc[k][4], acc[k][5], acc[k][6], acc[k][7]);
     }
   }
 }
 
-__global__ void colsum_partials_kernel(const float* __restrict__ part, int nparts, int d,
-                                       __nv_bfloat16* __restrict__ out_bf16, float* __restrict__ out_f32,
-                                       int accumulate) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d) return;
+// Column sums of the partial rows: 32 columns x 32 row groups a CTA (one thread a column walked all rows one after another: 16 us at 296
+// rows of 4096; with it [512, 512] backward took 21.5 us, now 13).
+__global__ void __launch_bounds__(1024) colsum_partials_kernel(const float* __restrict__ part, int nparts, int d,
+                                                               __nv_bfloat16* __restrict__ out_bf16, float* __restrict__ out_f32,
+                                                               int accumulate) {
+  __shared__ float red[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
   float s = 0.f;
-  for (int p = 0; p < nparts; ++p) s += part[(long long)p * d + c];
-  if (out_f32) out_f32[c] = accumulate ? out_f32[c] + s : s;
-  if (out_bf16) out_bf16[c] = __float2bfloat16(accumulate ? __bfloat162float(out_bf16[c]) + s : s);
+  if (c < d) {
+#pragma unroll 4
+    for (int p = ty; p < nparts; p += 32) s += part[(long long)p * d + c];
+  }
+  red[ty][tx] = s;
+  __syncthreads();
+  s = warp_sum(red[tx][ty]);             // warp ty adds column ty of the block
+  const int co = blockIdx.x * 32 + ty;
+  if (tx != 0 || co >= d) return;
+  if (out_f32) out_f32[co] = accumulate ? out_f32[co] + s : s;
+  if (out_bf16) out_bf16[co] = __float2bfloat16(accumulate ? __bfloat162float(out_bf16[co]) + s : s);
 }
 
 __global__ void __launch_bounds__(256) layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
@@ -297,34 +400,40 @@ extern "C" int sx_rmsnorm_fwd(const void* x, const void* res_in, const void* w, 
                               long long T, int d, float eps, cudaStream_t st) {
   if (d % 8) return -1;
   if (T == 0) return 0;
-  rmsnorm_fwd_kernel<<<(unsigned)T, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res_in,
-                                                  (const __nv_bfloat16*)w, (__nv_bfloat16*)y,
-                                                  (__nv_bfloat16*)res_out, rstd, d, eps);
+  const int nvec = d / 8;
+  auto run = [&](auto kern, int threads) {
+    kern<<<(unsigned)T, threads, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res_in, (const __nv_bfloat16*)w, (__nv_bfloat16*)y,
+                                          (__nv_bfloat16*)res_out, rstd, d, eps);
+  };
+  auto per = [&](int v) { return ((nvec + v - 1) / v + 31) / 32 * 32; };
+  // one vector a thread for rows up to 1024, two up to 8192; a CTA of 1024 threads has an SM to itself, and two passes over L2 are
+  // faster then ([1000, 16384]: 37 against 43 us)
+  if (nvec <= 128) run(rmsnorm_fwd_kernel<1>, per(1));
+  else if (nvec <= 1024) run(rmsnorm_fwd_kernel<2>, per(2));
+  else run(rmsnorm_fwd_long_kernel, 256);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 // dw_partial: scratch of nparts*d floats (nparts = value returned by sx_rmsnorm_bwd_parts()).
-extern "C" int sx_rmsnorm_bwd_parts() { return 296; }
+extern "C" int sx_rmsnorm_bwd_parts() { return 592; }
 
 extern "C" int sx_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const void* dres,
                               void* dx, float* dw_partial, void* dw_bf16, float* dw_f32, int accumulate, long long T,
                               int d, cudaStream_t st) {
   if (d % 8) return -1;
   if (T == 0) return 0;
-  const int parts = sx_rmsnorm_bwd_parts();
   const int nvec = d / 8;
-  const int need = (nvec + 255) / 256;
-  auto args = [&](auto kern) {
-    kern<<<parts, 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, rstd,
-                                (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, (int)T, d);
+  const int most = nvec <= 256 ? 592 : 296;      // short rows: four small CTAs an SM keep as much in flight as two large ones
+  const int parts = T < most ? (int)T : most;
+  auto run = [&](auto kern, int v) {
+    kern<<<parts, ((nvec + v - 1) / v + 31) / 32 * 32, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w,
+                                                               rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, (int)T, d);
   };
-  if (need <= 1) args(rmsnorm_bwd_kernel<1>);
-  else if (need <= 2) args(rmsnorm_bwd_kernel<2>);
-  else if (need <= 4) args(rmsnorm_bwd_kernel<4>);
-  else if (need <= 8) args(rmsnorm_bwd_kernel<8>);
+  if (nvec <= 128) run(rmsnorm_bwd_kernel<1>, 1);
+  else if (nvec <= 1024) run(rmsnorm_bwd_kernel<2>, 2);
+  else if (nvec <= 2048) run(rmsnorm_bwd_kernel<4>, 4);
   else return -2;
-  colsum_partials_kernel<<<(d + 255) / 256, 256, 0, st>>>(dw_partial, parts, d, (__nv_bfloat16*)dw_bf16, dw_f32,
-                                                          accumulate);
+  colsum_partials_kernel<<<(d + 31) / 32, 1024, 0, st>>>(dw_partial, parts, d, (__nv_bfloat16*)dw_bf16, dw_f32, accumulate);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
