@@ -274,22 +274,26 @@ extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, con
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
-// Number of partial rows the backward kernel writes for B sequences of L tokens.
-extern "C" int sx_conv1d_bwd_parts(int B, int L) {
+// Number of partial rows the backward kernel writes for B sequences of L tokens of C channels.
+extern "C" int sx_conv1d_bwd_parts(int B, int L, int C) {
   // four runs per warp (32 per CTA): the per-CTA prologue (taps, bias) and epilogue (partial row) cost about as much
-  // as one run
+  // as one run. Inputs that would leave SMs idle that way take as many CTAs as make one wave (two an SM), down to one
+  // run per warp ([4, 500, 1792]: 73 -> 32 us)
   const long long chunks = (long long)B * ((L + CONV_BTL - 1) / CONV_BTL);
-  const long long p = (chunks + 31) / 32;
+  const int cols = (C / CONV_BV + 31) / 32;
+  const long long wave = 296 / (cols > 0 ? cols : 1), most = (chunks + 7) / 8;
+  long long p = (chunks + 31) / 32;
+  if (p < wave) p = most < wave ? most : wave;
   return (int)(p < 1 ? 1 : (p > 512 ? 512 : p));
 }
 
-// partial: scratch of sx_conv1d_bwd_parts(B, L) * (K+1) * C floats; dwdb: fp32 [(K+1)*C] = dw [C][K] then db [C].
+// partial: scratch of sx_conv1d_bwd_parts(B, L, C) * (K+1) * C floats; dwdb: fp32 [(K+1)*C] = dw [C][K] then db [C].
 extern "C" int sx_conv1d_bwd(const void* dy, const void* x, const void* prev, const void* w, const void* bias, void* dx,
                              float* partial, float* dwdb, int B, int L, int C, int K, int act, long long xld,
                              cudaStream_t st) {
   if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C) return -1;
   if ((long long)B * L == 0) return 0;
-  const int parts = sx_conv1d_bwd_parts(B, L);
+  const int parts = sx_conv1d_bwd_parts(B, L, C);
   const dim3 grid((C / CONV_BV + 31) / 32, parts);
 #define SX_CONV_BWD(KK)                                                                                          \
   conv1d_bwd_kernel<KK><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,                  \

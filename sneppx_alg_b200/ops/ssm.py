@@ -54,7 +54,7 @@ class _Conv1dFn(torch.autograd.Function):
         K = w.shape[1]
         dy = dy.contiguous()
         dx = torch.empty(B, L, C, dtype=x.dtype, device=x.device)
-        parts = _lib.lib().sx_conv1d_bwd_parts(c_int(B), c_int(L))
+        parts = _lib.lib().sx_conv1d_bwd_parts(c_int(B), c_int(L), c_int(C))
         partial = torch.empty(parts * (K + 1) * C, dtype=torch.float32, device=x.device)
         dwdb = torch.empty((K + 1) * C, dtype=torch.float32, device=x.device)
         _lib.call("sx_conv1d_bwd", ptr(dy), ptr(x), ptr(prev if has_p else None), ptr(w), ptr(bias if has_b else None),
