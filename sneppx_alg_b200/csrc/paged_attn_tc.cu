@@ -55,14 +55,15 @@ struct PtItem {
   int b, hk, split, len, t0, n_steps;
 };
 
-// Work item `item` of the (split, KV head, sequence) space, sequences fastest so that neighbouring CTAs hold different
-// sequences; its tile range comes from the sequence length on the device.
+// Work item `item` of the (sequence, split, KV head) space, heads fastest: a cached position's heads lie side by side (256 bytes each), and
+// neighbouring CTAs that walk the same positions at the same time read whole DRAM pages together (48 sequences of 900 - 1800 positions, 8 heads:
+// 72 us with sequences fastest, 67 us). The tile range comes from the sequence length on the device.
 __device__ __forceinline__ PtItem pt_item(const PagedTcParams& p, int item) {
   PtItem w;
-  w.b = item % p.B;
-  const int rest = item / p.B;
-  w.hk = rest % p.Hkv;
-  w.split = rest / p.Hkv;
+  w.hk = item % p.Hkv;
+  const int rest = item / p.Hkv;
+  w.split = rest % p.nsplit;
+  w.b = rest / p.nsplit;
   w.len = p.seq_lens[w.b];
   const int tiles = (w.len + PT_BN - 1) / PT_BN;
   const int per = (tiles + p.nsplit - 1) / p.nsplit;
