@@ -43,6 +43,23 @@ class KVBlockPool:
         elif self.ref[b] < 0:
             raise RuntimeError(f"double free of KV block {b}")
 
+    def share_all(self, blocks) -> List[int]:
+        """``share`` of every block of a table."""
+        ref = self.ref
+        for b in blocks:
+            ref[b] += 1
+        return list(blocks)
+
+    def release_all(self, blocks) -> None:
+        """``release`` of every block of a table, in order."""
+        ref, free = self.ref, self.free
+        for b in blocks:
+            ref[b] = left = ref[b] - 1
+            if left <= 0:
+                if left < 0:
+                    raise RuntimeError(f"double free of KV block {b}")
+                free.append(b)
+
     @property
     def num_free(self) -> int:
         return len(self.free)
@@ -162,10 +179,9 @@ class PagedKVCache:
 
     def reserve(self, seq_id: int, n_new: int) -> List[int]:
         """Slots (block * block_size + offset) for the next ``n_new`` tokens, allocating / copying blocks as needed."""
-        table, n = self.tables[seq_id], self.lens[seq_id]
-        slots = []
-        for i in range(n, n + n_new):
-            bi, off = divmod(i, self.block_size)
+        table, n, bs = self.tables[seq_id], self.lens[seq_id], self.block_size
+        end, slots = n + n_new, []
+        for bi in range(n // bs, (end - 1) // bs + 1 if n_new > 0 else 0):
             if bi == len(table):
                 table.append(self.pool.allocate())
             elif self.pool.ref[table[bi]] > 1:      # shared block about to be written: copy on write
@@ -175,12 +191,13 @@ class PagedKVCache:
                     self.v[l][new].copy_(self.v[l][table[bi]])
                 self.pool.release(table[bi])
                 table[bi] = new
-            slots.append(table[bi] * self.block_size + off)
-        self.lens[seq_id] = n + n_new
+            first = (table[bi] - bi) * bs           # slot of position p: first + p
+            slots.extend(range(first + max(n, bi * bs), first + min(end, (bi + 1) * bs)))
+        self.lens[seq_id] = end
         return slots
 
     def fork(self, src_id: int, dst_id: int) -> None:
-        self.tables[dst_id] = [self.pool.share(b) for b in self.tables[src_id]]
+        self.tables[dst_id] = self.pool.share_all(self.tables[src_id])
         self.lens[dst_id] = self.lens[src_id]
 
     def free_sequence(self, seq_id: int, tokens=None) -> None:
@@ -188,8 +205,7 @@ class PagedKVCache:
         n = self.lens.pop(seq_id, 0)
         if self.prefix is not None and tokens is not None:
             self.prefix.insert(tokens[:n], table)
-        for b in table:
-            self.pool.release(b)
+        self.pool.release_all(table)
 
     def block_table_tensor(self, seq_ids, device=None) -> Tuple[torch.Tensor, torch.Tensor]:
         mb = max(1, max(len(self.tables[s]) for s in seq_ids))
