@@ -35,7 +35,8 @@ NVCC_FLAGS = [
 ]
 # Sources whose arithmetic follows IEEE single precision (no approximate division / square root / exponential, no
 # flush of denormals): recurrent state and the paths that also run models in 32-bit.
-PRECISE_SOURCES = {"decoder_ops.cu", "mamba_step.cu", "recurrence.cu", "ssd_serve.cu", "talking_attn.cu", "window_attn.cu"}
+PRECISE_SOURCES = {"decoder_ops.cu", "mamba_step.cu", "recurrence.cu", "ssd_mix.cu", "ssd_serve.cu", "talking_attn.cu",
+                   "window_attn.cu"}
 
 # Named subsets of the sources for programs that need only part of the library; each is linked on its own.
 CUDA_SUBSETS = {

@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(256) conv1d_fwd_kernel(const __nv_bfloat16* __
                                                          const __nv_bfloat16* __restrict__ bias,
                                                          __nv_bfloat16* __restrict__ y,
                                                          __nv_bfloat16* __restrict__ state_out, int B, int L, int C,
-                                                         int act, long long xld) {
+                                                         int act, long long xld, int Ly) {
   const int cv = C >> 3;
   const int lchunks = (L + CONV_TL - 1) / CONV_TL;
   const long long total = (long long)B * lchunks * cv;
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) conv1d_fwd_kernel(const __nv_bfloat16* __
 #pragma unroll
           for (int j = 0; j < 8; ++j) acc[j] = silu_f(acc[j]);
         }
-        st8(y + ((long long)b * L + l) * C + c, pack8(acc));
+        st8(y + ((long long)b * Ly + l) * C + c, pack8(acc));
         if (state_out && l >= L - (K - 1)) st8(state_out + ((long long)b * (K - 1) + (l - (L - (K - 1)))) * C + c, raw);
 #pragma unroll
         for (int i = 0; i < CONV_MAXK - 1; ++i)
@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const __nv_bfloat16*
                                                             const __nv_bfloat16* __restrict__ w,
                                                             const __nv_bfloat16* __restrict__ bias,
                                                             __nv_bfloat16* __restrict__ dx, float* __restrict__ partial,
-                                                            int B, int L, int C, int act, long long xld) {
+                                                            int B, int L, int C, int act, long long xld, int Ly,
+                                                            long long dxld) {
   constexpr int V = CONV_BV;
   __shared__ float s_acc[32][(CONV_MAXK + 1) * V + 1];
   const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const __nv_bfloat16*
           }
         if (l < L) {
           ld4(x + ((long long)b * L + l) * xld + c, xh[K - 1]);
-          ld4(dy + ((long long)b * L + l) * C + c, dph[K - 1]);
+          ld4(dy + ((long long)b * Ly + l) * C + c, dph[K - 1]);
           if (act) {
 #pragma unroll
             for (int j = 0; j < V; ++j) {
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const __nv_bfloat16*
             for (int k = 0; k < K; ++k) a += wv[k][j] * dph[K - 1 - k][j];
             dxa[j] = a;
           }
-          st4(dx + ((long long)b * L + lo) * C + c, dxa);
+          st4(dx + ((long long)b * L + lo) * dxld + c, dxa);
         }
       }
     }
@@ -254,16 +255,17 @@ __global__ void conv1d_reduce_partials(const float* __restrict__ part, int npart
 }  // namespace sx
 using namespace sx;
 
+// Sequences are L rows of pitch xld in x and Ly rows of pitch C in y (and in dy below; rows from L on are not touched).
 extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, const void* bias, void* y, void* state_out,
-                             int B, int L, int C, int K, int act, long long xld, cudaStream_t st) {
-  if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C) return -1;
+                             int B, int L, int C, int K, int act, long long xld, int Ly, cudaStream_t st) {
+  if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L) return -1;
   const long long total = (long long)B * ((L + CONV_TL - 1) / CONV_TL) * (C / 8);
   if (total == 0) return 0;
   const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
 #define SX_CONV_FWD(KK)                                                                                          \
   conv1d_fwd_kernel<KK><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)prev,              \
                                                 (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y, \
-                                                (__nv_bfloat16*)state_out, B, L, C, act, xld)
+                                                (__nv_bfloat16*)state_out, B, L, C, act, xld, Ly)
   switch (K) {
     case 1: SX_CONV_FWD(1); break;
     case 2: SX_CONV_FWD(2); break;
@@ -288,17 +290,18 @@ extern "C" int sx_conv1d_bwd_parts(int B, int L, int C) {
 }
 
 // partial: scratch of sx_conv1d_bwd_parts(B, L, C) * (K+1) * C floats; dwdb: fp32 [(K+1)*C] = dw [C][K] then db [C].
+// dx: rows of pitch dxld.
 extern "C" int sx_conv1d_bwd(const void* dy, const void* x, const void* prev, const void* w, const void* bias, void* dx,
-                             float* partial, float* dwdb, int B, int L, int C, int K, int act, long long xld,
-                             cudaStream_t st) {
-  if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C) return -1;
+                             float* partial, float* dwdb, int B, int L, int C, int K, int act, long long xld, int Ly,
+                             long long dxld, cudaStream_t st) {
+  if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L || dxld % 4 || dxld < C) return -1;
   if ((long long)B * L == 0) return 0;
   const int parts = sx_conv1d_bwd_parts(B, L, C);
   const dim3 grid((C / CONV_BV + 31) / 32, parts);
 #define SX_CONV_BWD(KK)                                                                                          \
   conv1d_bwd_kernel<KK><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,                  \
                                               (const __nv_bfloat16*)prev, (const __nv_bfloat16*)w,                \
-                                              (const __nv_bfloat16*)bias, (__nv_bfloat16*)dx, partial, B, L, C, act, xld)
+                                              (const __nv_bfloat16*)bias, (__nv_bfloat16*)dx, partial, B, L, C, act, xld, Ly, dxld)
   switch (K) {
     case 1: SX_CONV_BWD(1); break;
     case 2: SX_CONV_BWD(2); break;

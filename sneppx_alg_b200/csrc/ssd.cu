@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(256) ssd_bwd_rows2_kernel(const __nv_bfloat16*
                                                             const float* __restrict__ decay, const float* __restrict__ D,
                                                             __nv_bfloat16* __restrict__ dx, float* __restrict__ ddecay,
                                                             long long rows, int H, int Q, int vp, long long xld,
-                                                            int G) {
+                                                            int G, long long dxld) {
   const long long total = rows * vp;
   const long long span = ((total + 255) / 256) * 256;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < span; i += gridDim.x * 256ll) {
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(256) ssd_bwd_rows2_kernel(const __nv_bfloat16*
         o[j] = d * g[j] + dc * a[j] + b[j];
         s += a[j] * xv[j];
       }
-      st8(dx + i * 8, pack8(o));
+      st8(dx + t * dxld + (h * vp + pv) * 8, pack8(o));
     }
     s = seg_sum(s, vp);
     if (live && (i % vp) == 0) ddecay[r] = s;
@@ -320,16 +320,17 @@ __global__ void __launch_bounds__(256) ssd_heads_first_kernel(const __nv_bfloat1
   }
 }
 
-// Gate of the Mamba-2 block: out = y * silu(z), z read in place from a wider row-major tensor (row stride zld).
+// Gate of the Mamba-2 block: out = y * silu(z), z read in place from a wider row-major tensor (row stride zld). y (and dy) holds Lp rows for
+// every L rows of the others.
 __global__ void __launch_bounds__(256) gate_mul_fwd_kernel(const __nv_bfloat16* __restrict__ y,
                                                            const __nv_bfloat16* __restrict__ z, long long zld,
-                                                           __nv_bfloat16* __restrict__ out, long long rows, int cv) {
+                                                           __nv_bfloat16* __restrict__ out, long long rows, int cv, int L, int Lp) {
   const long long total = rows * cv;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
     const long long r = i / cv;
     const int c = (int)(i % cv) * 8;
     float a[8], b[8];
-    unpack8(ld8(y + i * 8), a);
+    unpack8(ld8(y + (r / L * Lp + r % L) * cv * 8 + c), a);
     unpack8(ld8(z + r * zld + c), b);
 #pragma unroll
     for (int j = 0; j < 8; ++j) a[j] *= b[j] / (1.f + __expf(-b[j]));
@@ -340,14 +341,14 @@ __global__ void __launch_bounds__(256) gate_mul_bwd_kernel(const __nv_bfloat16* 
                                                            const __nv_bfloat16* __restrict__ y,
                                                            const __nv_bfloat16* __restrict__ z, long long zld,
                                                            __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dz,
-                                                           long long rows, int cv) {
+                                                           long long rows, int cv, int L, int Lp, long long dzld) {
   const long long total = rows * cv;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
-    const long long r = i / cv;
+    const long long r = i / cv, yo = (r / L * Lp + r % L) * cv * 8;
     const int c = (int)(i % cv) * 8;
     float gv[8], a[8], b[8], oy[8], oz[8];
     unpack8(ld8(g + i * 8), gv);
-    unpack8(ld8(y + i * 8), a);
+    unpack8(ld8(y + yo + c), a);
     unpack8(ld8(z + r * zld + c), b);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -355,8 +356,8 @@ __global__ void __launch_bounds__(256) gate_mul_bwd_kernel(const __nv_bfloat16* 
       oy[j] = gv[j] * b[j] * sg;
       oz[j] = gv[j] * a[j] * sg * (1.f + b[j] * (1.f - sg));
     }
-    st8(dy + i * 8, pack8(oy));
-    st8(dz + i * 8, pack8(oz));
+    st8(dy + yo + c, pack8(oy));
+    st8(dz + r * dzld + c, pack8(oz));
   }
 }
 
@@ -445,32 +446,32 @@ extern "C" int sx_ssd_bwd_rows1(const void* dy, const void* x, const void* Yoff,
 
 extern "C" int sx_ssd_bwd_rows2(const void* dy, const void* x, const void* dxw, const void* dxi, const void* decay,
                                 const void* D, void* dx, void* ddecay, long long rows, int H, int Q, int P,
-                                long long xld, int G, cudaStream_t st) {
-  if (!vp_ok(P) || xld % 8 || H % G) return -1;
+                                long long xld, int G, long long dxld, cudaStream_t st) {
+  if (!vp_ok(P) || xld % 8 || dxld % 8 || H % G) return -1;
   if (rows == 0) return 0;
   ssd_bwd_rows2_kernel<<<row_grid(rows * (P / 8)), 256, 0, st>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dxw, (const __nv_bfloat16*)dxi,
       (const float*)decay,
-      (const float*)D, (__nv_bfloat16*)dx, (float*)ddecay, rows, H, Q, P / 8, xld, G);
+      (const float*)D, (__nv_bfloat16*)dx, (float*)ddecay, rows, H, Q, P / 8, xld, G, dxld);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 extern "C" int sx_gate_mul_fwd(const void* y, const void* z, long long zld, void* out, long long rows, int C,
-                               cudaStream_t st) {
-  if (C % 8 || zld % 8) return -1;
+                               int L, int Lp, cudaStream_t st) {
+  if (C % 8 || zld % 8 || L < 1 || Lp < L) return -1;
   if (rows == 0) return 0;
   gate_mul_fwd_kernel<<<row_grid(rows * (C / 8)), 256, 0, st>>>((const __nv_bfloat16*)y, (const __nv_bfloat16*)z, zld,
-                                                                 (__nv_bfloat16*)out, rows, C / 8);
+                                                                 (__nv_bfloat16*)out, rows, C / 8, L, Lp);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 extern "C" int sx_gate_mul_bwd(const void* g, const void* y, const void* z, long long zld, void* dy, void* dz,
-                               long long rows, int C, cudaStream_t st) {
-  if (C % 8 || zld % 8) return -1;
+                               long long rows, int C, int L, int Lp, long long dzld, cudaStream_t st) {
+  if (C % 8 || zld % 8 || dzld % 8 || L < 1 || Lp < L) return -1;
   if (rows == 0) return 0;
   gate_mul_bwd_kernel<<<row_grid(rows * (C / 8)), 256, 0, st>>>((const __nv_bfloat16*)g, (const __nv_bfloat16*)y,
                                                                  (const __nv_bfloat16*)z, zld, (__nv_bfloat16*)dy,
-                                                                 (__nv_bfloat16*)dz, rows, C / 8);
+                                                                 (__nv_bfloat16*)dz, rows, C / 8, L, Lp, dzld);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -53,7 +53,11 @@ class Mamba2Block(Module):
         incremental processing; it is updated in place when given."""
         B, L, _ = u.shape
         H, P, G, N = self.nheads, self.headdim, self.ngroups, self.d_state
-        z, xBC, dt = self.split(self.in_proj(u))
+        zx = self.in_proj(u)
+        mix = (self.conv_weight, self.conv_bias, self.dt_bias, self.A_log, self.D, H, P, G, N, min(self.chunk, 128))
+        if state is None and ssm.mixer_ok(zx, *mix):
+            return self.out_proj(self.norm(ssm.mamba2_mixer(zx, *mix)))
+        z, xBC, dt = self.split(zx)
         prev = state["conv"] if state is not None else None
         xBC_c = ssm.causal_conv1d(xBC, self.conv_weight, self.conv_bias, act=True, prev=prev)
         if state is not None:

@@ -11,6 +11,8 @@ of constant dt, B, C.
 """
 from __future__ import annotations
 
+import os
+
 import torch
 import torch.nn.functional as F
 
@@ -41,7 +43,7 @@ class _Conv1dFn(torch.autograd.Function):
             x = x.contiguous()
         y = torch.empty(B, L, C, dtype=x.dtype, device=x.device)
         _lib.call("sx_conv1d_fwd", ptr(x), ptr(prev), ptr(w), ptr(bias), ptr(y), ptr(None), c_int(B), c_int(L),
-                  c_int(C), c_int(K), c_int(int(act)), c_ll(x.stride(1)), stream())
+                  c_int(C), c_int(K), c_int(int(act)), c_ll(x.stride(1)), c_int(L), stream())
         ctx.save_for_backward(x, w, bias if bias is not None else torch.empty(0), prev if prev is not None else torch.empty(0))
         ctx.meta = (act, bias is not None, prev is not None)
         return y
@@ -59,7 +61,7 @@ class _Conv1dFn(torch.autograd.Function):
         dwdb = torch.empty((K + 1) * C, dtype=torch.float32, device=x.device)
         _lib.call("sx_conv1d_bwd", ptr(dy), ptr(x), ptr(prev if has_p else None), ptr(w), ptr(bias if has_b else None),
                   ptr(dx), ptr(partial), ptr(dwdb), c_int(B), c_int(L), c_int(C), c_int(K), c_int(int(act)),
-                  c_ll(x.stride(1)), stream())
+                  c_ll(x.stride(1)), c_int(L), c_ll(C), stream())
         dw = dwdb[: C * K].view(C, K).to(w.dtype)
         db = dwdb[C * K:].to(w.dtype) if has_b else None
         return dx, dw, db, None, None
@@ -79,7 +81,7 @@ class _GateMulFn(torch.autograd.Function):
         y = y.contiguous()
         zld = z.stride(-2)
         out = torch.empty_like(y)
-        _lib.call("sx_gate_mul_fwd", ptr(y), ptr(z), c_ll(zld), ptr(out), c_ll(rows), c_int(C_), stream())
+        _lib.call("sx_gate_mul_fwd", ptr(y), ptr(z), c_ll(zld), ptr(out), c_ll(rows), c_int(C_), c_int(1), c_int(1), stream())
         ctx.save_for_backward(y, z)
         return out
 
@@ -90,7 +92,7 @@ class _GateMulFn(torch.autograd.Function):
         g = g.contiguous()
         dy, dz = torch.empty_like(y), torch.empty(z.shape, dtype=z.dtype, device=z.device)
         _lib.call("sx_gate_mul_bwd", ptr(g), ptr(y), ptr(z), c_ll(z.stride(-2)), ptr(dy), ptr(dz),
-                  c_ll(y.numel() // C_), c_int(C_), stream())
+                  c_ll(y.numel() // C_), c_int(C_), c_int(1), c_int(1), c_ll(C_), stream())
         return dy, dz
 
 
@@ -330,13 +332,24 @@ def _bwd_rows2(dy5, x5, dxw, dxi, decay, D, cdt, G):
         ddecay = torch.empty(decay.shape, dtype=torch.float32, device=decay.device)
         _lib.call("sx_ssd_bwd_rows2", ptr(dy5), ptr(x5), ptr(dxw), ptr(dxi), ptr(decay),
                   ptr(D.float().contiguous() if D is not None else None), ptr(dx), ptr(ddecay), c_ll(decay.numel()),
-                  c_int(H), c_int(Q), c_int(P), c_ll(x5.stride(2)), c_int(G), stream())
+                  c_int(H), c_int(Q), c_int(P), c_ll(x5.stride(2)), c_int(G), c_ll(H * P), stream())
         return dx, ddecay
     dxw5 = _from_gf(dxw, x5.shape, G).float()
     dx = dxw5 * decay[..., None] + dxi.float().permute(0, 1, 3, 2, 4)
     if D is not None:
         dx = dx + dy5.float() * D.float().view(H, 1)
     return dx.to(cdt), (dxw5 * x5.float()).sum(-1)
+
+
+def _heads_first(t5):
+    """[B,nc,Q,H,P] -> contiguous [B*nc*H, Q, P]."""
+    B_, nc, Q, H, P = t5.shape
+    if t5.is_cuda and t5.dtype == torch.bfloat16 and _lib.available() and P % 8 == 0:
+        out = torch.empty(B_ * nc * H, Q, P, dtype=t5.dtype, device=t5.device)
+        _lib.call("sx_ssd_heads_first", ptr(t5), c_ll(t5.stride(2)), ptr(out), c_ll(out.shape[0] * Q), c_int(H), c_int(Q), c_int(P),
+                  stream())
+        return out
+    return t5.permute(0, 1, 3, 2, 4).contiguous().view(-1, Q, P)
 
 
 class _Chunks:
@@ -389,13 +402,7 @@ class _Chunks:
         return t.reshape(self.Bsz * self.nc * self.G, -1, self.N)
 
     def heads_first(self, t5):
-        """[B,nc,Q,H,P] -> contiguous [B*nc*H, Q, P]."""
-        if t5.is_cuda and t5.dtype == torch.bfloat16 and _lib.available() and self.P % 8 == 0:
-            out = torch.empty(self.Bsz * self.nc * self.H, self.Q, self.P, dtype=t5.dtype, device=t5.device)
-            _lib.call("sx_ssd_heads_first", ptr(t5), c_ll(t5.stride(2)), ptr(out), c_ll(out.shape[0] * self.Q),
-                      c_int(self.H), c_int(self.Q), c_int(self.P), stream())
-            return out
-        return t5.permute(0, 1, 3, 2, 4).contiguous().view(-1, self.Q, self.P)
+        return _heads_first(t5)
 
     def y_off(self, Hprev):
         B_, nc, Q, H, P, N = self.Bsz, self.nc, self.Q, self.H, self.P, self.N
@@ -413,7 +420,6 @@ def _chunk_fwd_fused(k, Bm, Cm, D, Hprev):
     group, M = C B^T o L o dt goes to the M X product straight from TMEM and the C Hprev^T term, the exp(cs) scaling
     and D x are applied in its epilogue. Covers chunk 128, state 128, headdim 64 without padding; returns None
     otherwise (``SX_SSD_FUSED=0`` forces the staged path)."""
-    import os
     if not (k.x5.is_cuda and k.cdt == torch.bfloat16 and k.Q == 128 and k.N == 128 and k.P == 64 and k.pad == 0
             and _lib.available() and k.Bsz * k.nc <= 65535 and os.environ.get("SX_SSD_FUSED", "1") != "0"
             and Bm.dtype == torch.bfloat16 and Cm.dtype == torch.bfloat16):
@@ -503,16 +509,170 @@ class _SSDFn(torch.autograd.Function):
                 dD.to(D.dtype) if D is not None else None, dinit if ctx.has_init else None, None)
 
 
-def ssd_scan(x, dt, A, Bm, Cm, D=None, chunk=64, init_state=None, return_state=False):
-    """Chunked SSD scan (forward and backward hand-written; see ``_SSDFn``). Same arguments as ``ssd_reference``."""
-    L = x.shape[1]
+def _chunk_size(chunk, L):
     chunk = max(8, min(int(chunk), 256))
     if chunk & (chunk - 1):
         chunk = 1 << (chunk.bit_length() - 1)          # the Q x Q kernels take power-of-two chunks
     while chunk > 8 and chunk // 2 >= L:
         chunk //= 2
-    y, final = _SSDFn.apply(x, dt, A, Bm, Cm, D, init_state, chunk)
+    return chunk
+
+
+def ssd_scan(x, dt, A, Bm, Cm, D=None, chunk=64, init_state=None, return_state=False):
+    """Chunked SSD scan (forward and backward hand-written; see ``_SSDFn``). Same arguments as ``ssd_reference``."""
+    y, final = _SSDFn.apply(x, dt, A, Bm, Cm, D, init_state, _chunk_size(chunk, x.shape[1]))
     return (y, final) if return_state else y
+
+
+# ----------------------------------------------------------------------------- the mixer of a Mamba-2 block in one node
+class _MixerFn(torch.autograd.Function):
+    """Convolution, step sizes, chunked scan, skip connection and output gate from the input projection's output to the gated rows, forward
+    and backward. The stages are the ones above; as one node they share buffers: the padded convolution output is what the scan reads in
+    place, every gradient is written into its columns of the projection's gradient, and nothing is padded, split or joined in between.
+    A block with its projections and norm, forward and backward: 122 -> 49 launches; width 768, 4 x 500 tokens 2.67 -> 1.59 ms (most of it
+    launches from the host), width 2560, 8192 tokens 4.37 -> 3.95 ms. Kept for backward: the projection's output, the convolution's output,
+    the scan's output and the chunk-entry states."""
+
+    @staticmethod
+    def _prep(zx, dt_bias, A_log, H, Q):
+        B_, L, W = zx.shape
+        nc = (L + Q - 1) // Q
+        f32 = lambda *s: torch.empty(s, dtype=torch.float32, device=zx.device)
+        dth, csh, E, decay, tot = f32(B_, nc, H, Q), f32(B_, nc, H, Q), f32(B_, nc, Q, H), f32(B_, nc, Q, H), f32(B_, nc, H)
+        raw = zx[..., W - H:]
+        _lib.call("sx_mix_prep", ptr(raw), c_ll(W), ptr(dt_bias), ptr(A_log), ptr(dth), ptr(csh), ptr(E), ptr(decay), ptr(tot), c_int(B_),
+                  c_int(nc), c_int(L), c_int(H), c_int(Q), stream())
+        return dth, csh, E, decay, tot
+
+    @staticmethod
+    def _bc(xbc, di, G, N, Q):
+        """B and C by (chunk, group) [B*nc*G, Q, N]: views of the convolution output for one group, a packed copy otherwise."""
+        C = xbc.shape[-1]
+        rows = xbc.view(-1, Q, C)
+        if G == 1:
+            return rows[..., di:di + N], rows[..., di + N:]
+        out = torch.empty(2, rows.shape[0] * G, Q, N, dtype=xbc.dtype, device=xbc.device)
+        src = xbc[..., di:]
+        _lib.call("sx_mix_pack", ptr(src), c_ll(C), ptr(out), c_ll(rows.shape[0] * Q), c_int(G), c_int(Q), c_int(N), stream())
+        return out[0], out[1]
+
+    @staticmethod
+    def forward(ctx, zx, conv_w, conv_b, dt_bias, A_log, D, sizes):
+        H, P, G, N, Q = sizes
+        B_, L, W = zx.shape
+        nc = (L + Q - 1) // Q
+        Lp, di, K, dev, cdt = nc * Q, H * P, conv_w.shape[1], zx.device, zx.dtype
+        C = di + 2 * G * N
+        xbc = torch.empty(B_, Lp, C, dtype=cdt, device=dev)
+        if Lp > L:
+            xbc[:, L:].zero_()
+        src = zx[..., di:di + C]
+        _lib.call("sx_conv1d_fwd", ptr(src), ptr(None), ptr(conv_w), ptr(conv_b), ptr(xbc), ptr(None), c_int(B_), c_int(L), c_int(C),
+                  c_int(K), c_int(1), c_ll(W), c_int(Lp), stream())
+        dth, csh, E, decay, tot = _MixerFn._prep(zx, dt_bias, A_log, H, Q)
+        x5 = xbc.view(B_, nc, Q, C)[..., :di].unflatten(-1, (H, P))
+        Bg, Cg = _MixerFn._bc(xbc, di, G, N, Q)
+        xw = _scale_rows(x5, decay, cdt, G)
+        S = gemm(xw, Bg, a_mn=True, b_mn=True, out_dtype=torch.float32)
+        Hprev, _ = _state_fwd(S.view(B_, nc, H, P, N), tot, None, cdt)
+        if Q == 128 and N == 128 and P == 64 and os.environ.get("SX_SSD_FUSED", "1") != "0":
+            y = torch.empty(B_, Lp, di, dtype=cdt, device=dev)
+            Cm, Bm = xbc[..., di + G * N:], xbc[..., di:]
+            _lib.call("sx_ssd_chunk_fwd", ptr(Cm), c_ll(C), ptr(Bm), c_ll(C), ptr(xbc), c_ll(C), ptr(Hprev), ptr(csh), ptr(dth), ptr(D), ptr(y),
+                      c_ll(B_ * nc), c_int(H), c_int(G), _lib.c_void_p(_lib.status_word(dev).data_ptr()), stream())
+        else:
+            CB = gemm(Cg, Bg, out_dtype=torch.float32).view(B_, nc, G, Q, Q)
+            M = _build_m(CB, csh, dth, H // G, cdt)
+            Yi = gemm(M.view(-1, Q, Q), _heads_first(x5), b_mn=True).view(B_, nc, H, Q, P)
+            y = _combine(Yi, gemm(Cg, Hprev.view(B_ * nc * G, -1, N)), x5, E, D, cdt, G)
+        out = torch.empty(B_, L, di, dtype=cdt, device=dev)
+        _lib.call("sx_gate_mul_fwd", ptr(y), ptr(zx), c_ll(W), ptr(out), c_ll(B_ * L), c_int(di), c_int(L), c_int(Lp), stream())
+        ctx.save_for_backward(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D)
+        ctx.sizes = sizes
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D = ctx.saved_tensors
+        H, P, G, N, Q = ctx.sizes
+        B_, L, W = zx.shape
+        nc, rep, di, K, dev, cdt = Hprev.shape[1], H // G, H * P, conv_w.shape[1], zx.device, zx.dtype
+        Lp, C, n = nc * Q, di + 2 * G * N, B_ * nc * G
+        f32 = torch.float32
+        g = g.contiguous()
+        dzx = torch.empty(B_, L, W, dtype=cdt, device=dev)
+        dy = torch.empty(B_, Lp, di, dtype=cdt, device=dev)
+        if Lp > L:
+            dy[:, L:].zero_()
+        _lib.call("sx_gate_mul_bwd", ptr(g), ptr(y), ptr(zx), c_ll(W), ptr(dy), ptr(dzx), c_ll(B_ * L), c_int(di), c_int(L), c_int(Lp),
+                  c_ll(W), stream())
+        dth, csh, E, decay, tot = _MixerFn._prep(zx, dt_bias, A_log, H, Q)
+        x5 = xbc.view(B_, nc, Q, C)[..., :di].unflatten(-1, (H, P))
+        dy5 = dy.view(B_, nc, Q, H, P)
+        Bg, Cg = _MixerFn._bc(xbc, di, G, N, Q)
+        Hg = Hprev.view(n, rep * P, N)
+        # contribution of earlier chunks, and through them the chunk states
+        dye, dcs, ddrow = _bwd_rows1(dy5, x5, gemm(Cg, Hg), E, cdt, G)
+        dC = gemm(dye, Hg, b_mn=True, out_dtype=f32)
+        dHprev = gemm(dye, Cg, a_mn=True, b_mn=True, out_dtype=f32)
+        dS, dtot, _ = _state_bwd(dHprev.view(B_, nc, H, P, N), tot, Hprev, None)
+        dSg = dS.view(n, rep * P, N)
+        dxw = gemm(Bg, dSg)
+        dB = gemm(_scale_rows(x5, decay, cdt, G), dSg, b_mn=True, out_dtype=f32)
+        # quadratic term within the chunk
+        dyh = _heads_first(dy5)
+        dM = gemm(dyh, _heads_first(x5))
+        CB = gemm(Cg, Bg, out_dtype=f32).view(B_, nc, G, Q, Q)
+        M, dGh, rowW, colU = _bwd_qq(dM.view(B_, nc, H, Q, Q), CB, csh, dth, rep, cdt)
+        dxi = gemm(M.view(-1, Q, Q), dyh, a_mn=True, b_mn=True)
+        dxbc = torch.empty(B_, Lp, C, dtype=cdt, device=dev)
+        ddecay = torch.empty(B_, nc, Q, H, dtype=f32, device=dev)
+        _lib.call("sx_ssd_bwd_rows2", ptr(dy), ptr(xbc), ptr(dxw), ptr(dxi), ptr(decay), ptr(D), ptr(dxbc), ptr(ddecay), c_ll(B_ * Lp * H),
+                  c_int(H), c_int(Q), c_int(P), c_ll(C), c_int(G), c_ll(C), stream())
+        dG = dGh.view(n * rep, Q, Q)
+        if rep > 1:
+            dG = torch.empty(n, Q, Q, dtype=cdt, device=dev)
+            _lib.call("sx_mix_sum", ptr(dGh), ptr(dG), c_ll(n), c_int(rep), c_int(Q * Q), stream())
+        gemm(dG, Bg, b_mn=True, out=dC, c=dC, beta=1.0)
+        gemm(dG, Cg, a_mn=True, b_mn=True, out=dB, c=dB, beta=1.0)
+        to = dxbc[..., di:]
+        _lib.call("sx_mix_unpack", ptr(dB), ptr(dC), ptr(to), c_ll(C), c_ll(B_ * Lp), c_int(G), c_int(Q), c_int(N), stream())
+        # convolution
+        parts = _lib.lib().sx_conv1d_bwd_parts(c_int(B_), c_int(L), c_int(C))
+        partial = torch.empty(parts * (K + 1) * C, dtype=f32, device=dev)
+        dwdb = torch.empty((K + 1) * C, dtype=f32, device=dev)
+        src, to = zx[..., di:di + C], dzx[..., di:di + C]
+        _lib.call("sx_conv1d_bwd", ptr(dxbc), ptr(src), ptr(None), ptr(conv_w), ptr(conv_b), ptr(to), ptr(partial), ptr(dwdb), c_int(B_),
+                  c_int(L), c_int(C), c_int(K), c_int(1), c_ll(W), c_int(Lp), c_ll(W), stream())
+        # step sizes
+        part = torch.empty(3, B_ * nc, H, dtype=f32, device=dev)
+        raw, to = zx[..., W - H:], dzx[..., W - H:]
+        _lib.call("sx_mix_finish", ptr(raw), c_ll(W), ptr(dt_bias), ptr(A_log), ptr(dth), ptr(csh), ptr(ddecay), ptr(dcs), ptr(ddrow),
+                  ptr(rowW), ptr(colU), ptr(dtot), ptr(tot), ptr(to), c_ll(W), ptr(part), c_int(B_), c_int(nc), c_int(L), c_int(H), c_int(Q),
+                  stream())
+        dA, dD, dbias = part.sum(1)
+        return dzx, dwdb[: C * K].view(C, K).to(cdt), dwdb[C * K:].to(cdt), dbias, dA, dD, None
+
+
+def mixer_ok(zx, conv_w, conv_b, dt_bias, A_log, D, H, P, G, N, chunk=128) -> bool:
+    """Whether ``mamba2_mixer`` takes these tensors: bf16 on a GPU with 32-bit step parameters, sizes that keep every column slice of the
+    projection on 16 bytes, head sizes of 8 times a power of two (the row kernels), at most four taps, and no more chunks than a grid has
+    rows."""
+    if not (zx.is_cuda and zx.dtype == torch.bfloat16 and zx.dim() == 3 and zx.numel() and zx.is_contiguous() and zx.data_ptr() % 16 == 0):
+        return False
+    (B_, L, W), C = zx.shape, H * P + 2 * G * N
+    Q = _chunk_size(chunk, L)
+    return (W == H * P + C + H and W % 8 == 0 and C % 8 == 0 and P % 8 == 0 and (P // 8) & (P // 8 - 1) == 0 and P <= 256 and N % 8 == 0
+            and H % G == 0 and conv_w.dim() == 2 and conv_w.shape[0] == C and 1 <= conv_w.shape[1] <= 4 and conv_b is not None
+            and conv_b.shape == (C,) and all(t.dtype == torch.bfloat16 and t.device == zx.device and t.is_contiguous() and t.data_ptr() % 16 == 0
+                                             for t in (conv_w, conv_b))
+            and all(t.dtype == torch.float32 and t.device == zx.device and t.shape == (H,) and t.is_contiguous() for t in (dt_bias, A_log, D))
+            and B_ * ((L + Q - 1) // Q) <= 65535 and _lib.available())
+
+
+def mamba2_mixer(zx, conv_w, conv_b, dt_bias, A_log, D, H, P, G, N, chunk=128):
+    """Gated rows [B, L, H P] of a Mamba-2 block from the input projection zx [B, L, z | x | B | C | dt]; see ``mixer_ok``."""
+    return _MixerFn.apply(zx, conv_w, conv_b, dt_bias, A_log, D, (H, P, G, N, _chunk_size(chunk, zx.shape[1])))
 
 
 def ssd_step(h, x, dt, A, Bm, Cm, D=None):

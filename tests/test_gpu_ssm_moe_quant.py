@@ -266,3 +266,49 @@ def test_grouped_fp8_expert_gemm_and_fp8_moe_layer():
     yr.backward(g.float())
     assert _rel(yy, yr) < 8e-2                       # e4m3 rounding of both operands of both GEMMs
     assert _rel(xx.grad, xr.grad) < 8e-2 and _rel(W1.grad, W1r.grad) < 8e-2 and _rel(W2.grad, W2r.grad) < 8e-2
+
+
+@pytest.mark.parametrize("B,L,H,P,G,N,K", [
+    (2, 256, 8, 64, 1, 128, 4), (1, 500, 8, 64, 2, 128, 4), (3, 129, 8, 64, 8, 128, 4), (2, 127, 8, 64, 1, 128, 4), (2, 1, 8, 64, 1, 128, 4),
+    (1, 40, 16, 32, 4, 64, 3), (2, 300, 8, 16, 1, 64, 2), (1, 77, 24, 64, 1, 64, 4), (1, 200, 8, 128, 2, 256, 1)])
+def test_mamba2_mixer(B, L, H, P, G, N, K, monkeypatch):
+    """The mixer as one node against the plain 32-bit recurrence: chunks that are full, end in padding or shorten with the sequence, one to
+    H groups, the fused and the staged output stage, one to four taps. Bound: rounding an operand to bf16 adds 2^-9 relative at random, at
+    most about twelve such roundings lie on the way to any result: sqrt(12) 2^-9 = 0.007 of its 2-norm; twice that, and four times for
+    the sums of mixed sign over tokens that the step parameters' gradients are."""
+    torch.manual_seed(B * L + N)
+    di, C = H * P, H * P + 2 * G * N
+    zx = torch.randn(B, L, di + C + H, device="cuda")
+    zx[..., di + C:] -= 2
+    args = [zx.bfloat16(), (0.5 * torch.randn(C, K, device="cuda")).bfloat16(), (0.1 * torch.randn(C, device="cuda")).bfloat16(),
+            torch.randn(H, device="cuda") - 1, torch.log(1 + 15 * torch.rand(H, device="cuda")), torch.randn(H, device="cuda")]
+    args = [t.requires_grad_() for t in args]
+    ref = [t.detach().double().requires_grad_() for t in args]
+    z, xbc, dt = torch.split(ref[0], [di, C, H], -1)
+    pad = torch.nn.functional.pad(xbc, (0, 0, K - 1, 0))
+    xbc = torch.nn.functional.silu(sum(pad[:, k:k + L] * ref[1][:, k] for k in range(K)) + ref[2])
+    x, Bm, Cm = torch.split(xbc, [di, G * N, G * N], -1)
+    x, Bm, Cm = x.view(B, L, H, P), Bm.view(B, L, G, N).repeat_interleave(H // G, 2), Cm.view(B, L, G, N).repeat_interleave(H // G, 2)
+    dt, h, ys = torch.nn.functional.softplus(dt + ref[3]), zx.new_zeros(B, H, P, N, dtype=torch.float64), []
+    for t in range(L):
+        h = h * torch.exp(-torch.exp(ref[4]) * dt[:, t])[..., None, None] + (dt[:, t, :, None] * x[:, t])[..., None] * Bm[:, t, :, None]
+        ys.append((h * Cm[:, t, :, None]).sum(-1) + ref[5][:, None] * x[:, t])
+    want = torch.stack(ys, 1).reshape(B, L, di) * torch.nn.functional.silu(z)
+    g = torch.randn(B, L, di, device="cuda").bfloat16()
+    wgrad = torch.autograd.grad(want, ref, g.double())
+    size = (H, P, G, N)
+    for fused in ("1", "0"):
+        monkeypatch.setenv("SX_SSD_FUSED", fused)
+        assert ssm.mixer_ok(*args, *size)
+        y = ssm.mamba2_mixer(*args, *size)
+        grads = torch.autograd.grad(y, args, g)
+        ops.check_status()
+        err = lambda a, b: ((a.double() - b).norm() / (b.norm() + 1e-30)).item()  # noqa: E731
+        assert y.shape == want.shape and err(y, want) < 0.014
+        for got, exp, t, name in zip(grads, wgrad, args, ("zx", "conv", "conv bias", "dt bias", "A_log", "D")):
+            if L == 1 and name == "A_log":      # nothing decays before a first token: exactly 0, here 32-bit terms below 100 that cancel
+                assert exp.abs().max() == 0 and got.abs().max() < 100 * 2.0 ** -20
+                continue
+            assert got.shape == t.shape and got.dtype == t.dtype and err(got, exp) < (0.014 if name == "zx" else 0.028), (name, err(got, exp))
+        for lo, hi, name in ((0, di, "z"), (di, di + di, "x"), (2 * di, 2 * di + 2 * G * N, "B, C"), (di + C, di + C + H, "dt")):
+            assert err(grads[0][..., lo:hi], wgrad[0][..., lo:hi]) < 0.028, (name, err(grads[0][..., lo:hi], wgrad[0][..., lo:hi]))
