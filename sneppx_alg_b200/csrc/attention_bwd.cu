@@ -8,10 +8,15 @@
 //   dV  += P^T dO  (A operand read from TMEM)   dK += dS^T Q       (128 x 128 accumulators in TMEM; dK scaled at the end)
 //   dQ^T = K^T dS^T         (128 x 64; staged through shared memory and added into dq_accum with bulk fp32
 //                            reductions, cp.reduce.async.bulk, by four drain warps; scaled when converted to bf16)
-// Pipeline: a loader warp keeps three (Q | dO) tiles and their LSE / delta rows in flight (the row statistics are
-// fetched two tiles ahead so that their global-load latency is hidden); one thread issues every MMA, S^T / dP^T of
-// tile i+1 ahead of the three accumulating GEMMs of tile i; sixteen softmax-gradient warps turn S^T / dP^T into
-// P^T / dS^T (double buffered, so they never wait for the accumulating GEMMs); the drain warps empty dQ^T while the
+// Pipeline: two tiles are in flight in TMEM, each with S^T and dP^T of its own. P^T takes the columns of S^T that it was computed from, dQ^T
+// those of dP^T once dS^T is out, so that both tiles fit beside the dV and dK accumulators (2 x 128 + 2 x 128 columns). One thread issues
+//   dV(i)  dQ(i)  dK(i)  S(i+2)  [dQ(i) drained]  dP(i+2)
+// while two groups of eight softmax-gradient warps turn S^T / dP^T into P^T / dS^T, the even and the odd tiles. A tile still takes 3400
+// cycles (3700 with one S^T / dP^T buffer and all sixteen warps on one tile; causal, 4096 tokens, 32 heads on 8: the kernel 523 -> 509 us,
+// 16384 tokens 7.0 - 7.2 ms either way), of which the tensor pipe is busy 2360 and multiplies 1280: the N = 64 products fetch A from shared
+// memory at half rate. Leaving out the dQ reductions or their staging changes nothing, leaving out the dQ products takes 15 % off. A loader
+// warp keeps up to four Q and three dO tiles and the LSE / delta rows in flight (dO is wanted later than Q;
+// the row statistics are fetched two tiles ahead so that their global-load latency is hidden); the drain warps empty dQ^T while the
 // next tile's GEMMs run. CTAs are ordered heaviest key tile first. All MN-major operand forms (dO, Q, K^T, dS^T) are
 // read from the very tiles TMA brought or the softmax warps wrote; no transposed copy exists. dK/dV need no atomics
 // because the whole GQA group is reduced inside the CTA.
@@ -28,8 +33,8 @@ namespace sx {
 constexpr int BWD_KV = 128;
 constexpr int BWD_Q = 64;
 constexpr int BWD_D = 128;
-// Warp roles: 0 loader (TMA + per-row statistics), 1 MMA issue, 2..17 softmax-gradient warps (4 column groups of 16
-// query columns x 4 TMEM lane quarters), 18..21 dQ drain warps (one per lane quarter).
+// Warp roles: 0 loader (TMA + per-row statistics), 1 MMA issue, 2..17 softmax-gradient warps (2 groups that take the tiles in turn, each 2
+// halves of 32 query columns x 4 TMEM lane quarters), 18..21 dQ drain warps (one per lane quarter).
 constexpr int BWD_SM_WARPS = 16;
 constexpr int BWD_DRAIN_WARPS = 4;
 constexpr int BWD_THREADS = 32 * (2 + BWD_SM_WARPS + BWD_DRAIN_WARPS);  // 704
@@ -49,21 +54,23 @@ struct AttnBwdParams {
 };
 
 struct BwdCfg {
-  static constexpr int STAGES = 3;                       // (Q | dO) tiles in flight: covers the TMA latency of ~1.5 us
+  static constexpr int Q_STAGES = 4, STAGES = 3;         // Q tiles; dO tiles and row statistics
   static constexpr int KV_BYTES = BWD_KV * BWD_D * 2;  // 32 KB
   static constexpr int Q_BYTES = BWD_Q * BWD_D * 2;    // 16 KB
   static constexpr int PT_BYTES = BWD_KV * BWD_Q * 2;  // 16 KB
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = KV_BYTES;
   static constexpr int OFF_Q = 2 * KV_BYTES;
-  static constexpr int OFF_DST = OFF_Q + STAGES * 2 * Q_BYTES;  // dS^T, double buffered
+  static constexpr int OFF_DO = OFF_Q + Q_STAGES * Q_BYTES;
+  static constexpr int OFF_DST = OFF_DO + STAGES * Q_BYTES;     // dS^T, double buffered
   static constexpr int OFF_DQS = OFF_DST + 2 * PT_BYTES;        // dQ staging: 4 drain warps x [32 query rows][32 head-dim] fp32
   static constexpr int DQS_BYTES = 4 * 4096;
   static constexpr int OFF_STAT = OFF_DQS + DQS_BYTES;          // STAGES x {lse * log2e, delta} x 64 floats
-  static constexpr int OFF_BAR = OFF_STAT + 2048;
+  static constexpr int OFF_BAR = OFF_STAT + STAGES * 512;
   static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
-  // TMEM columns: S^T, dP^T, dQ^T (64 each), P^T as packed bf16 pairs (2 x 32), dV, dK (128 each)
-  static constexpr uint32_t TM_S = 0, TM_DP = 64, TM_DQ = 128, TM_PT = 192, TM_DV = 256, TM_DK = 384;
+  // TMEM columns: two tiles of S^T and dP^T (64 each), dV, dK (128 each). P^T as packed bf16 pairs: the 16 query columns of a column group
+  // (one K step of dV) become the first 8 of the group's 16 columns of S^T, which only the warps of that group have read.
+  static constexpr uint32_t TM_S = 0, TM_DP = 64, TM_TILE = 128, TM_DV = 256, TM_DK = 384;
 };
 
 __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
@@ -73,20 +80,23 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   uint8_t* sK = smem + Cfg::OFF_K;
   uint8_t* sV = smem + Cfg::OFF_V;
   uint8_t* sQ = smem + Cfg::OFF_Q;
+  uint8_t* sdO = smem + Cfg::OFF_DO;
   uint8_t* sDST = smem + Cfg::OFF_DST;
   float* sStat = reinterpret_cast<float*>(smem + Cfg::OFF_STAT);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
   uint64_t* kv_full = bars;          // 1
-  uint64_t* qdo_full = bars + 1;     // [3]
-  uint64_t* qdo_empty = bars + 4;    // [3]
-  uint64_t* stat_full = bars + 7;    // [3], 1 arrival each
-  uint64_t* s_full = bars + 10;      // 1
-  uint64_t* dp_full = bars + 11;     // 1
-  uint64_t* pds_ready = bars + 12;   // 16 arrivals
-  uint64_t* dq_full = bars + 13;     // 1
-  uint64_t* dq_drained = bars + 14;  // 4 arrivals: the dQ^T accumulator has been read out of TMEM
-  uint64_t* all_done = bars + 15;    // 1: every MMA of the CTA has executed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* q_full = bars + 1;       // [4]
+  uint64_t* q_empty = bars + 5;      // [4]
+  uint64_t* do_full = bars + 9;      // [3]
+  uint64_t* do_empty = bars + 12;    // [3]
+  uint64_t* stat_full = bars + 15;   // [3], 1 arrival each
+  uint64_t* s_full = bars + 18;      // [2] by tile parity, as are the next two
+  uint64_t* dp_full = bars + 20;     // [2]
+  uint64_t* pds_ready = bars + 22;   // [2], 8 arrivals
+  uint64_t* dq_full = bars + 24;     // 1
+  uint64_t* dq_drained = bars + 25;  // 4 arrivals: the dQ^T accumulator has been read out of TMEM
+  uint64_t* all_done = bars + 26;    // 1: every MMA of the CTA has executed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -111,15 +121,21 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
+    for (int i = 0; i < Cfg::Q_STAGES; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+    }
     for (int i = 0; i < Cfg::STAGES; ++i) {
-      mbar_init(&qdo_full[i], 1);
-      mbar_init(&qdo_empty[i], 1);
+      mbar_init(&do_full[i], 1);
+      mbar_init(&do_empty[i], 1);
       mbar_init(&stat_full[i], 1);
     }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&dp_full[i], 1);
+      mbar_init(&pds_ready[i], BWD_SM_WARPS / 2);
+    }
     mbar_init(all_done, 1);
-    mbar_init(s_full, 1);
-    mbar_init(dp_full, 1);
-    mbar_init(pds_ready, BWD_SM_WARPS);
     mbar_init(dq_full, 1);
     mbar_init(dq_drained, BWD_DRAIN_WARPS);
     *s_abort = 0;
@@ -164,17 +180,24 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
       float cl0, cl1, cd0, cd1, nl0 = INFINITY, nl1 = INFINITY, nd0 = 0.f, nd1 = 0.f;
       load_stats(0, cl0, cl1, cd0, cd1);
       if (n_it > 1) load_stats(1, nl0, nl1, nd0, nd1);
-      for (int it = 0; it < n_it; ++it) {
-        const int s = it % Cfg::STAGES;
-        const uint32_t ph = (it / Cfg::STAGES) & 1;
-        const int head = kv_head * G + it / n_qt;
-        const int qrow0 = (qt_lo + it % n_qt) * BWD_Q;
-        if (!mbar_wait_warp(&qdo_empty[s], ph ^ 1, s_abort, p.status, ST_TIMEOUT_PRODUCER)) break;
+      auto load_q = [&](int it) {
+        const int s = it % Cfg::Q_STAGES;
+        if (!mbar_wait_warp(&q_empty[s], ((it / Cfg::Q_STAGES) & 1) ^ 1, s_abort, p.status, ST_TIMEOUT_PRODUCER)) return false;
         if (lane == 0) {
-          mbar_expect_tx(&qdo_full[s], 2 * Cfg::Q_BYTES);
-          tma5(sQ + s * 2 * Cfg::Q_BYTES, &p.tmQ, &qdo_full[s], qrow0, head, b);
-          tma5(sQ + s * 2 * Cfg::Q_BYTES + Cfg::Q_BYTES, &p.tmdO, &qdo_full[s], qrow0, head, b);
+          mbar_expect_tx(&q_full[s], Cfg::Q_BYTES);
+          tma5(sQ + s * Cfg::Q_BYTES, &p.tmQ, &q_full[s], (qt_lo + it % n_qt) * BWD_Q, kv_head * G + it / n_qt, b);
         }
+        return true;
+      };
+      bool ok = load_q(0);
+      for (int it = 0; it < n_it && ok; ++it) {
+        const int s = it % Cfg::STAGES;
+        if (!mbar_wait_warp(&do_empty[s], ((it / Cfg::STAGES) & 1) ^ 1, s_abort, p.status, ST_TIMEOUT_PRODUCER)) break;
+        if (lane == 0) {
+          mbar_expect_tx(&do_full[s], Cfg::Q_BYTES);
+          tma5(sdO + s * Cfg::Q_BYTES, &p.tmdO, &do_full[s], (qt_lo + it % n_qt) * BWD_Q, kv_head * G + it / n_qt, b);
+        }
+        if (it + 1 < n_it) ok = load_q(it + 1);
         float* st = sStat + s * 128;
         st[lane] = cl0; st[lane + 32] = cl1; st[64 + lane] = cd0; st[64 + lane + 32] = cd1;
         __syncwarp();
@@ -189,146 +212,163 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
       constexpr uint32_t idesc_acc = umma_idesc_f16(128, BWD_D, 1, 0, 1);    // P^T dO, dS^T Q
       constexpr uint32_t idesc_dq = umma_idesc_f16(128, BWD_Q, 1, 1, 1);     // K^T dS^T
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aDST0 = smem_u32(sDST);
-      auto issue_sdp = [&](int it) {
-        const uint32_t q = smem_u32(sQ + (it % Cfg::STAGES) * 2 * Cfg::Q_BYTES), dO = q + Cfg::Q_BYTES;
+      auto q_ready = [&](int it) {
+        return mbar_wait(&q_full[it % Cfg::Q_STAGES], (it / Cfg::Q_STAGES) & 1, s_abort, p.status, ST_TIMEOUT_MMA);
+      };
+      auto do_ready = [&](int it) {
+        return mbar_wait(&do_full[it % Cfg::STAGES], (it / Cfg::STAGES) & 1, s_abort, p.status, ST_TIMEOUT_MMA);
+      };
+      auto issue_s = [&](int it) {
+        const uint32_t q = smem_u32(sQ + (it % Cfg::Q_STAGES) * Cfg::Q_BYTES), t = tmem_base + Cfg::TM_S + (it & 1) * Cfg::TM_TILE;
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_f16_ss(tmem_base + Cfg::TM_S, umma_desc_sw128(aK + c * 16384 + k * 32, 16, 1024),
-                        umma_desc_sw128(q + c * 8192 + k * 32, 16, 1024), idesc_s, (c | k) ? 1u : 0u);
-        umma_commit(s_full);
+            umma_f16_ss(t, umma_desc_sw128(aK + c * 16384 + k * 32, 16, 1024), umma_desc_sw128(q + c * 8192 + k * 32, 16, 1024), idesc_s,
+                        (c | k) ? 1u : 0u);
+        umma_commit(&s_full[it & 1]);
+      };
+      auto issue_dp = [&](int it) {
+        const uint32_t dO = smem_u32(sdO + (it % Cfg::STAGES) * Cfg::Q_BYTES), t = tmem_base + Cfg::TM_DP + (it & 1) * Cfg::TM_TILE;
 #pragma unroll
         for (int c = 0; c < 2; ++c)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_f16_ss(tmem_base + Cfg::TM_DP, umma_desc_sw128(aV + c * 16384 + k * 32, 16, 1024),
-                        umma_desc_sw128(dO + c * 8192 + k * 32, 16, 1024), idesc_s, (c | k) ? 1u : 0u);
-        umma_commit(dp_full);
+            umma_f16_ss(t, umma_desc_sw128(aV + c * 16384 + k * 32, 16, 1024), umma_desc_sw128(dO + c * 8192 + k * 32, 16, 1024), idesc_s,
+                        (c | k) ? 1u : 0u);
+        umma_commit(&dp_full[it & 1]);
       };
       bool ok = mbar_wait(kv_full, 0, s_abort, p.status, ST_TIMEOUT_MMA);
-      if (ok) ok = mbar_wait(&qdo_full[0], 0, s_abort, p.status, ST_TIMEOUT_MMA);
-      if (ok) {
+      for (int it = 0; it < 2 && it < n_it && ok; ++it) {
+        ok = q_ready(it) && do_ready(it);
+        if (!ok) break;
         tc_fence_after();
-        issue_sdp(0);
+        issue_s(it);
+        issue_dp(it);
       }
       for (int it = 0; it < n_it && ok; ++it) {
-        if (!mbar_wait(pds_ready, it & 1, s_abort, p.status, ST_TIMEOUT_MMA)) { ok = false; break; }
-        if (it + 1 < n_it) {
-          const int jn = it + 1;
-          if (!mbar_wait(&qdo_full[jn % Cfg::STAGES], (jn / Cfg::STAGES) & 1, s_abort, p.status, ST_TIMEOUT_MMA)) {
-            ok = false;
-            break;
-          }
-        }
+        if (!mbar_wait(&pds_ready[it & 1], (it >> 1) & 1, s_abort, p.status, ST_TIMEOUT_MMA)) { ok = false; break; }
         tc_fence_after();
-        // S^T / dP^T of the next tile go first: the softmax warps work on them while the three GEMMs below run
-        if (it + 1 < n_it) issue_sdp(it + 1);
-        const uint32_t q = smem_u32(sQ + (it % Cfg::STAGES) * 2 * Cfg::Q_BYTES), dO = q + Cfg::Q_BYTES;
-        const uint32_t aDST = aDST0 + (it & 1) * Cfg::PT_BYTES;
-        const uint32_t tPT = tmem_base + Cfg::TM_PT + (it & 1) * 32;
-        // dV += P^T dO (P^T read from TMEM) ; dK += dS^T Q   (K = 64 query rows: 4 k-steps)
+        const uint32_t q = smem_u32(sQ + (it % Cfg::Q_STAGES) * Cfg::Q_BYTES), dO = smem_u32(sdO + (it % Cfg::STAGES) * Cfg::Q_BYTES);
+        const uint32_t aDST = aDST0 + (it & 1) * Cfg::PT_BYTES, tT = tmem_base + (it & 1) * Cfg::TM_TILE;
+        // dV += P^T dO (P^T read from TMEM)   (K = 64 query rows: 4 k-steps)
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          umma_f16_ts(tmem_base + Cfg::TM_DV, tPT + k * 8, umma_desc_sw128(dO + k * 2048, 8192, 1024), idesc_acc,
+          umma_f16_ts(tmem_base + Cfg::TM_DV, tT + Cfg::TM_S + k * 16, umma_desc_sw128(dO + k * 2048, 8192, 1024), idesc_acc,
                       (it | k) ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_f16_ss(tmem_base + Cfg::TM_DK, umma_desc_sw128(aDST + k * 32, 16, 1024),
-                      umma_desc_sw128(q + k * 2048, 8192, 1024), idesc_acc, (it | k) ? 1u : 0u);
-        // dQ^T = K^T dS^T  (K = 128 key rows: 8 k-steps); the accumulator of the previous iteration must be read out
-        if (it > 0) {
-          if (!mbar_wait(dq_drained, (it - 1) & 1, s_abort, p.status, ST_TIMEOUT_MMA)) { ok = false; break; }
-          tc_fence_after();
-        }
+        umma_commit(&do_empty[it % Cfg::STAGES]);
+        // dQ^T = K^T dS^T  (K = 128 key rows: 8 k-steps), over dP^T, which every softmax warp has read
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          umma_f16_ss(tmem_base + Cfg::TM_DQ, umma_desc_sw128(aK + k * 2048, 16384, 1024),
-                      umma_desc_sw128(aDST + k * 2048, 16384, 1024), idesc_dq, k ? 1u : 0u);
-        umma_commit(&qdo_empty[it % Cfg::STAGES]);
+          umma_f16_ss(tT + Cfg::TM_DP, umma_desc_sw128(aK + k * 2048, 16384, 1024), umma_desc_sw128(aDST + k * 2048, 16384, 1024), idesc_dq,
+                      k ? 1u : 0u);
         umma_commit(dq_full);
+        // dK += dS^T Q
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_f16_ss(tmem_base + Cfg::TM_DK, umma_desc_sw128(aDST + k * 32, 16, 1024), umma_desc_sw128(q + k * 2048, 8192, 1024), idesc_acc,
+                      (it | k) ? 1u : 0u);
+        umma_commit(&q_empty[it % Cfg::Q_STAGES]);
+        // S^T of tile it + 2 over P^T, which dV (issued before) has read
+        if (it + 2 < n_it) {
+          if (!q_ready(it + 2)) { ok = false; break; }
+          tc_fence_after();
+          issue_s(it + 2);
+        }
+        // every drain is waited for: its barrier advances one phase a tile
+        if (it + 1 < n_it && !mbar_wait(dq_drained, it & 1, s_abort, p.status, ST_TIMEOUT_MMA)) { ok = false; break; }
+        if (it + 2 < n_it) {
+          if (!do_ready(it + 2)) { ok = false; break; }
+          tc_fence_after();
+          issue_dp(it + 2);
+        }
       }
       if (ok) umma_commit(all_done);
     }
   } else if (warp < 2 + BWD_SM_WARPS) {
     // ------------------------------------------------------------ softmax-gradient warps
-    const int cg = (warp - 2) >> 2;     // column group: query columns [16*cg, 16*cg + 16) of the tile
+    const int cg = (warp - 2) >> 2;     // output columns in the end: halves of dV and dK
+    const int grp = cg >> 1;            // tiles of this group of eight warps: it % 2 == grp
     const int qd = warp & 3;            // TMEM lane quarter this warp may touch
     const int r = qd * 32 + lane;       // key row inside the tile == TMEM lane
     const int kv_idx = kv0 + r;
-    const int c0 = cg * 16;
     const uint32_t lane_addr = static_cast<uint32_t>(qd * 32) << 16;
     bool ok = n_it > 0;
-    for (int it = 0; it < n_it && ok; ++it) {
+    for (int it = grp; it < n_it && ok; it += 2) {
       const int qrow0 = (qt_lo + it % n_qt) * BWD_Q;
       const bool need_mask = (p.causal && kv0 + BWD_KV - 1 > qrow0 + offset) || (kv0 + BWD_KV > p.Skv) ||
                              (p.window > 0 && kv0 < qrow0 + BWD_Q - 1 + offset - p.window + 1);
       const int stg = it % Cfg::STAGES;
+      const uint32_t tile = tmem_base + grp * Cfg::TM_TILE + lane_addr;
+      uint8_t* dstb = sDST + grp * Cfg::PT_BYTES;
       if (!mbar_wait_warp(&stat_full[stg], (it / Cfg::STAGES) & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
-      const float* st = sStat + stg * 128 + c0;
-      float lse[16], dl[16];
-#pragma unroll
-      for (int i = 0; i < 16; i += 4) {
-        const float4 a4 = *reinterpret_cast<const float4*>(st + i);
-        const float4 d4 = *reinterpret_cast<const float4*>(st + 64 + i);
-        lse[i] = a4.x; lse[i + 1] = a4.y; lse[i + 2] = a4.z; lse[i + 3] = a4.w;
-        dl[i] = d4.x; dl[i + 1] = d4.y; dl[i + 2] = d4.z; dl[i + 3] = d4.w;
-      }
-      float pf[16];
-      uint32_t pt[8], ds[8];
-      if (!mbar_wait_warp(s_full, it & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[grp], (it >> 1) & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
-      {
-        uint32_t v[16];
-        tmem_ld16(tmem_base + Cfg::TM_S + lane_addr + c0, v);
-        tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) pf[i] = exp2f(fmaf(__uint_as_float(v[i]), p.scale_log2, -lse[i]));
-        if (need_mask) {
+      for (int h = 0; h < 2; ++h) {
+        const int cc0 = (cg & 1) * 2 + h, c0 = cc0 * 16;      // 16 query columns: one K step of dV
+        const float* st = sStat + stg * 128 + c0;
+        float pf[16];
+        uint32_t pt[8], ds[8];
+        {
+          uint32_t v[16];
+          tmem_ld16(tile + Cfg::TM_S + c0, v);
+          tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int qi = qrow0 + c0 + i + offset;
-            bool dead = kv_idx >= p.Skv;
-            if (p.causal && kv_idx > qi) dead = true;
-            if (p.window > 0 && kv_idx < qi - p.window + 1) dead = true;
-            if (dead) pf[i] = 0.f;
+          for (int i = 0; i < 16; i += 4) {
+            const float4 a4 = *reinterpret_cast<const float4*>(st + i);
+            pf[i] = exp2f(fmaf(__uint_as_float(v[i]), p.scale_log2, -a4.x));
+            pf[i + 1] = exp2f(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, -a4.y));
+            pf[i + 2] = exp2f(fmaf(__uint_as_float(v[i + 2]), p.scale_log2, -a4.z));
+            pf[i + 3] = exp2f(fmaf(__uint_as_float(v[i + 3]), p.scale_log2, -a4.w));
+          }
+          if (need_mask) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int qi = qrow0 + c0 + i + offset;
+              bool dead = kv_idx >= p.Skv;
+              if (p.causal && kv_idx > qi) dead = true;
+              if (p.window > 0 && kv_idx < qi - p.window + 1) dead = true;
+              if (dead) pf[i] = 0.f;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) pt[i / 2] = pack_bf16x2(pf[i], pf[i + 1]);
+        }
+        if (h == 0) {
+          ok = mbar_wait_warp(&dp_full[grp], (it >> 1) & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        {
+          uint32_t v[16];
+          tmem_ld16(tile + Cfg::TM_DP + c0, v);
+          // Buffer grp of P^T and dS^T was last read by the GEMMs of tile it - 2. Those were issued before S^T of this tile and the GEMMs
+          // of one thread execute in order, so s_full already covers them.
+          asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(tile + Cfg::TM_S + c0),
+                       "r"(pt[0]), "r"(pt[1]), "r"(pt[2]), "r"(pt[3]), "r"(pt[4]), "r"(pt[5]), "r"(pt[6]), "r"(pt[7])
+                       : "memory");
+          tmem_ld_wait();
+          // dS without the softmax scale: dK and dQ are scaled once when they are written out
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            const float4 d4 = *reinterpret_cast<const float4*>(st + 64 + i);
+            ds[i / 2] = pack_bf16x2(pf[i] * (__uint_as_float(v[i]) - d4.x), pf[i + 1] * (__uint_as_float(v[i + 1]) - d4.y));
+            ds[i / 2 + 1] = pack_bf16x2(pf[i + 2] * (__uint_as_float(v[i + 2]) - d4.z), pf[i + 3] * (__uint_as_float(v[i + 3]) - d4.w));
           }
         }
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) pt[i / 2] = pack_bf16x2(pf[i], pf[i + 1]);
+        for (int k = 0; k < 2; ++k) {
+          const int off = r * 128 + (((cc0 * 2 + k) ^ (r & 7)) << 4);
+          *reinterpret_cast<uint4*>(dstb + off) = make_uint4(ds[k * 4], ds[k * 4 + 1], ds[k * 4 + 2], ds[k * 4 + 3]);
+        }
       }
-      if (!mbar_wait_warp(dp_full, it & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
-      tc_fence_after();
-      {
-        uint32_t v[16];
-        tmem_ld16(tmem_base + Cfg::TM_DP + lane_addr + c0, v);
-        tmem_ld_wait();
-        // dS without the softmax scale: dK and dQ are scaled once when they are written out
-#pragma unroll
-        for (int i = 0; i < 16; i += 2)
-          ds[i / 2] = pack_bf16x2(pf[i] * (__uint_as_float(v[i]) - dl[i]), pf[i + 1] * (__uint_as_float(v[i + 1]) - dl[i + 1]));
-      }
-      // Buffer (it & 1) of P^T / dS^T was last read by the GEMMs of iteration it-2. Those were issued before the
-      // S^T GEMM of this iteration and tcgen05 GEMMs of one thread execute in order, so s_full already covers them.
-      {
-        uint32_t* w = pt;
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(
-                         tmem_base + Cfg::TM_PT + (it & 1) * 32 + lane_addr + cg * 8),
-                     "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                     : "memory");
-      }
-      uint8_t* dstb = sDST + (it & 1) * Cfg::PT_BYTES;
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int cc = cg * 2 + k;
-        const int off = r * 128 + ((cc ^ (r & 7)) << 4);
-        *reinterpret_cast<uint4*>(dstb + off) = make_uint4(ds[k * 4], ds[k * 4 + 1], ds[k * 4 + 2], ds[k * 4 + 3]);
-      }
+      if (!ok) break;
       tmem_st_wait();
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(pds_ready);
+      if (lane == 0) mbar_arrive(&pds_ready[grp]);
     }
     if (ok && n_it > 0) {
       if (mbar_wait_warp(all_done, 0, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) {
@@ -388,8 +428,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
       if (!mbar_wait_warp(dq_full, it & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
       uint32_t v0[32], v1[32];
-      tmem_ld32(tmem_base + Cfg::TM_DQ + lane_addr, v0);
-      tmem_ld32(tmem_base + Cfg::TM_DQ + lane_addr + 32, v1);
+      const uint32_t src = tmem_base + Cfg::TM_DP + (it & 1) * Cfg::TM_TILE + lane_addr;
+      tmem_ld32(src, v0);
+      tmem_ld32(src + 32, v1);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
@@ -422,27 +463,36 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   }
 }
 
-// delta[b,h,s] = sum_d dO * O ; one warp per (token, head).
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
-                                  float* __restrict__ delta, int B, int S, int H, int D, long long do_row_stride,
-                                  long long o_row_stride) {
-  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= (long long)B * S * H) return;
-  const int h = w % H;
-  const long long tok = w / H;  // b*S + s
-  const __nv_bfloat16* a = dO + tok * do_row_stride + (long long)h * D;
-  const __nv_bfloat16* c = O + tok * o_row_stride + (long long)h * D;
-  float s = 0.f;
-  for (int i = lane * 2; i < D; i += 64) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a + i));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(c + i));
-    s += x.x * y.x + x.y * y.y;
+// delta[b,h,s] = sum_d dO * O, and dq_accum zeroed. Bound: memory (dO and O read, dq_accum written once). 16 lanes a (token, head) row with a
+// 16-byte load each, four rows of a lane in flight: [1, 4096, 32, 128] 21 us, 45 us as a memset and a kernel with four bytes a lane.
+__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
+                                                         float* __restrict__ delta, float4* __restrict__ acc, long long acc4, unsigned rows,
+                                                         unsigned S, unsigned H, long long do_row_stride, long long o_row_stride) {
+  constexpr int R = 4;
+  const unsigned part = threadIdx.x & 15, r0 = (blockIdx.x * 16u + (threadIdx.x >> 4)) * R;
+  const long long threads = (long long)gridDim.x * 256;
+  bf16x8 a[R], c[R];
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    const unsigned r = min(r0 + k, rows - 1), h = r % H, tok = r / H;
+    a[k] = ld8(dO + tok * do_row_stride + h * BWD_D + part * 8);
+    c[k] = ld8(O + tok * o_row_stride + h * BWD_D + part * 8);
   }
-  s = warp_sum(s);
-  if (lane == 0) {
-    const long long bb = tok / S, ss = tok % S;
-    delta[(bb * H + h) * S + ss] = s;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < acc4; i += threads) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    float x[8], y[8], s = 0.f;
+    unpack8(a[k], x);
+    unpack8(c[k], y);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += x[j] * y[j];
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const unsigned r = r0 + k;
+    if (part == 0 && r < rows) {
+      const unsigned h = r % H, tok = r / H;
+      delta[((long long)(tok / S) * H + h) * S + tok % S] = s;
+    }
   }
 }
 
@@ -507,13 +557,11 @@ extern "C" int sx_attn_bwd(const SxAttnArgs* a, cudaStream_t st) {
   const int n_qt = (a->Sq + BWD_Q - 1) / BWD_Q;
   // dq_accum holds whole 64-row query tiles: B * Hq * n_qt * 64 * 128 floats
   const long long acc_floats = (long long)a->B * a->Hq * n_qt * BWD_Q * BWD_D;
-  cudaMemsetAsync(a->dq_accum, 0, sizeof(float) * acc_floats, st);
-  {
-    const long long warps = tokens * a->Hq;
-    const int blocks = (int)((warps * 32 + 255) / 256);
-    attn_delta_kernel<<<blocks, 256, 0, st>>>((const __nv_bfloat16*)a->dO, (const __nv_bfloat16*)a->O, a->delta, a->B,
-                                              a->Sq, a->Hq, a->D, a->do_row_stride, a->o_row_stride);
-  }
+  const long long rows = tokens * a->Hq;
+  if (rows <= 0 || rows > 0x7fffffffll || (a->o_row_stride % 8) || (reinterpret_cast<uintptr_t>(a->O) & 15)) return -5;
+  attn_delta_kernel<<<(unsigned)((rows + 63) / 64), 256, 0, st>>>((const __nv_bfloat16*)a->dO, (const __nv_bfloat16*)a->O, a->delta,
+                                                                  (float4*)a->dq_accum, acc_floats / 4, (unsigned)rows, (unsigned)a->Sq,
+                                                                  (unsigned)a->Hq, a->do_row_stride, a->o_row_stride);
   p.lse = a->lse; p.delta = a->delta; p.dq_accum = a->dq_accum;
   p.dK = (__nv_bfloat16*)a->dK; p.dV = (__nv_bfloat16*)a->dV;
   p.dk_row_stride = a->dk_row_stride; p.dv_row_stride = a->dv_row_stride;
