@@ -34,12 +34,14 @@ class LlamaAttention(Module):
         B, S, _ = x.shape
         H, Hk, D = self.H, self.Hk, self.D
         qkv = self.qkv_proj(x)
+        if kv_cache is None:
+            o = ops.rope_attention(qkv, rope[0], rope[1], H, Hk, D, positions, self.window)
+            return self.o_proj(o.reshape(B, S, H * D))
         qkv = ops.rope_qk_(qkv, rope[0], rope[1], H + Hk, D, positions)
         q = qkv[..., : H * D].view(B, S, H, D)
         k = qkv[..., H * D: (H + Hk) * D].view(B, S, Hk, D)
         v = qkv[..., (H + Hk) * D:].view(B, S, Hk, D)
-        if kv_cache is not None:
-            k, v = kv_cache.append(k, v)
+        k, v = kv_cache.append(k, v)
         o = ops.attention(q, k, v, causal=True, window=self.window)
         return self.o_proj(o.reshape(B, S, H * D))
 

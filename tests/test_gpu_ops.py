@@ -194,3 +194,63 @@ def test_differential_attention():
     a = F_.attention_reference(q.float(), k.float(), v.float(), True).view(B, S, H, 2, D)
     ref = a[..., 0, :] - lam.view(1, 1, -1, 1) * a[..., 1, :]
     assert _rel(o, ref) < 3e-2
+
+
+@pytest.mark.parametrize("B,S,H,Hk,window,pos", [(2, 77, 4, 2, 0, False), (1, 256, 8, 8, 0, True), (3, 130, 7, 1, 40, True), (1, 1, 4, 4, 0, False)])
+def test_rope_attention_is_rope_then_attention(B, S, H, Hk, window, pos):
+    """One node for rotation and attention against the two of them: the same kernels on the same operands, so outputs agree exactly and
+    gradients up to the order of the dQ additions and one more bf16 rounding (dQ and dK are rounded, then turned back: 2^-8 of a value)."""
+    torch.manual_seed(S)
+    D = 128
+    x = torch.randn(B, S, (H + 2 * Hk) * D, device="cuda", dtype=torch.bfloat16)
+    cos, sin = F_.rope_tables(512, D, 5e5, "cuda")
+    positions = torch.randint(0, 512, (B, S), device="cuda") if pos else None
+    a, b = x.clone().requires_grad_(True), x.clone().requires_grad_(True)
+    o = F_.rope_attention(a, cos, sin, H, Hk, D, positions, window)
+    q, k, v = F_._split_heads(F_.rope_qk_(b, cos, sin, H + Hk, D, positions), H, Hk, D)
+    ref = F_.attention(q, k, v, causal=True, window=window)
+    assert o.shape == (B, S, H, D) and torch.equal(o, ref) and torch.equal(a, x)
+    g = torch.randn_like(o)
+    o.backward(g)
+    ref.backward(g)
+    assert _rel(a.grad, b.grad) < 2.0 ** -7
+
+
+@pytest.mark.parametrize("heads,rot,D,interleaved,strided", [(6, 4, 128, False, False), (5, 5, 16, False, True), (3, 2, 24, False, False), (4, 2, 64, True, False)])
+def test_rope_to_new_buffer(heads, rot, D, interleaved, strided):
+    """Rotation into a new buffer and back: 16-byte kernel, a column slice of a wider tensor, and the sizes and layout that go through a copy.
+    Products and sums are 32-bit, so one bf16 rounding each way is left."""
+    torch.manual_seed(D)
+    B, S = 2, 33
+    wide = torch.randn(B, S, heads * D + 64, device="cuda", dtype=torch.bfloat16)
+    x = wide[..., :heads * D] if strided else wide[..., :heads * D].contiguous()
+    cos, sin = F_.rope_tables(S, D, 1e4, "cuda")
+    before = wide.clone()
+    y = F_.rope_qk_(x, cos, sin, rot, D, None, interleaved)
+    ref = F_.rope_reference(x[..., :rot * D].reshape(B, S, rot, D).float(), cos, sin, None, interleaved).reshape(B, S, -1)
+    assert torch.equal(wide, before) and torch.equal(y[..., rot * D:], x[..., rot * D:])
+    assert bool(((y[..., :rot * D].float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
+
+
+@pytest.mark.parametrize("T,d", [(1, 8), (3, 1024), (700, 1032), (2, 2048), (300, 2056), (5, 8192), (3, 8200), (2, 16384)])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_rmsnorm_row_sizes(T, d, with_res):
+    """Edges of the register forms (one and two vectors a thread, two passes beyond), fewer and more rows than backward CTAs, and weight
+    gradients from one to many partial rows. Inputs are bf16, everything else 32-bit: one rounding of each output, 2^-8 of its value plus
+    2^-8 of the residual sum that is rounded first; the weight gradient sums T products."""
+    torch.manual_seed(d)
+    x, r, g, gh = (torch.randn(T, d, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    w = (1 + 0.1 * torch.randn(d, device="cuda")).to(torch.bfloat16)
+    ins = [t.clone().requires_grad_(True) for t in ((x, w, r) if with_res else (x, w))]
+    y, h = F_.rmsnorm(ins[0], ins[1], 1e-5, ins[2] if with_res else None)
+    (((y * g).sum() + (h * gh).sum()) if with_res else (y * g).sum()).backward()
+    ref = [t.double().requires_grad_(True) for t in ((x, w, r) if with_res else (x, w))]
+    hr = (ref[0] + ref[2]) if with_res else ref[0]
+    hb = hr + (hr.detach().bfloat16().double() - hr.detach())          # the sum as it is stored
+    yr = hb * torch.rsqrt(hb.pow(2).mean(-1, keepdim=True) + 1e-5) * ref[1]
+    (((yr * g.double()).sum() + (hb * gh.double()).sum()) if with_res else (yr * g.double()).sum()).backward()
+    close = lambda a, b, extra=0.0: bool(((a.double() - b).abs() <= b.abs() * 2.0 ** -8 + extra).all())  # noqa: E731
+    assert close(y, yr.detach(), 1e-5)
+    top = ref[0].grad.abs().max().item()
+    assert close(ins[0].grad, ref[0].grad, 1e-4 * top)
+    assert close(ins[1].grad, ref[1].grad, 1e-4 * ref[1].grad.abs().max().item())

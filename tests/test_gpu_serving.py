@@ -220,3 +220,24 @@ def test_mamba2_decode_step(hidden, headdim, state, groups, taps, layers, batch)
     assert all(torch.equal(x[k], y[k]) for x, y in zip(kept, before) for k in x)
     a, b = run.decode([0, 0], [3, 3]), ref.decode([0, 0], [3, 3])
     assert close(a, b) and isinstance(run.states.entry(0), list)
+
+
+@pytest.mark.parametrize("T,Hq,Hkv,D,rotate", [(1, 4, 1, 128, True), (37, 28, 4, 128, True), (9, 40, 8, 256, True), (50, 6, 2, 16, True),
+                                               (50, 6, 2, 24, True), (33, 8, 8, 64, False)])
+def test_kv_append_sizes(T, Hq, Hkv, D, rotate):
+    """16-byte form (more items than a CTA has threads included) and the form for head sizes that are no multiple of 16; rows without a slot
+    are rotated and written nowhere. Products and sums are 32-bit: one bf16 rounding, 2^-8; copies are exact."""
+    torch.manual_seed(T)
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * D, device="cuda", dtype=torch.bfloat16)
+    kc = torch.randn(T // 4 + 2, 4, Hkv, D, device="cuda", dtype=torch.bfloat16)
+    vc = torch.randn_like(kc)
+    cos, sin = rope_tables(256, D, 1e4, "cuda")
+    pos = torch.randint(0, 256, (T,), device="cuda", dtype=torch.int32)
+    slot = torch.randperm(T, device="cuda").int() + 3
+    slot[::5] = -1
+    want = [t.double() for t in (qkv, kc, vc)]
+    paged.kv_append_reference(want[0], cos.double(), sin.double(), pos, slot, want[1], want[2], Hq, Hkv, D, rotate)
+    paged.kv_append_(qkv, cos, sin, pos, slot, kc, vc, Hq, Hkv, D, rotate)
+    for got, ref in zip((qkv, kc, vc), want):
+        assert bool(((got.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
+    assert torch.equal(vc.double(), want[2])
