@@ -17,109 +17,136 @@ __device__ __forceinline__ float silu_grad(float x) {
   return s * (1.f + x * (1.f - s));
 }
 
-// One thread: 8 channels x CONV_TL consecutive positions. The 8 x K weights and the bias live in registers and the
+// V channels of a row: V = 4 (8 bytes) forward, 2 backward.
+template <int V> struct ConvVec;
+template <> struct ConvVec<4> { typedef uint2 T; };
+template <> struct ConvVec<2> { typedef uint32_t T; };
+__device__ __forceinline__ float2 bf2(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); }
+__device__ __forceinline__ uint32_t pk2(float a, float b) {
+  const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&t);
+}
+__device__ __forceinline__ void conv_unpack(uint2 r, float (&f)[4]) {
+  const float2 a = bf2(r.x), b = bf2(r.y);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
+__device__ __forceinline__ void conv_unpack(uint32_t r, float (&f)[2]) {
+  const float2 a = bf2(r);
+  f[0] = a.x; f[1] = a.y;
+}
+__device__ __forceinline__ uint2 conv_pack(const float (&f)[4]) { return make_uint2(pk2(f[0], f[1]), pk2(f[2], f[3])); }
+__device__ __forceinline__ uint32_t conv_pack(const float (&f)[2]) { return pk2(f[0], f[1]); }
+template <int V> __device__ __forceinline__ typename ConvVec<V>::T conv_ld(const __nv_bfloat16* p) {
+  return *reinterpret_cast<const typename ConvVec<V>::T*>(p);
+}
+template <int V> __device__ __forceinline__ void conv_ld(const __nv_bfloat16* p, float (&f)[V]) { conv_unpack(conv_ld<V>(p), f); }
+template <int V> __device__ __forceinline__ void conv_st(__nv_bfloat16* p, const float (&f)[V]) {
+  *reinterpret_cast<typename ConvVec<V>::T*>(p) = conv_pack(f);
+}
+template <int K, int V>
+__device__ __forceinline__ void conv_taps(const __nv_bfloat16* w, int c, float (&wv)[K][V]) {
+  if (K == 4 && (reinterpret_cast<uintptr_t>(w) & 7) == 0) {   // a channel's four taps are 8 contiguous bytes
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      float t[4];
+      conv_ld<4>(w + (c + j) * 4, t);
+#pragma unroll
+      for (int k = 0; k < K; ++k) wv[k][j] = t[k];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int j = 0; j < V; ++j) wv[k][j] = __bfloat162float(w[(c + j) * K + k]);
+  }
+}
+
+// One thread: 4 channels x CONV_TL consecutive positions. The 4 x K weights and the bias live in registers and the
 // K-1 previous inputs slide through registers, so each input vector is loaded once and each output costs one 16-byte
 // load and one 16-byte store; consecutive threads own consecutive channel vectors (coalesced rows).
+// What bounds it is the latency of these chains (180 instructions for 8 channels of a row, half of them the sigmoid), so warps count: with
+// eight channels a thread and 128 registers an SM held 12 to 16. [8192, 7168]: 78 us, 100 with eight (36 us at copy bandwidth); [4, 500, 1792]
+// 14 and 16 us.
 constexpr int CONV_TL = 16;
 template <int K>
-__global__ void __launch_bounds__(256) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                         const __nv_bfloat16* __restrict__ prev,
-                                                         const __nv_bfloat16* __restrict__ w,
-                                                         const __nv_bfloat16* __restrict__ bias,
-                                                         __nv_bfloat16* __restrict__ y,
-                                                         __nv_bfloat16* __restrict__ state_out, int B, int L, int C,
-                                                         int act, long long xld, int Ly) {
-  const int cv = C >> 3;
+__global__ void __launch_bounds__(256, 3) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ prev,
+                                                            const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
+                                                            __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ state_out, int B,
+                                                            int L, int C, int act, long long xld, int Ly) {
+  constexpr int V = 4;
+  const int cv = C / V;
   const int lchunks = (L + CONV_TL - 1) / CONV_TL;
   const long long total = (long long)B * lchunks * cv;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % cv) * 8;
+  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
+    const int c = (int)(idx % cv) * V;
     const long long bl = idx / cv;
     const int l0 = (int)(bl % lchunks) * CONV_TL;
     const int b = (int)(bl / lchunks);
-    float wv[CONV_MAXK][8], bv[8];
-#pragma unroll
-    for (int k = 0; k < CONV_MAXK; ++k)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) wv[k][j] = (k < K) ? __bfloat162float(w[(c + j) * K + k]) : 0.f;
-    if (bias) unpack8(ld8(bias + c), bv);
+    const int l1 = min(L, l0 + CONV_TL);
+    const __nv_bfloat16* xp = x + ((long long)b * L + l0) * xld + c;
+    __nv_bfloat16* yp = y + ((long long)b * Ly + l0) * C + c;
+    float wv[K][V], bv[V];
+    conv_taps<K, V>(w, c, wv);
+    if (bias) conv_ld<V>(bias + c, bv);
     else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) bv[j] = 0.f;
+      for (int j = 0; j < V; ++j) bv[j] = 0.f;
     }
     // hist[i] = input at position l - (K-1) + i for the current l; hist[K-1] is the current input
-    float hist[CONV_MAXK][8];
+    float hist[K][V];
 #pragma unroll
-    for (int i = 0; i < CONV_MAXK; ++i)
+    for (int i = 0; i < K; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) hist[i][j] = 0.f;
+      for (int j = 0; j < V; ++j) hist[i][j] = 0.f;
+#pragma unroll
     for (int i = 0; i < K - 1; ++i) {
       const int ls = l0 - (K - 1) + i;
-      if (ls >= 0) unpack8(ld8(x + ((long long)b * L + ls) * xld + c), hist[i]);
-      else if (prev) unpack8(ld8(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c), hist[i]);
+      if (ls >= 0) conv_ld<V>(xp + (long long)(i - (K - 1)) * xld, hist[i]);
+      else if (prev) conv_ld<V>(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c, hist[i]);
     }
-    const int l1 = min(L, l0 + CONV_TL);
     for (int lb = l0; lb < l1; lb += 4) {
-      bf16x8 raw4[4];   // four independent 16-byte loads in flight per thread
+      uint2 raw4[4];   // four independent loads in flight per thread
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (lb + u < l1) raw4[u] = ld8(x + ((long long)b * L + lb + u) * xld + c);
+      for (int u = 0; u < 4; ++u, xp += xld)
+        if (lb + u < l1) raw4[u] = conv_ld<V>(xp);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 4; ++u, yp += C) {
         const int l = lb + u;
         if (l >= l1) break;
-        const bf16x8 raw = raw4[u];
-        unpack8(raw, hist[K - 1]);
-        float acc[8];
+        conv_unpack(raw4[u], hist[K - 1]);
+        float acc[V];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] = bv[j];
+        for (int j = 0; j < V; ++j) acc[j] = bv[j];
 #pragma unroll
-        for (int k = 0; k < CONV_MAXK; ++k)
-          if (k < K) {
+        for (int k = 0; k < K; ++k)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] = fmaf(hist[k][j], wv[k][j], acc[j]);
-          }
+          for (int j = 0; j < V; ++j) acc[j] = fmaf(hist[k][j], wv[k][j], acc[j]);
         if (act) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[j] = silu_f(acc[j]);
+          for (int j = 0; j < V; ++j) acc[j] = silu_f(acc[j]);
         }
-        st8(y + ((long long)b * Ly + l) * C + c, pack8(acc));
-        if (state_out && l >= L - (K - 1)) st8(state_out + ((long long)b * (K - 1) + (l - (L - (K - 1)))) * C + c, raw);
+        conv_st<V>(yp, acc);
+        if (state_out && l >= L - (K - 1))
+          *reinterpret_cast<uint2*>(state_out + ((long long)b * (K - 1) + (l - (L - (K - 1)))) * C + c) = raw4[u];
 #pragma unroll
-        for (int i = 0; i < CONV_MAXK - 1; ++i)
-          if (i < K - 1) {
+        for (int i = 0; i + 1 < K; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) hist[i][j] = hist[i + 1][j];
-          }
+          for (int j = 0; j < V; ++j) hist[i][j] = hist[i + 1][j];
       }
     }
   }
 }
 
-// dx and per-CTA partials of dw / dbias. A CTA is 32 channel groups of 4 (one per lane: 256 contiguous bytes per
-// row) by 8 runs of CONV_BTL consecutive positions (one per warp). A thread walks its run once: the last K inputs and
-// the last K pre-activation gradients slide through registers, so every x and dy value is loaded once (plus the K-1
-// row overlap between runs) and dx is stored once. Four channels per thread keep the kernel near 100 registers (two
-// CTAs per SM); with eight it needed 205 and ran at one. The 8 warps add their dw / db into shared memory and the CTA
-// writes one partial row; conv1d_reduce_partials sums the rows.
-constexpr int CONV_BTL = 16;
-constexpr int CONV_BV = 4;
-__device__ __forceinline__ void ld4(const __nv_bfloat16* p, float (&f)[CONV_BV]) {
-  const uint2 r = *reinterpret_cast<const uint2*>(p);
-  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
-  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
-}
-__device__ __forceinline__ void st4(__nv_bfloat16* p, const float (&f)[CONV_BV]) {
-  const __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
-  uint2 r;
-  r.x = *reinterpret_cast<const uint32_t*>(&a);
-  r.y = *reinterpret_cast<const uint32_t*>(&b);
-  *reinterpret_cast<uint2*>(p) = r;
-}
+// dx and per-CTA partials of dw / dbias. A CTA is 32 channel groups of 2 (one per lane: 128 contiguous bytes per row) by 8 runs of
+// CONV_BTL consecutive positions (one per warp). A thread walks its run once: the last K inputs and the last K pre-activation gradients
+// slide through registers, so every x and dy value is loaded once (plus the K-1 row overlap between runs) and dx is stored once. As above
+// warps count more than wide loads: two channels a thread keep the kernel near 64 registers, four CTAs an SM. [8192, 7168]: 247 us, 265 with
+// four channels and two CTAs an SM (54 us at copy bandwidth): the instructions of a row bound it. The 8 warps add their dw / db into shared memory and the CTA writes one
+// partial row; conv1d_reduce_partials sums the rows.
+constexpr int CONV_BTL = 16, BWD_CTAS = 4;
+constexpr int CONV_BV = 2;
 template <int K>
-__global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
+__global__ void __launch_bounds__(256, BWD_CTAS) conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                             const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ prev,
                                                             const __nv_bfloat16* __restrict__ w,
@@ -138,27 +165,14 @@ __global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const __nv_bfloat16*
   __syncthreads();
   if (live) {
     float wv[K][V], bv[V], dwacc[K][V], dbacc[V];
-    if (K == 4) {   // a channel's four taps are 8 contiguous bytes
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        float t[4];
-        ld4(w + (c + j) * 4, t);
-#pragma unroll
-        for (int k = 0; k < K; ++k) wv[k][j] = t[k];
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < K; ++k)
-#pragma unroll
-        for (int j = 0; j < V; ++j) wv[k][j] = __bfloat162float(w[(c + j) * K + k]);
-    }
+    conv_taps<K, V>(w, c, wv);
 #pragma unroll
     for (int k = 0; k < K; ++k)
 #pragma unroll
       for (int j = 0; j < V; ++j) dwacc[k][j] = 0.f;
 #pragma unroll
     for (int j = 0; j < V; ++j) dbacc[j] = bv[j] = 0.f;
-    if (bias) ld4(bias + c, bv);
+    if (bias) conv_ld<V>(bias + c, bv);
     const int lchunks = (L + CONV_BTL - 1) / CONV_BTL;
     const int nchunks = B * lchunks;
     for (int ch = blockIdx.y * 8 + sub; ch < nchunks; ch += gridDim.y * 8) {
@@ -172,8 +186,8 @@ __global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const __nv_bfloat16*
 #pragma unroll
       for (int i = 1; i < K; ++i) {
         const int ls = l0 - K + i;
-        if (ls >= 0) ld4(x + ((long long)b * L + ls) * xld + c, xh[i]);
-        else if (prev) ld4(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c, xh[i]);
+        if (ls >= 0) conv_ld<V>(x + ((long long)b * L + ls) * xld + c, xh[i]);
+        else if (prev) conv_ld<V>(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c, xh[i]);
       }
 #pragma unroll 4
       for (int l = l0; l < lend + K - 1; ++l) {
@@ -185,8 +199,8 @@ __global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const __nv_bfloat16*
             dph[i][j] = dph[i + 1][j];
           }
         if (l < L) {
-          ld4(x + ((long long)b * L + l) * xld + c, xh[K - 1]);
-          ld4(dy + ((long long)b * Ly + l) * C + c, dph[K - 1]);
+          conv_ld<V>(x + ((long long)b * L + l) * xld + c, xh[K - 1]);
+          conv_ld<V>(dy + ((long long)b * Ly + l) * C + c, dph[K - 1]);
           if (act) {
 #pragma unroll
             for (int j = 0; j < V; ++j) {
@@ -218,7 +232,7 @@ __global__ void __launch_bounds__(256, 2) conv1d_bwd_kernel(const __nv_bfloat16*
             for (int k = 0; k < K; ++k) a += wv[k][j] * dph[K - 1 - k][j];
             dxa[j] = a;
           }
-          st4(dx + ((long long)b * L + lo) * dxld + c, dxa);
+          conv_st<V>(dx + ((long long)b * L + lo) * dxld + c, dxa);
         }
       }
     }
@@ -259,7 +273,7 @@ using namespace sx;
 extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, const void* bias, void* y, void* state_out,
                              int B, int L, int C, int K, int act, long long xld, int Ly, cudaStream_t st) {
   if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L) return -1;
-  const long long total = (long long)B * ((L + CONV_TL - 1) / CONV_TL) * (C / 8);
+  const long long total = (long long)B * ((L + CONV_TL - 1) / CONV_TL) * (C / 4);
   if (total == 0) return 0;
   const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
 #define SX_CONV_FWD(KK)                                                                                          \
@@ -279,11 +293,11 @@ extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, con
 // Number of partial rows the backward kernel writes for B sequences of L tokens of C channels.
 extern "C" int sx_conv1d_bwd_parts(int B, int L, int C) {
   // four runs per warp (32 per CTA): the per-CTA prologue (taps, bias) and epilogue (partial row) cost about as much
-  // as one run. Inputs that would leave SMs idle that way take as many CTAs as make one wave (two an SM), down to one
+  // as one run. Inputs that would leave SMs idle that way take as many CTAs as make one wave, down to one
   // run per warp ([4, 500, 1792]: 73 -> 32 us)
   const long long chunks = (long long)B * ((L + CONV_BTL - 1) / CONV_BTL);
   const int cols = (C / CONV_BV + 31) / 32;
-  const long long wave = 296 / (cols > 0 ? cols : 1), most = (chunks + 7) / 8;
+  const long long wave = 148 * BWD_CTAS / (cols > 0 ? cols : 1), most = (chunks + 7) / 8;
   long long p = (chunks + 31) / 32;
   if (p < wave) p = most < wave ? most : wave;
   return (int)(p < 1 ? 1 : (p > 512 ? 512 : p));
