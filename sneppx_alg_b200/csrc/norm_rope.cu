@@ -423,10 +423,11 @@ extern "C" int sx_rmsnorm_fwd(const void* x, const void* res_in, const void* w, 
                                           (__nv_bfloat16*)res_out, rstd, d, eps);
   };
   auto per = [&](int v) { return ((nvec + v - 1) / v + 31) / 32 * 32; };
-  // one vector a thread for rows up to 1024, two up to 8192; a CTA of 1024 threads has an SM to itself, and two passes over L2 are
+  // 256 threads up to 4096 as long as they have a vector each (a thread's share then does not depend on how the row divides), more threads
+  // with two vectors up to 8192; a CTA of 1024 threads has an SM to itself, and two passes over L2 are
   // faster then ([1000, 16384]: 37 against 43 us)
-  if (nvec <= 128) run(rmsnorm_fwd_kernel<1>, per(1));
-  else if (nvec <= 1024) run(rmsnorm_fwd_kernel<2>, per(2));
+  if (nvec <= 256) run(rmsnorm_fwd_kernel<1>, per(1));
+  else if (nvec <= 1024) run(rmsnorm_fwd_kernel<2>, nvec <= 512 ? 256 : per(2));
   else run(rmsnorm_fwd_long_kernel, 256);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
@@ -443,10 +444,10 @@ extern "C" int sx_rmsnorm_bwd(const void* dy, const void* h, const void* w, cons
   const int most = nvec <= 256 ? 592 : 296;      // short rows: four small CTAs an SM keep as much in flight as two large ones
   const int parts = T < most ? (int)T : most;
   auto run = [&](auto kern, int v) {
-    kern<<<parts, ((nvec + v - 1) / v + 31) / 32 * 32, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w,
+    kern<<<parts, nvec > 256 && nvec <= 512 ? 256 : ((nvec + v - 1) / v + 31) / 32 * 32, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w,
                                                                rstd, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, dw_partial, (int)T, d);
   };
-  if (nvec <= 128) run(rmsnorm_bwd_kernel<1>, 1);
+  if (nvec <= 256) run(rmsnorm_bwd_kernel<1>, 1);
   else if (nvec <= 1024) run(rmsnorm_bwd_kernel<2>, 2);
   else if (nvec <= 2048) run(rmsnorm_bwd_kernel<4>, 4);
   else return -2;
