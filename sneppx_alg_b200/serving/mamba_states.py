@@ -127,7 +127,7 @@ def _sizes(model):
     H, P, N, G, taps = m.nheads, m.headdim, m.d_state, m.ngroups, m.d_conv
     inner, chan = H * P, H * P + 2 * G * N
     # sizes of 8, as the prompt form wants them; a lane of the step kernel owns four neighbouring state columns, two such pieces at most
-    if d % 8 or P % 8 or chan % 8 or N % 8 or N > 256 or P > 4096 or not 2 <= taps <= 4 or H % G or inner > 65536:
+    if d % 8 or P % 8 or chan % 8 or N % 8 or N > 256 or P > 1024 or not 2 <= taps <= 4 or H % G or inner > 65536:
         return None
     for layer in model.layers:
         sub = layer._modules
