@@ -39,6 +39,7 @@ struct PagedTcParams {
   float* ml_part;
   int* status;
   int B, Hq, Hkv, block_size, max_blocks, nsplit;
+  bool few_items;         // per CTA
   float scale_log2;
 };
 
@@ -55,15 +56,25 @@ struct PtItem {
   int b, hk, split, len, t0, n_steps;
 };
 
-// Work item `item` of the (sequence, split, KV head) space, heads fastest: a cached position's heads lie side by side (256 bytes each), and
-// neighbouring CTAs that walk the same positions at the same time read whole DRAM pages together (48 sequences of 900 - 1800 positions, 8 heads:
-// 72 us with sequences fastest, 67 us). The tile range comes from the sequence length on the device.
+// (sequence b, KV head hk, split) of item `item`, heads fastest: a cached position's heads lie side by side (256 bytes each), and neighbouring CTAs
+// that walk the same positions at the same time read whole DRAM pages together (48 sequences of 900 - 1800 positions, 8 heads: 87 us with
+// sequences fastest, 83 so). Splits slowest as long as a CTA has few items: the last splits of a sequence are shorter or empty and fill up
+// what the long ones leave, where otherwise some CTAs got long items only (16 sequences of 1000 positions, 4 heads: 30 us with splits before
+// sequences, 26 so; 128 of 4000, 2 heads, 10 items a CTA: 136 and 130). Odd splits walk the sequences backwards, so that a batch sorted by
+// length deals long and short items to the same CTA. With more than 12 items a CTA that evens out, and one sequence's splits side by side
+// are better (128 sequences of 1000 positions, 32 heads: 429 us, 441 with splits slowest).
+constexpr int PT_FEW_ITEMS = 12;
+__host__ __device__ __forceinline__ void pt_order(int item, int B, int Hkv, int nsplit, bool few, int* b, int* hk, int* split) {
+  const int rest = item / Hkv, d = few ? B : nsplit, q = rest / d, r = rest - q * d;
+  *hk = item - rest * Hkv;
+  *split = few ? q : r;
+  *b = few ? (q & 1 ? B - 1 - r : r) : q;
+}
+
+// The tile range of an item comes from the sequence length on the device.
 __device__ __forceinline__ PtItem pt_item(const PagedTcParams& p, int item) {
   PtItem w;
-  w.hk = item % p.Hkv;
-  const int rest = item / p.Hkv;
-  w.split = rest % p.nsplit;
-  w.b = rest / p.nsplit;
+  pt_order(item, p.B, p.Hkv, p.nsplit, p.few_items, &w.b, &w.hk, &w.split);
   w.len = p.seq_lens[w.b];
   const int tiles = (w.len + PT_BN - 1) / PT_BN;
   const int per = (tiles + p.nsplit - 1) / p.nsplit;
@@ -366,7 +377,7 @@ void paged_merge_launch(const float* o_part, const float* ml_part, void* out, lo
 }  // namespace sx
 using namespace sx;
 
-// Splits for the tensor-core kernel. It is persistent (one CTA per SM walks the (split, KV head, sequence) items), so
+// Splits for the tensor-core kernel. It is persistent (one CTA per SM walks the (sequence, KV head, split) items), so
 // splits only set the granularity: items of about six tiles keep the SMs evenly loaded, and there are at least two
 // items per SM when the batch is small.
 extern "C" int sx_paged_decode_tc_splits(int max_len, int ctas_per_split) {
@@ -377,6 +388,11 @@ extern "C" int sx_paged_decode_tc_splits(int max_len, int ctas_per_split) {
   if (s > tiles) s = tiles;
   if (s > 32) s = 32;
   return s < 1 ? 1 : s;
+}
+
+// The (sequence, KV head, split) of an item, for checks of the order on the host.
+extern "C" void sx_paged_decode_tc_item(int item, int B, int Hkv, int nsplit, int sms, int* b, int* hk, int* split) {
+  pt_order(item, B, Hkv, nsplit, (long long)B * Hkv * nsplit <= (long long)PT_FEW_ITEMS * sms, b, hk, split);
 }
 
 // Same contract as sx_paged_decode (o_part: fp32 [B, Hq, nsplit, D], ml_part: fp32 [B, Hq, nsplit, 2] scratch);
@@ -428,6 +444,7 @@ extern "C" int sx_paged_decode_tc(const void* q, long long q_row_stride, const v
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   }
   const long long items = (long long)B * Hkv * nsplit;
+  p.few_items = items <= (long long)PT_FEW_ITEMS * sms;
   paged_decode_tc_kernel<<<(unsigned)(items < sms ? items : sms), PT_THREADS, PT_SMEM, st>>>(p);
   paged_merge_launch(o_part, ml_part, out, out_row_stride, B, Hq, D, nsplit, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;

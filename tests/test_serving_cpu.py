@@ -179,3 +179,28 @@ def test_recurrent_states_leave_their_block_when_read():
     s, b = fresh()
     assert s.entry(7) is b and 7 in s and len(s) == 2 and s.get(9) is None
     assert s != {} and SequenceStates() == {}
+
+
+def test_paged_decode_deals_its_items_evenly():
+    """The decode kernel's CTAs take items c, c + n, ...: every (sequence, KV head, split) exactly once, and with few items a CTA none gets more
+    tiles of equal sequences than when the long items are dealt first."""
+    import ctypes as C
+    from sneppx_alg_b200 import _build
+    lib, n_cta = _build.load_cuda(), 148
+    for B, Hkv, n in ((16, 4, 1000), (16, 8, 1000), (16, 2, 4000), (128, 2, 4000), (48, 8, 4000), (3, 1, 200), (1, 1, 1), (128, 32, 1000)):
+        max_len = (n // 16 + 1) * 16
+        ns = lib.sx_paged_decode_tc_splits(C.c_int(max_len), C.c_int(B * Hkv))
+        tiles = (n + 127) // 128
+        per = -(-tiles // ns)
+        count = [max(0, min(tiles, (s + 1) * per) - s * per) for s in range(ns)]
+        b, hk, s = C.c_int(), C.c_int(), C.c_int()
+        seen, load = set(), [0] * n_cta
+        for i in range(B * Hkv * ns):
+            lib.sx_paged_decode_tc_item(i, B, Hkv, ns, n_cta, C.byref(b), C.byref(hk), C.byref(s))
+            seen.add((b.value, hk.value, s.value))
+            load[i % n_cta] += count[s.value]
+        assert seen == {(i, j, k) for i in range(B) for j in range(Hkv) for k in range(ns)}
+        best, longest = [0] * n_cta, sorted(count, reverse=True)
+        for i in range(B * Hkv * ns):
+            best[i % n_cta] += longest[i // (B * Hkv)]
+        assert max(load) == max(best) or B * Hkv * ns > 12 * n_cta, (B, Hkv, n, max(load), max(best))
