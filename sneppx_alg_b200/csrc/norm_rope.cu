@@ -1,6 +1,6 @@
 // N1: RMSNorm forward/backward with the residual add fused in, and LayerNorm forward.
-// R1: rotary position embedding (rotate-half and adjacent-pair conventions), in place on the
-//     fused QKV activation, forward and backward.
+// R1: rotary position embedding (rotate-half and adjacent-pair conventions) of the fused QKV activation,
+//     into a new buffer or in place, forward and backward.
 // SwiGLU / GeGLU gating forward and backward.
 // All bf16 in/out with fp32 math; rows are read with 128-bit loads. These replace the
 // reference's layernorm / rmsnorm / rope kernels (kernel/cuda/tensor_cuda.cu:393-441,
@@ -295,18 +295,20 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
   }
 }
 
-// Rotate-half layout from src to dst (which may be the same): one CTA per token, 8 rotation pairs per thread, i.e. two 16-byte loads of x (the
-// halves) and 2 x 32 bytes of cos / sin, which the heads of a token share in L1. Heads from `rot` on are copied. Bound: memory; rotating into
-// a new buffer replaces a copy followed by a rotation in place ([4096, 48 x 128]: 27 + 23 us before, 27 us).
+// Rotate-half layout from src to dst (which may be the same): 8 rotation pairs per thread, i.e. two 16-byte loads of x (the halves) and 2 x 32
+// bytes of cos / sin, which the heads of a token share in L1. Heads from `rot` on are copied. Launch shape: token_grid. Bound: memory; rotating into a new buffer replaces a copy followed by a rotation in place
+// ([4096, 48 x 128]: 27 + 23 us before, 27 us).
 __global__ void __launch_bounds__(512) rope_vec8_kernel(const __nv_bfloat16* src, __nv_bfloat16* dst, const float* __restrict__ cos_t,
-                                                        const float* __restrict__ sin_t, const int* __restrict__ pos, int seq, int heads,
-                                                        int rot, int D, long long src_stride, long long dst_stride, float sign) {
+                                                        const float* __restrict__ sin_t, const int* __restrict__ pos, unsigned tokens,
+                                                        int seq, int heads, int rot, int D, long long src_stride, long long dst_stride,
+                                                        float sign) {
   const int half = D >> 1, hv = half >> 3;
-  const long long t = blockIdx.x;
-  const long long p = pos ? pos[t] : (int)(t % seq);
+  const unsigned t = blockIdx.x * blockDim.y + threadIdx.y;
+  if (t >= tokens) return;
+  const long long p = pos ? pos[t] : (int)(t % (unsigned)seq);
   src += t * src_stride;
   dst += t * dst_stride;
-  for (int k = threadIdx.x; k < heads * hv; k += blockDim.x) {
+  for (int k = blockIdx.y * blockDim.x + threadIdx.x; k < heads * hv; k += gridDim.y * blockDim.x) {
     const int hd = k / hv, i = (k - hd * hv) * 8, o = hd * D + i;
     const bf16x8 pa = ld8(src + o), pb = ld8(src + o + half);
     if (hd >= rot) {
@@ -334,9 +336,11 @@ __global__ void __launch_bounds__(512) rope_vec8_kernel(const __nv_bfloat16* src
 }
 static int rope_vec8(const void* src, void* dst, const float* cos_t, const float* sin_t, const int* pos, long long tokens, int seq, int heads,
                      int rot, int D, long long src_stride, long long dst_stride, int backward, cudaStream_t st) {
-  const int items = heads * (D / 16);
-  rope_vec8_kernel<<<(unsigned)tokens, items < 512 ? (items + 31) / 32 * 32 : 512, 0, st>>>(
-      (const __nv_bfloat16*)src, (__nv_bfloat16*)dst, cos_t, sin_t, pos, seq, heads, rot, D, src_stride, dst_stride, backward ? -1.f : 1.f);
+  if (heads <= 0) return -11;
+  dim3 grid, block;
+  token_grid(tokens, heads * (D / 16), &grid, &block);
+  rope_vec8_kernel<<<grid, block, 0, st>>>((const __nv_bfloat16*)src, (__nv_bfloat16*)dst, cos_t, sin_t, pos, (unsigned)tokens, seq, heads, rot, D,
+                                           src_stride, dst_stride, backward ? -1.f : 1.f);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 static bool rope_vec8_ok(const void* src, const void* dst, const float* cos_t, const float* sin_t, long long tokens, int D, long long src_stride,

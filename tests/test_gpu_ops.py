@@ -5,7 +5,8 @@ import pytest
 import torch
 
 from sneppx_alg_b200 import ops
-from sneppx_alg_b200.ops import functional as F_
+from sneppx_alg_b200.ops import _lib, functional as F_
+from sneppx_alg_b200.ops._lib import c_int, c_ll, ptr, stream
 from sneppx_alg_b200.optim.fused import adamw_flat_, adamw_reference, grad_norm_
 
 pytestmark = pytest.mark.gpu
@@ -254,3 +255,51 @@ def test_rmsnorm_row_sizes(T, d, with_res):
     top = ref[0].grad.abs().max().item()
     assert close(ins[0].grad, ref[0].grad, 1e-4 * top)
     assert close(ins[1].grad, ref[1].grad, 1e-4 * ref[1].grad.abs().max().item())
+
+
+def _copy_us(nbytes):
+    """Time of a plain copy that reads and writes ``nbytes`` in all, buffers larger than L2."""
+    a = torch.empty(512 << 20, dtype=torch.uint8, device="cuda")
+    b = torch.empty_like(a)
+    return _median_us(lambda: b.copy_(a)) * nbytes / (2 * a.numel())
+
+
+def _median_us(fn, n=11):
+    for _ in range(3):
+        fn()
+    ts = []
+    for _ in range(n):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda._sleep(400000)          # the launches are queued before the first starts
+        a.record()
+        fn()
+        b.record()
+        torch.cuda.synchronize()
+        ts.append(a.elapsed_time(b) * 1e3)
+    return sorted(ts)[n // 2]
+
+
+@pytest.mark.parametrize("T,heads,rot,D", [(1, 1, 1, 16), (131, 1, 1, 16), (300, 3, 2, 48), (64, 15, 15, 128), (147, 16, 10, 128), (148, 16, 10, 128),
+                                           (5, 96, 80, 256), (200, 97, 90, 256)])
+def test_rope_launch_shapes(T, heads, rot, D):
+    """Tokens that share a CTA, with a last CTA that is not full; one CTA a token; a token over several CTAs. In place and into a new buffer,
+    against 64 bits: products and sums are 32-bit, one bf16 rounding."""
+    torch.manual_seed(T)
+    x = torch.randn(1, T, heads * D, device="cuda", dtype=torch.bfloat16)
+    cos, sin = F_.rope_tables(T, D, 1e4, "cuda")
+    ref = F_.rope_reference(x[..., :rot * D].reshape(1, T, rot, D).double(), cos.double(), sin.double()).reshape(1, T, -1)
+    y = F_.rope_qk_(x, cos, sin, rot, D)
+    assert bool(((y[..., :rot * D].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all()) and torch.equal(y[..., rot * D:], x[..., rot * D:])
+    z = x.clone()
+    _lib.call("sx_rope", ptr(z), ptr(cos), ptr(sin), ptr(None), c_ll(T), c_int(T), c_int(rot), c_int(D), c_ll(heads * D), c_int(0), c_int(0), stream())
+    assert torch.equal(z, y)
+
+
+def test_rope_of_small_tokens_keeps_up_with_a_copy():
+    """One head of 16 a token: 8 MB in and out. 74 us when a CTA held one token, 10 us now (both with the launch, from a cold cache)."""
+    T, D = 131072, 16
+    x = torch.randn(T, D, device="cuda", dtype=torch.bfloat16)
+    cos, sin = F_.rope_tables(8192, D, 1e4, "cuda")
+    us = _median_us(lambda: _lib.call("sx_rope", ptr(x), ptr(cos), ptr(sin), ptr(None), c_ll(T), c_int(8192), c_int(1), c_int(D), c_ll(D), c_int(0),
+                                      c_int(0), stream()))
+    assert us < 10 * _copy_us(2 * x.numel() * 2) + 15, us
