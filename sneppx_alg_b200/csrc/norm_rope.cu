@@ -296,8 +296,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 }
 
 // Rotate-half layout from src to dst (which may be the same): 8 rotation pairs per thread, i.e. two 16-byte loads of x (the halves) and 2 x 32
-// bytes of cos / sin, which the heads of a token share in L1. Heads from `rot` on are copied. Launch shape: token_grid. Bound: memory; rotating into a new buffer replaces a copy followed by a rotation in place
-// ([4096, 48 x 128]: 27 + 23 us before, 27 us).
+// bytes of cos / sin, which the heads of a token share in L1. Heads from `rot` on are copied. Launch shape: token_grid. Bound: memory; rotating
+// into a new buffer replaces a copy followed by a rotation in place ([4096, 48 x 128]: 27 + 23 us before, 27 us).
 __global__ void __launch_bounds__(512) rope_vec8_kernel(const __nv_bfloat16* src, __nv_bfloat16* dst, const float* __restrict__ cos_t,
                                                         const float* __restrict__ sin_t, const int* __restrict__ pos, unsigned tokens,
                                                         int seq, int heads, int rot, int D, long long src_stride, long long dst_stride,

@@ -171,31 +171,32 @@ __global__ void paged_merge_kernel(const float* __restrict__ o_part, const float
   if (d < D) out[(long long)b * out_row_stride + (long long)h * D + d] = __float2bfloat16(l > 0.f ? o / l : 0.f);
 }
 
-// One warp per (token, head). Heads [0, Hq) are queries (rotated in place), [Hq, Hq+Hkv) keys (rotated, written to the
-// cache), [Hq+Hkv, Hq+2Hkv) values (copied to the cache). qkv row = token, row stride in elements.
-// One CTA per token, one thread per 8 + 8 elements of a head (the two halves that rotate into one another), 16-byte loads and stores.
+// Heads [0, Hq) of a qkv row are queries (rotated in place), [Hq, Hq+Hkv) keys (rotated, written to the cache), [Hq+Hkv, Hq+2Hkv) values (copied
+// to the cache). qkv row = token, row stride in elements.
+// One thread per 8 + 8 elements of a head (the two halves that rotate into one another), 16-byte loads and stores, launch shape: token_grid.
 // Bound: memory (rows read once, queries and keys written back, keys and values written to the pool: 25 us at copy bandwidth for 6044
-// tokens of 32 + 2 x 8 heads). 41 us at that size, 92 us when a warp moved a head two bytes a lane.
+// tokens of 32 + 2 x 8 heads). 41 us at that size, 92 us when a warp moved a head two bytes a lane. Few tokens are bound by the
+// chain of position or slot, table and store: 16 tokens of 32 + 2 x 32 heads of 256 4.2 us, 6.2 with one CTA of 512 threads a token.
 __global__ void __launch_bounds__(512) kv_append_vec8_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride,
                                                              const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                                              const int* __restrict__ pos, const int* __restrict__ slot,
-                                                             __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
+                                                             __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int T,
                                                              int Hq, int Hkv, int D, int rotate) {
-  const int t = blockIdx.x, half = D >> 1, per = D >> 4, items = (Hq + 2 * Hkv) * per;
+  const int t = blockIdx.x * blockDim.y + threadIdx.y, half = D >> 1, per = D >> 4, items = (Hq + 2 * Hkv) * per;
+  if (t >= T) return;
   const int p = pos[t], sl = slot[t];
-  for (int i = threadIdx.x; i < items; i += blockDim.x) {
+  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < items; i += gridDim.y * blockDim.x) {
     const int h = i / per, e = (i - h * per) * 8;
+    if (!rotate && h < Hq) continue;
     __nv_bfloat16* row = qkv + (long long)t * row_stride + (long long)h * D + e;
+    bf16x8 pa = ld8(row), pb = ld8(row + half);
     if (h >= Hq + Hkv) {
       if (sl < 0) continue;
       __nv_bfloat16* dst = v_cache + ((long long)sl * Hkv + (h - Hq - Hkv)) * D + e;
-      const bf16x8 a = ld8(row), b = ld8(row + half);
-      st8(dst, a);
-      st8(dst + half, b);
+      st8(dst, pa);
+      st8(dst + half, pb);
       continue;
     }
-    if (!rotate && (h < Hq || sl < 0)) continue;
-    bf16x8 pa = ld8(row), pb = ld8(row + half);
     if (rotate) {
       float a[8], b[8], c[8], s[8];
       const float4* cp = reinterpret_cast<const float4*>(cos_t + (long long)p * half + e);
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(512) kv_append_vec8_kernel(__nv_bfloat16* __re
     }
   }
 }
-// Head sizes that are no multiple of 16 and rows or tables off a 16-byte boundary: a warp per head, one element a lane.
+// Head sizes that are no multiple of 16 and rows or tables off a 16-byte boundary: one warp per (token, head), one element a lane.
 __global__ void kv_append_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride, const float* __restrict__ cos_t,
                                  const float* __restrict__ sin_t, const int* __restrict__ pos,
                                  const int* __restrict__ slot, __nv_bfloat16* __restrict__ k_cache,
@@ -313,9 +314,10 @@ extern "C" int sx_kv_append(void* qkv, long long row_stride, const float* cos_t,
   auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if (D % 16 == 0 && row_stride % 8 == 0 && aligned(qkv) && aligned(k_cache) && aligned(v_cache) &&
       (!rotate || (aligned(cos_t) && aligned(sin_t)))) {
-    const int items = (Hq + 2 * Hkv) * (D / 16);
-    kv_append_vec8_kernel<<<T, items < 512 ? (items + 31) / 32 * 32 : 512, 0, st>>>(
-        (__nv_bfloat16*)qkv, row_stride, cos_t, sin_t, pos, slot, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, Hq, Hkv, D, rotate);
+    dim3 grid, block;
+    token_grid(T, (Hq + 2 * Hkv) * (D / 16), &grid, &block);
+    kv_append_vec8_kernel<<<grid, block, 0, st>>>((__nv_bfloat16*)qkv, row_stride, cos_t, sin_t, pos, slot, (__nv_bfloat16*)k_cache,
+                                                  (__nv_bfloat16*)v_cache, T, Hq, Hkv, D, rotate);
     return cudaGetLastError() == cudaSuccess ? 0 : -11;
   }
   const int blocks = (int)((warps * 32 + 255) / 256);

@@ -223,9 +223,10 @@ def test_mamba2_decode_step(hidden, headdim, state, groups, taps, layers, batch)
 
 
 @pytest.mark.parametrize("T,Hq,Hkv,D,rotate", [(1, 4, 1, 128, True), (37, 28, 4, 128, True), (9, 40, 8, 256, True), (50, 6, 2, 16, True),
-                                               (50, 6, 2, 24, True), (33, 8, 8, 64, False)])
+                                               (50, 6, 2, 24, True), (33, 8, 8, 64, False), (149, 12, 2, 128, True), (131, 1, 1, 16, True),
+                                               (160, 32, 32, 128, True), (9, 40, 8, 256, False)])
 def test_kv_append_sizes(T, Hq, Hkv, D, rotate):
-    """16-byte form (more items than a CTA has threads included) and the form for head sizes that are no multiple of 16; rows without a slot
+    """16-byte form (tokens that share a CTA, one CTA or several a token) and the form for head sizes that are no multiple of 16; rows without a slot
     are rotated and written nowhere. Products and sums are 32-bit: one bf16 rounding, 2^-8; copies are exact."""
     torch.manual_seed(T)
     qkv = torch.randn(T, (Hq + 2 * Hkv) * D, device="cuda", dtype=torch.bfloat16)
