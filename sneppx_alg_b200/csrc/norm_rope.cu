@@ -134,14 +134,16 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_long_kernel(const __nv_bfloat
 
 // dx = rstd * (w*dy) - h * rstd^3 * mean(w*dy*h) (+ dres) ; dw partial sums per CTA.
 // Each CTA walks rows blockIdx.x, blockIdx.x + gridDim.x, ... and keeps its dw partials in registers (thread t owns column vectors
-// t, t + blockDim, ...; at most V of them). Bound: memory; the loads of the next row are issued before the sum of this one, otherwise
+// t, t + blockDim, ...; at most V of them). Bound: memory. With V <= 2 the loads of the next row are issued before the sum of this one, otherwise
 // a CTA has one row in flight and the barrier's latency between rows. [4096, 4096] with dres: 46 us (20 us at copy bandwidth) with the
-// reduction of the partials, 75 us before; [8192, 5120]: 122 and 263 us.
+// reduction of the partials, 75 us before; [8192, 5120]: 122 and 263 us. Four vectors a thread (rows of more than 8192) leave no registers
+// for the next row: with it 264 bytes a thread are spilled. [8192, 12288] 180 us, 550 with the next row, 362 with eight vectors a thread.
 template <int V>
 __global__ void __launch_bounds__(512) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
                                                           const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                                                           const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                                                           float* __restrict__ dw_partial, int T, int d) {
+  constexpr bool AHEAD = V <= 2;
   __shared__ float red[2][32];
   const int nvec = d >> 3, t = threadIdx.x;
   float acc[V][8];
@@ -166,9 +168,10 @@ __global__ void __launch_bounds__(512) rmsnorm_bwd_kernel(const __nv_bfloat16* _
       }
     }
   };
-  if ((int)blockIdx.x < T) fetch(blockIdx.x);
+  if (AHEAD && (int)blockIdx.x < T) fetch(blockIdx.x);
   int buf = 0;
   for (long long row = blockIdx.x; row < T; row += gridDim.x, buf ^= 1) {
+    if (!AHEAD) fetch(row);
     const float r = rn;
 #pragma unroll
     for (int k = 0; k < V; ++k) {
@@ -176,7 +179,7 @@ __global__ void __launch_bounds__(512) rmsnorm_bwd_kernel(const __nv_bfloat16* _
       hv[k] = hn[k];
       ev[k] = en[k];
     }
-    if (row + gridDim.x < T) fetch(row + gridDim.x);
+    if (AHEAD && row + gridDim.x < T) fetch(row + gridDim.x);
     float dot = 0.f;
 #pragma unroll
     for (int k = 0; k < V; ++k) {

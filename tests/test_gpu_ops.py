@@ -233,7 +233,7 @@ def test_rope_to_new_buffer(heads, rot, D, interleaved, strided):
     assert bool(((y[..., :rot * D].float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
 
 
-@pytest.mark.parametrize("T,d", [(1, 8), (3, 1024), (700, 1032), (2, 2048), (300, 2056), (5, 8192), (3, 8200), (2, 16384)])
+@pytest.mark.parametrize("T,d", [(1, 8), (3, 1024), (700, 1032), (2, 2048), (300, 2056), (5, 8192), (3, 8200), (2, 16384), (300, 8200), (700, 16384)])
 @pytest.mark.parametrize("with_res", [False, True])
 def test_rmsnorm_row_sizes(T, d, with_res):
     """Edges of the register forms (one and two vectors a thread, two passes beyond), fewer and more rows than backward CTAs, and weight
@@ -303,3 +303,15 @@ def test_rope_of_small_tokens_keeps_up_with_a_copy():
     us = _median_us(lambda: _lib.call("sx_rope", ptr(x), ptr(cos), ptr(sin), ptr(None), c_ll(T), c_int(8192), c_int(1), c_int(D), c_ll(D), c_int(0),
                                       c_int(0), stream()))
     assert us < 10 * _copy_us(2 * x.numel() * 2) + 15, us
+
+
+@pytest.mark.parametrize("d", [8200, 12288, 16384])
+def test_rmsnorm_backward_of_long_rows_keeps_up_with_a_copy(d):
+    """Rows of more than 8192 read dy and the input and write dx: 2.4 to 2.7 times a copy's time, 5.6 to 6.9 when the kernel spilled registers."""
+    T = 8192
+    dy, x, dx = (torch.randn(T, d, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    w, dw, rstd = torch.randn(d, device="cuda").bfloat16(), torch.empty(d, device="cuda", dtype=torch.bfloat16), torch.ones(T, device="cuda")
+    part = torch.empty(_lib.lib().sx_rmsnorm_bwd_parts() * d, device="cuda")
+    us = _median_us(lambda: _lib.call("sx_rmsnorm_bwd", ptr(dy), ptr(x), ptr(w), ptr(rstd), ptr(None), ptr(dx), ptr(part), ptr(dw), ptr(None), c_int(0),
+                                      c_ll(T), c_int(d), stream()))
+    assert us < 4 * _copy_us(3 * T * d * 2), us
