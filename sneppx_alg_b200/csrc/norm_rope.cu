@@ -24,9 +24,9 @@ __device__ __forceinline__ float row_sum(float v, float* red) {
 // Bound: memory. A row stays in the registers of one CTA between the sum and the output (V vectors of 8 a thread), so it is read once and
 // all of its loads are in flight together; rows are spread over CTAs and overlap. Two vectors a thread keep CTAs small enough that
 // several share an SM. [4096, 4096] with residual: 31 us with a cold L2 full of dirty lines (read + write once: 20 us at copy
-// bandwidth), 37 us when a second pass
-// read the row again.
-template <int V>
+// bandwidth), 37 us when a second pass read the row again. RES: with a residual; without one the registers for it cost CTAs an SM
+// (60 and 40 a thread with V = 2; [8192, 6144] without residual 68 us with them, 64 with a second pass, 53 so).
+template <int V, bool RES>
 __global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in,
                                                            const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                                            __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd, int d, float eps) {
@@ -34,13 +34,13 @@ __global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* _
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const int nvec = d >> 3, t = threadIdx.x;
-  bf16x8 a[V], b[V], wv[V];
+  bf16x8 a[V], b[RES ? V : 1], wv[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) {
     const int i = t + k * blockDim.x;
     if (i < nvec) {
       a[k] = ld8(x + row * d + i * 8);
-      if (res_in) b[k] = ld8(res_in + row * d + i * 8);
+      if (RES) b[k] = ld8(res_in + row * d + i * 8);
     }
   }
 #pragma unroll
@@ -55,8 +55,8 @@ __global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* _
     if (i >= nvec) continue;
     unpack8(a[k], f[k]);
     float h[8];
-    if (res_in) {
-      unpack8(b[k], h);
+    if (RES) {
+      unpack8(b[RES ? k : 0], h);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[k][j] += h[j];
       // round through bf16 so that the statistics match what backward will re-read
@@ -431,11 +431,13 @@ extern "C" int sx_rmsnorm_fwd(const void* x, const void* res_in, const void* w, 
   };
   auto per = [&](int v) { return ((nvec + v - 1) / v + 31) / 32 * 32; };
   // 256 threads up to 4096 as long as they have a vector each (a thread's share then does not depend on how the row divides), more threads
-  // with two vectors up to 8192; a CTA of 1024 threads has an SM to itself, and two passes over L2 are
-  // faster then ([1000, 16384]: 37 against 43 us)
-  if (nvec <= 256) run(rmsnorm_fwd_kernel<1>, per(1));
-  else if (nvec <= 1024) run(rmsnorm_fwd_kernel<2>, nvec <= 512 ? 256 : per(2));
-  else run(rmsnorm_fwd_long_kernel, 256);
+  // with two vectors up to 8192; a CTA of 1024 threads has an SM to itself, and two passes over L2 are faster then ([1000, 16384]: 37
+  // against 43 us)
+  if (nvec <= 256) res_in ? run(rmsnorm_fwd_kernel<1, true>, per(1)) : run(rmsnorm_fwd_kernel<1, false>, per(1));
+  else if (nvec <= 1024) {
+    const int threads = nvec <= 512 ? 256 : per(2);
+    res_in ? run(rmsnorm_fwd_kernel<2, true>, threads) : run(rmsnorm_fwd_kernel<2, false>, threads);
+  } else run(rmsnorm_fwd_long_kernel, 256);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
