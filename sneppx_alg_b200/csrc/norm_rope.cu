@@ -441,16 +441,18 @@ extern "C" int sx_rmsnorm_fwd(const void* x, const void* res_in, const void* w, 
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
-// dw_partial: scratch of nparts*d floats (nparts = value returned by sx_rmsnorm_bwd_parts()).
-extern "C" int sx_rmsnorm_bwd_parts() { return 592; }
+// CTAs, and rows of partial weight gradients, of the backward pass: short rows keep as much in flight with four small CTAs an SM as longer ones
+// with two large.
+extern "C" int sx_rmsnorm_bwd_parts(int d) { return d <= 2048 ? 592 : 296; }
 
+// dw_partial: scratch of sx_rmsnorm_bwd_parts(d) * d floats.
 extern "C" int sx_rmsnorm_bwd(const void* dy, const void* h, const void* w, const float* rstd, const void* dres,
                               void* dx, float* dw_partial, void* dw_bf16, float* dw_f32, int accumulate, long long T,
                               int d, cudaStream_t st) {
   if (d % 8) return -1;
   if (T == 0) return 0;
   const int nvec = d / 8;
-  const int most = nvec <= 256 ? 592 : 296;      // short rows: four small CTAs an SM keep as much in flight as two large ones
+  const int most = sx_rmsnorm_bwd_parts(d);
   const int parts = T < most ? (int)T : most;
   auto run = [&](auto kern, int v) {
     kern<<<parts, nvec > 256 && nvec <= 512 ? 256 : ((nvec + v - 1) / v + 31) / 32 * 32, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w,

@@ -60,7 +60,7 @@ class _RMSNormFn(torch.autograd.Function):
         dy2 = dy.reshape(-1, d).contiguous()
         dres = dh.reshape(-1, d).contiguous() if dh is not None else None
         dx = torch.empty_like(h)
-        parts = _lib.lib().sx_rmsnorm_bwd_parts()
+        parts = _lib.lib().sx_rmsnorm_bwd_parts(c_int(d))
         scratch = torch.empty(parts * d, dtype=torch.float32, device=h.device)
         mg = getattr(w, "main_grad", None)
         if mg is not None:

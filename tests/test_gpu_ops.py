@@ -311,7 +311,19 @@ def test_rmsnorm_backward_of_long_rows_keeps_up_with_a_copy(d):
     T = 8192
     dy, x, dx = (torch.randn(T, d, device="cuda", dtype=torch.bfloat16) for _ in range(3))
     w, dw, rstd = torch.randn(d, device="cuda").bfloat16(), torch.empty(d, device="cuda", dtype=torch.bfloat16), torch.ones(T, device="cuda")
-    part = torch.empty(_lib.lib().sx_rmsnorm_bwd_parts() * d, device="cuda")
+    part = torch.empty(_lib.lib().sx_rmsnorm_bwd_parts(c_int(d)) * d, device="cuda")
     us = _median_us(lambda: _lib.call("sx_rmsnorm_bwd", ptr(dy), ptr(x), ptr(w), ptr(rstd), ptr(None), ptr(dx), ptr(part), ptr(dw), ptr(None), c_int(0),
                                       c_ll(T), c_int(d), stream()))
     assert us < 4 * _copy_us(3 * T * d * 2), us
+
+
+@pytest.mark.parametrize("d,rows", [(8, 592), (2048, 592), (2056, 296), (16384, 296)])
+def test_rmsnorm_backward_scratch(d, rows):
+    """The scratch is what the widths use: with it, rows behind the scratch stay as they are."""
+    assert _lib.lib().sx_rmsnorm_bwd_parts(c_int(d)) == rows
+    T = 1000
+    dy, x, dx = (torch.randn(T, d, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    w, dw, rstd = torch.randn(d, device="cuda").bfloat16(), torch.empty(d, device="cuda", dtype=torch.bfloat16), torch.ones(T, device="cuda")
+    part = torch.full((rows + 8, d), 7.0, device="cuda")
+    _lib.call("sx_rmsnorm_bwd", ptr(dy), ptr(x), ptr(w), ptr(rstd), ptr(None), ptr(dx), ptr(part), ptr(dw), ptr(None), c_int(0), c_ll(T), c_int(d), stream())
+    assert bool((part[rows:] == 7.0).all()) and not bool((part[:rows] == 7.0).all(1).any())
