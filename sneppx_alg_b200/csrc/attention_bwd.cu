@@ -464,7 +464,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
 }
 
 // delta[b,h,s] = sum_d dO * O, and dq_accum zeroed. Bound: memory (dO and O read, dq_accum written once). 16 lanes a (token, head) row with a
-// 16-byte load each, four rows of a lane in flight: [1, 4096, 32, 128] 21 us, 45 us as a memset and a kernel with four bytes a lane.
+// 16-byte load each, four rows of a lane in flight: [1, 4096, 32, 128] 21 us, 45 us as a memset and a kernel with four bytes a lane. dq_accum holds
+// whole tiles of 64 queries, so few queries leave more to zero than their rows have CTAs for: CTAs behind the last row only zero
+// ([1, 1, 32, 128], whole backward: 20 us, 36 with one CTA that zeroed 1 MB).
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
                                                          float* __restrict__ delta, float4* __restrict__ acc, long long acc4, unsigned rows,
                                                          unsigned S, unsigned H, long long do_row_stride, long long o_row_stride) {
@@ -559,9 +561,11 @@ extern "C" int sx_attn_bwd(const SxAttnArgs* a, cudaStream_t st) {
   const long long acc_floats = (long long)a->B * a->Hq * n_qt * BWD_Q * BWD_D;
   const long long rows = tokens * a->Hq;
   if (rows <= 0 || rows > 0x7fffffffll || (a->o_row_stride % 8) || (reinterpret_cast<uintptr_t>(a->O) & 15)) return -5;
-  attn_delta_kernel<<<(unsigned)((rows + 63) / 64), 256, 0, st>>>((const __nv_bfloat16*)a->dO, (const __nv_bfloat16*)a->O, a->delta,
-                                                                  (float4*)a->dq_accum, acc_floats / 4, (unsigned)rows, (unsigned)a->Sq,
-                                                                  (unsigned)a->Hq, a->do_row_stride, a->o_row_stride);
+  // CTAs for the rows, and for zeroing enough that a thread has at most 8 pieces, up to four an SM
+  const long long acc4 = acc_floats / 4, by_rows = (rows + 63) / 64, by_acc = (acc4 + 2047) / 2048 < 592 ? (acc4 + 2047) / 2048 : 592;
+  attn_delta_kernel<<<(unsigned)(by_rows > by_acc ? by_rows : by_acc), 256, 0, st>>>(
+      (const __nv_bfloat16*)a->dO, (const __nv_bfloat16*)a->O, a->delta, (float4*)a->dq_accum, acc4, (unsigned)rows, (unsigned)a->Sq,
+      (unsigned)a->Hq, a->do_row_stride, a->o_row_stride);
   p.lse = a->lse; p.delta = a->delta; p.dq_accum = a->dq_accum;
   p.dK = (__nv_bfloat16*)a->dK; p.dV = (__nv_bfloat16*)a->dV;
   p.dk_row_stride = a->dk_row_stride; p.dv_row_stride = a->dv_row_stride;

@@ -1,4 +1,5 @@
 """Bandwidth-bound kernels and attention against fp32 PyTorch references of the same ops."""
+import ctypes as C
 import math
 
 import pytest
@@ -327,3 +328,44 @@ def test_rmsnorm_backward_scratch(d, rows):
     part = torch.full((rows + 8, d), 7.0, device="cuda")
     _lib.call("sx_rmsnorm_bwd", ptr(dy), ptr(x), ptr(w), ptr(rstd), ptr(None), ptr(dx), ptr(part), ptr(dw), ptr(None), c_int(0), c_ll(T), c_int(d), stream())
     assert bool((part[rows:] == 7.0).all()) and not bool((part[:rows] == 7.0).all(1).any())
+
+
+def _attn_bwd_args(B, S, H, Hk, o=None):
+    """Arguments of a causal sx_attn_bwd call, with everything that it fills poisoned; and the tensors that they point to."""
+    D, bf = 128, torch.bfloat16
+    q, do = (torch.randn(B, S, H, D, device="cuda").to(bf) for _ in range(2))
+    k, v = (torch.randn(B, S, Hk, D, device="cuda").to(bf) for _ in range(2))
+    o_fwd, lse = F_.attention_with_lse(q, k, v, causal=True)
+    if o is not None:
+        o.copy_(o_fwd)
+    t = dict(q=q, k=k, v=v, do=do, o=o_fwd if o is None else o, lse=lse, acc=torch.full((B, H, (S + 63) // 64 * 64, D), float("nan"), device="cuda"),
+             delta=torch.full((B, H, S), float("nan"), device="cuda"), dq=torch.empty_like(q), dk=torch.empty_like(k), dv=torch.empty_like(v))
+    a = F_._attn_args(q, k, v, t["o"], lse, True, 0, D ** -0.5, 1)
+    a.dO, a.dQ, a.dK, a.dV = (t[n].data_ptr() for n in ("do", "dq", "dk", "dv"))
+    a.dq_accum, a.delta = t["acc"].data_ptr(), t["delta"].data_ptr()
+    a.do_row_stride = H * D
+    a.dq_row_stride, a.dk_row_stride, a.dv_row_stride = H * D, Hk * D, Hk * D
+    a.dq_batch_stride, a.dk_batch_stride, a.dv_batch_stride = S * H * D, S * Hk * D, S * Hk * D
+    return a, t
+
+
+@pytest.mark.parametrize("B,S,H,Hk", [(1, 1, 4, 1), (1, 1, 32, 32), (3, 2, 8, 8), (1, 63, 8, 2), (2, 65, 4, 4), (1, 300, 7, 1)])
+def test_attention_backward_prologue(B, S, H, Hk):
+    """The accumulator of dQ is zeroed, whole tiles also where they hold few queries, and delta is the sum of dO O. delta: 128 products in
+    32 bits, 2^-17 of the sum of magnitudes."""
+    a, t = _attn_bwd_args(B, S, H, Hk)
+    _lib.call("sx_attn_bwd", C.byref(a), stream())
+    ops.check_status()
+    prod = (t["do"].double() * t["o"].double()).permute(0, 2, 1, 3)
+    assert bool(((t["delta"].double() - prod.sum(-1)).abs() <= prod.abs().sum(-1) * 2.0 ** -17).all())
+    assert bool(t["acc"].isfinite().all()) and bool(t["dq"].isfinite().all())
+
+
+def test_attention_backward_of_one_query_zeroes_with_many_ctas():
+    """Sixteen times the heads of one query take little longer than one head: 64 heads hold 2 MB of accumulator tiles, 24 us more than one head when
+    one CTA zeroed them, 4 us now."""
+    us = []
+    for H in (4, 64):
+        a, t = _attn_bwd_args(1, 1, H, H)
+        us.append(_median_us(lambda: _lib.call("sx_attn_bwd", C.byref(a), stream())))
+    assert us[1] < us[0] + 14, us
