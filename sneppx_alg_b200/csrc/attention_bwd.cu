@@ -467,6 +467,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
 // 16-byte load each, four rows of a lane in flight: [1, 4096, 32, 128] 21 us, 45 us as a memset and a kernel with four bytes a lane. dq_accum holds
 // whole tiles of 64 queries, so few queries leave more to zero than their rows have CTAs for: CTAs behind the last row only zero
 // ([1, 1, 32, 128], whole backward: 20 us, 36 with one CTA that zeroed 1 MB).
+// WIDE: rows of O on 16 bytes; on 4 otherwise, which is all that a caller of sx_attn_bwd has to keep for O.
+template <bool WIDE>
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
                                                          float* __restrict__ delta, float4* __restrict__ acc, long long acc4, unsigned rows,
                                                          unsigned S, unsigned H, long long do_row_stride, long long o_row_stride) {
@@ -478,7 +480,12 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   for (int k = 0; k < R; ++k) {
     const unsigned r = min(r0 + k, rows - 1), h = r % H, tok = r / H;
     a[k] = ld8(dO + tok * do_row_stride + h * BWD_D + part * 8);
-    c[k] = ld8(O + tok * o_row_stride + h * BWD_D + part * 8);
+    const __nv_bfloat16* o = O + tok * o_row_stride + h * BWD_D + part * 8;
+    if constexpr (WIDE) c[k] = ld8(o);
+    else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) reinterpret_cast<uint32_t*>(&c[k])[j] = reinterpret_cast<const uint32_t*>(o)[j];
+    }
   }
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < acc4; i += threads) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -560,12 +567,16 @@ extern "C" int sx_attn_bwd(const SxAttnArgs* a, cudaStream_t st) {
   // dq_accum holds whole 64-row query tiles: B * Hq * n_qt * 64 * 128 floats
   const long long acc_floats = (long long)a->B * a->Hq * n_qt * BWD_Q * BWD_D;
   const long long rows = tokens * a->Hq;
-  if (rows <= 0 || rows > 0x7fffffffll || (a->o_row_stride % 8) || (reinterpret_cast<uintptr_t>(a->O) & 15)) return -5;
+  if (rows <= 0 || rows > 0x7fffffffll || (a->o_row_stride % 2) || (reinterpret_cast<uintptr_t>(a->O) & 3)) return -5;
   // CTAs for the rows, and for zeroing enough that a thread has at most 8 pieces, up to four an SM
   const long long acc4 = acc_floats / 4, by_rows = (rows + 63) / 64, by_acc = (acc4 + 2047) / 2048 < 592 ? (acc4 + 2047) / 2048 : 592;
-  attn_delta_kernel<<<(unsigned)(by_rows > by_acc ? by_rows : by_acc), 256, 0, st>>>(
-      (const __nv_bfloat16*)a->dO, (const __nv_bfloat16*)a->O, a->delta, (float4*)a->dq_accum, acc4, (unsigned)rows, (unsigned)a->Sq,
-      (unsigned)a->Hq, a->do_row_stride, a->o_row_stride);
+  const bool wide = a->o_row_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(a->O) & 15) == 0;
+  auto delta = [&](auto kern) {
+    kern<<<(unsigned)(by_rows > by_acc ? by_rows : by_acc), 256, 0, st>>>((const __nv_bfloat16*)a->dO, (const __nv_bfloat16*)a->O, a->delta,
+                                                                         (float4*)a->dq_accum, acc4, (unsigned)rows, (unsigned)a->Sq,
+                                                                         (unsigned)a->Hq, a->do_row_stride, a->o_row_stride);
+  };
+  wide ? delta(attn_delta_kernel<true>) : delta(attn_delta_kernel<false>);
   p.lse = a->lse; p.delta = a->delta; p.dq_accum = a->dq_accum;
   p.dK = (__nv_bfloat16*)a->dK; p.dV = (__nv_bfloat16*)a->dV;
   p.dk_row_stride = a->dk_row_stride; p.dv_row_stride = a->dv_row_stride;

@@ -361,6 +361,20 @@ def test_attention_backward_prologue(B, S, H, Hk):
     assert bool(t["acc"].isfinite().all()) and bool(t["dq"].isfinite().all())
 
 
+@pytest.mark.parametrize("shift,pad", [(2, 0), (0, 2), (6, 10), (8, 4)])
+def test_attention_backward_takes_an_output_on_four_bytes(shift, pad):
+    """Rows of O that start on 4 but not on 16 bytes give what aligned ones give, bit for bit (one key tile: no order of additions)."""
+    B, S, H, D = 2, 100, 4, 128
+    torch.manual_seed(shift + pad)
+    flat = torch.randn(B * S * (H * D + pad) + 64, device="cuda").bfloat16()
+    a, t = _attn_bwd_args(B, S, H, 2, flat[shift:].as_strided((B, S, H, D), (S * (H * D + pad), H * D + pad, D, 1)))
+    assert a.o_row_stride == H * D + pad
+    _lib.call("sx_attn_bwd", C.byref(a), stream())
+    want = F_.attention_backward(t["q"], t["k"], t["v"], t["o"].contiguous(), t["lse"], t["do"])
+    ops.check_status()
+    assert all(torch.equal(t[n], w) for n, w in zip(("dq", "dk", "dv"), want))
+
+
 def test_attention_backward_of_one_query_zeroes_with_many_ctas():
     """Sixteen times the heads of one query take little longer than one head: 64 heads hold 2 MB of accumulator tiles, 24 us more than one head when
     one CTA zeroed them, 4 us now."""
