@@ -169,7 +169,8 @@ def _block_of(entry, L, H, P, N, taps, chan, dev):
 def decode_step(model, states, seq_ids, last_tokens):
     """Logits [B, vocab] of one token for every sequence, its states advanced; None when model, batch or states are not ones that the
     step kernels take (another device or type, replaced or hooked modules, a sequence twice in the batch, more than 128 rows), in which
-    case nothing has changed. Everything is allocated before the first state is written."""
+    case nothing has changed. Everything is allocated before the first state is written, and a sequence moves on when every kernel has been
+    launched; where a launch fails, sequences whose states a kernel may have written are dropped and the others stay as they were."""
     B = len(seq_ids)
     if not (isinstance(states, SequenceStates) and isinstance(model, torch.nn.Module) and 0 < B <= MAX_ROWS and len(last_tokens) == B and len(set(seq_ids)) == B):
         return None
@@ -206,23 +207,31 @@ def decode_step(model, states, seq_ids, last_tokens):
     a.B, a.d, a.H, a.P, a.N, a.G, a.taps = B, d, H, P, N, G, taps
     a.table, a.status = table.data_ptr() + 8 * B, _lib.status_word(dev).data_ptr()
     half, stream = B * d * 2, _lib.stream()
+    try:
+        for i, layer in enumerate(model.layers):
+            m, own = layer.mixer, layer.mixer._parameters
+            # the residual of layer 0 is the embedding, then the two halves of `res` in turn; kernels write only the second of each pair
+            a.x = x.data_ptr() if i == 0 else out.data_ptr()
+            a.res_in = None if i == 0 else x.data_ptr() if i == 1 else res.data_ptr() + (i & 1) * half
+            a.res_out = None if i == 0 else res.data_ptr() + (1 - (i & 1)) * half
+            a.layer, a.eps, a.gate_eps = i, layer.norm.eps, m.norm.eps
+            a.norm_w, a.gate_norm_w = layer.norm.weight.data_ptr(), m.norm.weight.data_ptr()
+            a.in_w, a.out_w = m.in_proj.weight.data_ptr(), m.out_proj.weight.data_ptr()
+            a.conv_w, a.conv_b = own["conv_weight"].data_ptr(), own["conv_bias"].data_ptr()
+            a.dt_bias, a.a_log, a.D = own["dt_bias"].data_ptr(), own["A_log"].data_ptr(), own["D"].data_ptr()
+            _lib.call("sx_mamba2_step", C.byref(a), stream)
+        _lib.launch_count += 4 * L      # five kernels a call
+        last = x if L == 1 else res[1 - ((L - 1) & 1)]
+        _lib.call("sx_rmsnorm_fwd", _lib.ptr(out), _lib.ptr(last), _lib.ptr(model.norm.weight), _lib.ptr(hn), _lib.ptr(None), _lib.ptr(None),
+                  _lib.c_ll(B), _lib.c_int(d), _lib.c_float(model.norm.eps), stream)
+        gemm(hn, model.head_weight()[:model.config.vocab_size], out=logits)
+    except BaseException:
+        # kernels may have stepped states where they lie: those sequences are gone rather than half advanced. Lists are never written.
+        for sid, b in zip(seq_ids, blocks):
+            if dict.get(states, sid) is b:
+                dict.pop(states, sid)
+        raise
     for sid, b in zip(seq_ids, blocks):
         dict.__setitem__(states, sid, b)
         b.cur = 1 - b.cur
-    for i, layer in enumerate(model.layers):
-        m, own = layer.mixer, layer.mixer._parameters
-        # the residual of layer 0 is the embedding, then the two halves of `res` in turn; kernels write only the second of each pair
-        a.x = x.data_ptr() if i == 0 else out.data_ptr()
-        a.res_in = None if i == 0 else x.data_ptr() if i == 1 else res.data_ptr() + (i & 1) * half
-        a.res_out = None if i == 0 else res.data_ptr() + (1 - (i & 1)) * half
-        a.layer, a.eps, a.gate_eps = i, layer.norm.eps, m.norm.eps
-        a.norm_w, a.gate_norm_w = layer.norm.weight.data_ptr(), m.norm.weight.data_ptr()
-        a.in_w, a.out_w = m.in_proj.weight.data_ptr(), m.out_proj.weight.data_ptr()
-        a.conv_w, a.conv_b = own["conv_weight"].data_ptr(), own["conv_bias"].data_ptr()
-        a.dt_bias, a.a_log, a.D = own["dt_bias"].data_ptr(), own["A_log"].data_ptr(), own["D"].data_ptr()
-        _lib.call("sx_mamba2_step", C.byref(a), stream)
-    _lib.launch_count += 4 * L      # five kernels a call
-    last = x if L == 1 else res[1 - ((L - 1) & 1)]
-    _lib.call("sx_rmsnorm_fwd", _lib.ptr(out), _lib.ptr(last), _lib.ptr(model.norm.weight), _lib.ptr(hn), _lib.ptr(None), _lib.ptr(None),
-              _lib.c_ll(B), _lib.c_int(d), _lib.c_float(model.norm.eps), stream)
-    return gemm(hn, model.head_weight()[:model.config.vocab_size], out=logits)
+    return logits

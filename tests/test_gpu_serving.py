@@ -242,3 +242,38 @@ def test_kv_append_sizes(T, Hq, Hkv, D, rotate):
     for got, ref in zip((qkv, kc, vc), want):
         assert bool(((got.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
     assert torch.equal(vc.double(), want[2])
+
+
+def test_mamba2_decode_step_that_fails(monkeypatch):
+    """A launch that fails in the second layer: a sequence whose states were stepped where they lie is dropped, so that a retry fails instead of
+    going on from half-advanced states; one whose states came as lists keeps them and steps as if nothing had happened."""
+    from sneppx_alg_b200.models import ModelConfig, build_model
+    from sneppx_alg_b200.ops import _lib
+    from sneppx_alg_b200.serving.llm_engine import StatefulRunner
+    torch.manual_seed(0)
+    cfg = ModelConfig(architecture="mamba2", hidden_size=256, num_hidden_layers=3, vocab_size=500, ssm_state_size=128, ssm_expand=2, ssm_head_dim=64,
+                      ssm_ngroups=1, ssm_conv_kernel=4, rms_norm_eps=1e-5, tie_word_embeddings=True)
+    model = build_model(cfg, dtype=torch.bfloat16, device="cuda").eval()
+    run, other = StatefulRunner(model), StatefulRunner(model)
+    for r in (run, other):
+        for sid in (0, 1, 2):
+            r.prefill(sid, [3 + sid, 5, 7], 0)
+        r.decode([0, 2], [9, 9])
+    real, calls = _lib.call, []
+
+    def failing(name, *args):
+        calls.append(name)
+        if calls.count("sx_mamba2_step") == 2:
+            raise RuntimeError("no launch")
+        real(name, *args)
+
+    monkeypatch.setattr(_lib, "call", failing)
+    with pytest.raises(RuntimeError, match="no launch"):
+        run.decode([0, 1], [11, 12])
+    monkeypatch.setattr(_lib, "call", real)
+    with pytest.raises(KeyError):
+        run.decode([0, 1], [11, 12])
+    assert sorted(run.states.keys()) == [1, 2]
+    assert torch.equal(run.decode([1, 2], [12, 13]), other.decode([1, 2], [12, 13]))
+    assert torch.equal(run.decode([1, 2], [14, 15]), other.decode([1, 2], [14, 15]))
+    ops.check_status()
