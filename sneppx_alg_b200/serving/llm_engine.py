@@ -58,13 +58,18 @@ class Request:
 
 
 def _upload(values, dtype, device):
-    """A list of integers as a tensor on the device. The copy starts from pinned memory, so it queues behind what the stream holds: from
-    ordinary memory the host waits for the stream first, and the gap before the next launch is added to every call."""
-    try:
-        t = torch.frombuffer(array("q" if dtype is torch.long else "i", list(values)), dtype=dtype)   # a quarter of torch.tensor's time
-    except (TypeError, ValueError, OverflowError):                                                   # not integers, none at all, too large
+    """Integers as a tensor on the device: a list, or whatever else torch.tensor takes. The copy starts from pinned memory, so it queues behind
+    what the stream holds: from ordinary memory the host waits for the stream first, and the gap before the next launch is added to every
+    call."""
+    t = None
+    if type(values) is list:
+        try:
+            t = torch.frombuffer(array("q" if dtype is torch.long else "i", values), dtype=dtype)   # a quarter of torch.tensor's time
+        except (TypeError, ValueError, OverflowError):                                              # not integers, none at all, too large
+            pass
+    if t is None:       # arrays and tensors at once, not one value after another
         t = torch.tensor(values, dtype=dtype)
-    return t.pin_memory().to(device, non_blocking=True) if device.type == "cuda" else t.to(device)
+    return t.pin_memory().to(device, non_blocking=True) if device.type == "cuda" and not t.is_cuda else t.to(device)
 
 
 class LlamaPagedRunner:
@@ -126,7 +131,7 @@ class LlamaPagedRunner:
         dev = m.embedding.weight.device
         n, T = len(prompts), len(prompts[0])
         assert all(len(p) == T for p in prompts)
-        ids = _upload([t for p in prompts for t in p], torch.long, dev).view(n, T)
+        ids = _upload([t for p in prompts for t in p] if all(type(p) is list for p in prompts) else prompts, torch.long, dev).view(n, T)
         slots = _upload([s for sid in seq_ids for s in self.cache.reserve(sid, T)], torch.int32, dev)
         pos = torch.arange(T, dtype=torch.int32, device=dev).repeat(n)
         cos, sin = m.rope(dev, T)

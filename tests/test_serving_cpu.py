@@ -204,3 +204,37 @@ def test_paged_decode_deals_its_items_evenly():
         for i in range(B * Hkv * ns):
             best[i % n_cta] += longest[i // (B * Hkv)]
         assert max(load) == max(best) or B * Hkv * ns > 12 * n_cta, (B, Hkv, n, max(load), max(best))
+
+
+def test_prompts_are_uploaded_as_torch_tensor_takes_them():
+    """Lists of integers take a shorter way; everything else is what torch.tensor makes of it, refusals included, and arrays and tensors are
+    converted at once."""
+    import numpy as np
+    import pytest
+    from sneppx_alg_b200.serving.llm_engine import LlamaPagedRunner, _upload
+    dev = torch.device("cpu")
+    for values in ([], [3, 1, 2], [True, False], [1.0, 2.0], (4, 5), np.arange(6), np.arange(6, dtype=np.uint8), torch.arange(4), [np.int64(3), 4],
+                   [torch.tensor(7), 8], [[1, 2], [3, 4]], np.ones((2, 3), dtype=np.int32)):
+        for dtype in (torch.long, torch.int32):
+            want, got = torch.tensor(values, dtype=dtype), _upload(values, dtype, dev)
+            assert got.dtype == dtype and torch.equal(got, want), values
+    for values in ([2 ** 70], [None], ["a"], [torch.arange(3), torch.arange(3)]):
+        with pytest.raises(Exception) as ours:
+            _upload(values, torch.long, dev)
+        with pytest.raises(type(ours.value)):
+            torch.tensor(values, dtype=torch.long)
+
+    class Counted(np.ndarray):
+        def __iter__(self):
+            raise AssertionError("walked one value after another")
+
+    assert _upload(np.arange(5).view(Counted), torch.long, dev).tolist() == [0, 1, 2, 3, 4]
+    model, prompts = _model(), [[5, 6, 7, 8, 9], [10, 11, 12, 13, 14]]
+    outs = []
+    for form in (prompts, np.array(prompts), torch.tensor(prompts), [tuple(p) for p in prompts]):
+        cache = PagedKVCache(2, 16, 4, 2, 16, dtype=torch.float32, device="cpu")
+        runner = LlamaPagedRunner(model, cache)
+        for sid in (0, 1, 2):
+            cache.add_sequence(sid)
+        outs.append(torch.cat([runner.prefill_batch([0, 1], form), runner.prefill(2, form[0], 0)]))
+    assert all(torch.equal(o, outs[0]) for o in outs)
