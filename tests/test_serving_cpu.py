@@ -238,3 +238,82 @@ def test_prompts_are_uploaded_as_torch_tensor_takes_them():
             cache.add_sequence(sid)
         outs.append(torch.cat([runner.prefill_batch([0, 1], form), runner.prefill(2, form[0], 0)]))
     assert all(torch.equal(o, outs[0]) for o in outs)
+
+
+def test_slots_by_block_and_tables_shared_whole():
+    """Slots reserved by block against one token at a time, over full, partly filled and shared blocks and an exhausted pool; tables shared and
+    released whole against block by block."""
+    import random
+    import pytest
+
+    class Plain(PagedKVCache):
+        def reserve(self, seq_id, n_new):
+            table, slots = self.tables[seq_id], []
+            for i in range(self.lens[seq_id], self.lens[seq_id] + n_new):
+                at, off = divmod(i, self.block_size)
+                if at == len(table):
+                    table.append(self.pool.allocate())
+                elif self.pool.ref[table[at]] > 1:
+                    new = self.pool.allocate()
+                    self.k[0][new], self.v[0][new] = self.k[0][table[at]].clone(), self.v[0][table[at]].clone()
+                    self.pool.release(table[at])
+                    table[at] = new
+                slots.append(table[at] * self.block_size + off)
+            self.lens[seq_id] += n_new
+            return slots
+
+        def fork(self, src, dst):
+            self.tables[dst] = [self.pool.share(b) for b in self.tables[src]]
+            self.lens[dst] = self.lens[src]
+
+        def free_sequence(self, seq_id, tokens=None):
+            for b in self.tables.pop(seq_id, []):
+                self.pool.release(b)
+            self.lens.pop(seq_id, 0)
+
+    rng = random.Random(5)
+    for trial in range(20):
+        pair = [cls(1, 24, 4, 1, 8, dtype=torch.float32, device="cpu", enable_prefix_cache=False) for cls in (PagedKVCache, Plain)]
+        live, nxt = [], 0
+        for _ in range(40):
+            act = rng.random()
+            if act < 0.3 or not live:
+                for c in pair:
+                    c.add_sequence(nxt)
+                live.append(nxt)
+                nxt += 1
+            elif act < 0.7:
+                sid, n = rng.choice(live), rng.choice([0, 1, 3, 4, 5, 9])
+                got = []
+                for c in pair:
+                    try:
+                        got.append(c.reserve(sid, n))
+                    except MemoryError:
+                        got.append("exhausted")
+                assert got[0] == got[1]
+                if got[0] == "exhausted":
+                    break
+                for layer, value in (("k", 1.0 + nxt), ("v", 2.0 + nxt)):
+                    for c in pair:
+                        getattr(c, layer)[0].view(24 * 4, -1)[got[0]] = value
+            elif act < 0.85:
+                src = rng.choice(live)
+                for c in pair:
+                    c.fork(src, nxt)
+                live.append(nxt)
+                nxt += 1
+            else:
+                sid = live.pop(rng.randrange(len(live)))
+                for c in pair:
+                    c.free_sequence(sid)
+            a, b = pair
+            assert a.tables == b.tables and a.lens == b.lens and a.pool.free == b.pool.free and a.pool.ref == b.pool.ref
+            assert torch.equal(a.k[0], b.k[0]) and torch.equal(a.v[0], b.v[0])
+    pool = KVBlockPool(3)
+    blocks = [pool.allocate(), pool.allocate()]
+    pool.release_all(pool.share_all(blocks))
+    assert pool.num_free == 1
+    pool.release_all(blocks)
+    assert pool.num_free == 3 and pool.free[-2:] == blocks
+    with pytest.raises(RuntimeError, match="double free"):
+        pool.release_all(blocks)
