@@ -312,3 +312,28 @@ def test_mamba2_mixer(B, L, H, P, G, N, K, monkeypatch):
             assert got.shape == t.shape and got.dtype == t.dtype and err(got, exp) < (0.014 if name == "zx" else 0.028), (name, err(got, exp))
         for lo, hi, name in ((0, di, "z"), (di, di + di, "x"), (2 * di, 2 * di + 2 * G * N, "B, C"), (di + C, di + C + H, "dt")):
             assert err(grads[0][..., lo:hi], wgrad[0][..., lo:hi]) < 0.028, (name, err(grads[0][..., lo:hi], wgrad[0][..., lo:hi]))
+
+
+@pytest.mark.parametrize("C,L,Lp,wide", [(64, 1, 1, False), (1536, 1, 1, True), (320, 7, 7, True), (320, 7, 8, True), (64, 33, 64, False)])
+def test_gate_mul_padded_rows(C, L, Lp, wide):
+    """Dense and wider gradients of z, y with rows behind each sequence that are neither read nor written. 32-bit arithmetic and one bf16 rounding;
+    the sigmoid is within 2^-20, which the factor sig (1 + z (1 - sig)) of dz takes up to 1 + 2 |z| < 10 times, against |g y|."""
+    from sneppx_alg_b200.ops import _lib
+    from sneppx_alg_b200.ops._lib import c_int, c_ll, ptr, stream
+    torch.manual_seed(C + L)
+    n, bf = 3, torch.bfloat16
+    y = torch.full((n, Lp, C), float("nan"), device="cuda", dtype=bf)
+    y[:, :L] = torch.randn(n, L, C, device="cuda").to(bf)
+    z, g = torch.randn(n, L, C + 64, device="cuda").to(bf), torch.randn(n, L, C, device="cuda").to(bf)
+    out, dy = torch.empty(n, L, C, device="cuda", dtype=bf), torch.full_like(y, 3.0)
+    dz = torch.full((n, L, C + 64 if wide else C), 3.0, device="cuda", dtype=bf)
+    _lib.call("sx_gate_mul_fwd", ptr(y), ptr(z), c_ll(C + 64), ptr(out), c_ll(n * L), c_int(C), c_int(L), c_int(Lp), stream())
+    _lib.call("sx_gate_mul_bwd", ptr(g), ptr(y), ptr(z), c_ll(C + 64), ptr(dy), ptr(dz), c_ll(n * L), c_int(C), c_int(L), c_int(Lp), c_ll(dz.shape[-1]),
+              stream())
+    yr, zr = y[:, :L].double().requires_grad_(), z[..., :C].double().requires_grad_()
+    ref = yr * torch.nn.functional.silu(zr)
+    grads = torch.autograd.grad(ref, (yr, zr), g.double())
+    slack = 1e-5 * (1 + (g.double() * yr.detach()).abs())
+    close = lambda a, b: bool(((a.double() - b).abs() <= b.abs() * 2.0 ** -8 + slack).all())  # noqa: E731
+    assert close(out, ref.detach()) and close(dy[:, :L], grads[0]) and close(dz[..., :C], grads[1])
+    assert bool((dy[:, L:] == 3.0).all()) and bool((dz[..., C:] == 3.0).all())
