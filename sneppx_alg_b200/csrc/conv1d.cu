@@ -17,8 +17,9 @@ __device__ __forceinline__ float silu_grad(float x) {
   return s * (1.f + x * (1.f - s));
 }
 
-// V channels of a row: V = 4 (8 bytes) forward, 2 backward.
+// V channels of a row: 4 (8 bytes) or 2.
 template <int V> struct ConvVec;
+template <> struct ConvVec<8> { typedef uint4 T; };
 template <> struct ConvVec<4> { typedef uint2 T; };
 template <> struct ConvVec<2> { typedef uint32_t T; };
 __device__ __forceinline__ float2 bf2(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); }
@@ -34,6 +35,11 @@ __device__ __forceinline__ void conv_unpack(uint32_t r, float (&f)[2]) {
   const float2 a = bf2(r);
   f[0] = a.x; f[1] = a.y;
 }
+__device__ __forceinline__ void conv_unpack(uint4 r, float (&f)[8]) {
+  const float2 a = bf2(r.x), b = bf2(r.y), c = bf2(r.z), d = bf2(r.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
+__device__ __forceinline__ uint4 conv_pack(const float (&f)[8]) { return make_uint4(pk2(f[0], f[1]), pk2(f[2], f[3]), pk2(f[4], f[5]), pk2(f[6], f[7])); }
 __device__ __forceinline__ uint2 conv_pack(const float (&f)[4]) { return make_uint2(pk2(f[0], f[1]), pk2(f[2], f[3])); }
 __device__ __forceinline__ uint32_t conv_pack(const float (&f)[2]) { return pk2(f[0], f[1]); }
 template <int V> __device__ __forceinline__ typename ConvVec<V>::T conv_ld(const __nv_bfloat16* p) {
@@ -61,19 +67,18 @@ __device__ __forceinline__ void conv_taps(const __nv_bfloat16* w, int c, float (
   }
 }
 
-// One thread: 4 channels x CONV_TL consecutive positions. The 4 x K weights and the bias live in registers and the
-// K-1 previous inputs slide through registers, so each input vector is loaded once and each output costs one 16-byte
-// load and one 16-byte store; consecutive threads own consecutive channel vectors (coalesced rows).
+// One thread: V channels x CONV_TL consecutive positions. The V x K weights and the bias live in registers and the
+// K-1 previous inputs slide through registers, so each input vector is loaded once and each output costs one load and
+// one store of V channels; consecutive threads own consecutive channel vectors (coalesced rows).
 // What bounds it is the latency of these chains (180 instructions for 8 channels of a row, half of them the sigmoid), so warps count: with
 // eight channels a thread and 128 registers an SM held 12 to 16. [8192, 7168]: 78 us, 100 with eight (36 us at copy bandwidth); [4, 500, 1792]
 // 14 and 16 us.
 constexpr int CONV_TL = 16;
-template <int K>
+template <int K, int V>
 __global__ void __launch_bounds__(256, 3) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ prev,
                                                             const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
                                                             __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ state_out, int B,
                                                             int L, int C, int act, long long xld, int Ly) {
-  constexpr int V = 4;
   const int cv = C / V;
   const int lchunks = (L + CONV_TL - 1) / CONV_TL;
   const long long total = (long long)B * lchunks * cv;
@@ -105,7 +110,7 @@ __global__ void __launch_bounds__(256, 3) conv1d_fwd_kernel(const __nv_bfloat16*
       else if (prev) conv_ld<V>(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c, hist[i]);
     }
     for (int lb = l0; lb < l1; lb += 4) {
-      uint2 raw4[4];   // four independent loads in flight per thread
+      typename ConvVec<V>::T raw4[4];   // four independent loads in flight per thread
 #pragma unroll
       for (int u = 0; u < 4; ++u, xp += xld)
         if (lb + u < l1) raw4[u] = conv_ld<V>(xp);
@@ -127,7 +132,7 @@ __global__ void __launch_bounds__(256, 3) conv1d_fwd_kernel(const __nv_bfloat16*
         }
         conv_st<V>(yp, acc);
         if (state_out && l >= L - (K - 1))
-          *reinterpret_cast<uint2*>(state_out + ((long long)b * (K - 1) + (l - (L - (K - 1)))) * C + c) = raw4[u];
+          *reinterpret_cast<typename ConvVec<V>::T*>(state_out + ((long long)b * (K - 1) + (l - (L - (K - 1)))) * C + c) = raw4[u];
 #pragma unroll
         for (int i = 0; i + 1 < K; ++i)
 #pragma unroll
@@ -137,16 +142,18 @@ __global__ void __launch_bounds__(256, 3) conv1d_fwd_kernel(const __nv_bfloat16*
   }
 }
 
-// dx and per-CTA partials of dw / dbias. A CTA is 32 channel groups of 2 (one per lane: 128 contiguous bytes per row) by 8 runs of
+// dx and per-CTA partials of dw / dbias. A CTA is 32 channel groups of V (one per lane: 64 V contiguous bytes per row) by 8 runs of
 // CONV_BTL consecutive positions (one per warp). A thread walks its run once: the last K inputs and the last K pre-activation gradients
 // slide through registers, so every x and dy value is loaded once (plus the K-1 row overlap between runs) and dx is stored once. As above
-// warps count more than wide loads: two channels a thread keep the kernel near 64 registers, four CTAs an SM. [8192, 7168]: 247 us, 265 with
-// four channels and two CTAs an SM (54 us at copy bandwidth): the instructions of a row bound it. The 8 warps add their dw / db into shared memory and the CTA writes one
-// partial row; conv1d_reduce_partials sums the rows.
-constexpr int CONV_BTL = 16, BWD_CTAS = 4;
-constexpr int CONV_BV = 2;
-template <int K>
-__global__ void __launch_bounds__(256, BWD_CTAS) conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
+// warps count more than wide loads: two channels a thread keep the kernel near 64 registers, four CTAs an SM. [8192, 7168]: 247 us, 265
+// with four channels and two CTAs an SM (54 us at copy bandwidth): the instructions of a row bound it; three taps 247 and 263.
+// The 8 warps add their dw / db into shared memory and the CTA writes one partial row; conv1d_reduce_partials sums the rows.
+constexpr int CONV_BTL = 16;
+// From here on, where x and dy outgrow L2, the wider loads are better with one tap forward ([8192, 7168] 53 us with eight channels, 55 with four;
+// [8192, 1792] 22.5 and 20.5) and with two taps backward (194 us with four channels, 224 with two; [16384, 1792] 132 and 127).
+constexpr long long CONV_WIDE = 1ll << 25;
+template <int K, int V>
+__global__ void __launch_bounds__(256, 8 / V) conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                             const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ prev,
                                                             const __nv_bfloat16* __restrict__ w,
@@ -154,7 +161,6 @@ __global__ void __launch_bounds__(256, BWD_CTAS) conv1d_bwd_kernel(const __nv_bf
                                                             __nv_bfloat16* __restrict__ dx, float* __restrict__ partial,
                                                             int B, int L, int C, int act, long long xld, int Ly,
                                                             long long dxld) {
-  constexpr int V = CONV_BV;
   __shared__ float s_acc[32][(CONV_MAXK + 1) * V + 1];
   const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
   const int cv = C / V;
@@ -273,20 +279,20 @@ using namespace sx;
 extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, const void* bias, void* y, void* state_out,
                              int B, int L, int C, int K, int act, long long xld, int Ly, cudaStream_t st) {
   if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L) return -1;
-  const long long total = (long long)B * ((L + CONV_TL - 1) / CONV_TL) * (C / 4);
-  if (total == 0) return 0;
-  const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-#define SX_CONV_FWD(KK)                                                                                          \
-  conv1d_fwd_kernel<KK><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)prev,              \
-                                                (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y, \
-                                                (__nv_bfloat16*)state_out, B, L, C, act, xld, Ly)
+  if ((long long)B * L * C == 0) return 0;
+  auto run = [&](auto kern, int V) {
+    const long long total = (long long)B * ((L + CONV_TL - 1) / CONV_TL) * (C / V);
+    kern<<<(int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16), 256, 0, st>>>(
+        (const __nv_bfloat16*)x, (const __nv_bfloat16*)prev, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y,
+        (__nv_bfloat16*)state_out, B, L, C, act, xld, Ly);
+  };
+  const bool wide = (long long)B * L * C >= CONV_WIDE && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0;
   switch (K) {
-    case 1: SX_CONV_FWD(1); break;
-    case 2: SX_CONV_FWD(2); break;
-    case 3: SX_CONV_FWD(3); break;
-    default: SX_CONV_FWD(4); break;
+    case 1: wide ? run(conv1d_fwd_kernel<1, 8>, 8) : run(conv1d_fwd_kernel<1, 4>, 4); break;
+    case 2: run(conv1d_fwd_kernel<2, 4>, 4); break;
+    case 3: run(conv1d_fwd_kernel<3, 4>, 4); break;
+    default: run(conv1d_fwd_kernel<4, 4>, 4); break;
   }
-#undef SX_CONV_FWD
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -296,8 +302,8 @@ extern "C" int sx_conv1d_bwd_parts(int B, int L, int C) {
   // as one run. Inputs that would leave SMs idle that way take as many CTAs as make one wave, down to one
   // run per warp ([4, 500, 1792]: 73 -> 32 us)
   const long long chunks = (long long)B * ((L + CONV_BTL - 1) / CONV_BTL);
-  const int cols = (C / CONV_BV + 31) / 32;
-  const long long wave = 148 * BWD_CTAS / (cols > 0 ? cols : 1), most = (chunks + 7) / 8;
+  const int cols = (C / 2 + 31) / 32;             // of two channels with four CTAs an SM; four channels: half as many of both
+  const long long wave = 148 * 4 / (cols > 0 ? cols : 1), most = (chunks + 7) / 8;
   long long p = (chunks + 31) / 32;
   if (p < wave) p = most < wave ? most : wave;
   return (int)(p < 1 ? 1 : (p > 512 ? 512 : p));
@@ -311,18 +317,17 @@ extern "C" int sx_conv1d_bwd(const void* dy, const void* x, const void* prev, co
   if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L || dxld % 4 || dxld < C) return -1;
   if ((long long)B * L == 0) return 0;
   const int parts = sx_conv1d_bwd_parts(B, L, C);
-  const dim3 grid((C / CONV_BV + 31) / 32, parts);
-#define SX_CONV_BWD(KK)                                                                                          \
-  conv1d_bwd_kernel<KK><<<grid, 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,                  \
-                                              (const __nv_bfloat16*)prev, (const __nv_bfloat16*)w,                \
-                                              (const __nv_bfloat16*)bias, (__nv_bfloat16*)dx, partial, B, L, C, act, xld, Ly, dxld)
+  auto run = [&](auto kern, int V) {
+    kern<<<dim3((C / V + 31) / 32, parts), 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)prev,
+                                                         (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)dx, partial, B, L, C,
+                                                         act, xld, Ly, dxld);
+  };
   switch (K) {
-    case 1: SX_CONV_BWD(1); break;
-    case 2: SX_CONV_BWD(2); break;
-    case 3: SX_CONV_BWD(3); break;
-    default: SX_CONV_BWD(4); break;
+    case 1: run(conv1d_bwd_kernel<1, 2>, 2); break;
+    case 2: (long long)B * L * C >= CONV_WIDE ? run(conv1d_bwd_kernel<2, 4>, 4) : run(conv1d_bwd_kernel<2, 2>, 2); break;
+    case 3: run(conv1d_bwd_kernel<3, 2>, 2); break;
+    default: run(conv1d_bwd_kernel<4, 2>, 2); break;
   }
-#undef SX_CONV_BWD
   const int n = (K + 1) * C;
   cudaMemsetAsync(dwdb, 0, sizeof(float) * n, st);
   conv1d_reduce_partials<<<dim3((n + 255) / 256, parts < 8 ? parts : 8), 256, 0, st>>>(partial, parts, n, dwdb);

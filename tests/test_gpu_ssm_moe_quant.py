@@ -337,3 +337,35 @@ def test_gate_mul_padded_rows(C, L, Lp, wide):
     close = lambda a, b: bool(((a.double() - b).abs() <= b.abs() * 2.0 ** -8 + slack).all())  # noqa: E731
     assert close(out, ref.detach()) and close(dy[:, :L], grads[0]) and close(dz[..., :C], grads[1])
     assert bool((dy[:, L:] == 3.0).all()) and bool((dz[..., C:] == 3.0).all())
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 4])
+@pytest.mark.parametrize("B,L,C,act", [(2, 77, 72, True), (1, 1, 8, False), (3, 33, 200, True), (1, 300, 320, False), (1, 4856, 6912, True)])
+def test_conv1d_taps(K, B, L, C, act):
+    """One to four taps, below and above the size from which one and two take wider loads, channels that fill no warp, runs that end in a
+    sequence. Products and sums are 32-bit: one bf16
+    rounding of outputs, and of gradients (2^-8), with 2^-16 of the sum of magnitudes for sums and for the fast sigmoid."""
+    torch.manual_seed(K * C + L)
+    x, g = (torch.randn(B, L, C, device="cuda").bfloat16() for _ in range(2))
+    w, b = (0.5 * torch.randn(C, K, device="cuda")).bfloat16(), torch.randn(C, device="cuda").bfloat16()
+    ins = [t.clone().requires_grad_() for t in (x, w, b)]
+    y = ssm.causal_conv1d(*ins, act=act)
+    got = torch.autograd.grad(y, ins, g)
+    ref = [t.double().requires_grad_() for t in (x, w, b)]
+    pad = torch.nn.functional.pad(ref[0], (0, 0, K - 1, 0))
+    pre = sum(pad[:, k:k + L] * ref[1][:, k] for k in range(K)) + ref[2]
+    yr = torch.nn.functional.silu(pre) if act else pre
+    want = torch.autograd.grad(yr, ref, g.double(), retain_graph=True)
+    # magnitudes: the same sums over absolute values, the derivative of silu is below 1.1
+    up = 1.1 * g.double().abs()
+    xa = torch.nn.functional.pad(x.double().abs(), (0, 0, K - 1, 0))
+    wa = w.double().abs()
+    mag_y = sum(xa[:, k:k + L] * wa[:, k] for k in range(K)) + b.double().abs()
+    ua = torch.nn.functional.pad(up, (0, 0, 0, K - 1))
+    mag_x = sum(ua[:, K - 1 - k:K - 1 - k + L] * wa[:, k] for k in range(K))
+    mag_w = torch.stack([(xa[:, k:k + L] * up).sum((0, 1)) for k in range(K)], 1)
+    near = lambda a, e, m: bool(((a.double() - e).abs() <= e.abs() * 2.0 ** -8 + m * 2.0 ** -16 + 1e-30).all())  # noqa: E731
+    assert near(y, yr.detach(), mag_y)
+    # gradients before their rounding depend on the pre-activation through the sigmoid, which is steepest by |pre| / 4
+    k2 = 1 + mag_y.max()
+    assert near(got[0], want[0], mag_x * k2) and near(got[1], want[1], mag_w * k2) and near(got[2], want[2], up.sum((0, 1)) * k2)
