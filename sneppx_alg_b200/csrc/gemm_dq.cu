@@ -19,7 +19,7 @@
 // SMs idle and four converter warps wrote scaled bf16 tiles to shared memory. The floor (packed weights at copy bandwidth) is 9 and 4.5 us:
 // what bounds it now is the issue of K = 16 MMAs with a narrow N, about 70 cycles each.
 // The reference has quantise / dequantise kernels only (kernel/quantization/quantize_cuda.cu), no GEMM on them.
-#include <cuda_fp8.h>
+#include "dq_convert.cuh"
 #include "tc_common.cuh"
 #include "tmap.h"
 #include "sx_api.h"
@@ -68,29 +68,6 @@ __device__ __forceinline__ float4 dq_ld_peer(uint32_t local_addr, uint32_t rank)
                : "r"(ra)
                : "memory");
   return v;
-}
-
-// Eight nibbles (low first) -> four packed bf16 pairs of q - 8. 0x4300 | q is 128 + q in bf16, exactly.
-__device__ __forceinline__ void int4x8_to_bf16(uint32_t w, uint32_t* o) {
-  const uint32_t lo = w & 0x0f0f0f0fu, hi = (w >> 4) & 0x0f0f0f0fu;      // elements 0 2 4 6 / 1 3 5 7
-  const uint32_t a = __byte_perm(lo, hi, 0x5140), b = __byte_perm(lo, hi, 0x7362);   // 0 1 2 3 / 4 5 6 7
-  const uint32_t m = 0x43434343u;
-  uint32_t t[4] = {__byte_perm(a, m, 0x4140), __byte_perm(a, m, 0x4342), __byte_perm(b, m, 0x4140), __byte_perm(b, m, 0x4342)};
-  const __nv_bfloat162 off = __floats2bfloat162_rn(136.f, 136.f);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __nv_bfloat162 v = __hsub2(*reinterpret_cast<__nv_bfloat162*>(&t[i]), off);
-    o[i] = *reinterpret_cast<const uint32_t*>(&v);
-  }
-}
-// Four e4m3 bytes -> two packed bf16 pairs (e4m3 has three mantissa bits: exact).
-__device__ __forceinline__ void e4m3x4_to_bf16(uint32_t w, uint32_t* o) {
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> (16 * i)), __NV_E4M3);
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-    o[i] = pack_bf16x2(f.x, f.y);
-  }
 }
 
 __device__ __forceinline__ void dq_tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -339,6 +316,11 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
   }
 }
 
+// K of 128 or 256 and more tiles than one wave (gemm_dq_short.cu)
+bool gemm_dq_short_ok(int M, int N, int K, int sms);
+int gemm_dq_short(const void* X, long long ldx, const void* W, const float* scales, const float* bias, void* D, long long ldd, int M, int N, int K,
+                  int mode, int sms, int* status, cudaStream_t st);
+
 // CTAs of a cluster = slices of K: the fewest that fill the resident slots in as few waves as possible. A CTA costs its stages plus
 // a fixed part (set-up and reduction) worth about six of them, as in the bf16 decode kernel.
 static int dq_splits(int tiles, int stages, int slots) {
@@ -396,6 +378,10 @@ extern "C" int sx_gemm_dequant(const void* X, long long ldx, const void* W, cons
                                cudaStream_t st) {
   if (K % 128 || ldx % 8 || (reinterpret_cast<uintptr_t>(X) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return -1;
   if (M <= 0 || N <= 0) return 0;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (gemm_dq_short_ok(M, N, K, sms)) return gemm_dq_short(X, ldx, W, scales, bias, D, ldd, M, N, K, mode, sms, status, st);
   DqParams p;
   const int bt = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
   {
@@ -415,9 +401,6 @@ extern "C" int sx_gemm_dequant(const void* X, long long ldx, const void* W, cons
   }
   p.scales = scales; p.bias = bias; p.D = (__nv_bfloat16*)D; p.ldd = ldd;
   p.M = M; p.N = N; p.K = K; p.status = status; p.early_weights = static_weights;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (mode == 0) {
     if (bt == 16) return dq_launch<16, false>(p, sms, st);
     if (bt == 32) return dq_launch<32, false>(p, sms, st);

@@ -141,6 +141,56 @@ def test_dequant_gemm_tiles(mode, M, N, K):
     assert bool(((y.double() - ref).abs() <= bound).all())
 
 
+def _dequant_case(mode, M, N, K, bias=True):
+    torch.manual_seed(M + N)
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    if mode == "fp8":
+        q, s = quant.quant_fp8_128x128(w)
+        wd = q.double() * s.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+        q = q.view(torch.uint8)
+    else:
+        q, s = quant.quant_int4(w)
+        wd = (torch.stack([q & 15, q >> 4], -1).view(N, K).double() - 8) * s.double().repeat_interleave(128, 1)
+    return x, q, s, wd, torch.randn(N, device="cuda") if bias else None
+
+
+@pytest.mark.parametrize("mode", ["fp8", "int4"])
+@pytest.mark.parametrize("M,N,K,bias", [(148 * 128, 128, 128, True), (149 * 128, 128, 128, False), (19073, 128, 128, True), (2049, 1200, 128, True),
+                                        (5000, 1000, 256, True), (38017, 130, 256, False), (4096, 4104, 256, True)])
+def test_dequant_gemm_of_many_short_tiles(mode, M, N, K, bias):
+    """K of 128 and 256 with up to and more than one wave of tiles: the last rows and columns of ragged tiles, odd numbers of tiles a CTA. The bound is
+    that of test_dequant_gemm_tiles; rows in common with a call of few rows agree with it as far as two such results can."""
+    x, q, s, wd, b = _dequant_case(mode, M, N, K, bias)
+    y = quant.gemm_dequant(x, q, s, mode, b)
+    ops.check_status()
+    for r in (slice(0, 1024), slice(M - 700, M)):
+        ref = x[r].double() @ wd.t() + (b.double() if bias else 0.0)
+        mag = x[r].double().abs() @ wd.abs().t() + (b.abs().double() if bias else 0.0)
+        assert bool(((y[r].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + mag * 2.0 ** -20).all())
+    few = quant.gemm_dequant(x[M - 100:].contiguous(), q, s, mode, b)
+    assert bool(((y[M - 100:].double() - few.double()).abs() <= few.double().abs() * 2.0 ** -7 + mag[-100:] * 2.0 ** -19).all())
+
+
+def test_dequant_gemm_of_short_rows_keeps_up_with_its_output():
+    """16384 x 4096 outputs of K = 128 are bound by writing 134 MB: two to four times a copy's time, ten when every tile was a CTA of its own."""
+    x, q, s, _, _ = _dequant_case("int4", 16384, 4096, 128, False)
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    big = torch.empty(512 << 20, dtype=torch.uint8, device="cuda")
+    times = []
+    for fn in (lambda: quant.gemm_dequant(x, q, s, "int4"), lambda: big[:256 << 20].copy_(big[256 << 20:])):
+        ts = []
+        for _ in range(9):
+            torch.cuda._sleep(400000)
+            a.record()
+            fn()
+            b.record()
+            torch.cuda.synchronize()
+            ts.append(a.elapsed_time(b) * 1e3)
+        times.append(sorted(ts)[4])
+    assert times[0] < 6 * times[1] * (16384 * 4096 * 2 + x.numel() * 2) / (512 << 20), times
+
+
 def test_paged_engine_matches_cached_generation_gpu():
     from sneppx_alg_b200.models import ModelConfig, build_model
     from sneppx_alg_b200.serving.generation import generate
