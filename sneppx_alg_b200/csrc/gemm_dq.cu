@@ -382,6 +382,13 @@ extern "C" int sx_gemm_dequant(const void* X, long long ldx, const void* W, cons
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (gemm_dq_short_ok(M, N, K, sms)) return gemm_dq_short(X, ldx, W, scales, bias, D, ldd, M, N, K, mode, sms, status, st);
+  constexpr int MOST = 65535 * 128;      // rows of a launch: tiles of them are the grid's y
+  for (; M > MOST; M -= MOST) {
+    const int rc = sx_gemm_dequant(X, ldx, W, scales, bias, D, ldd, MOST, N, K, mode, static_weights, status, st);
+    if (rc) return rc;
+    X = (const __nv_bfloat16*)X + (long long)MOST * ldx;
+    D = (__nv_bfloat16*)D + (long long)MOST * ldd;
+  }
   DqParams p;
   const int bt = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
   {

@@ -191,6 +191,21 @@ def test_dequant_gemm_of_short_rows_keeps_up_with_its_output():
     assert times[0] < 6 * times[1] * (16384 * 4096 * 2 + x.numel() * 2) / (512 << 20), times
 
 
+@pytest.mark.parametrize("mode", ["fp8", "int4"])
+def test_dequant_gemm_of_more_rows_than_a_grid_has_tiles(mode):
+    """65535 tiles of 128 rows are one launch; the rows behind them come from a second one."""
+    M, N, K = 65535 * 128 + 77, 8, 384
+    x, q, s, wd, b = _dequant_case(mode, 256, N, K)
+    big = torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+    big[:128], big[-128:] = x[:128], x[128:]
+    y = quant.gemm_dequant(big, q, s, mode, b)
+    ops.check_status()
+    ref = x.double() @ wd.t() + b.double()
+    bound = ref.abs() * 2.0 ** -8 + (x.double().abs() @ wd.abs().t() + b.abs().double()) * 2.0 ** -20
+    assert bool(((torch.cat([y[:128], y[-128:]]).double() - ref).abs() <= bound).all())
+    assert torch.equal(y[128:-128], b.bfloat16().expand(M - 256, N))
+
+
 def test_paged_engine_matches_cached_generation_gpu():
     from sneppx_alg_b200.models import ModelConfig, build_model
     from sneppx_alg_b200.serving.generation import generate
