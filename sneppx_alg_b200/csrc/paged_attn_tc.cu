@@ -57,13 +57,13 @@ struct PtItem {
 };
 
 // (sequence b, KV head hk, split) of item `item`, heads fastest: a cached position's heads lie side by side (256 bytes each), and neighbouring CTAs
-// that walk the same positions at the same time read whole DRAM pages together (48 sequences of 900 - 1800 positions, 8 heads: 87 us with
-// sequences fastest, 83 so). Splits slowest as long as a CTA has few items: the last splits of a sequence are shorter or empty and fill up
-// what the long ones leave, where otherwise some CTAs got long items only (16 sequences of 1000 positions, 4 heads: 30 us with splits before
-// sequences, 26 so; 128 of 4000, 2 heads, 10 items a CTA: 136 and 130). Odd splits walk the sequences backwards, so that a batch sorted by
-// length deals long and short items to the same CTA. With more than 12 items a CTA that evens out, and one sequence's splits side by side
-// are better (128 sequences of 1000 positions, 32 heads: 429 us, 441 with splits slowest).
-constexpr int PT_FEW_ITEMS = 12;
+// that walk the same positions at the same time read whole DRAM pages together. Splits slowest as long as a CTA has few items: the last splits
+// of a sequence are shorter or empty and fill up what the long ones leave, where otherwise some CTAs got long items only (16 sequences of 1000
+// positions, 4 heads, 2 items a CTA: 30 us with splits before sequences, 26 so). Odd splits walk the sequences backwards, so that a batch
+// sorted by length deals long and short items to the same CTA. With more than 7 items a CTA that mostly evens out, and one sequence's splits
+// side by side are better: 48 sequences of 900 - 1800 positions, 8 heads, 81 us, 83 with splits slowest (87 with sequences fastest); 128 of 1000, 32
+// heads, 429 and 441. Equal lengths can still go the other way: 128 of 4000, 2 heads, 138 and 132.
+constexpr int PT_FEW_ITEMS = 7;
 __host__ __device__ __forceinline__ void pt_order(int item, int B, int Hkv, int nsplit, bool few, int* b, int* hk, int* split) {
   const int rest = item / Hkv, d = few ? B : nsplit, q = rest / d, r = rest - q * d;
   *hk = item - rest * Hkv;

@@ -203,7 +203,7 @@ def test_paged_decode_deals_its_items_evenly():
         best, longest = [0] * n_cta, sorted(count, reverse=True)
         for i in range(B * Hkv * ns):
             best[i % n_cta] += longest[i // (B * Hkv)]
-        assert max(load) == max(best) or B * Hkv * ns > 12 * n_cta, (B, Hkv, n, max(load), max(best))
+        assert max(load) == max(best) or B * Hkv * ns > 7 * n_cta, (B, Hkv, n, max(load), max(best))
 
 
 def test_prompts_are_uploaded_as_torch_tensor_takes_them():
