@@ -383,3 +383,46 @@ def test_attention_backward_of_one_query_zeroes_with_many_ctas():
         a, t = _attn_bwd_args(1, 1, H, H)
         us.append(_median_us(lambda: _lib.call("sx_attn_bwd", C.byref(a), stream())))
     assert us[1] < us[0] + 14, us
+
+
+def _attention64(q, k, v, do, causal, window):
+    """Output and gradients in 64 bits, and the probabilities' sum over the keys."""
+    q, k, v = (t.double().requires_grad_() for t in (q, k, v))
+    (B, Sq, H, D), Skv, rep = q.shape, k.shape[1], q.shape[2] // k.shape[2]
+    s = torch.einsum("bqhd,bkhd->bhqk", q, k.repeat_interleave(rep, 2)) / math.sqrt(D)
+    i = torch.arange(Sq, device="cuda").view(-1, 1) + Skv - Sq
+    j = torch.arange(Skv, device="cuda").view(1, -1)
+    hidden = (j > i if causal else torch.zeros_like(j > i)) | ((j <= i - window) if window else torch.zeros_like(j > i))
+    p = s.masked_fill(hidden, -math.inf).softmax(-1)
+    o = torch.einsum("bhqk,bkhd->bqhd", p, v.repeat_interleave(rep, 2))
+    pk = torch.einsum("bhqk,bkhd->bqhd", p, k.repeat_interleave(rep, 2)).detach()
+    return (o.detach(), *torch.autograd.grad(o, (q, k, v), do.double())), pk
+
+
+@pytest.mark.parametrize("H,Hk", [(2, 2), (7, 1)])
+@pytest.mark.parametrize("Sq,Skv,causal,window", [
+    (1, 1, True, 0), (63, 63, True, 0), (64, 64, True, 0), (65, 65, True, 0), (77, 77, True, 0), (129, 129, True, 0), (130, 130, False, 0), (257, 257, True, 0),
+    (1, 300, True, 0), (65, 129, True, 0), (77, 200, True, 0), (130, 1000, True, 0), (100, 260, False, 0), (260, 100, False, 0),
+    (64, 1024, True, 100), (192, 1000, True, 70), (700, 700, True, 64), (321, 321, True, 1)])
+def test_attention_backward_tiles(H, Hk, Sq, Skv, causal, window):
+    """One, two, three and more query tiles of a key tile, odd and even numbers of them over the heads of a group, key tiles that no query sees,
+    partial tiles of both, queries that follow cached keys. Every row of every result by itself: P, dS, O and the results are rounded to bf16
+    (2^-9 each, at random), so a row is within 2^-7 of its norm, and, where it cancels, of the root mean square of the rows. The rounding of O
+    moves delta, by 2^-9 sum |dO O| at most, which goes into a row of dQ with the factor scale |P K|; into dK with P and over the queries, at random,
+    below the terms before."""
+    B = 1 if Skv == 1 else 2
+    torch.manual_seed(Sq + Skv)
+    q, do = (torch.randn(B, Sq, H, 128, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Skv, Hk, 128, device="cuda").bfloat16() for _ in range(2))
+    if Sq == 1 and B == 2:
+        q, do, k, v = q[:1], do[:1], k[:1], v[:1]
+    ins = [t.clone().requires_grad_() for t in (q, k, v)]
+    o = F_.attention(*ins, causal=causal, window=window)
+    got = (o.detach(), *torch.autograd.grad(o, ins, do))
+    ops.check_status()
+    want, pk = _attention64(q, k, v, do, causal, window)
+    delta = 2.0 ** -9 * (do.double() * want[0]).abs().sum(-1) * pk.norm(dim=-1) / math.sqrt(128)
+    for name, a, e in zip(("o", "dq", "dk", "dv"), got, want):
+        err, norm = (a.double() - e).norm(dim=-1), e.norm(dim=-1)
+        bound = 2.0 ** -7 * norm + 2.0 ** -7 * norm.square().mean().sqrt() + 1e-4 + (delta if name == "dq" else 0.0)
+        assert bool((err <= bound).all()), (name, (err / bound).max().item())

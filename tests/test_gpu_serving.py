@@ -342,3 +342,78 @@ def test_mamba2_decode_step_that_fails(monkeypatch):
     assert torch.equal(run.decode([1, 2], [12, 13]), other.decode([1, 2], [12, 13]))
     assert torch.equal(run.decode([1, 2], [14, 15]), other.decode([1, 2], [14, 15]))
     ops.check_status()
+
+
+@pytest.mark.parametrize("mode", ["fp8", "int4"])
+@pytest.mark.parametrize("M", [1, 17, 64, 128])
+@pytest.mark.parametrize("N,K", [(128, 128), (128, 640), (200, 384), (4096, 4224), (1000, 3968)])
+def test_dequant_gemm_with_static_weights(mode, M, N, K):
+    """Weights and scales read ahead of the kernel that makes X, which lets its dependents start early: the same values as without, over several
+    calls in a row; rings of stages that hold all of a CTA's slice and more, slices of K that are empty."""
+    from sneppx_alg_b200.ops import functional as F_
+    from sneppx_alg_b200.ops.gemm import static_weights
+    x, q, s, wd, b = _dequant_case(mode, M, N, K)
+    w = torch.ones(K, device="cuda", dtype=torch.bfloat16)
+    want, rows = [], [x * (1 + i) for i in range(4)]
+    for r in rows:
+        h, _ = F_.rmsnorm(r, w)
+        want.append((h, quant.gemm_dequant(h, q, s, mode, b)))
+    got = []
+    with static_weights():
+        for r in rows:
+            h, _ = F_.rmsnorm(r, w)
+            got.append((h, quant.gemm_dequant(h, q, s, mode, b)))
+    ops.check_status()
+    for (h, y), (hw, yw) in zip(got, want):
+        assert torch.equal(h, hw) and torch.equal(y, yw)
+    ref = want[0][0].double() @ wd.t() + b.double()
+    mag = want[0][0].double().abs() @ wd.abs().t() + b.abs().double()
+    assert bool(((want[0][1].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + mag * 2.0 ** -20).all())
+
+
+def test_captured_decode_with_changing_batches():
+    """Rows of the captured step's block table are written when a table changes: sequences that swap rows, leave, come back shorter and grow over
+    blocks give the logits of the same steps without capture."""
+    from sneppx_alg_b200.models import ModelConfig, build_model
+    from sneppx_alg_b200.serving.kv_cache import PagedKVCache
+    from sneppx_alg_b200.serving.llm_engine import LlamaPagedRunner
+    torch.manual_seed(4)
+    cfg = ModelConfig(hidden_size=512, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=128, intermediate_size=512,
+                      vocab_size=300, max_position_embeddings=256, rms_norm_eps=1e-5)
+    model = build_model(cfg, dtype=torch.bfloat16, device="cuda").eval()
+    runners = []
+    for graphs in (True, False):
+        cache = PagedKVCache(2, 80, 8, 2, 128, device="cuda", enable_prefix_cache=False)
+        runners.append(LlamaPagedRunner(model, cache))
+        if graphs:
+            runners[0].enable_graphs(6, 128)
+
+    def start(sid, n):
+        for r in runners:
+            r.cache.add_sequence(sid)
+            r.prefill(sid, [(7 * sid + 3 * i) % 300 for i in range(n)], 0)
+
+    def stop(sid):
+        for r in runners:
+            r.cache.free_sequence(sid)
+
+    def steps(ids, n):
+        for t in range(n):
+            a, b = (r.decode(ids, [(11 * s + 5 * t) % 300 for s in ids]) for r in runners)
+            assert a.shape == b.shape and _rel(a, b) < 2e-2, (ids, t)
+
+    for sid, n in enumerate((5, 40, 17, 63, 8)):
+        start(sid, n)
+    steps([0, 1, 2, 3], 9)
+    steps([3, 0], 10)                 # fewer rows: another captured step
+    steps([2, 1, 0, 3, 4], 3)         # more of them, in other rows
+    stop(1)
+    start(1, 2)                       # a shorter table, of blocks that others have held, in a row that held a longer one
+    steps([2, 1, 0, 3, 4], 9)
+    stop(3)
+    start(5, 30)
+    for r in runners:                 # two sequences with one table, then one of them copies its last block
+        r.cache.fork(5, 6)
+    steps([5, 6, 1, 0], 9)
+    steps([6, 5, 2, 1, 0, 4], 4)
+    ops.check_status()
