@@ -17,7 +17,8 @@
 // Measured (B200, graph replay, cold weights), int4 [28672, 4096] at 1 / 16 / 32 / 64 / 128 rows: 29 / 29 / 31 / 40 / 62 us, [4096, 14336]
 // 16 / 16 / 17 / 19 / 28 us; 203 / 199 / 199 / 199 / 201 and 361 / 354 / 353 / 353 / 356 us before, when 128 x 128 output tiles left most
 // SMs idle and four converter warps wrote scaled bf16 tiles to shared memory. The floor (packed weights at copy bandwidth) is 9 and 4.5 us:
-// what bounds it now is the issue of K = 16 MMAs with a narrow N, about 70 cycles each.
+// what bounds it now are the K = 16 MMAs with a narrow N, about 70 cycles each, whether by their issue or by accumulating one after another into
+// one tile, which was not separated. K of 128 or 256 with more than one wave of tiles: gemm_dq_short.cu.
 // The reference has quantise / dequantise kernels only (kernel/quantization/quantize_cuda.cu), no GEMM on them.
 #include "dq_convert.cuh"
 #include "tc_common.cuh"
@@ -41,7 +42,11 @@ struct DqParams {
   int* status;
 };
 
-// BT rows of X per tile. Warps: PW promotion / epilogue, 8 converters, 1 MMA, 1 TMA.
+// BT rows of X per tile. Warps: PW promotion / epilogue, 4 NG converters, 2 MMA, 1 TMA.
+// Times below: cold, with the launch. PW: a promotion thread holds BT sums with four warps, and from 64 on they do not fit its registers beside the rest (120 bytes spilled at 64 rows,
+// int4 [28672, 4096] 57 us; 48 with eight); at 32 rows eight warps leave 48 registers for two CTAs an SM (43 us, 39 with four).
+// NG: four converter groups where one CTA an SM leaves room for them, 48 us at 64 rows, 53 with two; at 128 rows they leave 72 registers for
+// promotion threads of 64 sums (184 bytes spilled, 79 us; 72 with two).
 template <int BT>
 struct DqCfg {
   static constexpr int PW = BT >= 64 ? 8 : 4;           // from 64 columns on two warps per lane quadrant, half of the columns each

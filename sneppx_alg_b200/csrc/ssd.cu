@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(256) ssd_state_bwd_kernel(const float* __restr
 // Layouts of the [tokens, heads, P] tensors. Token-major row r = (bc * Q + q) * H + h. The operands of the GEMMs that
 // fold the heads of a B / C group into one matrix dimension are kept group-first, [bc][G][Q][H/G][P], so that
 // (bc, group) is one linear batch index; gf_row maps a token-major row to its group-first row (the identity for G = 1).
-// I: type of every index below, 32-bit unless a tensor has 2^31 elements or more. A 64-bit division is a call of some hundred instructions,
-// and a 16-byte piece takes six: [8192 tokens, 80 heads, 64] rows1 110 -> 65 us, scale_rows 49 -> 32, rows2 82 -> 73,
+// I: type of every index below, which count pieces of 16 bytes: 32-bit below 2^30 pieces; offsets in elements are 64-bit. A 64-bit division is a
+// call of some hundred instructions, and a piece takes six: [8192 tokens, 80 heads, 64] rows1 110 -> 65 us, scale_rows 49 -> 32, rows2 82 -> 73,
 // heads_first 38 -> 32.
 template <typename I>
 __device__ __forceinline__ I gf_row(I r, int H, int Q, int G) {
