@@ -39,7 +39,6 @@ struct PagedTcParams {
   float* ml_part;
   int* status;
   int B, Hq, Hkv, block_size, max_blocks, nsplit;
-  bool few_items;         // per CTA
   float scale_log2;
 };
 
@@ -64,17 +63,24 @@ struct PtItem {
 // side by side are better: 48 sequences of 900 - 1800 positions, 8 heads, 81 us, 83 with splits slowest (87 with sequences fastest); 128 of 1000, 32
 // heads, 429 and 441. Equal lengths can still go the other way: 128 of 4000, 2 heads, 138 and 132.
 constexpr int PT_FEW_ITEMS = 7;
-__host__ __device__ __forceinline__ void pt_order(int item, int B, int Hkv, int nsplit, bool few, int* b, int* hk, int* split) {
-  const int rest = item / Hkv, d = few ? B : nsplit, q = rest / d, r = rest - q * d;
-  *hk = item - rest * Hkv;
-  *split = few ? q : r;
-  *b = few ? (q & 1 ? B - 1 - r : r) : q;
+template <bool FEW>
+__host__ __device__ __forceinline__ void pt_order(int item, int B, int Hkv, int nsplit, int* b, int* hk, int* split) {
+  *hk = item % Hkv;
+  const int rest = item / Hkv;
+  if constexpr (FEW) {
+    *split = rest / B;
+    *b = *split & 1 ? B - 1 - rest % B : rest % B;
+  } else {
+    *split = rest % nsplit;
+    *b = rest / nsplit;
+  }
 }
 
 // The tile range of an item comes from the sequence length on the device.
+template <bool FEW>
 __device__ __forceinline__ PtItem pt_item(const PagedTcParams& p, int item) {
   PtItem w;
-  pt_order(item, p.B, p.Hkv, p.nsplit, p.few_items, &w.b, &w.hk, &w.split);
+  pt_order<FEW>(item, p.B, p.Hkv, p.nsplit, &w.b, &w.hk, &w.split);
   w.len = p.seq_lens[w.b];
   const int tiles = (w.len + PT_BN - 1) / PT_BN;
   const int per = (tiles + p.nsplit - 1) / p.nsplit;
@@ -87,6 +93,7 @@ __device__ __forceinline__ PtItem pt_item(const PagedTcParams& p, int item) {
 // Persistent: one CTA per SM walks items blockIdx.x, blockIdx.x + gridDim.x, ...; the TMA warp runs ahead across item
 // boundaries (the stage ring and every barrier phase are counted over the CTA's whole life), so the cache stream does
 // not stop while an item's result is written out.
+template <bool FEW>      // items a CTA, see pt_order
 __global__ void __launch_bounds__(PT_THREADS, 1) paged_decode_tc_kernel(const __grid_constant__ PagedTcParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -152,7 +159,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) paged_decode_tc_kernel(const __
     uint32_t gt = 0, qi = 0;             // tiles / non-empty items so far
     bool ok = true;
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-      const PtItem w = pt_item(p, item);
+      const PtItem w = pt_item<FEW>(p, item);
       if (w.n_steps == 0) continue;
       const int qb = qi & 1;
       if (!mbar_wait_warp(&q_empty[qb], ((qi >> 1) & 1) ^ 1, s_abort, p.status, ST_TIMEOUT_PRODUCER)) break;
@@ -192,7 +199,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) paged_decode_tc_kernel(const __
       uint32_t gt = 0, qi = 0;
       bool ok = true;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-        const PtItem w = pt_item(p, item);
+        const PtItem w = pt_item<FEW>(p, item);
         if (w.n_steps == 0) continue;
         const int qb = qi & 1;
         const uint32_t q0 = smem_u32(sQ + qb * PT_Q_BYTES);
@@ -237,7 +244,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) paged_decode_tc_kernel(const __
     bool ok = true;
     uint32_t gt = 0, qi = 0, rc = 0;    // tiles, non-empty items, uses of red_bar so far
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-      const PtItem w = pt_item(p, item);
+      const PtItem w = pt_item<FEW>(p, item);
       const long long row0 = ((long long)w.b * p.Hq + (long long)w.hk * G) * p.nsplit + w.split;   // + g * nsplit
       if (w.n_steps == 0) {
         for (int g = 0; g < G; ++g) {
@@ -392,7 +399,8 @@ extern "C" int sx_paged_decode_tc_splits(int max_len, int ctas_per_split) {
 
 // The (sequence, KV head, split) of an item, for checks of the order on the host.
 extern "C" void sx_paged_decode_tc_item(int item, int B, int Hkv, int nsplit, int sms, int* b, int* hk, int* split) {
-  pt_order(item, B, Hkv, nsplit, (long long)B * Hkv * nsplit <= (long long)PT_FEW_ITEMS * sms, b, hk, split);
+  if ((long long)B * Hkv * nsplit <= (long long)PT_FEW_ITEMS * sms) pt_order<true>(item, B, Hkv, nsplit, b, hk, split);
+  else pt_order<false>(item, B, Hkv, nsplit, b, hk, split);
 }
 
 // Same contract as sx_paged_decode (o_part: fp32 [B, Hq, nsplit, D], ml_part: fp32 [B, Hq, nsplit, 2] scratch);
@@ -432,8 +440,8 @@ extern "C" int sx_paged_decode_tc(const void* q, long long q_row_stride, const v
   p.scale_log2 = scale * 1.4426950408889634f;
   static bool set = false;
   if (!set) {
-    if (cudaFuncSetAttribute(paged_decode_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(paged_decode_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(paged_decode_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM) != cudaSuccess)
       return -10;
     set = true;
   }
@@ -444,8 +452,8 @@ extern "C" int sx_paged_decode_tc(const void* q, long long q_row_stride, const v
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   }
   const long long items = (long long)B * Hkv * nsplit;
-  p.few_items = items <= (long long)PT_FEW_ITEMS * sms;
-  paged_decode_tc_kernel<<<(unsigned)(items < sms ? items : sms), PT_THREADS, PT_SMEM, st>>>(p);
+  auto run = [&](auto kern) { kern<<<(unsigned)(items < sms ? items : sms), PT_THREADS, PT_SMEM, st>>>(p); };
+  items <= (long long)PT_FEW_ITEMS * sms ? run(paged_decode_tc_kernel<true>) : run(paged_decode_tc_kernel<false>);
   paged_merge_launch(o_part, ml_part, out, out_row_stride, B, Hq, D, nsplit, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
