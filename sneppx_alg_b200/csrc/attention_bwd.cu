@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // Heaviest key tiles first (under a causal mask tile 0 sees every query tile): kv head is the fastest block index.
   const int kv_tile = blockIdx.x / p.Hk, kv_head = blockIdx.x % p.Hk, b = blockIdx.z;
   const int G = p.Hq / p.Hk;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_it > 0) {
+    if (n_it > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_f16(128, BWD_Q, 1, 0, 0);      // K Q^T, V dO^T
       constexpr uint32_t idesc_acc = umma_idesc_f16(128, BWD_D, 1, 0, 1);    // P^T dO, dS^T Q
       constexpr uint32_t idesc_dq = umma_idesc_f16(128, BWD_Q, 1, 1, 1);     // K^T dS^T

@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // heavy (late) query tiles first: better tail behaviour under the causal mask
   const int pair = gridDim.x - 1 - blockIdx.x;
   const int head = blockIdx.y, b = blockIdx.z;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0 && elect_one()) {
       mbar_expect_tx(q_full, 2 * Cfg::Q_BYTES);
       tma5(sQ, &p.tmQ, q_full, q0, head, b);
       tma5(sQ + Cfg::Q_BYTES, &p.tmQ, q_full, q0 + ATT_BM, head, b);
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0 && elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc_f16(ATT_BM, ATT_BN, 1, 0, 0);
       constexpr uint32_t idesc_pv = umma_idesc_f16(ATT_BM, D, 1, 0, 1);
       auto issue_qk = [&](int x, int j) {

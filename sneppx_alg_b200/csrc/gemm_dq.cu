@@ -10,15 +10,15 @@
 //              is where the MMA reads its A operand: the expanded weights never touch shared memory. A group is one chain of
 //              dependent instructions (about 1 us a k-block), so several are in flight
 //   MMA        eight K = 16 steps per k-block into one of two accumulators, each with an issuing warp of its own: k-blocks do not
-//              accumulate into one another, and one thread's waits, issue and commits (about 1700 cycles a k-block) were the limit
+//              accumulate into one another, and one thread's waits, issue and commits were the limit
 //   promotion  acc[row][m] += scale[row, k-block] * partial in fp32 registers; the scale belongs to the thread's own row (TMEM lane),
 //              so it is one multiply-add per value. Products are therefore exact and nothing is rounded to bf16 before the output.
 // Two CTAs share an SM up to 32 rows of X, so that one converts while the other waits.
-// Measured (B200, graph replay, cold weights), int4 [28672, 4096] at 1 / 16 / 32 / 64 / 128 rows: 29 / 29 / 31 / 40 / 62 us, [4096, 14336]
-// 16 / 16 / 17 / 19 / 28 us; 203 / 199 / 199 / 199 / 201 and 361 / 354 / 353 / 353 / 356 us before, when 128 x 128 output tiles left most
-// SMs idle and four converter warps wrote scaled bf16 tiles to shared memory. The floor (packed weights at copy bandwidth) is 9 and 4.5 us:
-// what bounds it now are the K = 16 MMAs with a narrow N, about 70 cycles each, whether by their issue or by accumulating one after another into
-// one tile, which was not separated. K of 128 or 256 with more than one wave of tiles: gemm_dq_short.cu.
+// Measured (B200, graph replay, cold weights), int4 [28672, 4096] at 1 / 16 / 32 / 64 / 128 rows: 24 / 24 / 27 / 33 / 58 us, [4096, 14336]
+// 15 / 15 / 16 / 16 / 26 us; 28 / 28 / 30 / 39 / 62 and 16 / 17 / 17 / 19 / 28 us when operands were moved to uniform registers for each
+// MMA (tc_common.cuh), 203 / 199 / 199 / 199 / 201 and 361 / 354 / 353 / 353 / 356 us when 128 x 128 output tiles left most SMs idle and four
+// converter warps wrote scaled bf16 tiles to shared memory. The floor (packed weights at copy bandwidth) is 9 and 4.5 us. K of 128 or 256 with
+// more than one wave of tiles: gemm_dq_short.cu.
 // The reference has quantise / dequantise kernels only (kernel/quantization/quantize_cuda.cu), no GEMM on them.
 #include "dq_convert.cuh"
 #include "tc_common.cuh"
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   uint32_t S, r;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(S));
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
 
   if (warp == Cfg::MMA_WARP + 2) {
     // ------------------------------------------------------------ TMA
-    if (lane == 0) {
+    if (elect_one()) {
       auto load_w = [&](int i, int s) {
         mbar_expect_tx(&full[s], STAGE_BYTES);
         tma_load_2d(smem + s * STAGE_BYTES, &p.tmW, &full[s], (st0 + i) * 128, n0);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
     }
   } else if (warp >= Cfg::MMA_WARP) {
     // ------------------------------------------------------------ MMA: this warp's k-blocks i = buf, buf + 2, ...
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_f16(DQ_BM, BT, 1, 0, 0);
       const int buf = warp - Cfg::MMA_WARP;
       const uint32_t tD = tmem_base + Cfg::TM_D + buf * BT;

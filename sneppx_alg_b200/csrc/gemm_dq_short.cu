@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) gemm_dq_short_kernel(const __gr
   uint64_t* tempty = tfull + 2;               // [2] 4 epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < DS_STAGES; ++s) {
       mbar_init(&x_full[s], 1);
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) gemm_dq_short_kernel(const __gr
   const int kblks = p.K / 128, steps = p.K / DS_BK;      // steps of 64: two a k-block
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) gemm_dq_short_kernel(const __gr
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_f16(DS_BM, DS_BN, 1, 0, 0);
       int stage = 0, it = 0;
       uint32_t phase = 0;

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_f8_kernel(const __grid_con
   uint64_t* tempty = tfull + 2;                 // [2], 4 arrivals
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   constexpr int TCOLS = 2 * BT < 32 ? 32 : 2 * BT;
 
   if (threadIdx.x == 0) {
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_f8_kernel(const __grid_con
   const int s_row = grp * (p.tile_group ? (p.N + 127) / 128 : 0) + nb;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       for (int i = 0; i < nkb; ++i) {
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_f8_kernel(const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_f8(128, BT, 0, 0);
       int stage = 0;
       uint32_t phase = 0;

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_skinny_kernel(const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SK_MAX_STAGES + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int S = (int)cluster_size(), r = (int)cluster_rank();
   const int tile = blockIdx.x / S;
   const int n0 = tile * SK_BM;
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_skinny_kernel(const __grid
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       // weight tiles of the first ring pass may be fetched before the predecessor kernel has finished
       const int pre = (p.flags & 1) ? min(nk, p.stages) : 0;
       for (int i = 0; i < pre; ++i) {
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_skinny_kernel(const __grid
       }
     }
   } else if (warp == 4) {
-    if (lane == 0 && nk > 0) {
+    if (nk > 0 && elect_one()) {
       const uint32_t idesc = umma_idesc_f16(SK_BM, p.Mpad, 1, 0, 0);
       bool ok = true;
       for (int i = 0; i < nk; ++i) {

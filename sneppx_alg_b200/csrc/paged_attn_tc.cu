@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) paged_decode_tc_kernel(const __
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float (*s_red)[4][PT_MAX_G] = reinterpret_cast<float (*)[4][PT_MAX_G]>(smem + PT_OFF_BAR + 256);  // [2][4][G]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int G = p.Hq / p.Hkv;
   const int n_items = p.B * p.Hkv * p.nsplit;
 
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) paged_decode_tc_kernel(const __
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc_f16(PT_BN, PT_NQ, 1, 0, 0);   // A = K tile (K-major), B = Q (K-major)
       constexpr uint32_t idesc_pv = umma_idesc_f16(PT_D, PT_NQ, 1, 1, 0);    // A = V tile (MN-major), B = P^T (K-major)
       const uint32_t p0 = smem_u32(sP);

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(SF_THREADS, 1) ssd_chunk_fwd_kernel(const __gr
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int g = blockIdx.x;
   const long long bc = blockIdx.y;
   const int rep = p.H / p.G;
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(SF_THREADS, 1) ssd_chunk_fwd_kernel(const __gr
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(cb_full, 2 * Cfg::CB_BYTES);
       tma_load_4d(sC, &p.tmC, cb_full, 0, t0, 0, g);
       tma_load_4d(sB, &p.tmB, cb_full, 0, t0, 0, g);
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(SF_THREADS, 1) ssd_chunk_fwd_kernel(const __gr
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_g = umma_idesc_f16(SF_Q, SF_Q, 1, 0, 0);      // C B^T, both K-major
       constexpr uint32_t idesc_mx = umma_idesc_f16(SF_Q, SF_P, 1, 0, 1);     // M (TMEM) x X (MN-major)
       constexpr uint32_t idesc_yo = umma_idesc_f16(SF_Q, SF_P, 1, 0, 0);     // C x Hprev^T, both K-major

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) talk_tc_kernel(const __grid_con
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* s_ml = reinterpret_cast<float*>(sR);  // [2 streams][max, sum][128 rows], over the ring once it is drained
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tile = p.n_tiles - 1 - blockIdx.y, head = blockIdx.x;
   const int seq = p.tiles[2 * tile], r0 = p.tiles[2 * tile + 1];
   const int cu = p.rv.cu[seq], len = p.rv.cu[seq + 1] - cu, pos0 = p.rv.pos0[seq], base = p.kv_base[seq];
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) talk_tc_kernel(const __grid_con
 
   // order of the ring: K(0), K(1), then V(j), K(j + 2) for j = 0, 1, ..
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       if (p.resident) {
         mbar_expect_tx(q_full, p.nq * TT_SLICE);
         for (int c = 0; c < p.nq; ++c) tma_load_2d(sQ + c * TT_SLICE, &p.tmQ, q_full, (head * p.nq + c) * 64, t0);
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) talk_tc_kernel(const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_qk = umma_idesc_f16(TT_BM, TT_BN, 1, 0, 0);
       const uint32_t idesc_pv = umma_idesc_f16(TT_BM, (p.dv + 15) / 16 * 16, 1, 0, 1);
       int it = 0;

@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) win_tc_kernel(const __grid_cons
   float* s_ml = reinterpret_cast<float*>(sR);  // [2 streams][max, sum][128 rows], over the ring once it is drained
 
   const SxWinAttnArgs& a = p.a;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tile = a.n_tiles - 1 - blockIdx.y, head0 = PAIR ? 2 * blockIdx.x : blockIdx.x;
   const int seq = a.tiles[2 * tile], r0 = a.tiles[2 * tile + 1];
   const int cu = p.rv.cu[seq], len = p.rv.cu[seq + 1] - cu, pos0 = p.rv.pos0[seq];
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) win_tc_kernel(const __grid_cons
   // order of the ring. PAIR: K(0), then V(j), K(j + 1) for j = 0, 1, ..; else K(0), K(1), then V(j), K(j + 2)
   constexpr int AHEAD = PAIR ? 1 : 2;
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const int n_q = (PAIR ? 2 : 1) * nq;
       mbar_expect_tx(q_full, n_q * WT_SLICE);
       for (int c = 0; c < n_q; ++c) tma_load_2d(sQ + c * WT_SLICE, &p.tmQ, q_full, (head0 * nq + c) * 64, t0);
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) win_tc_kernel(const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_qk = umma_idesc_f16(WT_BM, WT_BN, 1, 0, 0);
       const uint32_t idesc_pv = umma_idesc_f16(WT_BM, (a.dv + 15) / 16 * 16, 1, 0, 1);
       int it = 0;
