@@ -2,18 +2,23 @@
 //
 // One CTA owns 256 query rows of one (batch, head) as two 128-row tiles X in {A, B}, each served
 // by its own softmax warpgroup, and walks the visible 128-row KV tiles:
-//   S_X = Q_X K^T       tcgen05.mma SS, fp32 in TMEM
-//   P_X = exp2(S_X - m) one query row per thread (TMEM lane == row, no shuffles); P is written back
-//                       as packed bf16 over the S columns it came from
+//   S   = Q_X K^T       tcgen05.mma SS, fp32 in TMEM
+//   P_X = exp2(S - m)   one query row per thread (TMEM lane == row, no shuffles), packed bf16 in TMEM
 //   O_X += P_X V        tcgen05.mma TS: P straight from TMEM, V consumed MN-major from its [kv, d] tile
-// The MMA warp ping-pongs the two tiles (PV(A,j), QK(A,j+1), PV(B,j), QK(B,j+1), ...), so the tensor
-// pipe works on one tile while the other tile's warpgroup does its softmax. tcgen05.mma executes in
-// issue order, which is what makes the S/P aliasing safe. The running max is only refreshed when
-// it grew by more than 2^8, so rescaling O in TMEM is rare. Causal / sliding-window masks, GQA head
+// Both tiles take turns with one S: a warpgroup has its scores in registers (setmaxnreg: 216 a thread) before it works on them, so that the next
+// product may follow at once, and P has columns of its own. A tile's scores are then ready when its warpgroup is, and the row's chain of maximum,
+// 128 exponentials and sum is all that a step of it waits for. With P over S, S had to wait for O += P V of the step before, which was a third of
+// a step, whatever the exponentials cost (half of them as polynomials: slower; 16 softmax warps, half a row each: slower). The MMA warp issues the
+// score products two items (tile, step) ahead of P V, in a fixed order: taking whichever is ready first was slower, the tiles fall into step.
+// The running max is only refreshed when it grew by more than 2^8, so rescaling O in TMEM is rare.
+// Causal / sliding-window masks, GQA head
 // mapping and the differential-attention V mapping (two score heads share one V head) are index
 // arithmetic; nothing is materialised. An optional block mask (one byte per 128 x 128 score tile, per head or
 // shared) removes whole tiles from the walk: a step whose tile is masked for both query tiles is neither loaded nor
 // multiplied (block-sparse / flex-attention patterns at tile granularity).
+// Bound: exponentials (16 a cycle and SM: 2048 cycles for a step of both tiles, as many as its products take). B200, warm, before -> now:
+// [1, 4096, 32 / 8 heads, 128] causal 187 -> 127 us, [1, 8192, 8 / 2] full 288 -> 238, [8, 512, 28 / 4] causal 53 -> 43, [1, 16384, 32 / 8] causal
+// 2.28 -> 1.98 ms (1100 TFLOP/s, at the power cap).
 // Takes the place of the reference's SIMT flash-attention forward, GQA and block-sparse kernels
 // (kernel/cuda/attention_cuda.cu:37-328, 498-573, 1154-1230) and its empty "v3" kernel (:1262-1286).
 #include <limits.h>
@@ -25,7 +30,9 @@ namespace sx {
 
 constexpr int ATT_BM = 128;   // rows per q tile (two per CTA)
 constexpr int ATT_BN = 128;
-constexpr int ATT_THREADS = 320;  // TMA warp, MMA warp, 2 x 4 softmax warps
+// 2 x 4 softmax warps, TMA warp, MMA warp, two idle ones: the last four give registers to the softmax warps, which hold a row of 128 scores
+// (2 x 128 x 216 + 128 x 72 = 384 x 168, what the block is launched with)
+constexpr int ATT_THREADS = 384, ATT_TMA_WARP = 8, ATT_MMA_WARP = 9;
 
 struct AttnFwdParams {
   CUtensorMap tmQ, tmK, tmV;
@@ -36,6 +43,7 @@ struct AttnFwdParams {
   int B, Sq, Skv, Hq, Hk;
   int v_head_div;  // V head = (K head) / v_head_div
   int causal, window;  // window <= 0: unlimited
+  int pairs, batch_first;   // pairs of query tiles; order of blocks
   float scale_log2;    // softmax scale * log2(e)
   const uint8_t* block_mask;   // optional [B or 1][Hq or 1][q tiles][kv tiles], non-zero = tile takes part
   long long bm_batch_stride, bm_head_stride;
@@ -50,7 +58,8 @@ struct AttnCfg {
   static constexpr int OFF_V = OFF_K + 2 * KV_BYTES;
   static constexpr int OFF_BAR = OFF_V + 2 * KV_BYTES;
   static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
-  static constexpr int TMEM_COLS = 512;  // per tile: S/P at +0 (128 cols), O at +128; tile B at +256
+  // TMEM columns: S of whichever tile's turn it is, P of tiles A and B (bf16 pairs), O of both
+  static constexpr uint32_t TMEM_COLS = 512, TM_S = 0, TM_P = 128, TM_O = 256;
 };
 
 // Visible KV tile range [lo, hi) of a 128-row q tile starting at q0.
@@ -86,14 +95,16 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
   uint64_t* v_empty = bars + 7;       // [2]
   uint64_t* s_full = bars + 9;        // [2 tiles]
   uint64_t* p_full = bars + 11;       // [2 tiles]
-  uint64_t* o_done = bars + 13;       // [2 tiles]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* pv_done = bars + 13;      // [2 tiles]
+  uint64_t* s_free = bars + 15;       // 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  // heavy (late) query tiles first: better tail behaviour under the causal mask
-  const int pair = gridDim.x - 1 - blockIdx.x;
-  const int head = blockIdx.y, b = blockIdx.z;
+  // blocks by head, then by sequence and pair of query tiles, or the other way round: see sx_attn_fwd
+  const int head = blockIdx.x % p.Hq, rest = blockIdx.x / p.Hq, inner = p.batch_first ? p.B : p.pairs;
+  const int b = p.batch_first ? rest % inner : rest / inner;
+  const int pair = p.pairs - 1 - (p.batch_first ? rest / inner : rest % inner);
   const int kv_head = head / (p.Hq / p.Hk);
   const int v_head = kv_head / p.v_head_div;
   const int q0 = pair * 2 * ATT_BM;
@@ -135,15 +146,16 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
       mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 4);
-      mbar_init(&o_done[i], 1);
+      mbar_init(&pv_done[i], 1);
     }
+    mbar_init(s_free, 4);
     *s_abort = 0;
     mbar_fence_init();
     tma_prefetch_desc(&p.tmQ);
     tma_prefetch_desc(&p.tmK);
     tma_prefetch_desc(&p.tmV);
   }
-  if (warp == 1) tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+  if (warp == ATT_MMA_WARP) tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -157,125 +169,137 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
         : "memory");
   };
 
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (n_steps > 0 && elect_one()) {
-      mbar_expect_tx(q_full, 2 * Cfg::Q_BYTES);
-      tma5(sQ, &p.tmQ, q_full, q0, head, b);
-      tma5(sQ + Cfg::Q_BYTES, &p.tmQ, q_full, q0 + ATT_BM, head, b);
-      int j = 0;   // steps taken so far
-      for (int jt = first_step; jt >= 0; jt = next_step(jt), ++j) {
-        const int s = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        const int kv0 = jt * ATT_BN;
-        if (!mbar_wait(&k_empty[s], ph ^ 1, s_abort, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&k_full[s], Cfg::KV_BYTES);
-        tma5(sK + s * Cfg::KV_BYTES, &p.tmK, &k_full[s], kv0, kv_head, b);
-        if (!mbar_wait(&v_empty[s], ph ^ 1, s_abort, p.status, ST_TIMEOUT_PRODUCER)) break;
-        mbar_expect_tx(&v_full[s], Cfg::KV_BYTES);
-        tma5(sV + s * Cfg::KV_BYTES, &p.tmV, &v_full[s], kv0, v_head, b);
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (n_steps > 0 && elect_one()) {
-      constexpr uint32_t idesc_qk = umma_idesc_f16(ATT_BM, ATT_BN, 1, 0, 0);
-      constexpr uint32_t idesc_pv = umma_idesc_f16(ATT_BM, D, 1, 0, 1);
-      auto issue_qk = [&](int x, int j) {
-        const uint32_t a0 = smem_u32(sQ + x * Cfg::Q_BYTES), b0 = smem_u32(sK + (j & 1) * Cfg::KV_BYTES);
-        const uint32_t d = tmem_base + x * 256;
-#pragma unroll
-        for (int c = 0; c < D / 64; ++c)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f16_ss(d, umma_desc_sw128(a0 + c * (ATT_BM * 128) + k * 32, 16, 1024),
-                        umma_desc_sw128(b0 + c * (ATT_BN * 128) + k * 32, 16, 1024), idesc_qk, (c | k) ? 1u : 0u);
-        umma_commit(&s_full[x]);
-      };
-      // steps each tile takes part in: total, and so far (gives barrier parities and accumulate flags)
-      int total[2] = {0, 0}, cnt[2] = {0, 0};
-      for (int jt = first_step; jt >= 0; jt = next_step(jt))
-        for (int x = 0; x < 2; ++x) total[x] += on(x, jt) ? 1 : 0;
-      bool ok = mbar_wait(q_full, 0, s_abort, p.status, ST_TIMEOUT_MMA);
-      if (ok) ok = mbar_wait(&k_full[0], 0, s_abort, p.status, ST_TIMEOUT_MMA);
-      if (ok) {
-        tc_fence_after();
-        for (int x = 0; x < 2; ++x)
-          if (on(x, first_step)) issue_qk(x, 0);
-        umma_commit(&k_empty[0]);
-      }
-      int j = 0;   // steps taken so far; K / V ring slot and phase follow it
-      for (int jt = first_step; jt >= 0 && ok; ++j) {
-        const int nxt = next_step(jt);
-        const bool more = nxt >= 0;
-        if (!mbar_wait(&v_full[j & 1], (j >> 1) & 1, s_abort, p.status, ST_TIMEOUT_MMA)) { ok = false; break; }
-        if (more && !mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1, s_abort, p.status, ST_TIMEOUT_MMA)) {
-          ok = false;
-          break;
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == ATT_TMA_WARP) {
+      // ------------------------------------------------------------ TMA producer
+      if (n_steps > 0 && elect_one()) {
+        mbar_expect_tx(q_full, 2 * Cfg::Q_BYTES);
+        tma5(sQ, &p.tmQ, q_full, q0, head, b);
+        tma5(sQ + Cfg::Q_BYTES, &p.tmQ, q_full, q0 + ATT_BM, head, b);
+        int j = 0;   // steps taken so far
+        for (int jt = first_step; jt >= 0; jt = next_step(jt), ++j) {
+          const int s = j & 1;
+          const uint32_t ph = (j >> 1) & 1;
+          const int kv0 = jt * ATT_BN;
+          if (!mbar_wait(&k_empty[s], ph ^ 1, s_abort, p.status, ST_TIMEOUT_PRODUCER)) break;
+          mbar_expect_tx(&k_full[s], Cfg::KV_BYTES);
+          tma5(sK + s * Cfg::KV_BYTES, &p.tmK, &k_full[s], kv0, kv_head, b);
+          if (!mbar_wait(&v_empty[s], ph ^ 1, s_abort, p.status, ST_TIMEOUT_PRODUCER)) break;
+          mbar_expect_tx(&v_full[s], Cfg::KV_BYTES);
+          tma5(sV + s * Cfg::KV_BYTES, &p.tmV, &v_full[s], kv0, v_head, b);
         }
-        for (int x = 0; x < 2 && ok; ++x) {
-          if (on(x, jt)) {
-            if (!mbar_wait(&p_full[x], cnt[x] & 1, s_abort, p.status, ST_TIMEOUT_MMA)) { ok = false; break; }
+      }
+    } else if (warp == ATT_MMA_WARP) {
+      // ------------------------------------------------------------ MMA issuer
+      if (n_steps > 0 && elect_one()) {
+        constexpr uint32_t idesc_qk = umma_idesc_f16(ATT_BM, ATT_BN, 1, 0, 0);
+        constexpr uint32_t idesc_pv = umma_idesc_f16(ATT_BM, D, 1, 0, 1);
+        bool ok = mbar_wait(q_full, 0, s_abort, p.status, ST_TIMEOUT_MMA);
+        int cnt_a = 0, cnt_b = 0;                // products P V so far
+        // O_x += P_x V of the step in ring slot j & 1; `last`: nobody else multiplies this V
+        auto do_pv = [&](int x, int j, bool last) -> bool {
+          const int done = x ? cnt_b : cnt_a;
+          if (!mbar_wait(&v_full[j & 1], (j >> 1) & 1, s_abort, p.status, ST_TIMEOUT_MMA) ||
+              !mbar_wait(&p_full[x], done & 1, s_abort, p.status, ST_TIMEOUT_MMA)) return false;
+          tc_fence_after();
+          const uint32_t b0 = smem_u32(sV + (j & 1) * Cfg::KV_BYTES);
+          const uint32_t dO = tmem_base + Cfg::TM_O + x * 128, aP = tmem_base + Cfg::TM_P + x * 64;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            umma_f16_ts(dO, aP + k * 8, umma_desc_sw128(b0 + k * 2048, ATT_BN * 128, 1024), idesc_pv, (done | k) ? 1u : 0u);
+          umma_commit(&pv_done[x]);
+          if (last) umma_commit(&v_empty[j & 1]);
+          cnt_a += x ^ 1;
+          cnt_b += x;
+          return true;
+        };
+        // Products S = Q K^T in the order A, B, A, B ... of the tiles that take part in a step, two ahead of the products P V
+        int i = 0, x1 = 0, j1 = 0, x2 = 0, j2 = 0;
+        int j = 0;
+        for (int jt = first_step; jt >= 0 && ok; jt = next_step(jt), ++j) {
+          if (!mbar_wait(&k_full[j & 1], (j >> 1) & 1, s_abort, p.status, ST_TIMEOUT_MMA)) { ok = false; break; }
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            if (!ok || !on(x, jt)) continue;
+            if (i > 0 && !mbar_wait(s_free, (i - 1) & 1, s_abort, p.status, ST_TIMEOUT_MMA)) { ok = false; continue; }
             tc_fence_after();
-            const uint32_t b0 = smem_u32(sV + (j & 1) * Cfg::KV_BYTES);
-            const uint32_t dO = tmem_base + x * 256 + 128, aP = tmem_base + x * 256;
+            const uint32_t a0 = smem_u32(sQ + x * Cfg::Q_BYTES), b0 = smem_u32(sK + (j & 1) * Cfg::KV_BYTES);
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              umma_f16_ts(dO, aP + k * 8, umma_desc_sw128(b0 + k * 2048, ATT_BN * 128, 1024), idesc_pv,
-                          (cnt[x] | k) ? 1u : 0u);
-            ++cnt[x];
-            if (cnt[x] == total[x]) umma_commit(&o_done[x]);  // last step of this tile
+            for (int c = 0; c < D / 64; ++c)
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                umma_f16_ss(tmem_base + Cfg::TM_S, umma_desc_sw128(a0 + c * (ATT_BM * 128) + k * 32, 16, 1024),
+                            umma_desc_sw128(b0 + c * (ATT_BN * 128) + k * 32, 16, 1024), idesc_qk, (c | k) ? 1u : 0u);
+            umma_commit(&s_full[x]);
+            if (i >= 2) ok = do_pv(x2, j2, j1 != j2);
+            x2 = x1; j2 = j1; x1 = x; j1 = j;
+            ++i;
           }
-          if (more && on(x, nxt)) issue_qk(x, j + 1);
+          if (ok) umma_commit(&k_empty[j & 1]);
         }
-        umma_commit(&v_empty[j & 1]);
-        if (more) umma_commit(&k_empty[(j + 1) & 1]);
-        jt = nxt;
+        if (ok && i >= 2) ok = do_pv(x2, j2, j1 != j2);
+        if (ok && i >= 1) do_pv(x1, j1, true);
       }
     }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     // ------------------------------------------------------------ softmax warpgroups
-    const int x = (warp - 2) >> 2;          // which q tile
+    const int x = warp >> 2;                // which q tile
     const int qd = warp & 3;                // TMEM lane quadrant of this warp
     const int row = qd * 32 + lane;         // row inside the tile == TMEM lane
     const int q_idx = q0 + x * ATT_BM + row;
     const int offset = p.Skv - p.Sq;
     const uint32_t lane_addr = static_cast<uint32_t>(qd * 32) << 16;
-    const uint32_t tS = tmem_base + x * 256 + lane_addr;
-    const uint32_t tO = tS + 128;
+    const uint32_t tS = tmem_base + Cfg::TM_S + lane_addr, tP = tmem_base + Cfg::TM_P + x * 64 + lane_addr;
+    const uint32_t tO = tmem_base + Cfg::TM_O + x * 128 + lane_addr;
+    const int my_lo = x ? lo[1] : lo[0], my_hi = x ? hi[1] : hi[0];
+    auto mine = [&](int jt) -> bool {
+      if constexpr (!MASK) return true;
+      else return bm[(long long)(pair * 2 + x) * p.bm_kv_tiles + jt] != 0;
+    };
     int n_mine = 0;   // steps this tile takes part in
-    for (int jt = lo[x]; jt < hi[x]; ++jt) n_mine += on(x, jt) ? 1 : 0;
+    for (int jt = my_lo; jt < my_hi; ++jt) n_mine += mine(jt) ? 1 : 0;
     float m_used = -INFINITY;  // running (possibly stale) max, log2 domain
     float l = 0.f;
     bool ok = true;
-    int hi_k = p.Skv - 1;  // last visible key index for this row
-    if (p.causal) hi_k = min(hi_k, q_idx + offset);
-    const int lo_k = p.window > 0 ? q_idx + offset - p.window + 1 : INT_MIN;
-    for (int jt = lo[x], j = 0; jt < hi[x] && ok; ++jt) {
-      if (!on(x, jt)) continue;
-      const int kv0 = jt * ATT_BN;
+    // visible keys of this row: [lo_k, hi_k]
+    const int hi_k = p.causal ? min(p.Skv - 1, q_idx + offset) : p.Skv - 1;
+    const int lo_k = p.window > 0 ? (int)max((long long)q_idx + offset - p.window + 1, -1ll) : -1;
+    const int qt0 = q0 + x * ATT_BM;
+    // tiles from this one on have keys that some row does not see; before lo_full, too, where there is a window
+    const int hi_full = (min(p.Skv, p.causal ? qt0 + offset + 1 : p.Skv)) / ATT_BN;
+    const int lo_full = p.window > 0 ? (int)max((long long)qt0 + ATT_BM - 1 + offset - p.window + 1, 0ll) : 0;
+    const uint64_t scale2 = pack_f32x2(p.scale_log2, p.scale_log2);
+    for (int jt = my_lo, j = 0; jt < my_hi && ok; ++jt) {
+      if (!mine(jt)) continue;
       if (!mbar_wait_warp(&s_full[x], j & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
       tc_fence_after();
-      const int qt0 = q0 + x * ATT_BM;
-      const bool need_mask = (p.causal && kv0 + ATT_BN - 1 > qt0 + offset) || (kv0 + ATT_BN > p.Skv) ||
-                             (p.window > 0 && kv0 < qt0 + ATT_BM - 1 + offset - p.window + 1);
+      const bool need_mask = jt >= hi_full || jt * ATT_BN < lo_full;
       uint32_t r[ATT_BN];
 #pragma unroll
-      for (int c = 0; c < ATT_BN / 32; ++c) tmem_ld32(tS + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[c * 32]));
+      for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[c * 32]));
       tmem_ld_wait();
-      float mx = -INFINITY;
-      if (need_mask) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(s_free);      // the other tile's scores may follow
+      // four chains of three-operand maxima: one chain of 128 dependent ones takes as long as the exponentials of half a tile
+      float mc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int i = 0; i < ATT_BN; ++i) {
-          const int kv = kv0 + i;
-          if (kv > hi_k || kv < lo_k) r[i] = 0xff800000u;  // -inf
-          mx = fmaxf(mx, __uint_as_float(r[i]));
+      for (int c = 0; c < 4; ++c) {
+        if (need_mask) {
+          const int h = hi_k - jt * ATT_BN - c * 32, w = lo_k - jt * ATT_BN - c * 32;
+          const uint32_t seen = (h >= 31 ? 0xffffffffu : h < 0 ? 0u : (2u << h) - 1u) & (w <= 0 ? 0xffffffffu : w > 31 ? 0u : 0xffffffffu << w);
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (!(seen & (1u << i))) r[c * 32 + i] = 0xff800000u;  // -inf
         }
-      } else {
 #pragma unroll
-        for (int i = 0; i < ATT_BN; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
+        for (int i = 0; i < 32; i += 8)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mc[k] = fmax3(mc[k], __uint_as_float(r[c * 32 + i + 2 * k]), __uint_as_float(r[c * 32 + i + 2 * k + 1]));
       }
-      mx *= p.scale_log2;
+      const float mx = fmaxf(fmax3(mc[0], mc[1], mc[2]), mc[3]) * p.scale_log2;
       float alpha = 1.f;
       bool rescale = false;
       if ((mx > m_used + 8.f || m_used == -INFINITY) && mx != -INFINITY) {
@@ -284,40 +308,52 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
         m_used = mx;
       }
       l *= alpha;
-      const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
-      float lsum = 0.f;
-#pragma unroll
-      for (int i = 0; i < ATT_BN; i += 2) {
-        const float v0 = exp2f(fmaf(__uint_as_float(r[i]), p.scale_log2, -m_sub));
-        const float v1 = exp2f(fmaf(__uint_as_float(r[i + 1]), p.scale_log2, -m_sub));
-        const uint32_t pb = pack_bf16x2(v0, v1);
-        r[i / 2] = pb;
-        // row sum from the rounded values so that l matches what P V sees
-        lsum += __uint_as_float(pb << 16) + __uint_as_float(pb & 0xffff0000u);
-      }
-      l += lsum;
-      // s_full(j) was committed after P V of step j-1 (in-order pipe), so O and the S/P columns are ours
       if (j > 0 && __any_sync(0xffffffffu, rescale)) {
+        if (!mbar_wait_warp(&pv_done[x], (j - 1) & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
+        tc_fence_after();
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld32(tO + c * 32, o);
+        for (int c = 0; c < D / 16; ++c) {
+          uint32_t o[16];
+          tmem_ld16(tO + c * 16, o);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st32(tO + c * 32, o);
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st16(tO + c * 16, o);
         }
       }
-      tmem_st32(tS, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-      tmem_st32(tS + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+      const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
+      const uint64_t m2 = pack_f32x2(-m_sub, -m_sub);
+      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      auto exps = [&](int i0, int i1) {
+#pragma unroll
+        for (int i = i0; i < i1; i += 2) {
+          const uint64_t e = fma_f32x2(pack_f32x2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), scale2, m2);
+          float v0, v1;
+          unpack_f32x2(e, v0, v1);
+          const uint32_t pb = pack_bf16x2(exp2f(v0), exp2f(v1));
+          r[i / 2] = pb;
+          // row sum from the rounded values so that l matches what P V sees
+          add_bf16x2(ls[i & 2], ls[(i & 2) + 1], pb);
+        }
+      };
+      exps(0, 64);
+      // P V of the step before has read P
+      if (j > 0) {
+        if (!mbar_wait_warp(&pv_done[x], (j - 1) & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; break; }
+        tc_fence_after();
+      }
+      tmem_st32(tP, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+      exps(64, 128);
+      tmem_st32(tP + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[x]);
+      l += (ls[0] + ls[2]) + (ls[1] + ls[3]);
       ++j;
     }
     if (ok && n_mine > 0) {
-      if (mbar_wait_warp(&o_done[x], 0, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) {
+      if (mbar_wait_warp(&pv_done[x], (n_mine - 1) & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) {
         tc_fence_after();
         const float inv_l = l > 0.f ? 1.f / l : 0.f;
         const bool row_ok = q_idx < p.Sq;
@@ -356,7 +392,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
   tc_fence_before();
   __syncthreads();
   if (*s_abort) bounded_delay_ns(2000000);
-  if (warp == 1) {
+  if (warp == ATT_MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
@@ -399,7 +435,14 @@ extern "C" int sx_attn_fwd(const SxAttnArgs* a, cudaStream_t st) {
   p.bm_batch_stride = a->bm_batch_stride;
   p.bm_head_stride = a->bm_head_stride;
   p.bm_kv_tiles = (a->Skv + ATT_BN - 1) / ATT_BN;
-  dim3 grid((a->Sq + 2 * ATT_BM - 1) / (2 * ATT_BM), a->Hq, a->B);
+  // Blocks start heaviest first, so that the last ones to start are short: under a causal mask the last pair of query tiles walks the most keys.
+  // Over the whole batch where its keys and values stay in L2; otherwise one sequence after another, where the pairs of tiles that run at the
+  // same time share what they read.
+  p.pairs = (a->Sq + 2 * ATT_BM - 1) / (2 * ATT_BM);
+  p.batch_first = (long long)a->B * a->Skv * (a->Hk + v_heads) * a->D * 2 <= (64ll << 20);
+  const long long blocks = (long long)p.pairs * a->Hq * a->B;
+  if (blocks <= 0 || blocks > INT_MAX) return -4;
+  const dim3 grid((unsigned)blocks);
   if (a->D == 128) {
     static bool set = false;
     if (!set) {

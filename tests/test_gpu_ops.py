@@ -426,3 +426,33 @@ def test_attention_backward_tiles(H, Hk, Sq, Skv, causal, window):
         err, norm = (a.double() - e).norm(dim=-1), e.norm(dim=-1)
         bound = 2.0 ** -7 * norm + 2.0 ** -7 * norm.square().mean().sqrt() + 1e-4 + (delta if name == "dq" else 0.0)
         assert bool((err <= bound).all()), (name, (err / bound).max().item())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_attention_forward_of_a_batch_is_that_of_its_sequences(D):
+    """Keys and values of more than 64 MB take the blocks one sequence after another, a sequence by itself starts heads and tiles heaviest first: the
+    same bits, last partial tile and log-sum-exp included."""
+    B, Sq, Skv, H = 5, 300, 4096, 16
+    torch.manual_seed(D)
+    q = torch.randn(B, Sq, H, D, device="cuda").bfloat16()
+    k, v = (torch.randn(B, Skv, H, D, device="cuda").bfloat16() for _ in range(2))
+    o, lse = F_.attention_with_lse(q, k, v, causal=True)
+    for b in range(B):
+        ob, lb = F_.attention_with_lse(q[b:b + 1], k[b:b + 1], v[b:b + 1], causal=True)
+        assert torch.equal(ob[0], o[b]) and torch.equal(lb[0], lse[b])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("key", [0, 70, 127, 128, 300])
+def test_attention_forward_passes_nan_scores_on(key):
+    """A key of NaN makes every query that sees it NaN and leaves the others as they are; queries that see no key are zero."""
+    S, H = 333, 4
+    torch.manual_seed(key)
+    q, k, v = (torch.randn(1, S, H, 128, device="cuda").bfloat16() for _ in range(3))
+    want = F_.attention_with_lse(q, k, v, causal=True)[0]
+    k[:, key] = float("nan")
+    o = F_.attention_with_lse(q, k, v, causal=True)[0]
+    assert bool(o[:, key:].isnan().all()) and torch.equal(o[:, :key], want[:, :key])
+    none = F_.attention_with_lse(q, k[:, :100], v[:, :100], causal=True)[0]      # the first 233 queries come before every key
+    assert bool((none[:, :S - 100] == 0).all())
+    ops.check_status()
