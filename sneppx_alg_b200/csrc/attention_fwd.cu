@@ -17,8 +17,8 @@
 // shared) removes whole tiles from the walk: a step whose tile is masked for both query tiles is neither loaded nor
 // multiplied (block-sparse / flex-attention patterns at tile granularity).
 // Bound: exponentials (16 a cycle and SM: 2048 cycles for a step of both tiles, as many as its products take). B200, warm, before -> now:
-// [1, 4096, 32 / 8 heads, 128] causal 187 -> 127 us, [1, 8192, 8 / 2] full 288 -> 238, [8, 512, 28 / 4] causal 53 -> 43, [1, 16384, 32 / 8] causal
-// 2.28 -> 1.98 ms (1100 TFLOP/s, at the power cap).
+// [1, 4096, 32 / 8 heads, 128] causal 187 -> 130 us, [1, 8192, 8 / 2] full 288 -> 245, [8, 512, 28 / 4] causal 53 -> 44, [1, 16384, 32 / 8] causal
+// 2.28 -> 2.00 ms (1100 TFLOP/s, at the power cap).
 // Takes the place of the reference's SIMT flash-attention forward, GQA and block-sparse kernels
 // (kernel/cuda/attention_cuda.cu:37-328, 498-573, 1154-1230) and its empty "v3" kernel (:1262-1286).
 #include <limits.h>
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
       }
       const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
       const uint64_t m2 = pack_f32x2(-m_sub, -m_sub);
-      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      float lsum = 0.f;
       auto exps = [&](int i0, int i1) {
 #pragma unroll
         for (int i = i0; i < i1; i += 2) {
@@ -332,8 +332,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
           unpack_f32x2(e, v0, v1);
           const uint32_t pb = pack_bf16x2(exp2f(v0), exp2f(v1));
           r[i / 2] = pb;
-          // row sum from the rounded values so that l matches what P V sees
-          add_bf16x2(ls[i & 2], ls[(i & 2) + 1], pb);
+          // row sum from the rounded values so that l matches what P V sees, in the order of the keys
+          lsum += add_bf16x2(pb);
         }
       };
       exps(0, 64);
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[x]);
-      l += (ls[0] + ls[2]) + (ls[1] + ls[3]);
+      l += lsum;
       ++j;
     }
     if (ok && n_mine > 0) {

@@ -318,9 +318,11 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// a += low half of v, b += its high half: bf16 added to fp32 as it is
-__device__ __forceinline__ void add_bf16x2(float& a, float& b, uint32_t v) {
-  asm("{\n .reg .b16 lo, hi;\n mov.b32 {lo, hi}, %2;\n add.f32.bf16 %0, lo, %0;\n add.f32.bf16 %1, hi, %1;\n}" : "+f"(a), "+f"(b) : "r"(v));
+// low half of v + its high half in fp32
+__device__ __forceinline__ float add_bf16x2(uint32_t v) {
+  float r;
+  asm("{\n .reg .b16 lo, hi;\n mov.b32 {lo, hi}, %1;\n add.f32.bf16 %0, lo, %2;\n}" : "=f"(r) : "r"(v), "f"(__uint_as_float(v & 0xffff0000u)));
+  return r;
 }
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float r;
