@@ -46,7 +46,7 @@ typedef struct SxAttnArgs {
   float* lse;              // [B, Hq, Sq] natural-log LSE (forward: out; backward: in)
   const void* dO;          // backward only
   void* dQ; void* dK; void* dV;  // backward outputs (bf16), same strides as Q / K / V
-  float* dq_accum;         // backward scratch: [B, Sq, Hq, D] fp32, zero-filled by the call
+  float* dq_accum;         // backward scratch: B * Hq * ceil(Sq / 64) * 64 * D fp32, zero-filled by the call
   float* delta;            // backward scratch: [B, Hq, Sq] fp32
   long long q_row_stride, k_row_stride, v_row_stride, o_row_stride;
   long long q_batch_stride, k_batch_stride, v_batch_stride;

@@ -456,3 +456,21 @@ def test_attention_forward_passes_nan_scores_on(key):
     none = F_.attention_with_lse(q, k[:, :100], v[:, :100], causal=True)[0]      # the first 233 queries come before every key
     assert bool((none[:, :S - 100] == 0).all())
     ops.check_status()
+
+
+@pytest.mark.parametrize("S,H,Hk", [(1, 2, 1), (64, 3, 3), (65, 4, 2), (127, 2, 2), (128, 5, 1), (150, 4, 4), (193, 2, 1), (256, 3, 1), (513, 2, 2)])
+def test_attention_backward_stays_inside_its_accumulator(S, H, Hk):
+    """The last query tile may reach behind the accumulator, which holds multiples of 64 queries: nothing is added there, and the results are those
+    of 64 bits. Three roundings to bf16 lie between (P or dS, an operand's and the result's, 2^-9 each): 2^-7 of the norm."""
+    torch.manual_seed(S)
+    a, t = _attn_bwd_args(1, S, H, Hk)
+    n = H * ((S + 63) // 64 * 64) * 128
+    acc = torch.full((n + 64 * 128,), 7.0, device="cuda")
+    a.dq_accum = acc.data_ptr()
+    _lib.call("sx_attn_bwd", C.byref(a), stream())
+    ops.check_status()
+    assert bool((acc[n:] == 7.0).all())
+    want, _ = _attention64(t["q"], t["k"], t["v"], t["do"], True, 0)
+    for name, e in zip(("dq", "dk", "dv"), want[1:]):
+        if e.norm() > 1e-6:         # one key: no gradient of the scores
+            assert (t[name].double() - e).norm() <= 2.0 ** -7 * e.norm(), name
