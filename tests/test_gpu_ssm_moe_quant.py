@@ -118,6 +118,38 @@ def test_ssd_fused_chunk_kernel_matches_staged_path(monkeypatch):
     assert _rel(y1, y0) < 1e-2 and torch.equal(f1, f0)
 
 
+@pytest.mark.parametrize("H,G", [(1, 1), (2, 1), (3, 1), (5, 1), (24, 1), (9, 3), (16, 8)])
+def test_ssd_chunk_kernel_deals_heads_out(H, G):
+    """One chunk deals its heads out over many CTAs, odd numbers and a last short share among them; two hundred copies of it take one CTA a group:
+    the same bits. Against 64 bits: M is rounded to bf16 before its product and the sum to bf16 after it, 2^-9 of their magnitudes each."""
+    from sneppx_alg_b200.ops import _lib
+    from sneppx_alg_b200.ops._lib import c_int, c_ll, ptr, stream
+    torch.manual_seed(H + G)
+    Q, P, N, n = 128, 64, 128, 200
+    rows = torch.randn(Q, H * P + 2 * G * N, device="cuda").bfloat16()
+    state = torch.randn(H, P, N, device="cuda").bfloat16()
+    dt = torch.rand(H, Q, device="cuda") * 0.1
+    cs = torch.cumsum(-dt * (1 + 15 * torch.rand(H, 1, device="cuda")), -1)
+    D = torch.randn(H, device="cuda")
+    ys = []
+    for bc in (1, n):
+        u = rows.repeat(bc, 1)
+        W, B_, C_ = u.shape[1], u[:, H * P:], u[:, H * P + G * N:]
+        hp, cs_, dt_ = (t.repeat(bc, *[1] * (t.dim() - 1)) for t in (state, cs, dt))
+        y = torch.full((bc * Q, H * P), float("nan"), device="cuda").bfloat16()
+        _lib.call("sx_ssd_chunk_fwd", ptr(C_), c_ll(W), ptr(B_), c_ll(W), ptr(u), c_ll(W), ptr(hp), ptr(cs_), ptr(dt_), ptr(D), ptr(y), c_ll(bc),
+                  c_int(H), c_int(G), ptr(_lib.status_word("cuda")), stream())
+        ys.append(y.view(bc, Q, H, P))
+    ops.check_status()
+    assert bool((ys[1] == ys[0]).all())
+    x = rows[:, :H * P].double().view(Q, H, P)
+    Bm, Cm = (rows[:, o:o + G * N].double().view(Q, G, N).repeat_interleave(H // G, 1) for o in (H * P, H * P + G * N))
+    M = torch.einsum("lhn,shn->hls", Cm, Bm) * (cs.double()[:, :, None] - cs.double()[:, None]).exp().tril() * dt.double()[:, None]
+    terms = [torch.einsum("hls,shp->lhp", M, x), torch.einsum("lhn,hpn->lhp", Cm, state.double()) * cs.double().exp().t()[..., None], D.double()[:, None] * x]
+    size = torch.einsum("hls,shp->lhp", M.abs(), x.abs()) + terms[0].abs() + terms[1].abs() + terms[2].abs()
+    assert bool(((ys[0][0].double() - sum(terms)).abs() <= 2.0 ** -8 * size + 1e-6).all())
+
+
 def test_router_and_moe_layer():
     torch.manual_seed(0)
     T, d, E, k, Fd = 1000, 256, 16, 4, 192
