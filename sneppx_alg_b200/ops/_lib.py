@@ -177,16 +177,24 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_cuda = False   # a GPU and the library have been found: neither goes away again
+
+
 def available() -> bool:
-    """True when CUDA tensors can be served by the native library."""
-    if not torch.cuda.is_available():
-        return False
-    lib()  # raises if the library cannot be built / loaded: no silent fallback on a GPU box
+    """True when CUDA tensors can be served by the native library. Asked several times a launch: torch.cuda.is_available() reads the
+    environment each time (2 us)."""
+    global _cuda
+    if not _cuda:
+        if not torch.cuda.is_available():
+            return False
+        lib()  # raises if the library cannot be built / loaded: no silent fallback on a GPU box
+        _cuda = True
     return True
 
 
 def stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    """Current stream of the current device, without a Stream object around it (0.4 us instead of 3)."""
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def ptr(t) -> c_void_p:
@@ -195,8 +203,8 @@ def ptr(t) -> c_void_p:
 
 def status_word(device=None) -> torch.Tensor:
     """Per-device int32 word the waiting kernels write their timeout codes into."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
+    dev = None if device is None else device if isinstance(device, torch.device) else torch.device(device)
+    key = torch.cuda.current_device() if dev is None or dev.index is None else dev.index
     t = _status.get(key)
     if t is None:
         t = torch.zeros(4, dtype=torch.int32, device=torch.device("cuda", key))

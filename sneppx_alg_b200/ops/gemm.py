@@ -15,6 +15,7 @@ import threading
 import torch
 
 from . import _lib
+from . import debug as _dbg
 
 ACT = {None: 0, "none": 0, "gelu": 1, "silu": 2, "relu": 3, "relu2": 5}
 
@@ -202,11 +203,9 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, c=None, beta
         shape = (batch, M, N) if (batch > 1 or a.dim() == 3 or (b.dim() == 3 and tile_group is None) or
                                   k_ranges is not None) else (M, N)
         out = torch.empty(shape, dtype=odt, device=a.device)
-        from . import debug as _dbg
         if _dbg.ENABLED and tile_group is None and k_ranges is None:
             _dbg.poison_(out)      # debug-bounds mode: every element must be written by the kernel
     if tile_group is not None:
-        from . import debug as _dbg
         if _dbg.ENABLED:
             _dbg.check_indices(tile_group, -1, b.shape[0], _dbg.SITE_TILE_GROUP)
     assert out.stride(-1) == 1
@@ -214,22 +213,24 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, c=None, beta
     sD = out.stride(0) if out.dim() == 3 else 0
     args = _lib.SxGemmArgs()
     args.A, args.B, args.D = a.data_ptr(), b.data_ptr(), out.data_ptr()
-    args.C = c.data_ptr() if (c is not None and beta != 0.0) else None
-    args.bias = bias.float().data_ptr() if bias is not None else None
     if bias is not None:
         _keep = bias.float()
         args.bias = _keep.data_ptr()
     args.M, args.N, args.K, args.batch = M, N, K, batch
     args.lda, args.ldb, args.ldd = lda, ldb, ldd
-    args.ldc = c.stride(-2) if c is not None else 0
     args.strideA, args.strideB, args.strideD = sA, sB, sD
-    args.strideC = (c.stride(0) if (c is not None and c.dim() == 3) else 0)
-    args.a_mn, args.b_mn = int(a_mn), int(b_mn)
-    args.out_fp32 = int(out.dtype == torch.float32)
-    args.c_fp32 = int(c is not None and c.dtype == torch.float32)
+    args.a_mn, args.b_mn = a_mn, b_mn
+    args.out_fp32 = out.dtype == torch.float32
+    if c is not None:          # fields that are not set are zero
+        if beta != 0.0:
+            args.C = c.data_ptr()
+        args.ldc = c.stride(-2)
+        if c.dim() == 3:
+            args.strideC = c.stride(0)
+        args.c_fp32 = c.dtype == torch.float32
     if isinstance(act, (XIELU, SoftCap)):
         args.act, args.act_a, args.act_b = act.code, act.a, act.b
-    else:
+    elif act is not None:
         args.act = ACT[act] if not isinstance(act, int) else act
     args.alpha, args.beta = float(alpha), float(beta)
     if tile_group is not None:
@@ -240,9 +241,12 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, c=None, beta
         args.k_ranges = k_ranges.data_ptr()
         args.k_total = k_total
     args.status = _lib.status_word(a.device).data_ptr()
-    args.sm_limit = sm_limit
-    args.force_bn = force_bn
-    args.flags = 1 if _static.on else 0
+    if sm_limit:
+        args.sm_limit = sm_limit
+    if force_bn:
+        args.force_bn = force_bn
+    if _static.on:
+        args.flags = 1
     _lib.call("sx_gemm_bf16", C.byref(args), _lib.stream())
     return out
 
