@@ -38,6 +38,28 @@ typedef struct SxGemmArgs {
 } SxGemmArgs;
 int sx_gemm_bf16(const SxGemmArgs* args, cudaStream_t stream);
 
+// ------------------------------------------------------------------ mixer of a Mamba-2 block (mixer.cu)
+// zx [B, L, W = z | x | B | C | dt] bf16 contiguous, 16-byte aligned; conv_w [channels, K], conv_b bf16; dt_bias, a_log, D [H] fp32.
+// Chunks of Q tokens, nc of them a sequence, Lp = nc * Q.
+typedef struct SxMixerArgs {
+  const void* zx; const void* conv_w; const void* conv_b;
+  const float* dt_bias; const float* a_log; const float* D;
+  void* xbc;      // [B, Lp, channels] bf16: convolution output (forward: out; backward: in), as the next two
+  void* y;        // [B, Lp, H P] bf16: scan output
+  void* hprev;    // [B, nc, H, P, N] bf16: states entering the chunks
+  void* out;      // forward: [B, L, H P] bf16
+  const void* g;  // backward: gradient of out, contiguous
+  void* dzx;      // backward: [B, L, W] bf16
+  float* dwdb;    // backward: [(K + 1) * channels], taps' gradient by channel, then the bias'
+  float* part;    // backward: [3][B * nc][H] terms of the gradients of a_log, D and dt_bias
+  void* work; long long work_bytes;
+  int B, L, H, P, G, N, Q, K, fused;   // fused: sx_ssd_chunk_fwd (Q = N = 128, P = 64) for the scan's output
+  int* status;
+} SxMixerArgs;
+long long sx_mixer_workspace(const SxMixerArgs* args, int backward);
+int sx_mixer_fwd(const SxMixerArgs* args, cudaStream_t stream);
+int sx_mixer_bwd(const SxMixerArgs* args, cudaStream_t stream);
+
 // ------------------------------------------------------------------ A1 / A2 flash attention
 // Q [B, Sq, Hq, D], K [B, Skv, Hk, D], V [B, Skv, Hk / v_head_div, D], O [B, Sq, Hq, D]; bf16; each given as a
 // base pointer plus token (row) and batch strides in elements, so slices of a fused QKV buffer work in place.

@@ -129,6 +129,15 @@ class SxSsdArgs(C.Structure):
     ]
 
 
+class SxMixerArgs(C.Structure):
+    _fields_ = [
+        ("zx", c_void_p), ("conv_w", c_void_p), ("conv_b", c_void_p), ("dt_bias", c_void_p), ("a_log", c_void_p), ("D", c_void_p),
+        ("xbc", c_void_p), ("y", c_void_p), ("hprev", c_void_p), ("out", c_void_p), ("g", c_void_p), ("dzx", c_void_p), ("dwdb", c_void_p),
+        ("part", c_void_p), ("work", c_void_p), ("work_bytes", c_ll), ("B", c_int), ("L", c_int), ("H", c_int), ("P", c_int), ("G", c_int),
+        ("N", c_int), ("Q", c_int), ("K", c_int), ("fused", c_int), ("status", c_void_p),
+    ]
+
+
 class SxMambaStepArgs(C.Structure):
     _fields_ = [
         ("x", c_void_p), ("res_in", c_void_p), ("res_out", c_void_p), ("norm_w", c_void_p), ("hn", c_void_p), ("in_w", c_void_p),

@@ -11,12 +11,14 @@ of constant dt, B, C.
 """
 from __future__ import annotations
 
+import ctypes
 import os
 
 import torch
 import torch.nn.functional as F
 
 from . import _lib
+from . import debug as _dbg
 from ._lib import c_int, c_ll, ptr, stream
 from .gemm import bmm, gemm
 
@@ -530,8 +532,33 @@ class _MixerFn(torch.autograd.Function):
     and backward. The stages are the ones above; as one node they share buffers: the padded convolution output is what the scan reads in
     place, every gradient is written into its columns of the projection's gradient, and nothing is padded, split or joined in between.
     A block with its projections and norm, forward and backward: 122 -> 49 launches; width 768, 4 x 500 tokens 2.67 -> 1.59 ms (most of it
-    launches from the host), width 2560, 8192 tokens 4.37 -> 3.95 ms. Kept for backward: the projection's output, the convolution's output,
+    launches from the host), width 2560, 8192 tokens 4.37 -> 3.95 ms. Sizes that csrc/mixer.cu takes launch from one native call each way
+    (width 768: 1.26 -> 0.78 ms). Kept for backward: the projection's output, the convolution's output,
     the scan's output and the chunk-entry states."""
+
+    @staticmethod
+    def _native(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D, sizes):
+        """Arguments of the whole sequence as one call (csrc/mixer.cu), for the sizes that it takes; else None."""
+        H, P, G, N, Q = sizes
+        if Q not in (64, 128) or P % 64 or N % 64 or _dbg.ENABLED:
+            return None
+        a = _lib.SxMixerArgs()
+        a.zx, a.xbc, a.y, a.hprev = zx.data_ptr(), xbc.data_ptr(), y.data_ptr(), Hprev.data_ptr()
+        a.conv_w, a.conv_b, a.dt_bias, a.a_log, a.D = (t.data_ptr() for t in (conv_w, conv_b, dt_bias, A_log, D))
+        a.B, a.L = zx.shape[:2]
+        a.H, a.P, a.G, a.N, a.Q, a.K = H, P, G, N, Q, conv_w.shape[1]
+        a.fused = Q == 128 and N == 128 and P == 64 and os.environ.get("SX_SSD_FUSED", "1") != "0"
+        a.status = _lib.status_word(zx.device).data_ptr()
+        return a
+
+    @staticmethod
+    def _native_call(a, name, backward, device):
+        size = _lib.lib().sx_mixer_workspace
+        size.restype = _lib.c_ll
+        a.work_bytes = size(ctypes.byref(a), c_int(backward))
+        work = torch.empty(a.work_bytes, dtype=torch.uint8, device=device)
+        a.work = work.data_ptr()
+        _lib.call(name, ctypes.byref(a), stream())
 
     @staticmethod
     def _prep(zx, dt_bias, A_log, H, Q):
@@ -564,6 +591,15 @@ class _MixerFn(torch.autograd.Function):
         Lp, di, K, dev, cdt = nc * Q, H * P, conv_w.shape[1], zx.device, zx.dtype
         C = di + 2 * G * N
         xbc = torch.empty(B_, Lp, C, dtype=cdt, device=dev)
+        y, Hprev = torch.empty(B_, Lp, di, dtype=cdt, device=dev), torch.empty(B_, nc, H, P, N, dtype=cdt, device=dev)
+        a = _MixerFn._native(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D, sizes)
+        if a is not None:
+            out = torch.empty(B_, L, di, dtype=cdt, device=dev)
+            a.out = out.data_ptr()
+            _MixerFn._native_call(a, "sx_mixer_fwd", 0, dev)
+            ctx.save_for_backward(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D)
+            ctx.sizes = sizes
+            return out
         if Lp > L:
             xbc[:, L:].zero_()
         src = zx[..., di:di + C]
@@ -576,7 +612,6 @@ class _MixerFn(torch.autograd.Function):
         S = gemm(xw, Bg, a_mn=True, b_mn=True, out_dtype=torch.float32)
         Hprev, _ = _state_fwd(S.view(B_, nc, H, P, N), tot, None, cdt)
         if Q == 128 and N == 128 and P == 64 and os.environ.get("SX_SSD_FUSED", "1") != "0":
-            y = torch.empty(B_, Lp, di, dtype=cdt, device=dev)
             Cm, Bm = xbc[..., di + G * N:], xbc[..., di:]
             _lib.call("sx_ssd_chunk_fwd", ptr(Cm), c_ll(C), ptr(Bm), c_ll(C), ptr(xbc), c_ll(C), ptr(Hprev), ptr(csh), ptr(dth), ptr(D), ptr(y),
                       c_ll(B_ * nc), c_int(H), c_int(G), _lib.c_void_p(_lib.status_word(dev).data_ptr()), stream())
@@ -601,6 +636,13 @@ class _MixerFn(torch.autograd.Function):
         f32 = torch.float32
         g = g.contiguous()
         dzx = torch.empty(B_, L, W, dtype=cdt, device=dev)
+        a = _MixerFn._native(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D, ctx.sizes)
+        if a is not None:
+            dwdb, part = torch.empty((K + 1) * C, dtype=f32, device=dev), torch.empty(3, B_ * nc, H, dtype=f32, device=dev)
+            a.g, a.dzx, a.dwdb, a.part = g.data_ptr(), dzx.data_ptr(), dwdb.data_ptr(), part.data_ptr()
+            _MixerFn._native_call(a, "sx_mixer_bwd", 1, dev)
+            dA, dD, dbias = part.sum(1)
+            return dzx, dwdb[: C * K].view(C, K).to(cdt), dwdb[C * K:].to(cdt), dbias, dA, dD, None
         dy = torch.empty(B_, Lp, di, dtype=cdt, device=dev)
         if Lp > L:
             dy[:, L:].zero_()

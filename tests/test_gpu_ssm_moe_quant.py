@@ -346,6 +346,38 @@ def test_mamba2_mixer(B, L, H, P, G, N, K, monkeypatch):
             assert err(grads[0][..., lo:hi], wgrad[0][..., lo:hi]) < 0.028, (name, err(grads[0][..., lo:hi], wgrad[0][..., lo:hi]))
 
 
+@pytest.mark.parametrize("B,L,H,P,G,N,fused", [(1, 33, 8, 64, 1, 64, True), (2, 64, 8, 64, 2, 128, True), (1, 65, 8, 64, 1, 128, True), (3, 200, 24, 64, 3, 128, True),
+                                               (2, 128, 8, 128, 1, 64, True), (1, 300, 16, 64, 2, 128, False), (40, 128, 8, 64, 1, 128, True)])
+def test_mixer_in_one_call_is_the_mixer_by_entry_points(monkeypatch, B, L, H, P, G, N, fused):
+    """Chunks of 64 and 128, ragged tails, one and several groups, the fused and the staged output: the same launches in the same order. The same bits
+    but where sums are added atomically (the decay's gradient over a state, the taps'), two orders of which are 2^-16 of the sums' terms apart and
+    then rounded to bf16 (2^-8 of a value between the two)."""
+    from sneppx_alg_b200.ops import _lib
+    monkeypatch.setenv("SX_SSD_FUSED", "1" if fused else "0")
+    torch.manual_seed(L + H)
+    di, C = H * P, H * P + 2 * G * N
+    zx = torch.randn(B, L, di + C + H, device="cuda")
+    zx[..., di + C:] -= 2
+    args = [zx.bfloat16(), (0.5 * torch.randn(C, 4, device="cuda")).bfloat16(), (0.1 * torch.randn(C, device="cuda")).bfloat16(),
+            torch.randn(H, device="cuda") - 1, torch.log(1 + 15 * torch.rand(H, device="cuda")), torch.randn(H, device="cuda")]
+    args = [t.requires_grad_() for t in args]
+    assert ssm.mixer_ok(*args, H, P, G, N)
+    g = torch.randn(B, L, di, device="cuda").bfloat16()
+    got = []
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(ssm._MixerFn, "_native", staticmethod(lambda *a: None))
+        n = _lib.launch_count
+        y = ssm.mamba2_mixer(*args, H, P, G, N)
+        assert (_lib.launch_count - n == 1) == native
+        got.append((y, *torch.autograd.grad(y, args, g)))
+    ops.check_status()
+    (y1, z1, *rest1), (y0, z0, *rest0) = got
+    assert torch.equal(y1, y0) and torch.equal(z1[..., :di + C], z0[..., :di + C])
+    close = lambda a, b: bool(((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + 2.0 ** -12 * b.float().abs().max()).all())  # noqa: E731
+    assert close(z1, z0) and all(a.dtype == b.dtype and close(a, b) for a, b in zip(rest1, rest0))
+
+
 @pytest.mark.parametrize("C,L,Lp,wide", [(64, 1, 1, False), (1536, 1, 1, True), (320, 7, 7, True), (320, 7, 8, True), (64, 33, 64, False)])
 def test_gate_mul_padded_rows(C, L, Lp, wide):
     """Dense and wider gradients of z, y with rows behind each sequence that are neither read nor written. 32-bit arithmetic and one bf16 rounding;
