@@ -68,6 +68,28 @@ __device__ __forceinline__ float block_max(float v, float* red) {
   return red[32];
 }
 
+// Launch of a kernel that begins with after_predecessor(): its blocks may be set up while the kernel before it on the stream still runs (programmatic
+// dependent launch), so that what lies between the two is the wait, not a launch. In a decode step of an 8B-width model half of the kernels take
+// 2 to 3 us, most of it that.
+__device__ __forceinline__ void after_predecessor() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the same for the kernel after this one
+  asm volatile("griddepcontrol.wait;" ::: "memory");                // all that kernels before this one wrote is there
+}
+template <typename... K, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<K>(args)...);
+}
+
 // Launch shape of a kernel whose thread takes one of `items` pieces of a token: block (pieces, tokens), grid (tokens, pieces). Tokens of fewer
 // than 128 pieces share a CTA, so that it has 8 warps (one token each left 32 threads to a CTA: rotating 131072 tokens of one head of 16 took
 // 72 us, 6 so). Larger ones go over several CTAs, of 128 threads where tokens are few, because a thread that takes pieces one after another

@@ -30,7 +30,7 @@ template <int V, bool RES>
 __global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in,
                                                            const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                                            __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd, int d, float eps) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a dependent launch may start its prologue
+  after_predecessor();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const int nvec = d >> 3, t = threadIdx.x;
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_long_kernel(const __nv_bfloat
                                                                const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                                                __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd, int d,
                                                                float eps) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  after_predecessor();
   __shared__ float red[33];
   const long long row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * d;
@@ -378,7 +378,7 @@ __device__ __forceinline__ float gate_act_grad(float g, int act) {
 
 __global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long long T,
                                int F, int act) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a dependent launch may start its prologue
+  after_predecessor();
   const int fv = F >> 3;
   const long long total = T * fv;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
@@ -426,8 +426,8 @@ extern "C" int sx_rmsnorm_fwd(const void* x, const void* res_in, const void* w, 
   if (T == 0) return 0;
   const int nvec = d / 8;
   auto run = [&](auto kern, int threads) {
-    kern<<<(unsigned)T, threads, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)res_in, (const __nv_bfloat16*)w, (__nv_bfloat16*)y,
-                                          (__nv_bfloat16*)res_out, rstd, d, eps);
+    launch_dependent(kern, (unsigned)T, threads, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res_in, (const __nv_bfloat16*)w,
+                     (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, rstd, d, eps);
   };
   auto per = [&](int v) { return ((nvec + v - 1) / v + 31) / 32 * 32; };
   // 256 threads up to 4096 as long as they have a vector each (a thread's share then does not depend on how the row divides), more threads
@@ -499,7 +499,7 @@ extern "C" int sx_glu_fwd(const void* gu, void* h, long long T, int F, int act, 
   if (T == 0) return 0;
   const long long total = T * (F / 8);
   const int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-  glu_fwd_kernel<<<blocks, 256, 0, st>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)h, T, F, act);
+  launch_dependent(glu_fwd_kernel, blocks, 256, 0, st, (const __nv_bfloat16*)gu, (__nv_bfloat16*)h, T, F, act);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(PA_TILE) paged_decode_kernel(
 
 __global__ void paged_merge_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part,
                                    __nv_bfloat16* __restrict__ out, long long out_row_stride, int Hq, int D, int nsplit) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a dependent launch may start its prologue
+  after_predecessor();
   const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const long long base = ((long long)b * Hq + h) * nsplit;
   float m = -INFINITY;
@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(512) kv_append_vec8_kernel(__nv_bfloat16* __re
                                                              const int* __restrict__ pos, const int* __restrict__ slot,
                                                              __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int T,
                                                              int Hq, int Hkv, int D, int rotate) {
+  after_predecessor();
   const int t = blockIdx.x * blockDim.y + threadIdx.y, half = D >> 1, per = D >> 4, items = (Hq + 2 * Hkv) * per;
   if (t >= T) return;
   const int p = pos[t], sl = slot[t];
@@ -265,7 +266,7 @@ __global__ void kv_append_kernel(__nv_bfloat16* __restrict__ qkv, long long row_
 // Shared with the tensor-core decode kernel (paged_attn_tc.cu).
 void paged_merge_launch(const float* o_part, const float* ml_part, void* out, long long out_row_stride, int B, int Hq,
                         int D, int nsplit, cudaStream_t st) {
-  paged_merge_kernel<<<dim3(B, Hq), D, 0, st>>>(o_part, ml_part, (__nv_bfloat16*)out, out_row_stride, Hq, D, nsplit);
+  launch_dependent(paged_merge_kernel, dim3(B, Hq), D, 0, st, o_part, ml_part, (__nv_bfloat16*)out, out_row_stride, Hq, D, nsplit);
 }
 
 }  // namespace sx
@@ -316,8 +317,8 @@ extern "C" int sx_kv_append(void* qkv, long long row_stride, const float* cos_t,
       (!rotate || (aligned(cos_t) && aligned(sin_t)))) {
     dim3 grid, block;
     token_grid(T, (Hq + 2 * Hkv) * (D / 16), &grid, &block);
-    kv_append_vec8_kernel<<<grid, block, 0, st>>>((__nv_bfloat16*)qkv, row_stride, cos_t, sin_t, pos, slot, (__nv_bfloat16*)k_cache,
-                                                  (__nv_bfloat16*)v_cache, T, Hq, Hkv, D, rotate);
+    launch_dependent(kv_append_vec8_kernel, grid, block, 0, st, (__nv_bfloat16*)qkv, row_stride, cos_t, sin_t, pos, slot, (__nv_bfloat16*)k_cache,
+                     (__nv_bfloat16*)v_cache, T, Hq, Hkv, D, rotate);
     return cudaGetLastError() == cudaSuccess ? 0 : -11;
   }
   const int blocks = (int)((warps * 32 + 255) / 256);

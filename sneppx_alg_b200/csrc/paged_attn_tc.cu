@@ -11,6 +11,7 @@
 // query heads of the KV head and there are no shuffles on the score path, which is what bounded the SIMT kernel
 // (paged_attn.cu); here the kernel is bound by the TMA stream. Splits are merged by paged_merge_kernel.
 // Serves the role of the reference's paged decode kernels (kernel/cuda/attention_cuda.cu:602-690).
+#include "common.cuh"
 #include "tc_common.cuh"
 #include "tmap.h"
 #include "sx_api.h"
@@ -133,6 +134,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) paged_decode_tc_kernel(const __
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tS = tmem_base, tO = tmem_base + 16;
+  // No launch_dependents: the merge kernel and, behind it, the next product's blocks would take their places on SMs that are done first and draw
+  // weights against the cache stream (a decode step of 48 sequences: 15.0 ms, 14.4 so).
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   auto tma5 = [](void* dst, const CUtensorMap* m, uint64_t* bar, int c1, int c2, int c3, int c4) {
     asm volatile(
@@ -443,7 +447,7 @@ extern "C" int sx_paged_decode_tc(const void* q, long long q_row_stride, const v
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   }
   const long long items = (long long)B * Hkv * nsplit;
-  auto run = [&](auto kern) { kern<<<(unsigned)(items < sms ? items : sms), PT_THREADS, PT_SMEM, st>>>(p); };
+  auto run = [&](auto kern) { launch_dependent(kern, (unsigned)(items < sms ? items : sms), PT_THREADS, PT_SMEM, st, p); };
   items <= (long long)PT_FEW_ITEMS * sms ? run(paged_decode_tc_kernel<true>) : run(paged_decode_tc_kernel<false>);
   paged_merge_launch(o_part, ml_part, out, out_row_stride, B, Hq, D, nsplit, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
