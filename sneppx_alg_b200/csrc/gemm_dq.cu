@@ -14,8 +14,8 @@
 //   promotion  acc[row][m] += scale[row, k-block] * partial in fp32 registers; the scale belongs to the thread's own row (TMEM lane),
 //              so it is one multiply-add per value. Products are therefore exact and nothing is rounded to bf16 before the output.
 // Two CTAs share an SM up to 32 rows of X, so that one converts while the other waits.
-// Measured (B200, graph replay, cold weights), int4 [28672, 4096] at 1 / 16 / 32 / 64 / 128 rows: 24 / 24 / 27 / 33 / 58 us, [4096, 14336]
-// 15 / 15 / 16 / 16 / 26 us; 28 / 28 / 30 / 39 / 62 and 16 / 17 / 17 / 19 / 28 us when operands were moved to uniform registers for each
+// Measured (B200, graph replay, cold weights), int4 [28672, 4096] at 1 / 16 / 32 / 64 / 128 rows: 24 / 24 / 27 / 33 / 51 us, [4096, 14336]
+// 15 / 15 / 16 / 16 / 23 us; 28 / 28 / 30 / 39 / 62 and 16 / 17 / 17 / 19 / 28 us when operands were moved to uniform registers for each
 // MMA (tc_common.cuh), 203 / 199 / 199 / 199 / 201 and 361 / 354 / 353 / 353 / 356 us when 128 x 128 output tiles left most SMs idle and four
 // converter warps wrote scaled bf16 tiles to shared memory. The floor (packed weights at copy bandwidth) is 9 and 4.5 us. K of 128 or 256 with
 // more than one wave of tiles: gemm_dq_short.cu.
@@ -51,13 +51,19 @@ template <int BT>
 struct DqCfg {
   static constexpr int PW = BT >= 64 ? 8 : 4;           // from 64 columns on two warps per lane quadrant, half of the columns each
   static constexpr int COLS = BT / (PW / 4);            // columns of a promotion thread
-  static constexpr int NG = BT == 64 ? 4 : 2;           // converter groups = A buffers
+  static constexpr int NG = BT == 64 ? 4 : 2;           // converter groups
+  // A buffers, k-block i in buffer i % NA: an even number, so that a buffer and its barriers belong to one group and one MMA warp (a phase's parity
+  // says nothing to a warp that missed the phase before). Two for each group at 128 rows, whose converters otherwise wait for the MMA of their
+  // last k-block: 58 -> 51 us. Up to 32 rows TMEM has room for three in two CTAs; with barriers for each group that gained nothing (24 us).
+  static constexpr int NA = BT >= 64 ? 4 : 2;
+  static_assert(NA % NG == 0, "a buffer belongs to one group");
   static constexpr int MMA_WARP = PW + 4 * NG;          // two MMA warps, then the TMA warp
   static constexpr int THREADS = 32 * (MMA_WARP + 3);
   static constexpr int CTAS = BT <= 32 ? 2 : 1;         // resident per SM
   static constexpr int X_BYTES = BT * DQ_BK * 2;        // X of one k-block: two 64-column slabs
-  static constexpr int TM_D = NG * 64;                  // TMEM: A buffers of 64 columns, then two accumulators
+  static constexpr int TM_D = NA * 64;                  // TMEM: A buffers of 64 columns, then two accumulators
   static constexpr int TMEM_COLS = TM_D + 2 * BT <= 256 ? 256 : 512;
+  static_assert(CTAS * TMEM_COLS <= 512 && TM_D + 2 * BT <= TMEM_COLS, "TMEM");
   static constexpr int BUDGET = CTAS == 2 ? 98304 : 196608;
 };
 
@@ -95,9 +101,9 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.stages * STAGE_BYTES);
   uint64_t* full = bars;
   uint64_t* empty = bars + DQ_MAX_STAGES;                             // four converter warps and one MMA warp a k-block
-  uint64_t* a_full = bars + 2 * DQ_MAX_STAGES;                        // [NG] four converter warps
-  uint64_t* a_empty = a_full + Cfg::NG;                               // [NG] MMA
-  uint64_t* d_full = a_empty + Cfg::NG;                               // [2] MMA
+  uint64_t* a_full = bars + 2 * DQ_MAX_STAGES;                        // [NA] four converter warps
+  uint64_t* a_empty = a_full + Cfg::NA;                               // [NA] MMA
+  uint64_t* d_full = a_empty + Cfg::NA;                               // [2] MMA
   uint64_t* d_empty = d_full + 2;                                     // [2] promotion warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -118,7 +124,7 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 5 * KPS);
     }
-    for (int i = 0; i < Cfg::NG; ++i) {
+    for (int i = 0; i < Cfg::NA; ++i) {
       mbar_init(&a_full[i], 4);
       mbar_init(&a_empty[i], 1);
     }
@@ -170,15 +176,16 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
       const uint32_t tD = tmem_base + Cfg::TM_D + buf * BT;
       const uint32_t sm0 = smem_u32(smem);
       int s = INT4 ? 0 : buf;                                          // stage and its phase, followed without a division
-      uint32_t sph = 0, dph = 1;
+      uint32_t sph = 0, dph = 1, aph = 0;
+      int g = buf;                                                     // A buffer and its phase
       for (int i = buf; i < nk; i += 2) {
-        const int g = i % Cfg::NG;
+        if (g >= Cfg::NA) { g -= Cfg::NA; aph ^= 1; }
         if (s >= p.stages) { s -= p.stages; sph ^= 1; }
         // a_full follows full of the stage (the converters read it), but the X tile arrived through the async proxy: wait for it here too
         if (!mbar_wait(&full[s], sph, s_abort, p.status, ST_TIMEOUT_MMA)) break;
         if (!mbar_wait(&d_empty[buf], dph, s_abort, p.status, ST_TIMEOUT_MMA)) break;
         const uint64_t x0 = umma_desc_sw128(sm0 + s * STAGE_BYTES + DQ_W_BYTES + (INT4 ? buf : 0) * Cfg::X_BYTES, 16, 1024);
-        if (!mbar_wait(&a_full[g], (i / Cfg::NG) & 1, s_abort, p.status, ST_TIMEOUT_MMA)) break;
+        if (!mbar_wait(&a_full[g], aph, s_abort, p.status, ST_TIMEOUT_MMA)) break;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 8; ++k)
@@ -187,6 +194,7 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
         umma_commit(&a_empty[g]);
         umma_commit(&empty[s]);
         s += INT4 ? 1 : 2;
+        g += 2;
         dph ^= 1;
       }
     }
@@ -194,10 +202,11 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
     // ------------------------------------------------------------ converters: group g takes the k-blocks i with i % NG == g
     const int g = (warp - Cfg::PW) >> 2, q = warp & 3;                // q: TMEM lane quadrant of this warp (PW is a multiple of 4)
     const int row = q * 32 + lane;
-    const uint32_t tA = tmem_base + g * 64 + (static_cast<uint32_t>(q * 32) << 16);
-    int s = g / KPS;
-    uint32_t sph = 0;
-    for (int i = g, n = 0; i < nk; i += Cfg::NG, ++n, s += Cfg::NG / KPS) {
+    int s = g / KPS, ab = g;
+    uint32_t sph = 0, aph = 1;
+    for (int i = g; i < nk; i += Cfg::NG, s += Cfg::NG / KPS, ab += Cfg::NG) {
+      if (ab >= Cfg::NA) { ab -= Cfg::NA; aph ^= 1; }
+      const uint32_t tA = tmem_base + ab * 64 + (static_cast<uint32_t>(q * 32) << 16);
       while (s >= p.stages) { s -= p.stages; sph ^= 1; }
       if (!mbar_wait_warp(&full[s], sph, s_abort, p.status, ST_TIMEOUT_CONVERT)) break;
       const uint8_t* src = smem + s * STAGE_BYTES + row * 128;
@@ -215,7 +224,7 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
           if (lane == 0) mbar_arrive(&empty[s]);
         }
         if (h == 0) {
-          ok = mbar_wait_warp(&a_empty[g], (n & 1) ^ 1, s_abort, p.status, ST_TIMEOUT_CONVERT);
+          ok = mbar_wait_warp(&a_empty[ab], aph, s_abort, p.status, ST_TIMEOUT_CONVERT);
           if (!ok) break;
           tc_fence_after();
         }
@@ -241,7 +250,7 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&a_full[g]);
+      if (lane == 0) mbar_arrive(&a_full[ab]);
     }
   } else {
     // ------------------------------------------------------------ promotion: thread = weight row (TMEM lane)

@@ -172,6 +172,20 @@ def test_dequant_gemm_of_many_short_tiles(mode, M, N, K, bias):
     assert bool(((y[M - 100:].double() - few.double()).abs() <= few.double().abs() * 2.0 ** -7 + mag[-100:] * 2.0 ** -19).all())
 
 
+@pytest.mark.parametrize("mode,M,N,K", [("int4", 16, 28672, 4096), ("int4", 32, 4096, 14336), ("int4", 1, 3584, 18944), ("int4", 128, 6144, 4096),
+                                        ("fp8", 16, 4096, 14336), ("fp8", 32, 6144, 4096), ("fp8", 100, 4096, 4096)])
+def test_dequant_gemm_repeats_itself(mode, M, N, K):
+    """Converters, MMA and promotion warps run ahead of one another by up to the buffers between them, how far depends on what the memory does: calls
+    on cold weights, one behind the other, give the same bits each time, and those of the dequantised product (one rounding of 32-bit sums)."""
+    x, q, s, wd, _ = _dequant_case(mode, M, N, K, False)
+    want = (x.double() @ wd.double().t())
+    ws = [(q.clone(), s.clone()) for _ in range(max(2, (200 << 20) // q.numel()))]
+    ys = [quant.gemm_dequant(x, *w, mode) for _ in range(3) for w in ws]
+    ops.check_status()
+    assert (ys[0].double() - want).norm() < 2.0 ** -8 * want.norm()
+    assert all(torch.equal(y, ys[0]) for y in ys)
+
+
 def test_dequant_gemm_of_short_rows_keeps_up_with_its_output():
     """16384 x 4096 outputs of K = 128 are bound by writing 134 MB: two to four times a copy's time, ten when every tile was a CTA of its own."""
     x, q, s, _, _ = _dequant_case("int4", 16384, 4096, 128, False)
