@@ -5,6 +5,7 @@
 // The reference's conv kernels limit L to one thread block (algorithms/hss/cuda/hss_cuda_extended.cu:208-226)
 // and its Mamba-2 block copies instead of convolving (kernel/arch/mamba2.c:82-84).
 #include "common.cuh"
+#include "tc_common.cuh"
 #include "sx_api.h"
 
 namespace sx {
@@ -49,6 +50,7 @@ template <int V> __device__ __forceinline__ void conv_ld(const __nv_bfloat16* p,
 template <int V> __device__ __forceinline__ void conv_st(__nv_bfloat16* p, const float (&f)[V]) {
   *reinterpret_cast<typename ConvVec<V>::T*>(p) = conv_pack(f);
 }
+__device__ __forceinline__ uint64_t bf16x2_f32x2(uint32_t v) { return pack_f32x2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
 template <int K, int V>
 __device__ __forceinline__ void conv_taps(const __nv_bfloat16* w, int c, float (&wv)[K][V]) {
   if (K == 4 && (reinterpret_cast<uintptr_t>(w) & 7) == 0) {   // a channel's four taps are 8 contiguous bytes
@@ -142,120 +144,135 @@ __global__ void __launch_bounds__(256, 3) conv1d_fwd_kernel(const __nv_bfloat16*
   }
 }
 
-// dx and per-CTA partials of dw / dbias. A CTA is 32 channel groups of V (one per lane: 64 V contiguous bytes per row) by 8 runs of
-// CONV_BTL consecutive positions (one per warp). A thread walks its run once: the last K inputs and the last K pre-activation gradients
-// slide through registers, so every x and dy value is loaded once (plus the K-1 row overlap between runs) and dx is stored once. As above
-// warps count more than wide loads: two channels a thread keep the kernel near 64 registers, four CTAs an SM. [8192, 7168]: 247 us, 265
-// with four channels and two CTAs an SM (54 us at copy bandwidth): the instructions of a row bound it; three taps 247 and 263.
+// dx and per-CTA partials of dw / dbias. A CTA is 32 pairs of channels (one per lane: 128 contiguous bytes per row) by 8 runs of `run` consecutive
+// positions (one per warp). A thread walks its run once: the last K inputs and the last K pre-activation gradients slide through registers, so
+// every x and dy value is loaded once (plus the K-1 row overlap between runs) and dx is stored once.
+// Bound: the instructions of a row, so both channels go through one packed multiply-add (fma.f32x2), addresses advance by a row, and the rows that
+// only warm up, only finish or do both are loops of their own. [8192, 7168], four taps: 159 us, 247 with two scalar channels and conditions in
+// every row, 265 with four channels and fewer warps (54 us at copy bandwidth).
 // The 8 warps add their dw / db into shared memory and the CTA writes one partial row; conv1d_reduce_partials sums the rows.
-constexpr int CONV_BTL = 16;
-// From here on, where x and dy outgrow L2, the wider loads are better with one tap forward ([8192, 7168] 53 us with eight channels, 55 with four;
-// [8192, 1792] 22.5 and 20.5) and with two taps backward (194 us with four channels, 224 with two; [16384, 1792] 132 and 127).
-constexpr long long CONV_WIDE = 1ll << 25;
-template <int K, int V>
-__global__ void __launch_bounds__(256, 8 / V) conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                            const __nv_bfloat16* __restrict__ x,
-                                                            const __nv_bfloat16* __restrict__ prev,
-                                                            const __nv_bfloat16* __restrict__ w,
-                                                            const __nv_bfloat16* __restrict__ bias,
-                                                            __nv_bfloat16* __restrict__ dx, float* __restrict__ partial,
-                                                            int B, int L, int C, int act, long long xld, int Ly,
-                                                            long long dxld) {
-  __shared__ float s_acc[32][(CONV_MAXK + 1) * V + 1];
+template <int K>
+__global__ void __launch_bounds__(256, K == 4 ? 4 : 3) conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                                                            const __nv_bfloat16* __restrict__ prev, const __nv_bfloat16* __restrict__ w,
+                                                            const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ dx,
+                                                            float* __restrict__ partial, int B, int L, int C, int act, long long xld, int Ly,
+                                                            long long dxld, int run) {
+  __shared__ float s_acc[32][(CONV_MAXK + 1) * 2 + 1];
   const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5;
-  const int cv = C / V;
   const int v = blockIdx.x * 32 + lane;
-  const bool live = v < cv;
-  const int c = v * V;
-  for (int i = threadIdx.x; i < 32 * ((CONV_MAXK + 1) * V + 1); i += 256) (&s_acc[0][0])[i] = 0.f;
+  const bool live = v < C / 2;
+  const int c = v * 2;
+  for (int i = threadIdx.x; i < 32 * ((CONV_MAXK + 1) * 2 + 1); i += 256) (&s_acc[0][0])[i] = 0.f;
   __syncthreads();
   if (live) {
-    float wv[K][V], bv[V], dwacc[K][V], dbacc[V];
-    conv_taps<K, V>(w, c, wv);
+    uint64_t wv[K], dw[K], db = 0, bv = 0;
+    {
+      float t[K][2];
+      conv_taps<K, 2>(w, c, t);
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-#pragma unroll
-      for (int j = 0; j < V; ++j) dwacc[k][j] = 0.f;
-#pragma unroll
-    for (int j = 0; j < V; ++j) dbacc[j] = bv[j] = 0.f;
-    if (bias) conv_ld<V>(bias + c, bv);
-    const int lchunks = (L + CONV_BTL - 1) / CONV_BTL;
+      for (int k = 0; k < K; ++k) { wv[k] = pack_f32x2(t[k][0], t[k][1]); dw[k] = 0; }
+      if (bias) bv = bf16x2_f32x2(conv_ld<2>(bias + c));
+    }
+    const int lchunks = (L + run - 1) / run;
     const int nchunks = B * lchunks;
     for (int ch = blockIdx.y * 8 + sub; ch < nchunks; ch += gridDim.y * 8) {
-      const int b = ch / lchunks, l0 = (ch % lchunks) * CONV_BTL;
-      const int lend = min(l0 + CONV_BTL, L);
-      float xh[K][V], dph[K][V];
+      const int b = ch / lchunks, l0 = (ch % lchunks) * run;
+      const int lend = min(l0 + run, L);
+      // xh[i], dp[i]: input and pre-activation gradient of the position K - 1 - i before the current one
+      uint64_t xh[K], dp[K];
 #pragma unroll
-      for (int i = 0; i < K; ++i)
-#pragma unroll
-        for (int j = 0; j < V; ++j) xh[i][j] = dph[i][j] = 0.f;
+      for (int i = 0; i < K; ++i) xh[i] = dp[i] = 0;
 #pragma unroll
       for (int i = 1; i < K; ++i) {
         const int ls = l0 - K + i;
-        if (ls >= 0) conv_ld<V>(x + ((long long)b * L + ls) * xld + c, xh[i]);
-        else if (prev) conv_ld<V>(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c, xh[i]);
+        if (ls >= 0) xh[i] = bf16x2_f32x2(conv_ld<2>(x + ((long long)b * L + ls) * xld + c));
+        else if (prev) xh[i] = bf16x2_f32x2(conv_ld<2>(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c));
       }
-#pragma unroll 4
-      for (int l = l0; l < lend + K - 1; ++l) {
+      const __nv_bfloat16* xp = x + ((long long)b * L + l0) * xld + c;
+      const __nv_bfloat16* gp = dy + ((long long)b * Ly + l0) * C + c;
+      __nv_bfloat16* op = dx + ((long long)b * L + l0) * dxld + c;
+      // one position: its pre-activation gradient into dp[K - 1]
+      auto enter = [&](uint32_t xr, uint32_t gr) {
 #pragma unroll
-        for (int i = 0; i + 1 < K; ++i)
+        for (int i = 0; i + 1 < K; ++i) { xh[i] = xh[i + 1]; dp[i] = dp[i + 1]; }
+        xh[K - 1] = bf16x2_f32x2(xr);
+        uint64_t g = bf16x2_f32x2(gr);
+        if (act) {
+          uint64_t pre = bv;
 #pragma unroll
-          for (int j = 0; j < V; ++j) {
-            xh[i][j] = xh[i + 1][j];
-            dph[i][j] = dph[i + 1][j];
-          }
-        if (l < L) {
-          conv_ld<V>(x + ((long long)b * L + l) * xld + c, xh[K - 1]);
-          conv_ld<V>(dy + ((long long)b * Ly + l) * C + c, dph[K - 1]);
-          if (act) {
-#pragma unroll
-            for (int j = 0; j < V; ++j) {
-              float pre = bv[j];
-#pragma unroll
-              for (int k = 0; k < K; ++k) pre += xh[k][j] * wv[k][j];
-              dph[K - 1][j] *= silu_grad(pre);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < V; ++j) xh[K - 1][j] = dph[K - 1][j] = 0.f;
+          for (int k = 0; k < K; ++k) pre = fma_f32x2(xh[k], wv[k], pre);
+          float p0, p1;
+          unpack_f32x2(pre, p0, p1);
+          g = mul_f32x2(g, pack_f32x2(silu_grad(p0), silu_grad(p1)));
         }
-        if (l < lend) {   // this run's own rows: dw[k] += dpre[l] x[l-(K-1)+k], db += dpre[l]
+        dp[K - 1] = g;
+      };
+      auto sums = [&] {   // of the run's own positions: dw[k] += dpre[l] x[l-(K-1)+k], db += dpre[l]
+        db = add_f32x2(db, dp[K - 1]);
 #pragma unroll
-          for (int j = 0; j < V; ++j) {
-            dbacc[j] += dph[K - 1][j];
+        for (int k = 0; k < K; ++k) dw[k] = fma_f32x2(dp[K - 1], xh[k], dw[k]);
+      };
+      auto leave = [&] {  // dx of the position K - 1 before: sum_k w[k] dpre[l - k]
+        uint64_t a = 0;
 #pragma unroll
-            for (int k = 0; k < K; ++k) dwacc[k][j] += dph[K - 1][j] * xh[k][j];
-          }
+        for (int k = 0; k < K; ++k) a = fma_f32x2(wv[k], dp[K - 1 - k], a);
+        float a0, a1;
+        unpack_f32x2(a, a0, a1);
+        *reinterpret_cast<uint32_t*>(op) = pk2(a0, a1);
+        op += dxld;
+      };
+      int l = l0;
+#pragma unroll
+      for (int i = 0; i < K - 1; ++i)
+        if (l < lend) {
+          enter(conv_ld<2>(xp), conv_ld<2>(gp));
+          sums();
+          xp += xld; gp += C; ++l;
         }
-        const int lo = l - (K - 1);   // dx[lo] = sum_k w[k] dpre[lo + (K-1) - k]
-        if (lo >= l0) {
-          float dxa[V];
+      for (; l + 4 <= lend; l += 4) {
+        uint32_t xr[4], gr[4];
 #pragma unroll
-          for (int j = 0; j < V; ++j) {
-            float a = 0.f;
+        for (int u = 0; u < 4; ++u, xp += xld, gp += C) { xr[u] = conv_ld<2>(xp); gr[u] = conv_ld<2>(gp); }
 #pragma unroll
-            for (int k = 0; k < K; ++k) a += wv[k][j] * dph[K - 1 - k][j];
-            dxa[j] = a;
-          }
-          conv_st<V>(dx + ((long long)b * L + lo) * dxld + c, dxa);
+        for (int u = 0; u < 4; ++u) {
+          enter(xr[u], gr[u]);
+          sums();
+          leave();
         }
+      }
+      for (; l < lend; ++l, xp += xld, gp += C) {
+        enter(conv_ld<2>(xp), conv_ld<2>(gp));
+        sums();
+        leave();
+      }
+      // the positions behind the run, which its last ones feed: zero gradient behind the sequence
+      const int short_by = max(0, K - 1 - (lend - l0));      // a run of fewer than K - 1 positions has not left its first ones yet
+#pragma unroll
+      for (int i = 0; i < K - 1; ++i, ++l, xp += xld, gp += C) {
+        if (l < L) enter(conv_ld<2>(xp), conv_ld<2>(gp));
+        else {
+#pragma unroll
+          for (int k = 0; k + 1 < K; ++k) dp[k] = dp[k + 1];
+          dp[K - 1] = 0;
+        }
+        if (i >= short_by) leave();
       }
     }
 #pragma unroll
-    for (int j = 0; j < V; ++j) {
-#pragma unroll
-      for (int k = 0; k < K; ++k) atomicAdd(&s_acc[lane][k * V + j], dwacc[k][j]);
-      atomicAdd(&s_acc[lane][K * V + j], dbacc[j]);
+    for (int k = 0; k <= K; ++k) {
+      float a0, a1;
+      unpack_f32x2(k < K ? dw[k < K ? k : 0] : db, a0, a1);
+      atomicAdd(&s_acc[lane][k * 2], a0);
+      atomicAdd(&s_acc[lane][k * 2 + 1], a1);
     }
   }
   __syncthreads();
   // partial layout: [part][(K+1) * C]: dw as [c][k] flattened (C*K) then db (C)
   float* pp = partial + (long long)blockIdx.y * (K + 1) * C;
-  for (int i = threadIdx.x; i < 32 * (K + 1) * V; i += 256) {
-    const int ln = i / ((K + 1) * V), r = i % ((K + 1) * V);
-    const int k = r / V, j = r % V;
-    const int cc = (blockIdx.x * 32 + ln) * V + j;
+  for (int i = threadIdx.x; i < 32 * (K + 1) * 2; i += 256) {
+    const int ln = i / ((K + 1) * 2), r = i % ((K + 1) * 2);
+    const int k = r / 2, j = r % 2;
+    const int cc = (blockIdx.x * 32 + ln) * 2 + j;
     if (cc >= C) continue;
     if (k < K) pp[(long long)cc * K + k] = s_acc[ln][r];
     else pp[(long long)C * K + cc] = s_acc[ln][r];
@@ -274,6 +291,10 @@ __global__ void conv1d_reduce_partials(const float* __restrict__ part, int npart
 
 }  // namespace sx
 using namespace sx;
+
+// From here on, where x and y outgrow L2, wider loads are better with one tap forward ([8192, 7168] 53 us with eight channels, 55 with four;
+// [8192, 1792] 22.5 and 20.5).
+constexpr long long CONV_WIDE = 1ll << 25;
 
 // Sequences are L rows of pitch xld in x and Ly rows of pitch C in y (and in dy below; rows from L on are not touched).
 extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, const void* bias, void* y, void* state_out,
@@ -296,16 +317,22 @@ extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, con
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
+// Positions of a run: the K - 1 positions behind it are computed twice, so long ones where the runs still fill the SMs twice over ([8192, 7168]
+// 159 us, 167 with 32, 4 taps; 126 and 136, 2 taps).
+static int conv_bwd_run(int B, int L, int C) { return (long long)B * ((L + 63) / 64) * ((C / 2 + 31) / 32) >= 148ll * 32 * 2 ? 64 : 16; }
+
 // Number of partial rows the backward kernel writes for B sequences of L tokens of C channels.
 extern "C" int sx_conv1d_bwd_parts(int B, int L, int C) {
   // four runs per warp (32 per CTA): the per-CTA prologue (taps, bias) and epilogue (partial row) cost about as much
   // as one run. Inputs that would leave SMs idle that way take as many CTAs as make one wave, down to one
   // run per warp ([4, 500, 1792]: 73 -> 32 us)
-  const long long chunks = (long long)B * ((L + CONV_BTL - 1) / CONV_BTL);
-  const int cols = (C / 2 + 31) / 32;             // of two channels with four CTAs an SM; four channels: half as many of both
+  const int run = conv_bwd_run(B, L, C);
+  const long long chunks = (long long)B * ((L + run - 1) / run);
+  const int cols = (C / 2 + 31) / 32;             // four CTAs an SM
   const long long wave = 148 * 4 / (cols > 0 ? cols : 1), most = (chunks + 7) / 8;
-  long long p = (chunks + 31) / 32;
+  long long p = (chunks * run / 16 + 31) / 32;
   if (p < wave) p = most < wave ? most : wave;
+  if (p > most) p = most;
   return (int)(p < 1 ? 1 : (p > 512 ? 512 : p));
 }
 
@@ -317,16 +344,16 @@ extern "C" int sx_conv1d_bwd(const void* dy, const void* x, const void* prev, co
   if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L || dxld % 4 || dxld < C) return -1;
   if ((long long)B * L == 0) return 0;
   const int parts = sx_conv1d_bwd_parts(B, L, C);
-  auto run = [&](auto kern, int V) {
-    kern<<<dim3((C / V + 31) / 32, parts), 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)prev,
+  auto run = [&](auto kern) {
+    kern<<<dim3((C / 2 + 31) / 32, parts), 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)prev,
                                                          (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)dx, partial, B, L, C,
-                                                         act, xld, Ly, dxld);
+                                                         act, xld, Ly, dxld, conv_bwd_run(B, L, C));
   };
   switch (K) {
-    case 1: run(conv1d_bwd_kernel<1, 2>, 2); break;
-    case 2: (long long)B * L * C >= CONV_WIDE ? run(conv1d_bwd_kernel<2, 4>, 4) : run(conv1d_bwd_kernel<2, 2>, 2); break;
-    case 3: run(conv1d_bwd_kernel<3, 2>, 2); break;
-    default: run(conv1d_bwd_kernel<4, 2>, 2); break;
+    case 1: run(conv1d_bwd_kernel<1>); break;
+    case 2: run(conv1d_bwd_kernel<2>); break;
+    case 3: run(conv1d_bwd_kernel<3>); break;
+    default: run(conv1d_bwd_kernel<4>); break;
   }
   const int n = (K + 1) * C;
   cudaMemsetAsync(dwdb, 0, sizeof(float) * n, st);

@@ -433,3 +433,21 @@ def test_conv1d_taps(K, B, L, C, act):
     # gradients before their rounding depend on the pre-activation through the sigmoid, which is steepest by |pre| / 4
     k2 = 1 + mag_y.max()
     assert near(got[0], want[0], mag_x * k2) and near(got[1], want[1], mag_w * k2) and near(got[2], want[2], up.sum((0, 1)) * k2)
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 4])
+@pytest.mark.parametrize("L", [1, 2, 3, 63, 65, 130])
+def test_conv1d_backward_runs(K, L):
+    """A batch large enough for runs of 64 positions gives each sequence the bits that runs of 16 give it alone, sequences shorter than the taps and
+    ends of runs included; the taps' gradients are sums of 200 equal terms in 32 bits, rounded to bf16."""
+    torch.manual_seed(10 * L + K)
+    C, n = 1024, 200 * max(1, 128 // L)
+    x, g = (torch.randn(1, L, C, device="cuda").bfloat16() for _ in range(2))
+    w, b = (0.5 * torch.randn(C, K, device="cuda")).bfloat16(), torch.randn(C, device="cuda").bfloat16()
+    grads = []
+    for B in (1, n):
+        ins = [x.repeat(B, 1, 1).requires_grad_(), w.clone().requires_grad_(), b.clone().requires_grad_()]
+        grads.append(torch.autograd.grad(ssm.causal_conv1d(*ins, act=True), ins, g.repeat(B, 1, 1)))
+    assert bool((grads[1][0] == grads[0][0]).all())
+    for a, e in zip(grads[1][1:], grads[0][1:]):
+        assert bool(((a.double() / n - e.double()).abs() <= 2.0 ** -7 * e.double().abs() + 2.0 ** -14 * e.double().abs().max()).all())
