@@ -31,8 +31,9 @@ namespace sx {
 constexpr int ATT_BM = 128;   // rows per q tile (two per CTA)
 constexpr int ATT_BN = 128;
 // 2 x 4 softmax warps, TMA warp, MMA warp, two idle ones: the last four give registers to the softmax warps, which hold a row of 128 scores
-// (2 x 128 x 216 + 128 x 72 = 384 x 168, what the block is launched with)
+// (2 x 128 x 216 + 128 x 72 = 384 x 168, what the block is launched with; more than that would never be granted, so the launch checks it)
 constexpr int ATT_THREADS = 384, ATT_TMA_WARP = 8, ATT_MMA_WARP = 9;
+constexpr int ATT_REGS = 168;
 
 struct AttnFwdParams {
   CUtensorMap tmQ, tmK, tmV;
@@ -408,6 +409,20 @@ static int make_attn_map(CUtensorMap* tm, const void* base, int B, int S, int H,
   return make_tmap(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, base, dims, strides, box);
 }
 
+template <int D, bool MASK>
+static int attn_fwd_launch(const AttnFwdParams& p, dim3 grid, cudaStream_t st) {
+  static bool set = false;
+  if (!set) {
+    cudaFuncAttributes fa;
+    if (cudaFuncSetAttribute(attn_fwd_kernel<D, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::SMEM_BYTES) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, attn_fwd_kernel<D, MASK>) != cudaSuccess) return -10;
+    if (fa.numRegs < ATT_REGS) return -12;
+    set = true;
+  }
+  attn_fwd_kernel<D, MASK><<<grid, ATT_THREADS, AttnCfg<D>::SMEM_BYTES, st>>>(p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
 }  // namespace sx
 using namespace sx;
 
@@ -443,28 +458,7 @@ extern "C" int sx_attn_fwd(const SxAttnArgs* a, cudaStream_t st) {
   const long long blocks = (long long)p.pairs * a->Hq * a->B;
   if (blocks <= 0 || blocks > INT_MAX) return -4;
   const dim3 grid((unsigned)blocks);
-  if (a->D == 128) {
-    static bool set = false;
-    if (!set) {
-      if (cudaFuncSetAttribute(attn_fwd_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               AttnCfg<128>::SMEM_BYTES) != cudaSuccess ||
-          cudaFuncSetAttribute(attn_fwd_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               AttnCfg<128>::SMEM_BYTES) != cudaSuccess) return -10;
-      set = true;
-    }
-    if (p.block_mask) attn_fwd_kernel<128, true><<<grid, ATT_THREADS, AttnCfg<128>::SMEM_BYTES, st>>>(p);
-    else attn_fwd_kernel<128, false><<<grid, ATT_THREADS, AttnCfg<128>::SMEM_BYTES, st>>>(p);
-  } else {
-    static bool set = false;
-    if (!set) {
-      if (cudaFuncSetAttribute(attn_fwd_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               AttnCfg<64>::SMEM_BYTES) != cudaSuccess ||
-          cudaFuncSetAttribute(attn_fwd_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               AttnCfg<64>::SMEM_BYTES) != cudaSuccess) return -10;
-      set = true;
-    }
-    if (p.block_mask) attn_fwd_kernel<64, true><<<grid, ATT_THREADS, AttnCfg<64>::SMEM_BYTES, st>>>(p);
-    else attn_fwd_kernel<64, false><<<grid, ATT_THREADS, AttnCfg<64>::SMEM_BYTES, st>>>(p);
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+  const bool masked = p.block_mask != nullptr;
+  if (a->D == 128) return masked ? attn_fwd_launch<128, true>(p, grid, st) : attn_fwd_launch<128, false>(p, grid, st);
+  return masked ? attn_fwd_launch<64, true>(p, grid, st) : attn_fwd_launch<64, false>(p, grid, st);
 }
