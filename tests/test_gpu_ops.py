@@ -458,6 +458,24 @@ def test_attention_forward_passes_nan_scores_on(key):
     ops.check_status()
 
 
+@pytest.mark.parametrize("B,S,H,Hk,pad", [(1, 1, 1, 1, 0), (2, 31, 4, 2, 4), (3, 32, 3, 1, 12), (2, 33, 28, 4, 4), (2, 65, 2, 2, 0), (3, 129, 6, 3, 8)])
+def test_attention_backward_converts_its_accumulator(B, S, H, Hk, pad):
+    """dQ is the accumulator (pieces of 32 queries, groups of 4 columns, queries, columns), scaled and rounded once: equal bits; nothing is written
+    between the rows of a dQ whose row stride is a multiple of 4 elements."""
+    torch.manual_seed(S)
+    a, t = _attn_bwd_args(B, S, H, Hk)
+    P = (S + 63) // 64 * 2
+    acc = torch.empty(B, H, P, 32, 32, 4, device="cuda")
+    dq = torch.full((B, S, H * 128 + pad), 7.0, dtype=torch.bfloat16, device="cuda")
+    a.dq_accum, a.dQ, a.dq_row_stride, a.dq_batch_stride = acc.data_ptr(), dq.data_ptr(), dq.stride(1), dq.stride(0)
+    _lib.call("sx_attn_bwd", C.byref(a), stream())
+    ops.check_status()
+    want = (acc * torch.tensor(a.scale, dtype=torch.float32, device="cuda")).bfloat16()
+    want = want.permute(0, 2, 4, 1, 3, 5).reshape(B, P * 32, H * 128)[:, :S]
+    assert torch.equal(dq[..., :H * 128].view(torch.int16), want.view(torch.int16))
+    assert bool((dq[..., H * 128:] == 7.0).all())
+
+
 @pytest.mark.parametrize("S,H,Hk", [(1, 2, 1), (64, 3, 3), (65, 4, 2), (127, 2, 2), (128, 5, 1), (150, 4, 4), (193, 2, 1), (256, 3, 1), (513, 2, 2)])
 def test_attention_backward_stays_inside_its_accumulator(S, H, Hk):
     """The last query tile may reach behind the accumulator, which holds multiples of 64 queries: nothing is added there, and the results are those
