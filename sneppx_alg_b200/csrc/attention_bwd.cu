@@ -17,8 +17,9 @@
 // atomics because the whole GQA group is reduced inside the CTA.
 // Bound: shared memory. The 40 products of a tile are 2560 cycles of the tensor pipe, their operands, the tiles, dS and the staged dQ 512 KB,
 // 4096 cycles at 128 bytes; a tile takes about 4000. With query tiles of 64 (two in flight) it was 6800 for as many queries: a product of N = 64
-// takes its A as often as one of N = 128. B200, warm, whole backward, before -> now: [1, 4096, 32 / 8 heads] causal 549 -> 418 us,
-// [1, 16384, 32 / 8] 7.59 -> 5.63 ms, [1, 8192, 8 / 2] full 1013 -> 700 us, [8, 512, 28 / 4] 157 -> 125 us.
+// takes its A as often as one of N = 128. B200, warm, whole backward as called (delta, this kernel, conversion),
+// before -> now: [1, 4096, 32 / 8 heads] causal 550 -> 367 us, [1, 16384, 32 / 8] 7.4 -> 5.1 ms, [1, 8192, 8 / 2] full 1084 -> 800 us,
+// [8, 512, 28 / 4] 185 -> 152 us.
 // dQ by 16-byte reductions from registers instead of staging and bulk reductions: 25 cycles per 512 bytes, 64 KB a tile, and shared memory
 // accesses queue behind them (488 us at 4096, 425 staged by four warps). The accumulator's columns have to be read before dP^T of the next tile:
 // eight drain warps take them into registers at once.
