@@ -20,7 +20,6 @@ __device__ __forceinline__ float silu_grad(float x) {
 
 // V channels of a row: 4 (8 bytes) or 2.
 template <int V> struct ConvVec;
-template <> struct ConvVec<8> { typedef uint4 T; };
 template <> struct ConvVec<4> { typedef uint2 T; };
 template <> struct ConvVec<2> { typedef uint32_t T; };
 __device__ __forceinline__ float2 bf2(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); }
@@ -36,11 +35,6 @@ __device__ __forceinline__ void conv_unpack(uint32_t r, float (&f)[2]) {
   const float2 a = bf2(r);
   f[0] = a.x; f[1] = a.y;
 }
-__device__ __forceinline__ void conv_unpack(uint4 r, float (&f)[8]) {
-  const float2 a = bf2(r.x), b = bf2(r.y), c = bf2(r.z), d = bf2(r.w);
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-}
-__device__ __forceinline__ uint4 conv_pack(const float (&f)[8]) { return make_uint4(pk2(f[0], f[1]), pk2(f[2], f[3]), pk2(f[4], f[5]), pk2(f[6], f[7])); }
 __device__ __forceinline__ uint2 conv_pack(const float (&f)[4]) { return make_uint2(pk2(f[0], f[1]), pk2(f[2], f[3])); }
 __device__ __forceinline__ uint32_t conv_pack(const float (&f)[2]) { return pk2(f[0], f[1]); }
 template <int V> __device__ __forceinline__ typename ConvVec<V>::T conv_ld(const __nv_bfloat16* p) {
@@ -69,76 +63,155 @@ __device__ __forceinline__ void conv_taps(const __nv_bfloat16* w, int c, float (
   }
 }
 
-// One thread: V channels x CONV_TL consecutive positions. The V x K weights and the bias live in registers and the
-// K-1 previous inputs slide through registers, so each input vector is loaded once and each output costs one load and
-// one store of V channels; consecutive threads own consecutive channel vectors (coalesced rows).
-// What bounds it is the latency of these chains (180 instructions for 8 channels of a row, half of them the sigmoid), so warps count: with
-// eight channels a thread and 128 registers an SM held 12 to 16. [8192, 7168]: 78 us, 100 with eight (36 us at copy bandwidth); [4, 500, 1792]
-// 14 and 16 us.
-constexpr int CONV_TL = 16;
-template <int K, int V>
-__global__ void __launch_bounds__(256, 3) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ prev,
+// One thread: 4 channels x `run` consecutive positions. The K taps and the bias live in registers and the K-1 previous inputs slide through
+// registers, so each input vector is loaded once and each output costs one load and one store of 4 channels; consecutive threads own consecutive
+// channel vectors (coalesced rows).
+// Bound: the instructions of a row (half of them the sigmoid), so pairs of channels go through one packed multiply-add, rounded like two scalar
+// ones, and the rows that no state is made of are a loop without conditions. Cold, scalar with conditions -> now, four taps: [8192, 7168]
+// 79.9 -> 67.6 us (36 at copy bandwidth), [8192, 5376] 63.5 -> 55.3, [16, 4096, 4352] 348 -> 263, [4, 2048, 1792] 30.7 -> 26.6; [8192, 7168] with
+// three taps 70 -> 63.5, two 59 -> 51, one 53 either way. Three CTAs an SM: four (64 registers) spill 64 bytes and take 71.7 us with three or four
+// taps, but 51 instead of 57 with two. A 32-bit division for the index spills as well (77.8 us).
+template <int K>
+__global__ void __launch_bounds__(256, K >= 3 ? 3 : 4) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ prev,
                                                             const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
                                                             __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ state_out, int B,
-                                                            int L, int C, int act, long long xld, int Ly) {
-  const int cv = C / V;
-  const int lchunks = (L + CONV_TL - 1) / CONV_TL;
+                                                            int L, int C, int act, long long xld, int Ly, int run) {
+  typedef uint2 T;
+  constexpr int V = 4, P = V / 2;
+  const unsigned cv = C / V, lchunks = (L + run - 1) / run;
   const long long total = (long long)B * lchunks * cv;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
     const int c = (int)(idx % cv) * V;
-    const long long bl = idx / cv;
-    const int l0 = (int)(bl % lchunks) * CONV_TL;
-    const int b = (int)(bl / lchunks);
-    const int l1 = min(L, l0 + CONV_TL);
+    const unsigned bl = (unsigned)(idx / cv);
+    const int l0 = (int)(bl % lchunks) * run, b = (int)(bl / lchunks);
+    const int l1 = min(L, l0 + run);
     const __nv_bfloat16* xp = x + ((long long)b * L + l0) * xld + c;
     __nv_bfloat16* yp = y + ((long long)b * Ly + l0) * C + c;
-    float wv[K][V], bv[V];
-    conv_taps<K, V>(w, c, wv);
-    if (bias) conv_ld<V>(bias + c, bv);
+    uint64_t wv[K][P], bv[P], xh[K][P];   // pairs of channels; xh[i]: input of the position K - 1 - i before the current one
+    {
+      float t[K][V], f[V];
+      conv_taps<K, V>(w, c, t);
+      if (bias) conv_ld<V>(bias + c, f);
+#pragma unroll
+      for (int j = 0; j < P; ++j) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) { wv[k][j] = pack_f32x2(t[k][2 * j], t[k][2 * j + 1]); xh[k][j] = 0; }
+        bv[j] = bias ? pack_f32x2(f[2 * j], f[2 * j + 1]) : 0;
+      }
+    }
+    auto take = [&](T r, uint64_t (&h)[P]) {
+#pragma unroll
+      for (int j = 0; j < P; ++j) h[j] = bf16x2_f32x2(reinterpret_cast<const uint32_t*>(&r)[j]);
+    };
+#pragma unroll
+    for (int i = 1; i < K; ++i) {
+      const int ls = l0 - K + i;
+      if (ls >= 0) take(conv_ld<V>(xp + (long long)(i - K) * xld), xh[i]);
+      else if (prev) take(conv_ld<V>(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c), xh[i]);
+    }
+    auto row = [&](T r) {
+#pragma unroll
+      for (int i = 0; i + 1 < K; ++i)
+#pragma unroll
+        for (int j = 0; j < P; ++j) xh[i][j] = xh[i + 1][j];
+      take(r, xh[K - 1]);
+      float f[V];
+#pragma unroll
+      for (int j = 0; j < P; ++j) {
+        uint64_t a = bv[j];
+#pragma unroll
+        for (int k = 0; k < K; ++k) a = fma_f32x2(xh[k][j], wv[k][j], a);
+        unpack_f32x2(a, f[2 * j], f[2 * j + 1]);
+      }
+      if (act) {
+#pragma unroll
+        for (int j = 0; j < V; ++j) f[j] = silu_f(f[j]);
+      }
+      conv_st<V>(yp, f);
+      yp += C;
+    };
+    const int plain = state_out ? min(l1, L - (K - 1)) : l1;   // from here on rows are of the state too
+    int l = l0;
+    for (; l + 4 <= plain; l += 4) {
+      T r[4];   // four independent loads in flight per thread
+#pragma unroll
+      for (int u = 0; u < 4; ++u, xp += xld) r[u] = conv_ld<V>(xp);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) row(r[u]);
+    }
+    for (; l < l1; l += 4) {
+      T r[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u, xp += xld)
+        if (l + u < l1) r[u] = conv_ld<V>(xp);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (l + u < l1) {
+          row(r[u]);
+          if (state_out && l + u >= L - (K - 1)) *reinterpret_cast<T*>(state_out + ((long long)b * (K - 1) + (l + u - (L - (K - 1)))) * C + c) = r[u];
+        }
+    }
+  }
+}
+
+// The same for sequences of few positions (one token of each in a decoding step): a thread walks all of them, scalar, and has no division by runs.
+// The packed form's taps and main loop stand in front of its first rows. Four taps: [16, 4, 1792] 2.83 us, 3.46 packed (3.17 when this walk served
+// every length); [16, 1, 1792] 2.40 (2.70). From 8 positions on the packed form is as fast as that walk was (4.0 us) and then faster (4.8 and 5.6 at 15).
+constexpr int CONV_SHORT = 8;
+template <int K>
+__global__ void __launch_bounds__(256, 3) conv1d_short_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ prev,
+                                                              const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
+                                                              __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ state_out, int B,
+                                                              int L, int C, int act, long long xld, int Ly) {
+  const int cv = C / 4;
+  const long long total = (long long)B * cv;
+  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
+    const int c = (int)(idx % cv) * 4;
+    const long long b = idx / cv;
+    const __nv_bfloat16* xp = x + b * L * xld + c;
+    __nv_bfloat16* yp = y + b * Ly * C + c;
+    float wv[K][4], bv[4], hist[K][4];   // hist[i]: input of the position K - 1 - i before the current one
+    conv_taps<K, 4>(w, c, wv);
+    if (bias) conv_ld<4>(bias + c, bv);
     else {
 #pragma unroll
-      for (int j = 0; j < V; ++j) bv[j] = 0.f;
+      for (int j = 0; j < 4; ++j) bv[j] = 0.f;
     }
-    // hist[i] = input at position l - (K-1) + i for the current l; hist[K-1] is the current input
-    float hist[K][V];
 #pragma unroll
     for (int i = 0; i < K; ++i)
 #pragma unroll
-      for (int j = 0; j < V; ++j) hist[i][j] = 0.f;
+      for (int j = 0; j < 4; ++j) hist[i][j] = 0.f;
+    if (prev) {
 #pragma unroll
-    for (int i = 0; i < K - 1; ++i) {
-      const int ls = l0 - (K - 1) + i;
-      if (ls >= 0) conv_ld<V>(xp + (long long)(i - (K - 1)) * xld, hist[i]);
-      else if (prev) conv_ld<V>(prev + ((long long)b * (K - 1) + (K - 1 + ls)) * C + c, hist[i]);
+      for (int i = 0; i < K - 1; ++i) conv_ld<4>(prev + (b * (K - 1) + i) * C + c, hist[i]);
     }
-    for (int lb = l0; lb < l1; lb += 4) {
-      typename ConvVec<V>::T raw4[4];   // four independent loads in flight per thread
+    for (int lb = 0; lb < L; lb += 4) {
+      uint2 raw[4];   // four independent loads in flight per thread
 #pragma unroll
       for (int u = 0; u < 4; ++u, xp += xld)
-        if (lb + u < l1) raw4[u] = conv_ld<V>(xp);
+        if (lb + u < L) raw[u] = conv_ld<4>(xp);
 #pragma unroll
       for (int u = 0; u < 4; ++u, yp += C) {
         const int l = lb + u;
-        if (l >= l1) break;
-        conv_unpack(raw4[u], hist[K - 1]);
-        float acc[V];
+        if (l >= L) break;
+        conv_unpack(raw[u], hist[K - 1]);
+        float acc[4];
 #pragma unroll
-        for (int j = 0; j < V; ++j) acc[j] = bv[j];
+        for (int j = 0; j < 4; ++j) acc[j] = bv[j];
 #pragma unroll
         for (int k = 0; k < K; ++k)
 #pragma unroll
-          for (int j = 0; j < V; ++j) acc[j] = fmaf(hist[k][j], wv[k][j], acc[j]);
+          for (int j = 0; j < 4; ++j) acc[j] = fmaf(hist[k][j], wv[k][j], acc[j]);
         if (act) {
 #pragma unroll
-          for (int j = 0; j < V; ++j) acc[j] = silu_f(acc[j]);
+          for (int j = 0; j < 4; ++j) acc[j] = silu_f(acc[j]);
         }
-        conv_st<V>(yp, acc);
-        if (state_out && l >= L - (K - 1))
-          *reinterpret_cast<typename ConvVec<V>::T*>(state_out + ((long long)b * (K - 1) + (l - (L - (K - 1)))) * C + c) = raw4[u];
+        conv_st<4>(yp, acc);
+        if (state_out && l >= L - (K - 1)) *reinterpret_cast<uint2*>(state_out + (b * (K - 1) + (l - (L - (K - 1)))) * C + c) = raw[u];
 #pragma unroll
         for (int i = 0; i + 1 < K; ++i)
 #pragma unroll
-          for (int j = 0; j < V; ++j) hist[i][j] = hist[i + 1][j];
+          for (int j = 0; j < 4; ++j) hist[i][j] = hist[i + 1][j];
       }
     }
   }
@@ -292,27 +365,27 @@ __global__ void conv1d_reduce_partials(const float* __restrict__ part, int npart
 }  // namespace sx
 using namespace sx;
 
-// From here on, where x and y outgrow L2, wider loads are better with one tap forward ([8192, 7168] 53 us with eight channels, 55 with four;
-// [8192, 1792] 22.5 and 20.5).
-constexpr long long CONV_WIDE = 1ll << 25;
-
 // Sequences are L rows of pitch xld in x and Ly rows of pitch C in y (and in dy below; rows from L on are not touched).
 extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, const void* bias, void* y, void* state_out,
                              int B, int L, int C, int K, int act, long long xld, int Ly, cudaStream_t st) {
   if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L) return -1;
   if ((long long)B * L * C == 0) return 0;
-  auto run = [&](auto kern, int V) {
-    const long long total = (long long)B * ((L + CONV_TL - 1) / CONV_TL) * (C / V);
-    kern<<<(int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16), 256, 0, st>>>(
+  // Runs of 32 read fewer rows twice, but only where they still fill the SMs twice over ([8192, 7168] 71.7 us with 16, 67.6 with 32; [4, 500, 1792]
+  // 14 and 18).
+  const long long threads = (long long)B * ((L + 31) / 32) * (C / 4);
+  const int run = threads >= 2ll * 148 * 768 ? 32 : 16;
+  auto go = [&](auto kern, auto... more) {
+    const long long blocks = ((long long)B * (sizeof...(more) ? (L + run - 1) / run : 1) * (C / 4) + 255) / 256;
+    kern<<<(int)(blocks < 148 * 1024 ? blocks : 148 * 1024), 256, 0, st>>>(
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)prev, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y,
-        (__nv_bfloat16*)state_out, B, L, C, act, xld, Ly);
+        (__nv_bfloat16*)state_out, B, L, C, act, xld, Ly, more...);
   };
-  const bool wide = (long long)B * L * C >= CONV_WIDE && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0;
+  const bool few = L < CONV_SHORT;
   switch (K) {
-    case 1: wide ? run(conv1d_fwd_kernel<1, 8>, 8) : run(conv1d_fwd_kernel<1, 4>, 4); break;
-    case 2: run(conv1d_fwd_kernel<2, 4>, 4); break;
-    case 3: run(conv1d_fwd_kernel<3, 4>, 4); break;
-    default: run(conv1d_fwd_kernel<4, 4>, 4); break;
+    case 1: go(conv1d_fwd_kernel<1>, run); break;
+    case 2: few ? go(conv1d_short_kernel<2>) : go(conv1d_fwd_kernel<2>, run); break;
+    case 3: few ? go(conv1d_short_kernel<3>) : go(conv1d_fwd_kernel<3>, run); break;
+    default: few ? go(conv1d_short_kernel<4>) : go(conv1d_fwd_kernel<4>, run); break;
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from sneppx_alg_b200 import ops
-from sneppx_alg_b200.ops import moe, quant, ssm
+from sneppx_alg_b200.ops import _lib, moe, quant, ssm
 
 pytestmark = pytest.mark.gpu
 
@@ -433,6 +433,44 @@ def test_conv1d_taps(K, B, L, C, act):
     # gradients before their rounding depend on the pre-activation through the sigmoid, which is steepest by |pre| / 4
     k2 = 1 + mag_y.max()
     assert near(got[0], want[0], mag_x * k2) and near(got[1], want[1], mag_w * k2) and near(got[2], want[2], up.sum((0, 1)) * k2)
+
+
+@pytest.mark.parametrize("act", [0, 1])
+@pytest.mark.parametrize("K", [1, 2, 3, 4])
+@pytest.mark.parametrize("L", [1, 2, 3, 5, 7, 8, 15, 16, 17, 31, 33, 64, 67])
+def test_conv1d_forward_runs(K, L, act):
+    """Few positions, runs of 16 and runs of 32 (a batch that fills the SMs) give a sequence the same bits, and write the state of its last positions
+    and nothing else. Against 64 bits: one rounding to bf16, 2^-8 of the value, and K + 8 roundings to 32 bits of the sum of magnitudes, below 2^-16."""
+    torch.manual_seed(100 * L + K)
+    C, W = 1024, 1024 + 64
+    x = torch.randn(1, L, W, device="cuda").bfloat16()
+    prev = torch.randn(1, max(K - 1, 1), C, device="cuda").bfloat16()
+    w, b = torch.randn(C, K, device="cuda").bfloat16(), torch.randn(C, device="cuda").bfloat16()
+
+    def run(x, prev, n, state=True):
+        B, Ly = x.shape[0], n + 2
+        y, s = torch.full((B, Ly, C), 7.0, device="cuda").bfloat16(), torch.full((B, max(K - 1, 1), C), 7.0, device="cuda").bfloat16()
+        assert x.is_contiguous() and x.shape[1] == n
+        _lib.call("sx_conv1d_fwd", _lib.ptr(x), _lib.ptr(prev if K > 1 else None), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), _lib.ptr(s if state else None),
+                  _lib.c_int(B), _lib.c_int(n), _lib.c_int(C), _lib.c_int(K), _lib.c_int(act), _lib.c_ll(W), _lib.c_int(Ly), _lib.stream())
+        assert bool((y[:, n:] == 7.0).all())
+        return y[:, :n], s
+
+    y, s = run(x, prev, L)
+    ext = torch.cat([prev[:, prev.shape[1] - (K - 1):] if K > 1 else prev[:, :0], x[..., :C]], dim=1).double()
+    terms = torch.stack([ext[:, k:k + L] * w[:, k].double() for k in range(K)] + [b.double().expand(1, L, C)])
+    want = terms.sum(0)
+    want = torch.nn.functional.silu(want) if act else want
+    assert bool(((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16 * terms.abs().sum(0)).all())
+    for i in range(K - 1):                                      # the state's rows: positions L - (K - 1) + i
+        l = L - (K - 1) + i
+        assert torch.equal(s[0, i], x[0, l, :C]) if l >= 0 else bool((s[0, i] == 7.0).all())
+    n = (2 * 148 * 768 * 4) // (C * ((L + 31) // 32)) + 1       # sequences that make runs of 32
+    yb, sb = run(x.repeat(n, 1, 1), prev.repeat(n, 1, 1), L)
+    assert bool((yb == y).all()) and bool((sb == s).all())
+    assert torch.equal(run(x, prev, L, state=False)[0], y)
+    longer = torch.cat([x, torch.randn(1, 40, W, device="cuda").bfloat16()], dim=1)
+    assert torch.equal(run(longer, prev, L + 40)[0][:, :L], y)
 
 
 @pytest.mark.parametrize("K", [1, 2, 3, 4])
