@@ -68,9 +68,14 @@ __device__ __forceinline__ float block_max(float v, float* red) {
   return red[32];
 }
 
-// Launch of a kernel that begins with after_predecessor(): its blocks may be set up while the kernel before it on the stream still runs (programmatic
-// dependent launch), so that what lies between the two is the wait, not a launch. In a decode step of an 8B-width model half of the kernels take
-// 2 to 3 us, most of it that.
+// Launch of a kernel whose blocks may be set up while the kernel before it on the stream still runs (programmatic dependent launch), so that what lies
+// between the two is the wait, not a launch. In a decode step of an 8B-width model half of the kernels take 2 to 3 us, most of it that.
+// The kernel executes griddepcontrol.wait before it touches anything that an earlier kernel writes or reads. Its pointers are not __restrict__: that
+// would promise the compiler that nobody else writes the memory while the kernel runs, and let it load around the cache's coherence or ahead of the
+// wait, but until the wait returns the kernel before does write it. Whether it lets its own successor start early is up to it: after_predecessor()
+// does, the paged decode kernel does not.
+// A chain of kernels that do holds nothing back. Loads in front of a wait (the static weights of a decode product) may pass all of them, up to the last
+// kernel that was not launched this way or did not signal: no kernel behind that one may write what is loaded so.
 __device__ __forceinline__ void after_predecessor() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the same for the kernel after this one
   asm volatile("griddepcontrol.wait;" ::: "memory");                // all that kernels before this one wrote is there

@@ -6,7 +6,8 @@
 // projections' weights (gemm_skinny.cu). One CTA per (head, sequence) keeps its P x N state in registers between the read and the
 // write: a warp owns whole rows, a lane four neighbouring values of N, so rows move as 512-byte pieces and y needs one warp sum a row.
 // The state is fetched before griddepcontrol.wait: no kernel between the last step's and this one writes it, so the fetch runs under the
-// input projection, and so does all of the convolution but the newest token. Four CTAs an SM (64 registers): with two, 1280 CTAs were
+// input projection, and so does all of the convolution but the newest token. This kernel does not signal its successor, so whatever starts early
+// behind it, the next step's fetch too, starts when the states have been written. Four CTAs an SM (64 registers): with two, 1280 CTAs were
 // more than four rounds of one chain of loads each (40 us a launch under a profiler, 29 now). Convolution inputs are read from one buffer and the shifted ones written to another, because the heads of a group
 // share B and C and run in no order.
 // Measured (B200, 8 layers of width 2560, 16 sequences, one step with embedding, head and argmax): 0.76 ms against 9.3 ms when every step
@@ -142,11 +143,13 @@ static int mamba_gemm(const void* x, const void* w, void* y, int M, int N, int K
   a.lda = K; a.ldb = K; a.ldd = N;
   a.alpha = 1.f;
   a.status = status;
-  a.flags = 1;      // weights are not written by a kernel of this step
+  a.flags = 1;      // see sx_mamba2_step
   return sx_gemm_bf16(&a, st);
 }
 
-// Five launches. The sizes are those that the front-end has checked (serving/mamba_states.py).
+// Five launches. The sizes are those that the front-end has checked (serving/mamba_states.py). The weights of both projections are declared static, and
+// the norm in front lets their first loads pass it: no kernel in front of the call may write them, unless one that is launched ordinarily lies between
+// (the lookup of the tokens in a decode step).
 extern "C" int sx_mamba2_step(const SxMambaStepArgs* a, cudaStream_t st) {
   if (a->B <= 0) return 0;
   if (a->B > 65535 || a->H <= 0 || a->G <= 0 || a->H % a->G || a->P <= 0 || a->N <= 0 || a->N % 4 || a->N > 256 || a->taps < 2 || a->taps > 4 || a->d % 8)

@@ -20,32 +20,37 @@ __device__ __forceinline__ float row_sum(float v, float* red) {
   return warp_sum(lane < nw ? red[lane] : 0.f);
 }
 
+// Rows that are read once: they leave the weights' place in L1 alone. (What these kernels read may be written until their wait returns, so the
+// non-coherent loads that would do that are not open to them.)
+__device__ __forceinline__ bf16x8 ld8_once(const __nv_bfloat16* p) {
+  bf16x8 v;
+  uint32_t* u = reinterpret_cast<uint32_t*>(&v);
+  asm volatile("ld.global.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "l"(p) : "memory");
+  return v;
+}
+
 // y = rmsnorm(x + res_in) * w ; res_out = x + res_in ; rstd saved for backward.
 // Bound: memory. A row stays in the registers of one CTA between the sum and the output (V vectors of 8 a thread), so it is read once and
 // all of its loads are in flight together; rows are spread over CTAs and overlap. Two vectors a thread keep CTAs small enough that
-// several share an SM. [4096, 4096] with residual: 31 us with a cold L2 full of dirty lines (read + write once: 20 us at copy
-// bandwidth), 37 us when a second pass read the row again. RES: with a residual; without one the registers for it cost CTAs an SM
-// (60 and 40 a thread with V = 2; [8192, 6144] without residual 68 us with them, 64 with a second pass, 53 so).
+// several share an SM; the weights come from L1 or L2 when the sum is there, because registers for them cost CTAs, too. Warm, with / without a
+// residual: [8192, 6144] 64 / 46 us (85 / 47 with the weights fetched first, through the read-only path), [8192, 2560] 30 / 21 (37 / 23),
+// [4096, 4096] 22 / 14 (26 / 16). RES: with a residual; without one the registers for it cost CTAs an SM.
 template <int V, bool RES>
-__global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in,
-                                                           const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                                           __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd, int d, float eps) {
+__global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* res_in, const __nv_bfloat16* w,
+                                                          __nv_bfloat16* y, __nv_bfloat16* res_out, float* rstd, int d, float eps) {
   after_predecessor();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const int nvec = d >> 3, t = threadIdx.x;
-  bf16x8 a[V], b[RES ? V : 1], wv[V];
+  bf16x8 a[V], b[RES ? V : 1];
 #pragma unroll
   for (int k = 0; k < V; ++k) {
     const int i = t + k * blockDim.x;
     if (i < nvec) {
-      a[k] = ld8(x + row * d + i * 8);
-      if (RES) b[k] = ld8(res_in + row * d + i * 8);
+      a[k] = ld8_once(x + row * d + i * 8);
+      if (RES) b[k] = ld8_once(res_in + row * d + i * 8);
     }
   }
-#pragma unroll
-  for (int k = 0; k < V; ++k)
-    if (t + k * blockDim.x < nvec) wv[k] = ld8(w + (t + k * blockDim.x) * 8);
   float f[V][8], ss = 0.f;
 #pragma unroll
   for (int k = 0; k < V; ++k) {
@@ -74,6 +79,10 @@ __global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* _
     for (int j = 0; j < 8; ++j) ss += h[j] * h[j];
   }
   ss = row_sum(ss, red);
+  bf16x8 wv[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k)
+    if (t + k * blockDim.x < nvec) wv[k] = ld8(w + (t + k * blockDim.x) * 8);
   const float r = rsqrtf(ss / d + eps);
   if (t == 0 && rstd) rstd[row] = r;
 #pragma unroll
@@ -88,10 +97,8 @@ __global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* _
   }
 }
 // Rows longer than 8192: two passes.
-__global__ void __launch_bounds__(256) rmsnorm_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in,
-                                                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                                                               __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd, int d,
-                                                               float eps) {
+__global__ void __launch_bounds__(256) rmsnorm_fwd_long_kernel(const __nv_bfloat16* x, const __nv_bfloat16* res_in, const __nv_bfloat16* w,
+                                                               __nv_bfloat16* y, __nv_bfloat16* res_out, float* rstd, int d, float eps) {
   after_predecessor();
   __shared__ float red[33];
   const long long row = blockIdx.x;
@@ -376,8 +383,7 @@ __device__ __forceinline__ float gate_act_grad(float g, int act) {
   return g > 0.f ? 1.f : 0.f;
 }
 
-__global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ h, long long T,
-                               int F, int act) {
+__global__ void glu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* h, long long T, int F, int act) {
   after_predecessor();
   const int fv = F >> 3;
   const long long total = T * fv;

@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(PA_TILE) paged_decode_kernel(
   }
 }
 
-__global__ void paged_merge_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part,
-                                   __nv_bfloat16* __restrict__ out, long long out_row_stride, int Hq, int D, int nsplit) {
+__global__ void paged_merge_kernel(const float* o_part, const float* ml_part, __nv_bfloat16* out, long long out_row_stride, int Hq, int D,
+                                   int nsplit) {
   after_predecessor();
   const int b = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
   const long long base = ((long long)b * Hq + h) * nsplit;
@@ -177,11 +177,9 @@ __global__ void paged_merge_kernel(const float* __restrict__ o_part, const float
 // Bound: memory (rows read once, queries and keys written back, keys and values written to the pool: 25 us at copy bandwidth for 6044
 // tokens of 32 + 2 x 8 heads). 41 us at that size, 92 us when a warp moved a head two bytes a lane. Few tokens are bound by the
 // chain of position or slot, table and store: 16 tokens of 32 + 2 x 32 heads of 256 4.2 us, 6.2 with one CTA of 512 threads a token.
-__global__ void __launch_bounds__(512) kv_append_vec8_kernel(__nv_bfloat16* __restrict__ qkv, long long row_stride,
-                                                             const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                             const int* __restrict__ pos, const int* __restrict__ slot,
-                                                             __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int T,
-                                                             int Hq, int Hkv, int D, int rotate) {
+__global__ void __launch_bounds__(512) kv_append_vec8_kernel(__nv_bfloat16* qkv, long long row_stride, const float* cos_t, const float* sin_t,
+                                                             const int* pos, const int* slot, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
+                                                             int T, int Hq, int Hkv, int D, int rotate) {
   after_predecessor();
   const int t = blockIdx.x * blockDim.y + threadIdx.y, half = D >> 1, per = D >> 4, items = (Hq + 2 * Hkv) * per;
   if (t >= T) return;

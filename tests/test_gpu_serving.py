@@ -186,6 +186,84 @@ def test_dequant_gemm_repeats_itself(mode, M, N, K):
     assert all(torch.equal(y, ys[0]) for y in ys)
 
 
+@pytest.mark.parametrize("Hq,Hkv,D", [(8, 2, 128), (4, 4, 64)])
+@pytest.mark.parametrize("d", [512, 4096, 8704])
+def test_kernels_that_start_early_keep_the_order_of_the_stream(d, Hq, Hkv, D):
+    """The kernels of a decode step wait for their predecessors inside. Layers of one after the other over the same buffers, for inputs that change,
+    give the bits that the same calls give when each is waited for, launched one by one and as a graph: norms of short, ordinary and long rows,
+    products of bf16 and int4 weights that are fetched early, KV append, both decode kernels (head size 64: not on tensor cores), their merge, SwiGLU."""
+    from sneppx_alg_b200.ops import _lib
+    from sneppx_alg_b200.ops._lib import c_float, c_int, c_ll, ptr, stream
+    from sneppx_alg_b200.ops.gemm import gemm, static_weights
+    torch.manual_seed(d + D)
+    B, L, F, bs, n, rounds = 16, 3, 1024, 16, 700, 4
+    wide = (Hq + 2 * Hkv) * D
+    rand = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    weights = [dict(n1=rand(d), n2=rand(d), qkv=rand(wide, d) * d ** -0.5, o=rand(d, Hq * D) * (Hq * D) ** -0.5, gu=quant.quant_int4(rand(2 * F, d) * d ** -0.5),
+                    down=rand(d, F) * F ** -0.5) for _ in range(L)]
+    blocks = (n + rounds) // bs + 1
+    table = torch.randperm(B * blocks, device="cuda").view(B, blocks).int()
+    caches0 = rand(L, 2, B * blocks, bs, Hkv, D)
+    cos, sin = rope_tables(1024, D, 1e4, "cuda")
+    pos = [torch.full((B,), n + t, dtype=torch.int32, device="cuda") for t in range(rounds)]
+    lens = [p + 1 for p in pos]
+    slots = [table[:, (n + t) // bs] * bs + (n + t) % bs for t in range(rounds)]
+    xs = [rand(B, d) for _ in range(rounds)]
+    hn, out, o, qkv, h = rand(B, d), rand(B, d), rand(B, d), rand(B, wide), rand(B, F)
+    res = [rand(B, d), rand(B, d)]
+    kept, caches = torch.zeros(rounds, 2, B, d, device="cuda").bfloat16(), caches0.clone()
+
+    def run(done):
+        def norm(x, r_in, w, r_out):
+            _lib.call("sx_rmsnorm_fwd", ptr(x), ptr(r_in), ptr(w), ptr(hn), ptr(r_out), ptr(None), c_ll(B), c_int(d), c_float(1e-5), stream())
+            done()
+        with static_weights():
+            for t in range(rounds):
+                out.copy_(xs[t])
+                res[0].zero_()
+                for w, (kc, vc) in zip(weights, caches):
+                    norm(out, res[0], w["n1"], res[1])
+                    gemm(hn, w["qkv"], out=qkv)
+                    done()
+                    paged.kv_append_(qkv, cos, sin, pos[t], slots[t], kc, vc, Hq, Hkv, D)
+                    done()
+                    a = paged.paged_decode(qkv[:, :Hq * D].view(B, Hq, D), kc, vc, table, lens[t])
+                    done()
+                    gemm(a.view(B, -1), w["o"], out=o)
+                    done()
+                    norm(o, res[1], w["n2"], res[0])
+                    gu = quant.gemm_dequant(hn, *w["gu"], "int4")
+                    done()
+                    _lib.call("sx_glu_fwd", ptr(gu), ptr(h), c_ll(B), c_int(F), c_int(0), stream())
+                    done()
+                    gemm(h, w["down"], out=out)
+                    done()
+                kept[t, 0].copy_(out)
+                kept[t, 1].copy_(res[0])
+
+    def result():
+        torch.cuda.synchronize()
+        ops.check_status()
+        both = kept.clone(), caches.clone()
+        kept.zero_()
+        caches.copy_(caches0)
+        return both
+
+    run(torch.cuda.synchronize)
+    want = result()
+    assert bool(want[0].isfinite().all())
+    for _ in range(3):
+        run(lambda: None)
+        assert all(torch.equal(a, e) for a, e in zip(result(), want))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(lambda: None)
+    result()
+    for _ in range(3):
+        graph.replay()
+        assert all(torch.equal(a, e) for a, e in zip(result(), want))
+
+
 def test_dequant_gemm_of_short_rows_keeps_up_with_its_output():
     """16384 x 4096 outputs of K = 128 are bound by writing 134 MB: two to four times a copy's time, ten when every tile was a CTA of its own."""
     x, q, s, _, _ = _dequant_case("int4", 16384, 4096, 128, False)

@@ -1,0 +1,27 @@
+"""Rules for the CUDA sources that no compiler checks."""
+import re
+
+from sneppx_alg_b200 import _build
+
+
+def _kernels(text):
+    """(name, parameters, body) of the __global__ functions of a source file."""
+    for m in re.finditer(r"__global__\s+void\s+(?:__cluster_dims__\([^)]*\)\s*)?(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(([^)]*)\)\s*\{", text):
+        yield m.group(1), m.group(2), text[m.end():text.find("\n}\n", m.end())]
+
+
+def test_kernels_that_start_early_promise_nothing_about_their_inputs():
+    """A kernel that waits for its predecessor inside (griddepcontrol.wait) runs while that one still writes: a __restrict__ pointer would tell the
+    compiler that nobody does, and let it load ahead of the wait. And whatever is launched that way waits."""
+    waiting, launched = {}, set()
+    for src in _build.cuda_sources():
+        text = re.sub(r"//[^\n]*", "", src.read_text())
+        for name, params, body in _kernels(text):
+            if re.search(r"after_predecessor\(\)|griddepcontrol\.wait|griddep_wait\(\)", body):
+                waiting[name] = params
+        launched |= set(re.findall(r"launch_dependent\((\w+_kernel)", text))
+        for m in re.finditer(r"auto run = \[&\]\(auto kern[^{]*\{\s*launch_dependent\(kern", text):
+            launched |= set(re.findall(r"run\((\w+_kernel)", text[m.end():m.end() + 2000].split('\nextern "C"')[0]))
+    assert {"rmsnorm_fwd_kernel", "rmsnorm_fwd_long_kernel", "glu_fwd_kernel", "paged_merge_kernel", "kv_append_vec8_kernel", "paged_decode_tc_kernel"} <= launched
+    assert {"gemm_skinny_kernel", "gemm_dq_kernel", "mamba_step_kernel"} <= set(waiting) and launched <= set(waiting)
+    assert not [n for n, params in waiting.items() if "__restrict__" in params]
