@@ -215,7 +215,10 @@ __global__ void __launch_bounds__(SF_THREADS, 1) ssd_chunk_fwd_kernel(const __gr
       __syncwarp();
       if (lane == 0) mbar_arrive(&m_full[grp]);
       // ---- epilogue of this head
-      if (!mbar_wait_warp(&y_full[grp], n & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; continue; }
+      // x is read from the tile that TMA brought: its own barrier is waited for, too, which the product's end does not stand for (it has flipped by then,
+      // and flips again only when these warps have freed the tile)
+      if (!mbar_wait_warp(&y_full[grp], n & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE) ||
+          !mbar_wait_warp(&xh_full[grp], n & 1, s_abort, p.status, ST_TIMEOUT_EPILOGUE)) { ok = false; continue; }
       tc_fence_after();
       const float e = __expf(cs_l);
       const float dh = p.D ? p.D[h] : 0.f;

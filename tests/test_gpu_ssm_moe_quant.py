@@ -150,6 +150,37 @@ def test_ssd_chunk_kernel_deals_heads_out(H, G):
     assert bool(((ys[0][0].double() - sum(terms)).abs() <= 2.0 ** -8 * size + 1e-6).all())
 
 
+@pytest.mark.parametrize("H,G", [(24, 1), (80, 8)])
+def test_ssd_chunk_kernel_repeats_itself(H, G):
+    """The skip connection reads x from the tile that TMA brought while other tiles are on their way: calls over rows that change in between, one
+    behind the other, give the bits of calls that are waited for. The skip connection outweighs the rest a thousand times, so that a row which came late shows."""
+    from sneppx_alg_b200.ops._lib import c_int, c_ll, ptr, stream
+    torch.manual_seed(H)
+    Q, P, N, bc = 128, 64, 128, 40
+    u = [torch.randn(bc * Q, H * P + 2 * G * N, device="cuda").bfloat16() for _ in range(4)]
+    W, state = u[0].shape[1], torch.randn(bc, H, P, N, device="cuda").bfloat16()
+    dt = torch.rand(bc, H, Q, device="cuda") * 0.1
+    cs, D = torch.cumsum(-dt, -1), 1000 * torch.randn(H, device="cuda")
+    rows = torch.empty_like(u[0])
+
+    def call(x):
+        rows.copy_(x)
+        y = torch.empty(bc * Q, H * P, dtype=torch.bfloat16, device="cuda")
+        _lib.call("sx_ssd_chunk_fwd", ptr(rows[:, H * P + G * N:]), c_ll(W), ptr(rows[:, H * P:]), c_ll(W), ptr(rows), c_ll(W), ptr(state), ptr(cs), ptr(dt),
+                  ptr(D), ptr(y), c_ll(bc), c_int(H), c_int(G), ptr(_lib.status_word("cuda")), stream())
+        return y
+
+    want = []
+    for x in u:
+        want.append(call(x))
+        torch.cuda.synchronize()
+    got = [call(u[i % 4]) for i in range(24)]
+    _lib.check_status()
+    assert all(torch.equal(y, want[i % 4]) for i, y in enumerate(got))
+    skip = D.repeat_interleave(P) * u[0][:, :H * P].float()
+    assert (want[0].float() - skip).norm() < 0.02 * skip.norm()
+
+
 def test_router_and_moe_layer():
     torch.manual_seed(0)
     T, d, E, k, Fd = 1000, 256, 16, 4, 192

@@ -25,3 +25,11 @@ def test_kernels_that_start_early_promise_nothing_about_their_inputs():
     assert {"rmsnorm_fwd_kernel", "rmsnorm_fwd_long_kernel", "glu_fwd_kernel", "paged_merge_kernel", "kv_append_vec8_kernel", "paged_decode_tc_kernel"} <= launched
     assert {"gemm_skinny_kernel", "gemm_dq_kernel", "mamba_step_kernel"} <= set(waiting) and launched <= set(waiting)
     assert not [n for n, params in waiting.items() if "__restrict__" in params]
+
+
+def test_ssd_output_stage_waits_for_the_tile_that_its_epilogue_reads():
+    """The epilogue warps read x from shared memory that TMA filled: they wait for that transfer's barrier themselves, not only for the product's."""
+    text = (_build.CSRC / "ssd_fwd.cu").read_text()
+    body = next(body for name, _, body in _kernels(text) if name == "ssd_chunk_fwd_kernel")
+    epilogue = body[body.index("epilogue of this head"):]
+    assert epilogue.index("mbar_wait_warp(&xh_full[grp], n & 1") < epilogue.index("const uint8_t* xrow = sX")
