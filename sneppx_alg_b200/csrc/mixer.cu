@@ -36,13 +36,13 @@ namespace sx {
 
 typedef uint16_t h16;   // bf16 storage
 
-// One walk over the sequence: with `run` off it only adds up the scratch.
+// One walk over the sequence: with `run` off it only finds out how much scratch it takes.
 struct Mixer {
   const SxMixerArgs& a;
   cudaStream_t st;
   const bool run;
   int rc = 0;
-  long long used = 0;
+  long long used = 0;   // bytes of scratch
   // sizes: chunks of a sequence, (chunk, group) matrices, heads of a group, inner width, convolution channels, projection width
   const int nc, rep, di, C;
   const long long n, W, Lp, BC, rP;
@@ -52,12 +52,31 @@ struct Mixer {
         C(args.H * args.P + 2 * args.G * args.N), n((long long)args.B * nc * args.G), W((long long)di + C + args.H), Lp((long long)nc * args.Q),
         BC((long long)args.B * nc), rP((long long)rep * args.P) {}
 
+  // Buffers in the order of their addresses: take() fills the first gap that is wide enough, drop() gives one back when the last launch that reads it
+  // has been issued (they run one after another).
+  struct Range { long long at, end; } held[48];
+  int n_held = 0;
+  char* base() const { return a.work ? static_cast<char*>(a.work) : reinterpret_cast<char*>(256); }   // without scratch: sizes only
   template <typename T>
   T* take(long long count) {
-    T* p = a.work ? reinterpret_cast<T*>(static_cast<char*>(a.work) + used) : nullptr;
-    used += (count * (long long)sizeof(T) + 255) / 256 * 256;
-    return p;
+    const long long bytes = (count * (long long)sizeof(T) + 255) / 256 * 256;
+    long long at = 0;
+    int i = 0;
+    for (; i < n_held && held[i].at - at < bytes; ++i) at = held[i].end;
+    if (n_held == (int)(sizeof(held) / sizeof(held[0]))) { rc = -3; return nullptr; }
+    for (int j = n_held++; j > i; --j) held[j] = held[j - 1];
+    held[i] = {at, at + bytes};
+    if (at + bytes > used) used = at + bytes;
+    return reinterpret_cast<T*>(base() + at);
   }
+  void drop(const void* p) {
+    int i = 0;
+    while (i < n_held && base() + held[i].at != p) ++i;
+    if (i == n_held) { rc = -3; return; }
+    for (--n_held; i < n_held; ++i) held[i] = held[i + 1];
+  }
+  template <typename... P>
+  void drop(const void* p, P... more) { drop(p); drop(more...); }
   template <typename F>
   void go(F&& f) {
     if (run && rc == 0) rc = f();
@@ -125,9 +144,12 @@ struct Mixer {
     go([&] { return sx_conv1d_fwd((const h16*)a.zx + di, nullptr, a.conv_w, a.conv_b, a.xbc, nullptr, a.B, a.L, C, a.K, 1, W, (int)Lp, st); });
     prep();
     float* S = take<float>(n * rP * N);
-    gemm(dense(scaled_rows(), Q, rP, true), mn(Bg), S, rP, N, Q, n, true);
+    h16* xw = scaled_rows();
+    gemm(dense(xw, Q, rP, true), mn(Bg), S, rP, N, Q, n, true);
+    drop(xw, decay);
     float* fin = take<float>((long long)a.B * H * P * N);
     go([&] { return sx_ssd_state_fwd(S, tot, nullptr, a.hprev, fin, a.B, nc, H, P * N, st); });
+    drop(S, fin);
     const h16* x = (const h16*)a.xbc;
     if (a.fused) {
       go([&] { return sx_ssd_chunk_fwd(x + di + a.G * N, C, x + di, C, x, C, a.hprev, csh, dth, a.D, a.y, BC, H, a.G, a.status, st); });
@@ -136,8 +158,11 @@ struct Mixer {
       gemm(Cg, Bg, CB, Q, Q, N, n, true);
       h16* M = take<h16>(BC * H * Q * Q);
       go([&] { return sx_ssd_build_m(CB, csh, dth, M, BC, H, a.G, Q, st); });
-      h16 *xh = heads_first(x, C), *Yi = take<h16>(BC * Q * di), *Yo = take<h16>(BC * Q * di);
+      drop(CB);
+      h16 *xh = heads_first(x, C), *Yi = take<h16>(BC * Q * di);
       gemm(dense(M, Q, Q), dense(xh, Q, P, true), Yi, Q, P, Q, BC * H, false);
+      drop(M, xh);
+      h16* Yo = take<h16>(BC * Q * di);
       gemm(Cg, dense(a.hprev, rP, N), Yo, Q, rP, N, n, false);
       go([&] { return sx_ssd_combine(Yi, Yo, x, E, a.D, a.y, BC * Q * H, H, Q, P, C, a.G, st); });
     }
@@ -157,29 +182,38 @@ struct Mixer {
     float *dcs = take<float>(vec), *ddrow = take<float>(vec);
     gemm(Cg, dense(a.hprev, rP, N), Yo, Q, rP, N, n, false);
     go([&] { return sx_ssd_bwd_rows1(dy, x, Yo, E, dye, dcs, ddrow, vec, P, H, C, Q, a.G, st); });
+    drop(Yo, E);
     float *dC = take<float>(n * Q * N), *dHp = take<float>(states);
     gemm(dense(dye, Q, rP), dense(a.hprev, rP, N, true), dC, Q, N, rP, n, true);
     gemm(dense(dye, Q, rP, true), mn(Cg), dHp, rP, N, Q, n, true);
+    drop(dye);
     h16* dS = take<h16>(states);
     float *dtot = take<float>(BC * H), *dinit = take<float>((long long)a.B * H * P * N);
     if (run) check(cudaMemsetAsync(dtot, 0, BC * H * sizeof(float), st));
     go([&] { return sx_ssd_state_bwd(dHp, tot, a.hprev, nullptr, dS, dtot, dinit, a.B, nc, H, P * N, st); });
+    drop(dHp, dinit);
     h16* dxw = take<h16>(toks);
     gemm(Bg, dense(dS, rP, N), dxw, Q, rP, N, n, false);
     float* dB = take<float>(n * Q * N);
-    gemm(dense(scaled_rows(), Q, rP), dense(dS, rP, N, true), dB, Q, N, rP, n, true);
+    h16* xw = scaled_rows();
+    gemm(dense(xw, Q, rP), dense(dS, rP, N, true), dB, Q, N, rP, n, true);
+    drop(xw, dS);
     // quadratic term within the chunk
     h16 *dyh = heads_first(dy, di), *xh = heads_first(x, C), *dM = take<h16>(BC * H * Q * Q);
     gemm(dense(dyh, Q, P), dense(xh, Q, P), dM, Q, Q, P, BC * H, false);
+    drop(xh);
     float *CB = take<float>(n * Q * Q), *rowW = take<float>(vec), *colU = take<float>(vec);
     gemm(Cg, Bg, CB, Q, Q, N, n, true);
     h16 *M = take<h16>(BC * H * Q * Q), *dGh = take<h16>(BC * H * Q * Q);
     go([&] { return sx_ssd_bwd_qq(dM, CB, csh, dth, M, dGh, rowW, colU, BC, H, a.G, Q, st); });
+    drop(dM, CB);
     h16* dxi = take<h16>(toks);
     gemm(dense(M, Q, Q, true), dense(dyh, Q, P, true), dxi, Q, P, Q, BC * H, false);
+    drop(M, dyh);
     h16* dxbc = take<h16>(BC * Q * C);
     float* ddecay = take<float>(vec);
     go([&] { return sx_ssd_bwd_rows2(dy, x, dxw, dxi, decay, a.D, dxbc, ddecay, vec, H, Q, P, C, a.G, C, st); });
+    drop(dy, dxw, dxi);
     const h16* dG = dGh;
     if (rep > 1) {
       h16* sum = take<h16>(n * Q * Q);
@@ -210,6 +244,7 @@ static int mixer_call(const SxMixerArgs& a, cudaStream_t st, bool back) {
   if (!mixer_ok(a) || !a.work) return -1;
   Mixer size(a, st, false);
   back ? size.backward() : size.forward();
+  if (size.rc) return size.rc;
   if (size.used > a.work_bytes) return -2;
   Mixer m(a, st, true);
   back ? m.backward() : m.forward();
@@ -223,7 +258,7 @@ extern "C" long long sx_mixer_workspace(const SxMixerArgs* a, int backward) {
   if (!sx::mixer_ok(*a)) return -1;
   sx::Mixer m(*a, nullptr, false);
   backward ? m.backward() : m.forward();
-  return m.used;
+  return m.rc ? m.rc : m.used;
 }
 extern "C" int sx_mixer_fwd(const SxMixerArgs* a, cudaStream_t st) { return sx::mixer_call(*a, st, false); }
 extern "C" int sx_mixer_bwd(const SxMixerArgs* a, cudaStream_t st) { return sx::mixer_call(*a, st, true); }

@@ -537,13 +537,13 @@ class _MixerFn(torch.autograd.Function):
     the scan's output and the chunk-entry states."""
 
     @staticmethod
-    def _native(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D, sizes):
+    def _native(zx, xbc, conv_w, conv_b, dt_bias, A_log, D, sizes):
         """Arguments of the whole sequence as one call (csrc/mixer.cu), for the sizes that it takes; else None."""
         H, P, G, N, Q = sizes
         if Q not in (64, 128) or P % 64 or N % 64 or _dbg.ENABLED:
             return None
         a = _lib.SxMixerArgs()
-        a.zx, a.xbc, a.y, a.hprev = zx.data_ptr(), xbc.data_ptr(), y.data_ptr(), Hprev.data_ptr()
+        a.zx, a.xbc = zx.data_ptr(), xbc.data_ptr()
         a.conv_w, a.conv_b, a.dt_bias, a.a_log, a.D = (t.data_ptr() for t in (conv_w, conv_b, dt_bias, A_log, D))
         a.B, a.L = zx.shape[:2]
         a.H, a.P, a.G, a.N, a.Q, a.K = H, P, G, N, Q, conv_w.shape[1]
@@ -591,11 +591,11 @@ class _MixerFn(torch.autograd.Function):
         Lp, di, K, dev, cdt = nc * Q, H * P, conv_w.shape[1], zx.device, zx.dtype
         C = di + 2 * G * N
         xbc = torch.empty(B_, Lp, C, dtype=cdt, device=dev)
-        y, Hprev = torch.empty(B_, Lp, di, dtype=cdt, device=dev), torch.empty(B_, nc, H, P, N, dtype=cdt, device=dev)
-        a = _MixerFn._native(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D, sizes)
+        a = _MixerFn._native(zx, xbc, conv_w, conv_b, dt_bias, A_log, D, sizes)
         if a is not None:
+            y, Hprev = torch.empty(B_, Lp, di, dtype=cdt, device=dev), torch.empty(B_, nc, H, P, N, dtype=cdt, device=dev)
             out = torch.empty(B_, L, di, dtype=cdt, device=dev)
-            a.out = out.data_ptr()
+            a.y, a.hprev, a.out = y.data_ptr(), Hprev.data_ptr(), out.data_ptr()
             _MixerFn._native_call(a, "sx_mixer_fwd", 0, dev)
             ctx.save_for_backward(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D)
             ctx.sizes = sizes
@@ -612,6 +612,7 @@ class _MixerFn(torch.autograd.Function):
         S = gemm(xw, Bg, a_mn=True, b_mn=True, out_dtype=torch.float32)
         Hprev, _ = _state_fwd(S.view(B_, nc, H, P, N), tot, None, cdt)
         if Q == 128 and N == 128 and P == 64 and os.environ.get("SX_SSD_FUSED", "1") != "0":
+            y = torch.empty(B_, Lp, di, dtype=cdt, device=dev)
             Cm, Bm = xbc[..., di + G * N:], xbc[..., di:]
             _lib.call("sx_ssd_chunk_fwd", ptr(Cm), c_ll(C), ptr(Bm), c_ll(C), ptr(xbc), c_ll(C), ptr(Hprev), ptr(csh), ptr(dth), ptr(D), ptr(y),
                       c_ll(B_ * nc), c_int(H), c_int(G), _lib.c_void_p(_lib.status_word(dev).data_ptr()), stream())
@@ -636,9 +637,10 @@ class _MixerFn(torch.autograd.Function):
         f32 = torch.float32
         g = g.contiguous()
         dzx = torch.empty(B_, L, W, dtype=cdt, device=dev)
-        a = _MixerFn._native(zx, xbc, y, Hprev, conv_w, conv_b, dt_bias, A_log, D, ctx.sizes)
+        a = _MixerFn._native(zx, xbc, conv_w, conv_b, dt_bias, A_log, D, ctx.sizes)
         if a is not None:
             dwdb, part = torch.empty((K + 1) * C, dtype=f32, device=dev), torch.empty(3, B_ * nc, H, dtype=f32, device=dev)
+            a.y, a.hprev = y.data_ptr(), Hprev.data_ptr()
             a.g, a.dzx, a.dwdb, a.part = g.data_ptr(), dzx.data_ptr(), dwdb.data_ptr(), part.data_ptr()
             _MixerFn._native_call(a, "sx_mixer_bwd", 1, dev)
             dA, dD, dbias = part.sum(1)

@@ -409,6 +409,33 @@ def test_mixer_in_one_call_is_the_mixer_by_entry_points(monkeypatch, B, L, H, P,
     assert close(z1, z0) and all(a.dtype == b.dtype and close(a, b) for a, b in zip(rest1, rest0))
 
 
+def test_mixer_in_one_call_holds_no_more_memory(monkeypatch):
+    """Scratch of the pass as one call against that of its entry points one by one, at a size where both are far above the allocator's rounding."""
+    torch.manual_seed(0)
+    B, L, H, P, G, N = 1, 4096, 40, 64, 4, 128
+    di, C = H * P, H * P + 2 * G * N
+    zx = torch.randn(B, L, di + C + H, device="cuda").bfloat16().requires_grad_()
+    args = [zx, (0.5 * torch.randn(C, 4, device="cuda")).bfloat16(), torch.randn(C, device="cuda").bfloat16(), torch.randn(H, device="cuda") - 3,
+            torch.rand(H, device="cuda"), torch.randn(H, device="cuda")]
+    g, peaks = torch.randn(B, L, di, device="cuda").bfloat16(), []
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(ssm._MixerFn, "_native", staticmethod(lambda *a: None))
+        for step in range(2):
+            torch.cuda.empty_cache()
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            y = ssm.mamba2_mixer(*args, H, P, G, N)
+            forward = torch.cuda.max_memory_allocated() - before
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            torch.autograd.grad(y, zx, g)
+            backward = torch.cuda.max_memory_allocated() - before
+            del y
+        peaks.append((forward, backward))
+    assert all(a <= b for a, b in zip(*peaks)), peaks
+
+
 @pytest.mark.parametrize("C,L,Lp,wide", [(64, 1, 1, False), (1536, 1, 1, True), (320, 7, 7, True), (320, 7, 8, True), (64, 33, 64, False)])
 def test_gate_mul_padded_rows(C, L, Lp, wide):
     """Dense and wider gradients of z, y with rows behind each sequence that are neither read nor written. 32-bit arithmetic and one bf16 rounding;

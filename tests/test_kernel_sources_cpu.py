@@ -1,7 +1,11 @@
-"""Rules for the CUDA sources that no compiler checks."""
+"""Rules for the CUDA sources that no compiler checks, and host code of the library that needs no GPU."""
+import ctypes
 import re
 
+import pytest
+
 from sneppx_alg_b200 import _build
+from sneppx_alg_b200.ops import _lib
 
 
 def _kernels(text):
@@ -33,3 +37,20 @@ def test_ssd_output_stage_waits_for_the_tile_that_its_epilogue_reads():
     body = next(body for name, _, body in _kernels(text) if name == "ssd_chunk_fwd_kernel")
     epilogue = body[body.index("epilogue of this head"):]
     assert epilogue.index("mbar_wait_warp(&xh_full[grp], n & 1") < epilogue.index("const uint8_t* xrow = sX")
+
+
+@pytest.mark.parametrize("B,L,H,P,G,N,Q", [(1, 8192, 80, 64, 8, 128, 128), (4, 8192, 80, 64, 8, 128, 128), (4, 500, 24, 64, 1, 128, 128), (1, 4096, 16, 128, 1, 64, 128),
+                                           (2, 60, 8, 64, 2, 64, 64)])
+def test_mixer_scratch_is_used_again(B, L, H, P, G, N, Q):
+    """The backward of the mixer as one call takes no more scratch than its stages one by one hold while they work on the Q x Q matrices, where
+    they hold the most: dy, dye, dxw and dy by heads; dM, M and dG; the chunk states' gradients in 32 and 16 bits; dB, dC, C B^T, B and C by
+    group; eight vectors. Every buffer is rounded up to 256 bytes."""
+    nc = (L + Q - 1) // Q
+    n, vec = B * nc * G, B * nc * Q * H
+    held = 4 * vec * P * 2 + 3 * vec * Q * 2 + vec // Q * P * N * 6 + n * Q * (2 * N * 4 + Q * 4 + 2 * N * 2) + 8 * vec * 4
+    size = _lib.lib().sx_mixer_workspace
+    size.restype = ctypes.c_longlong
+    a = _lib.SxMixerArgs()
+    a.B, a.L, a.H, a.P, a.G, a.N, a.Q, a.K, a.fused = B, L, H, P, G, N, Q, 4, int((Q, N, P) == (128, 128, 64))
+    back, forward = size(ctypes.byref(a), 1), size(ctypes.byref(a), 0)
+    assert 0 < forward < back <= held + 40 * 256, (back, held)
