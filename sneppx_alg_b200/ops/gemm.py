@@ -219,7 +219,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, out_dtype=None, c=None, beta
     args.M, args.N, args.K, args.batch = M, N, K, batch
     args.lda, args.ldb, args.ldd = lda, ldb, ldd
     args.strideA, args.strideB, args.strideD = sA, sB, sD
-    args.a_mn, args.b_mn = a_mn, b_mn
+    args.a_mn, args.b_mn = int(a_mn), int(b_mn)      # numpy truth values, too
     args.out_fp32 = out.dtype == torch.float32
     if c is not None:          # fields that are not set are zero
         if beta != 0.0:

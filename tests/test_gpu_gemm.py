@@ -138,3 +138,12 @@ def test_gemm_mn_major_a_with_ragged_rows():
     gemm(g, x, a_mn=True, b_mn=True, out=acc, c=acc, beta=1.0)
     ops.check_status()
     assert _rel(acc, want) < 1e-2
+
+
+def test_gemm_takes_truth_values_of_numpy():
+    """Layouts read off numpy arrays are numpy's truth values."""
+    import numpy as np
+    torch.manual_seed(0)
+    a, b = (torch.randn(128, 192, device="cuda").bfloat16() for _ in range(2))
+    assert torch.equal(gemm(a, b, a_mn=np.True_, b_mn=np.True_), gemm(a, b, a_mn=True, b_mn=True))
+    assert torch.equal(gemm(a, b, a_mn=np.False_, b_mn=np.bool_(False)), gemm(a, b))
