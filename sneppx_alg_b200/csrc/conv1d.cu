@@ -18,8 +18,9 @@ __device__ __forceinline__ float silu_grad(float x) {
   return s * (1.f + x * (1.f - s));
 }
 
-// V channels of a row: 4 (8 bytes) or 2.
+// V channels of a row: 8 (16 bytes), 4 or 2.
 template <int V> struct ConvVec;
+template <> struct ConvVec<8> { typedef uint4 T; };
 template <> struct ConvVec<4> { typedef uint2 T; };
 template <> struct ConvVec<2> { typedef uint32_t T; };
 __device__ __forceinline__ float2 bf2(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); }
@@ -31,10 +32,15 @@ __device__ __forceinline__ void conv_unpack(uint2 r, float (&f)[4]) {
   const float2 a = bf2(r.x), b = bf2(r.y);
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
 }
+__device__ __forceinline__ void conv_unpack(uint4 r, float (&f)[8]) {
+  const float2 a = bf2(r.x), b = bf2(r.y), c = bf2(r.z), d = bf2(r.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
 __device__ __forceinline__ void conv_unpack(uint32_t r, float (&f)[2]) {
   const float2 a = bf2(r);
   f[0] = a.x; f[1] = a.y;
 }
+__device__ __forceinline__ uint4 conv_pack(const float (&f)[8]) { return make_uint4(pk2(f[0], f[1]), pk2(f[2], f[3]), pk2(f[4], f[5]), pk2(f[6], f[7])); }
 __device__ __forceinline__ uint2 conv_pack(const float (&f)[4]) { return make_uint2(pk2(f[0], f[1]), pk2(f[2], f[3])); }
 __device__ __forceinline__ uint32_t conv_pack(const float (&f)[2]) { return pk2(f[0], f[1]); }
 template <int V> __device__ __forceinline__ typename ConvVec<V>::T conv_ld(const __nv_bfloat16* p) {
@@ -63,21 +69,21 @@ __device__ __forceinline__ void conv_taps(const __nv_bfloat16* w, int c, float (
   }
 }
 
-// One thread: 4 channels x `run` consecutive positions. The K taps and the bias live in registers and the K-1 previous inputs slide through
-// registers, so each input vector is loaded once and each output costs one load and one store of 4 channels; consecutive threads own consecutive
+// One thread: V channels (4, or 8 with one tap, see sx_conv1d_fwd) x `run` consecutive positions. The K taps and the bias live in registers and the K-1 previous inputs slide through
+// registers, so each input vector is loaded once and each output costs one load and one store of V channels; consecutive threads own consecutive
 // channel vectors (coalesced rows).
 // Bound: the instructions of a row (half of them the sigmoid), so pairs of channels go through one packed multiply-add, rounded like two scalar
 // ones, and the rows that no state is made of are a loop without conditions. Cold, scalar with conditions -> now, four taps: [8192, 7168]
 // 79.9 -> 67.6 us (36 at copy bandwidth), [8192, 5376] 63.5 -> 55.3, [16, 4096, 4352] 348 -> 263, [4, 2048, 1792] 30.7 -> 26.6; [8192, 7168] with
 // three taps 70 -> 63.5, two 59 -> 51, one 53 either way. Three CTAs an SM: four (64 registers) spill 64 bytes and take 71.7 us with three or four
 // taps, but 51 instead of 57 with two. A 32-bit division for the index spills as well (77.8 us).
-template <int K>
-__global__ void __launch_bounds__(256, K >= 3 ? 3 : 4) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ prev,
+template <int K, int V>
+__global__ void __launch_bounds__(256, V == 8 || K >= 3 ? 3 : 4) conv1d_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ prev,
                                                             const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
                                                             __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ state_out, int B,
                                                             int L, int C, int act, long long xld, int Ly, int run) {
-  typedef uint2 T;
-  constexpr int V = 4, P = V / 2;
+  typedef typename ConvVec<V>::T T;
+  constexpr int P = V / 2;
   const unsigned cv = C / V, lchunks = (L + run - 1) / run;
   const long long total = (long long)B * lchunks * cv;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
@@ -224,8 +230,11 @@ __global__ void __launch_bounds__(256, 3) conv1d_short_kernel(const __nv_bfloat1
 // only warm up, only finish or do both are loops of their own. [8192, 7168], four taps: 159 us, 247 with two scalar channels and conditions in
 // every row, 265 with four channels and fewer warps (54 us at copy bandwidth).
 // The 8 warps add their dw / db into shared memory and the CTA writes one partial row; conv1d_reduce_partials sums the rows.
-template <int K>
-__global__ void __launch_bounds__(256, K == 4 ? 4 : 3) conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+// One tap: rows one by one and four CTAs an SM ([8192, 7168] 82 and 89 us with SiLU; 92 and 98 four at a time, 88 and 98 scalar). FEW: sequences of
+// fewer than CONV_FEW positions, without the loop of four (512 of one position and 7168 channels, four taps: 27.7 us, 32 with it, 28.4 scalar).
+constexpr int CONV_FEW = 5;
+template <int K, bool FEW>
+__global__ void __launch_bounds__(256, K == 4 || K == 1 ? 4 : 3) conv1d_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ prev, const __nv_bfloat16* __restrict__ w,
                                                             const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ dx,
                                                             float* __restrict__ partial, int B, int L, int C, int act, long long xld, int Ly,
@@ -302,15 +311,17 @@ __global__ void __launch_bounds__(256, K == 4 ? 4 : 3) conv1d_bwd_kernel(const _
           sums();
           xp += xld; gp += C; ++l;
         }
-      for (; l + 4 <= lend; l += 4) {
-        uint32_t xr[4], gr[4];
+      if constexpr (!FEW) {
+        for (; l + 4 <= lend; l += 4) {
+          uint32_t xr[4], gr[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u, xp += xld, gp += C) { xr[u] = conv_ld<2>(xp); gr[u] = conv_ld<2>(gp); }
+          for (int u = 0; u < 4; ++u, xp += xld, gp += C) { xr[u] = conv_ld<2>(xp); gr[u] = conv_ld<2>(gp); }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          enter(xr[u], gr[u]);
-          sums();
-          leave();
+          for (int u = 0; u < 4; ++u) {
+            enter(xr[u], gr[u]);
+            sums();
+            leave();
+          }
         }
       }
       for (; l < lend; ++l, xp += xld, gp += C) {
@@ -370,22 +381,26 @@ extern "C" int sx_conv1d_fwd(const void* x, const void* prev, const void* w, con
                              int B, int L, int C, int K, int act, long long xld, int Ly, cudaStream_t st) {
   if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L) return -1;
   if ((long long)B * L * C == 0) return 0;
+  const bool few = L < CONV_SHORT;
+  // With one tap a row is hardly more than its load and its store: from here on, where x and y outgrow L2, 16-byte ones are better ([8192, 7168] 40.2
+  // and 43.4 us, with SiLU 43.8 and 46.4; [8192, 1792] 8.4 and 7.6).
+  const bool wide = K == 1 && !few && (long long)B * L * C >= 1ll << 25 &&
+                    ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0;
+  const int V = wide ? 8 : 4;
   // Runs of 32 read fewer rows twice, but only where they still fill the SMs twice over ([8192, 7168] 71.7 us with 16, 67.6 with 32; [4, 500, 1792]
-  // 14 and 18).
-  const long long threads = (long long)B * ((L + 31) / 32) * (C / 4);
-  const int run = threads >= 2ll * 148 * 768 ? 32 : 16;
+  // 14 and 18). With one tap no row is read twice.
+  const int run = K > 1 && (long long)B * ((L + 31) / 32) * (C / 4) >= 2ll * 148 * 768 ? 32 : 16;
   auto go = [&](auto kern, auto... more) {
-    const long long blocks = ((long long)B * (sizeof...(more) ? (L + run - 1) / run : 1) * (C / 4) + 255) / 256;
+    const long long blocks = ((long long)B * (sizeof...(more) ? (L + run - 1) / run : 1) * (C / V) + 255) / 256;
     kern<<<(int)(blocks < 148 * 1024 ? blocks : 148 * 1024), 256, 0, st>>>(
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)prev, (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y,
         (__nv_bfloat16*)state_out, B, L, C, act, xld, Ly, more...);
   };
-  const bool few = L < CONV_SHORT;
   switch (K) {
-    case 1: go(conv1d_fwd_kernel<1>, run); break;
-    case 2: few ? go(conv1d_short_kernel<2>) : go(conv1d_fwd_kernel<2>, run); break;
-    case 3: few ? go(conv1d_short_kernel<3>) : go(conv1d_fwd_kernel<3>, run); break;
-    default: few ? go(conv1d_short_kernel<4>) : go(conv1d_fwd_kernel<4>, run); break;
+    case 1: few ? go(conv1d_short_kernel<1>) : wide ? go(conv1d_fwd_kernel<1, 8>, run) : go(conv1d_fwd_kernel<1, 4>, run); break;
+    case 2: few ? go(conv1d_short_kernel<2>) : go(conv1d_fwd_kernel<2, 4>, run); break;
+    case 3: few ? go(conv1d_short_kernel<3>) : go(conv1d_fwd_kernel<3, 4>, run); break;
+    default: few ? go(conv1d_short_kernel<4>) : go(conv1d_fwd_kernel<4, 4>, run); break;
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
@@ -396,14 +411,15 @@ static int conv_bwd_run(int B, int L, int C) { return (long long)B * ((L + 63) /
 
 // Number of partial rows the backward kernel writes for B sequences of L tokens of C channels.
 extern "C" int sx_conv1d_bwd_parts(int B, int L, int C) {
-  // four runs per warp (32 per CTA): the per-CTA prologue (taps, bias) and epilogue (partial row) cost about as much
-  // as one run. Inputs that would leave SMs idle that way take as many CTAs as make one wave, down to one
+  // 64 positions per warp, four runs of 16 or one of 64: the per-CTA prologue (taps, bias) and epilogue (partial row) cost about as much as 16.
+  // Sequences of few positions are counted by those, longer ones by the runs of 16 that they would have (512 sequences of one position and 7168
+  // channels: 27.7 us, 47 counted as runs of 64). Inputs that would leave SMs idle that way take as many CTAs as make one wave, down to one
   // run per warp ([4, 500, 1792]: 73 -> 32 us)
   const int run = conv_bwd_run(B, L, C);
   const long long chunks = (long long)B * ((L + run - 1) / run);
   const int cols = (C / 2 + 31) / 32;             // four CTAs an SM
   const long long wave = 148 * 4 / (cols > 0 ? cols : 1), most = (chunks + 7) / 8;
-  long long p = (chunks * run / 16 + 31) / 32;
+  long long p = ((L < CONV_FEW ? ((long long)B * L + 15) / 16 : (long long)B * ((L + 15) / 16)) + 31) / 32;
   if (p < wave) p = most < wave ? most : wave;
   if (p > most) p = most;
   return (int)(p < 1 ? 1 : (p > 512 ? 512 : p));
@@ -417,16 +433,17 @@ extern "C" int sx_conv1d_bwd(const void* dy, const void* x, const void* prev, co
   if (C % 8 || K > CONV_MAXK || K < 1 || xld % 8 || xld < C || Ly < L || dxld % 4 || dxld < C) return -1;
   if ((long long)B * L == 0) return 0;
   const int parts = sx_conv1d_bwd_parts(B, L, C);
+  const bool few = L < CONV_FEW;
   auto run = [&](auto kern) {
     kern<<<dim3((C / 2 + 31) / 32, parts), 256, 0, st>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)prev,
                                                          (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, (__nv_bfloat16*)dx, partial, B, L, C,
                                                          act, xld, Ly, dxld, conv_bwd_run(B, L, C));
   };
   switch (K) {
-    case 1: run(conv1d_bwd_kernel<1>); break;
-    case 2: run(conv1d_bwd_kernel<2>); break;
-    case 3: run(conv1d_bwd_kernel<3>); break;
-    default: run(conv1d_bwd_kernel<4>); break;
+    case 1: run(conv1d_bwd_kernel<1, true>); break;
+    case 2: few ? run(conv1d_bwd_kernel<2, true>) : run(conv1d_bwd_kernel<2, false>); break;
+    case 3: few ? run(conv1d_bwd_kernel<3, true>) : run(conv1d_bwd_kernel<3, false>); break;
+    default: few ? run(conv1d_bwd_kernel<4, true>) : run(conv1d_bwd_kernel<4, false>); break;
   }
   const int n = (K + 1) * C;
   cudaMemsetAsync(dwdb, 0, sizeof(float) * n, st);

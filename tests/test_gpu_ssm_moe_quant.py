@@ -547,3 +547,27 @@ def test_conv1d_backward_runs(K, L):
     assert bool((grads[1][0] == grads[0][0]).all())
     for a, e in zip(grads[1][1:], grads[0][1:]):
         assert bool(((a.double() / n - e.double()).abs() <= 2.0 ** -7 * e.double().abs() + 2.0 ** -14 * e.double().abs().max()).all())
+
+
+@pytest.mark.parametrize("act", [0, 1])
+@pytest.mark.parametrize("L,shift", [(16, 0), (33, 0), (100, 0), (33, 4)])
+def test_conv1d_one_tap_of_large_inputs(L, shift, act):
+    """One tap on inputs that outgrow L2 takes 16-byte loads where the tensors lie on 16 bytes: the bits of a sequence by itself, which takes 8-byte ones."""
+    torch.manual_seed(L + shift)
+    C = 2048
+    n = (1 << 25) // (L * C) + 1
+    flat = torch.randn(n * L * C + 8, device="cuda").bfloat16()
+    x, w, b = flat[shift:shift + n * L * C].view(n, L, C), torch.randn(C, 1, device="cuda").bfloat16(), torch.randn(C, device="cuda").bfloat16()
+
+    def run(x):
+        y = torch.full((x.shape[0], L + 1, C), 7.0, device="cuda").bfloat16()
+        _lib.call("sx_conv1d_fwd", _lib.ptr(x), _lib.ptr(None), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), _lib.ptr(None), _lib.c_int(x.shape[0]), _lib.c_int(L),
+                  _lib.c_int(C), _lib.c_int(1), _lib.c_int(act), _lib.c_ll(C), _lib.c_int(L + 1), _lib.stream())
+        assert bool((y[:, L:] == 7.0).all())
+        return y[:, :L]
+
+    y = run(x)
+    assert all(torch.equal(y[i:i + 1], run(x[i:i + 1])) for i in (0, 1, n // 2, n - 1))
+    want = x.double() * w[:, 0].double() + b.double()
+    want = torch.nn.functional.silu(want) if act else want
+    assert bool(((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16 * ((x.double() * w[:, 0].double()).abs() + b.double().abs())).all())

@@ -54,3 +54,11 @@ def test_mixer_scratch_is_used_again(B, L, H, P, G, N, Q):
     a.B, a.L, a.H, a.P, a.G, a.N, a.Q, a.K, a.fused = B, L, H, P, G, N, Q, 4, int((Q, N, P) == (128, 128, 64))
     back, forward = size(ctypes.byref(a), 1), size(ctypes.byref(a), 0)
     assert 0 < forward < back <= held + 40 * 256, (back, held)
+
+
+@pytest.mark.parametrize("B,L,C", [(512, 1, 7168), (512, 7, 7168), (4096, 3, 256), (64, 64, 4096), (40, 130, 3584), (1, 8192, 7168), (4, 500, 1792), (1, 1, 64)])
+def test_conv1d_backward_takes_a_partial_row_for_512_positions(B, L, C):
+    """Runs of 64 positions are counted by what the sequences hold: 32 runs of 16 a partial row, or as many rows as make one wave of four CTAs an SM."""
+    parts = _lib.lib().sx_conv1d_bwd_parts(B, L, C)
+    runs, wave = B * ((L + 15) // 16), 148 * 4 // ((C // 2 + 31) // 32)
+    assert 1 <= parts <= max((runs + 31) // 32, wave, 1)
