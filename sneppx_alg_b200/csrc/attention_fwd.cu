@@ -16,9 +16,10 @@
 // arithmetic; nothing is materialised. An optional block mask (one byte per 128 x 128 score tile, per head or
 // shared) removes whole tiles from the walk: a step whose tile is masked for both query tiles is neither loaded nor
 // multiplied (block-sparse / flex-attention patterns at tile granularity).
-// Bound: exponentials (16 a cycle and SM: 2048 cycles for a step of both tiles, as many as its products take). B200, warm, before -> now:
-// [1, 4096, 32 / 8 heads, 128] causal 187 -> 130 us, [1, 8192, 8 / 2] full 288 -> 245, [8, 512, 28 / 4] causal 53 -> 44, [1, 16384, 32 / 8] causal
-// 2.28 -> 2.00 ms (1100 TFLOP/s, at the power cap).
+// Bound: exponentials (16 a cycle and SM: 2048 cycles for a step of both tiles, as many as its products take). B200, warm, captured calls, with one S a
+// tile -> now: [1, 4096, 32 / 8 heads, 128] causal 191 -> 135 us, [1, 8192, 8 / 2] full 281 -> 240, [8, 512, 28 / 4] causal 55 -> 43, [1, 16384, 32 / 8]
+// causal 2.28 -> 2.00 ms (1100 TFLOP/s, at the power cap). A block of one step is a chain from launch to store: [64, 128, 32 / 8] full 92 us either
+// way, 101 when the first loads came behind the block's set-up and each quarter of a row asked for a mask.
 // Takes the place of the reference's SIMT flash-attention forward, GQA and block-sparse kernels
 // (kernel/cuda/attention_cuda.cu:37-328, 498-573, 1154-1230) and its empty "v3" kernel (:1262-1286).
 #include <limits.h>
@@ -44,7 +45,7 @@ struct AttnFwdParams {
   int B, Sq, Skv, Hq, Hk;
   int v_head_div;  // V head = (K head) / v_head_div
   int causal, window;  // window <= 0: unlimited
-  int pairs, batch_first;   // pairs of query tiles; order of blocks
+  int pairs, order;    // pairs of query tiles; what the grid's axes are, see sx_attn_fwd
   float scale_log2;    // softmax scale * log2(e)
   const uint8_t* block_mask;   // optional [B or 1][Hq or 1][q tiles][kv tiles], non-zero = tile takes part
   long long bm_batch_stride, bm_head_stride;
@@ -102,10 +103,10 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  // blocks by head, then by sequence and pair of query tiles, or the other way round: see sx_attn_fwd
-  const int head = blockIdx.x % p.Hq, rest = blockIdx.x / p.Hq, inner = p.batch_first ? p.B : p.pairs;
-  const int b = p.batch_first ? rest % inner : rest / inner;
-  const int pair = p.pairs - 1 - (p.batch_first ? rest / inner : rest % inner);
+  const unsigned ax = blockIdx.x, ay = blockIdx.y, az = blockIdx.z;
+  const int head = p.order < 2 ? ax : ay;
+  const int b = p.order == 0 ? ay : p.order == 2 ? ax : az;
+  const int pair = p.pairs - 1 - (int)(p.order == 1 ? ay : p.order == 3 ? ax : az);
   const int kv_head = head / (p.Hq / p.Hk);
   const int v_head = kv_head / p.v_head_div;
   const int q0 = pair * 2 * ATT_BM;
@@ -138,7 +139,17 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
   const int first_step = jhi > jlo ? next_step(jlo - 1) : -1;
   const int n_steps = first_step >= 0 ? 1 : 0;   // only "are there any" is used below
 
-  if (threadIdx.x == 0) {
+  auto tma5 = [](void* dst, const CUtensorMap* m, uint64_t* bar, int c1, int c3, int c4) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(0), "r"(c1), "r"(0),
+        "r"(c3), "r"(c4)
+        : "memory");
+  };
+
+  // The loader sets up the barriers and sends for the first tiles while the other warps get TMEM and meet: a block of one step takes 12 thousand cycles,
+  // 1.5 of them up to there.
+  if (warp == ATT_TMA_WARP && elect_one()) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1);
@@ -152,34 +163,31 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
     mbar_init(s_free, 4);
     *s_abort = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&p.tmQ);
-    tma_prefetch_desc(&p.tmK);
-    tma_prefetch_desc(&p.tmV);
+    fence_proxy_async_smem();
+    if (n_steps > 0) {
+      mbar_expect_tx(q_full, 2 * Cfg::Q_BYTES);
+      tma5(sQ, &p.tmQ, q_full, q0, head, b);
+      tma5(sQ + Cfg::Q_BYTES, &p.tmQ, q_full, q0 + ATT_BM, head, b);
+      mbar_expect_tx(&k_full[0], Cfg::KV_BYTES);
+      tma5(sK, &p.tmK, &k_full[0], first_step * ATT_BN, kv_head, b);
+      mbar_expect_tx(&v_full[0], Cfg::KV_BYTES);
+      tma5(sV, &p.tmV, &v_full[0], first_step * ATT_BN, v_head, b);
+    }
   }
+  __syncwarp();
   if (warp == ATT_MMA_WARP) tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  auto tma5 = [](void* dst, const CUtensorMap* m, uint64_t* bar, int c1, int c3, int c4) {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(0), "r"(c1), "r"(0),
-        "r"(c3), "r"(c4)
-        : "memory");
-  };
-
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == ATT_TMA_WARP) {
       // ------------------------------------------------------------ TMA producer
       if (n_steps > 0 && elect_one()) {
-        mbar_expect_tx(q_full, 2 * Cfg::Q_BYTES);
-        tma5(sQ, &p.tmQ, q_full, q0, head, b);
-        tma5(sQ + Cfg::Q_BYTES, &p.tmQ, q_full, q0 + ATT_BM, head, b);
-        int j = 0;   // steps taken so far
-        for (int jt = first_step; jt >= 0; jt = next_step(jt), ++j) {
+        int j = 1;   // steps taken so far: the first one is on its way
+        for (int jt = next_step(first_step); jt >= 0; jt = next_step(jt), ++j) {
           const int s = j & 1;
           const uint32_t ph = (j >> 1) & 1;
           const int kv0 = jt * ATT_BN;
@@ -286,20 +294,20 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
       if (lane == 0) mbar_arrive(s_free);      // the other tile's scores may follow
       // four chains of three-operand maxima: one chain of 128 dependent ones takes as long as the exponentials of half a tile
       float mc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (need_mask) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (need_mask) {
+        for (int c = 0; c < 4; ++c) {
           const int h = hi_k - jt * ATT_BN - c * 32, w = lo_k - jt * ATT_BN - c * 32;
           const uint32_t seen = (h >= 31 ? 0xffffffffu : h < 0 ? 0u : (2u << h) - 1u) & (w <= 0 ? 0xffffffffu : w > 31 ? 0u : 0xffffffffu << w);
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             if (!(seen & (1u << i))) r[c * 32 + i] = 0xff800000u;  // -inf
         }
-#pragma unroll
-        for (int i = 0; i < 32; i += 8)
-#pragma unroll
-          for (int k = 0; k < 4; ++k) mc[k] = fmax3(mc[k], __uint_as_float(r[c * 32 + i + 2 * k]), __uint_as_float(r[c * 32 + i + 2 * k + 1]));
       }
+#pragma unroll
+      for (int i = 0; i < ATT_BN; i += 8)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mc[k] = fmax3(mc[k], __uint_as_float(r[i + 2 * k]), __uint_as_float(r[i + 2 * k + 1]));
       const float mx = fmaxf(fmax3(mc[0], mc[1], mc[2]), mc[3]) * p.scale_log2;
       float alpha = 1.f;
       bool rescale = false;
@@ -451,13 +459,15 @@ extern "C" int sx_attn_fwd(const SxAttnArgs* a, cudaStream_t st) {
   p.bm_head_stride = a->bm_head_stride;
   p.bm_kv_tiles = (a->Skv + ATT_BN - 1) / ATT_BN;
   // Blocks start heaviest first, so that the last ones to start are short: under a causal mask the last pair of query tiles walks the most keys.
-  // Over the whole batch where its keys and values stay in L2; otherwise one sequence after another, where the pairs of tiles that run at the
-  // same time share what they read.
+  // Heads are next to one another. Then the whole batch where its keys and values stay in L2; otherwise one sequence after another, where the pairs
+  // of tiles that run at the same time share what they read. The grid's axes are the three indices themselves (three divisions less in front of a
+  // block's first load, 450 cycles); only x holds more than 65535.
   p.pairs = (a->Sq + 2 * ATT_BM - 1) / (2 * ATT_BM);
-  p.batch_first = (long long)a->B * a->Skv * (a->Hk + v_heads) * a->D * 2 <= (64ll << 20);
-  const long long blocks = (long long)p.pairs * a->Hq * a->B;
-  if (blocks <= 0 || blocks > INT_MAX) return -4;
-  const dim3 grid((unsigned)blocks);
+  const bool batch_first = (long long)a->B * a->Skv * (a->Hk + v_heads) * a->D * 2 <= (64ll << 20);
+  p.order = a->B > 65535 ? 2 : p.pairs > 65535 ? 3 : batch_first ? 0 : 1;
+  const dim3 grids[4] = {dim3(a->Hq, a->B, p.pairs), dim3(a->Hq, p.pairs, a->B), dim3(a->B, a->Hq, p.pairs), dim3(p.pairs, a->Hq, a->B)};
+  const dim3 grid = grids[p.order];
+  if (grid.x == 0 || grid.y == 0 || grid.z == 0 || grid.y > 65535 || grid.z > 65535 || (long long)grid.x * grid.y * grid.z > INT_MAX) return -4;
   const bool masked = p.block_mask != nullptr;
   if (a->D == 128) return masked ? attn_fwd_launch<128, true>(p, grid, st) : attn_fwd_launch<128, false>(p, grid, st);
   return masked ? attn_fwd_launch<64, true>(p, grid, st) : attn_fwd_launch<64, false>(p, grid, st);

@@ -443,6 +443,33 @@ def test_attention_forward_of_a_batch_is_that_of_its_sequences(D):
     ops.check_status()
 
 
+@pytest.mark.parametrize("causal", [True, False])
+def test_attention_forward_of_many_short_sequences(causal):
+    """More sequences than the second axis of a grid holds: the bits that a few of them give alone."""
+    torch.manual_seed(3)
+    B, S = 65536 + 70, 3
+    q = torch.randn(B, S, 2, 64, device="cuda").bfloat16()
+    k, v = (torch.randn(B, S, 1, 64, device="cuda").bfloat16() for _ in range(2))
+    with torch.no_grad():
+        o = F_.attention(q, k, v, causal=causal)
+        for r in (slice(0, 40), slice(65520, 65560), slice(B - 40, B)):
+            assert torch.equal(o[r], F_.attention(q[r], k[r], v[r], causal=causal))
+    ops.check_status()
+
+
+def test_attention_forward_of_many_queries():
+    """More pairs of query tiles than the second axis of a grid holds, on three keys: the bits that the first and the last queries give alone."""
+    torch.manual_seed(4)
+    S = 65536 * 256 + 300
+    q = torch.randn(1, S, 1, 64, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.randn(1, 3, 1, 64, device="cuda").bfloat16() for _ in range(2))
+    with torch.no_grad():
+        o = F_.attention(q, k, v, causal=False)
+        for r in (slice(0, 600), slice(1 << 23, (1 << 23) + 600), slice(S - 600, S)):
+            assert torch.equal(o[:, r], F_.attention(q[:, r].contiguous(), k, v, causal=False))
+    ops.check_status()
+
+
 @pytest.mark.parametrize("key", [0, 70, 127, 128, 300])
 def test_attention_forward_passes_nan_scores_on(key):
     """A key of NaN makes every query that sees it NaN and leaves the others as they are; queries that see no key are zero."""
