@@ -385,6 +385,28 @@ def test_attention_backward_of_one_query_zeroes_with_many_ctas():
     assert us[1] < us[0] + 14, us
 
 
+@pytest.mark.parametrize("Sq,Skv,causal,window", [(1, 200, True, 0), (33, 33, True, 0), (64, 300, False, 0), (65, 65, True, 0), (128 + 1, 129, True, 0), (128 + 64, 400, True, 0),
+                                                  (128 + 65, 193, False, 0), (256 + 40, 296, True, 50)])
+def test_attention_backward_reads_no_column_behind_the_last_query(Sq, Skv, causal, window):
+    """A last tile of at most 64 queries leaves half of the probabilities' and their gradients' columns as they were. What lay there before, values of
+    another call or NaN of one whose inputs were NaN, does not show: the bits of a call after one of finite values."""
+    torch.manual_seed(Sq)
+    H, Hk = 6, 2
+    q, do = (torch.randn(1, Sq, H, 128, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(1, Skv, Hk, 128, device="cuda").bfloat16() for _ in range(2))
+    o, lse = F_.attention_with_lse(q, k, v, causal=causal, window=window)
+    bad = [torch.full((1, 1024, 37 * 4, 128), float("nan"), device="cuda").bfloat16() for _ in range(2)]
+    got = []
+    for poison in (False, True, True):
+        if poison:      # every SM's shared memory and TMEM
+            F_.attention_backward(bad[0], bad[0], bad[0], bad[0], torch.zeros(1, 37 * 4, 1024, device="cuda"), bad[1], causal=False)
+        got.append(F_.attention_backward(q, k, v, o, lse, do, causal=causal, window=window))
+    ops.check_status()
+    for g in got[1:]:
+        assert torch.equal(g[1], got[0][1]) and torch.equal(g[2], got[0][2])          # dK and dV keep their bits, dQ is summed in any order
+        assert (g[0].float() - got[0][0].float()).norm() <= 2.0 ** -8 * got[0][0].float().norm()
+
+
 def _attention64(q, k, v, do, causal, window):
     """Output and gradients in 64 bits, and the probabilities' sum over the keys."""
     q, k, v = (t.double().requires_grad_() for t in (q, k, v))
