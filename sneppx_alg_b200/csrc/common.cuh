@@ -74,11 +74,18 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // would promise the compiler that nobody else writes the memory while the kernel runs, and let it load around the cache's coherence or ahead of the
 // wait, but until the wait returns the kernel before does write it. Whether it lets its own successor start early is up to it: after_predecessor()
 // does, the paged decode kernel does not.
-// A chain of kernels that do holds nothing back. Loads in front of a wait (the static weights of a decode product) may pass all of them, up to the last
-// kernel that was not launched this way or did not signal: no kernel behind that one may write what is loaded so.
-__device__ __forceinline__ void after_predecessor() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the same for the kernel after this one
+// A chain of kernels that signal before they wait holds nothing back. Loads in front of a wait (the static weights of a decode product) may pass all of
+// them, up to the last kernel that was not launched this way or did not signal: no kernel behind that one may write what is loaded so.
+// When to let the successor start: at once where this kernel leaves the SMs nearly empty, so that the successor's set-up and first loads of weights lie
+// under the wait (eight norms and products of one row of 768: 78 us, 83 behind the wait; a step of an 8B decoder for one sequence 7.9 and 8.2 ms); behind the
+// wait from three warps an SM on, because kernels that wait hold places, and what follows is dealt out unevenly around them (eight norms of 300 rows of
+// 16384 106 and 69 us, 73 launched ordinarily). `most` CTAs: above that not at all, for the same reason where a CTA's share is long (600 rows: 159 us, 111).
+__device__ __forceinline__ void after_predecessor(unsigned most = 0xffffffffu) {
+  const unsigned ctas = gridDim.x * gridDim.y * gridDim.z;
+  const bool small = (unsigned long long)ctas * (blockDim.x * blockDim.y) <= 148 * 96;
+  if (small) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");                // all that kernels before this one wrote is there
+  if (!small && ctas <= most) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... K, typename... A>
 inline cudaError_t launch_dependent(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {

@@ -38,7 +38,7 @@ __device__ __forceinline__ bf16x8 ld8_once(const __nv_bfloat16* p) {
 template <int V, bool RES>
 __global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* res_in, const __nv_bfloat16* w,
                                                           __nv_bfloat16* y, __nv_bfloat16* res_out, float* rstd, int d, float eps) {
-  after_predecessor();
+  after_predecessor(2 * 148);
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const int nvec = d >> 3, t = threadIdx.x;
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(512) rmsnorm_fwd_kernel(const __nv_bfloat16* x
 // Rows longer than 8192: two passes.
 __global__ void __launch_bounds__(256) rmsnorm_fwd_long_kernel(const __nv_bfloat16* x, const __nv_bfloat16* res_in, const __nv_bfloat16* w,
                                                                __nv_bfloat16* y, __nv_bfloat16* res_out, float* rstd, int d, float eps) {
-  after_predecessor();
+  after_predecessor(2 * 148);
   __shared__ float red[33];
   const long long row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * d;

@@ -280,6 +280,32 @@ def _median_us(fn, n=11):
     return sorted(ts)[n // 2]
 
 
+@pytest.mark.parametrize("T,d", [(16, 4096), (128, 4096), (300, 16384), (600, 16384), (1000, 768)])
+def test_norms_in_a_row_gain_by_starting_early(T, d):
+    """Norms that are set up while their predecessors run are not slower for it: sixteen in a row take no longer than with an ordinarily launched kernel
+    between each two, which they would wait for. With every norm signalling at once 16 of [300, 16384] took 212 us, 160 so."""
+    x, w = torch.randn(T, d, device="cuda").bfloat16(), torch.ones(d, device="cuda").bfloat16()
+    y, one = torch.empty_like(x), torch.zeros(1, device="cuda")
+
+    def norms(spaced):
+        for _ in range(8):
+            for a, b in ((x, y), (y, x)):
+                _lib.call("sx_rmsnorm_fwd", _lib.ptr(a), _lib.ptr(None), _lib.ptr(w), _lib.ptr(b), _lib.ptr(None), _lib.ptr(None), _lib.c_ll(T), _lib.c_int(d),
+                          _lib.c_float(1e-5), stream())
+                if spaced:
+                    one.zero_()
+
+    us = []
+    for spaced in (False, True):
+        norms(spaced)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            norms(spaced)
+        us.append(_median_us(graph.replay))
+    assert us[0] <= us[1] * 1.05, us
+
+
 @pytest.mark.parametrize("T,heads,rot,D", [(1, 1, 1, 16), (131, 1, 1, 16), (300, 3, 2, 48), (64, 15, 15, 128), (147, 16, 10, 128), (148, 16, 10, 128),
                                            (5, 96, 80, 256), (200, 97, 90, 256)])
 def test_rope_launch_shapes(T, heads, rot, D):

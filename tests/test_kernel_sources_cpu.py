@@ -21,7 +21,7 @@ def test_kernels_that_start_early_promise_nothing_about_their_inputs():
     for src in _build.cuda_sources():
         text = re.sub(r"//[^\n]*", "", src.read_text())
         for name, params, body in _kernels(text):
-            if re.search(r"after_predecessor\(\)|griddepcontrol\.wait|griddep_wait\(\)", body):
+            if re.search(r"after_predecessor\(|griddepcontrol\.wait|griddep_wait\(\)", body):
                 waiting[name] = params
         launched |= set(re.findall(r"launch_dependent\((\w+_kernel)", text))
         for m in re.finditer(r"auto run = \[&\]\(auto kern[^{]*\{\s*launch_dependent\(kern", text):
