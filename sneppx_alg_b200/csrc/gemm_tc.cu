@@ -1031,9 +1031,6 @@ static int launch_cfg2_any(const GemmKernelParams& kp, int am, int bm, int sms, 
 
 }  // namespace sx
 
-extern "C" int sx_gemm_skinny_ok(const SxGemmArgs* a);
-extern "C" int sx_gemm_skinny(const SxGemmArgs* a, cudaStream_t st);
-
 static int gemm_launch(const SxGemmArgs* a, const SxGemmCommArgs* cm, cudaStream_t st) {
   using namespace sx;
   if (a->M <= 0 || a->N <= 0 || a->batch <= 0) return 0;

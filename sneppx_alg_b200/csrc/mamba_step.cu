@@ -133,9 +133,6 @@ __global__ void __launch_bounds__(32 * MS_WARPS, 4) mamba_step_kernel(const SxMa
 }  // namespace sx
 using namespace sx;
 
-extern "C" int sx_rmsnorm_fwd(const void* x, const void* res_in, const void* w, void* y, void* res_out, float* rstd, long long T, int d,
-                              float eps, cudaStream_t st);
-
 static int mamba_gemm(const void* x, const void* w, void* y, int M, int N, int K, int* status, cudaStream_t st) {
   SxGemmArgs a = {};
   a.A = x; a.B = w; a.D = y;

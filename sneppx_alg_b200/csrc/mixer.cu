@@ -5,33 +5,6 @@
 // of a block of width 768 whose kernels take 0.4 ms. Scratch is one block that the caller allocates (sx_mixer_workspace).
 #include "sx_api.h"
 
-extern "C" {
-int sx_conv1d_fwd(const void*, const void*, const void*, const void*, void*, void*, int, int, int, int, int, long long, int, cudaStream_t);
-int sx_conv1d_bwd_parts(int, int, int);
-int sx_conv1d_bwd(const void*, const void*, const void*, const void*, const void*, void*, float*, float*, int, int, int, int, int, long long, int,
-                  long long, cudaStream_t);
-int sx_ssd_build_m(const void*, const void*, const void*, void*, long long, int, int, int, cudaStream_t);
-int sx_ssd_bwd_qq(const void*, const void*, const void*, const void*, void*, void*, void*, void*, long long, int, int, int, cudaStream_t);
-int sx_ssd_state_fwd(const void*, const void*, const void*, void*, void*, int, int, int, int, cudaStream_t);
-int sx_ssd_state_bwd(const void*, const void*, const void*, const void*, void*, void*, void*, int, int, int, int, cudaStream_t);
-int sx_ssd_scale_rows(const void*, const void*, void*, long long, int, int, long long, int, int, cudaStream_t);
-int sx_ssd_combine(const void*, const void*, const void*, const void*, const void*, void*, long long, int, int, int, long long, int, cudaStream_t);
-int sx_ssd_bwd_rows1(const void*, const void*, const void*, const void*, void*, void*, void*, long long, int, int, long long, int, int, cudaStream_t);
-int sx_ssd_bwd_rows2(const void*, const void*, const void*, const void*, const void*, const void*, void*, void*, long long, int, int, int, long long,
-                     int, long long, cudaStream_t);
-int sx_ssd_heads_first(const void*, long long, void*, long long, int, int, int, cudaStream_t);
-int sx_ssd_chunk_fwd(const void*, long long, const void*, long long, const void*, long long, const void*, const void*, const void*, const void*, void*,
-                     long long, int, int, int*, cudaStream_t);
-int sx_gate_mul_fwd(const void*, const void*, long long, void*, long long, int, int, int, cudaStream_t);
-int sx_gate_mul_bwd(const void*, const void*, const void*, long long, void*, void*, long long, int, int, int, long long, cudaStream_t);
-int sx_mix_prep(const void*, long long, const float*, const float*, float*, float*, float*, float*, float*, int, int, int, int, int, cudaStream_t);
-int sx_mix_finish(const void*, long long, const float*, const float*, const float*, const float*, const float*, const float*, const float*, const float*,
-                  const float*, const float*, const float*, void*, long long, float*, int, int, int, int, int, cudaStream_t);
-int sx_mix_pack(const void*, long long, void*, long long, int, int, int, cudaStream_t);
-int sx_mix_unpack(const float*, const float*, void*, long long, long long, int, int, int, cudaStream_t);
-int sx_mix_sum(const void*, void*, long long, int, int, cudaStream_t);
-}
-
 namespace sx {
 
 typedef uint16_t h16;   // bf16 storage

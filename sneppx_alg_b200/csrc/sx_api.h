@@ -38,6 +38,44 @@ typedef struct SxGemmArgs {
 } SxGemmArgs;
 int sx_gemm_bf16(const SxGemmArgs* args, cudaStream_t stream);
 
+// ------------------------------------------------------------------ entry points that others call in C (norm_rope.cu, conv1d.cu, ssd*.cu, gemm_skinny.cu)
+// Declared once, before their definitions: with C linkage the linker would not notice arguments that differ.
+int sx_gemm_skinny_ok(const SxGemmArgs* args);
+int sx_gemm_skinny(const SxGemmArgs* args, cudaStream_t stream);
+int sx_rmsnorm_fwd(const void* x, const void* res_in, const void* w, void* y, void* res_out, float* rstd, long long T, int d, float eps, cudaStream_t stream);
+int sx_conv1d_fwd(const void* x, const void* prev, const void* w, const void* bias, void* y, void* state_out, int B, int L, int C, int K, int act,
+                  long long xld, int Ly, cudaStream_t stream);
+int sx_conv1d_bwd_parts(int B, int L, int C);
+int sx_conv1d_bwd(const void* dy, const void* x, const void* prev, const void* w, const void* bias, void* dx, float* partial, float* dwdb, int B, int L,
+                  int C, int K, int act, long long xld, int Ly, long long dxld, cudaStream_t stream);
+int sx_ssd_build_m(const void* CB, const void* cs, const void* dt, void* M, long long BC, int H, int G, int Q, cudaStream_t stream);
+int sx_ssd_bwd_qq(const void* dM, const void* CB, const void* cs, const void* dt, void* M, void* dGh, void* rowW, void* colU, long long BC, int H,
+                  int G, int Q, cudaStream_t stream);
+int sx_ssd_state_fwd(const void* S, const void* tot, const void* init, void* Hprev, void* fin, int B, int nc, int H, int PN, cudaStream_t stream);
+int sx_ssd_state_bwd(const void* dHprev, const void* tot, const void* Hprev, const void* dfin, void* dS, void* dtot, void* dinit, int B, int nc,
+                     int H, int PN, cudaStream_t stream);
+int sx_ssd_scale_rows(const void* a, const void* scale, void* out, long long rows, int P, int H, long long ald, int Q, int G, cudaStream_t stream);
+int sx_ssd_combine(const void* Yi, const void* Yoff, const void* x, const void* E, const void* D, void* y, long long rows, int H, int Q, int P,
+                   long long xld, int G, cudaStream_t stream);
+int sx_ssd_bwd_rows1(const void* dy, const void* x, const void* Yoff, const void* E, void* dye, void* dcs, void* ddrow, long long rows, int P, int H,
+                     long long xld, int Q, int G, cudaStream_t stream);
+int sx_ssd_bwd_rows2(const void* dy, const void* x, const void* dxw, const void* dxi, const void* decay, const void* D, void* dx, void* ddecay,
+                     long long rows, int H, int Q, int P, long long xld, int G, long long dxld, cudaStream_t stream);
+int sx_ssd_heads_first(const void* in, long long ild, void* out, long long rows, int H, int Q, int P, cudaStream_t stream);
+int sx_ssd_chunk_fwd(const void* C, long long c_ld, const void* B, long long b_ld, const void* x, long long x_ld, const void* Hprev, const void* cs,
+                     const void* dt, const void* D, void* y, long long BC, int H, int G, int* status, cudaStream_t stream);
+int sx_gate_mul_fwd(const void* y, const void* z, long long zld, void* out, long long rows, int C, int L, int Lp, cudaStream_t stream);
+int sx_gate_mul_bwd(const void* g, const void* y, const void* z, long long zld, void* dy, void* dz, long long rows, int C, int L, int Lp,
+                    long long dzld, cudaStream_t stream);
+int sx_mix_prep(const void* raw, long long ld, const float* bias, const float* a_log, float* dth, float* csh, float* E, float* decay, float* tot,
+                int B, int nc, int L, int H, int Q, cudaStream_t stream);
+int sx_mix_finish(const void* raw, long long ld, const float* bias, const float* a_log, const float* dth, const float* csh, const float* ddecay,
+                  const float* dcs, const float* ddrow, const float* rowW, const float* colU, const float* dtot, const float* tot, void* draw,
+                  long long dld, float* part, int B, int nc, int L, int H, int Q, cudaStream_t stream);
+int sx_mix_pack(const void* in, long long ld, void* out, long long rows, int G, int Q, int N, cudaStream_t stream);
+int sx_mix_unpack(const float* dB, const float* dC, void* out, long long ld, long long rows, int G, int Q, int N, cudaStream_t stream);
+int sx_mix_sum(const void* in, void* out, long long n, int rep, int M, cudaStream_t stream);
+
 // ------------------------------------------------------------------ mixer of a Mamba-2 block (mixer.cu)
 // zx [B, L, W = z | x | B | C | dt] bf16 contiguous, 16-byte aligned; conv_w [channels, K], conv_b bf16; dt_bias, a_log, D [H] fp32.
 // Chunks of Q tokens, nc of them a sequence, Lp = nc * Q.

@@ -31,6 +31,15 @@ def test_kernels_that_start_early_promise_nothing_about_their_inputs():
     assert not [n for n, params in waiting.items() if "__restrict__" in params]
 
 
+def test_entry_points_are_declared_in_one_place():
+    """C linkage: a declaration beside a caller would link to whatever has the name. What one source calls of another is in the header that both include."""
+    for src in _build.cuda_sources():
+        text = src.read_text()
+        assert not re.findall(r'^extern "C"[^{;]*;', text, re.M), src.name
+        for block in re.findall(r'^extern "C" \{(.*?)^\}', text, re.M | re.S):
+            assert not re.findall(r"^\w[^{};()]*\([^{}()]*\);", block, re.M), src.name
+
+
 def test_ssd_output_stage_waits_for_the_tile_that_its_epilogue_reads():
     """The epilogue warps read x from shared memory that TMA filled: they wait for that transfer's barrier themselves, not only for the product's."""
     text = (_build.CSRC / "ssd_fwd.cu").read_text()
