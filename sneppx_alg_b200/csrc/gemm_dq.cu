@@ -15,8 +15,8 @@
 //              so it is one multiply-add per value. Products are therefore exact and nothing is rounded to bf16 before the output.
 // Two CTAs share an SM up to 32 rows of X, so that one converts while the other waits.
 // Measured (B200, graph replay, cold weights), int4 [28672, 4096] at 1 / 16 / 32 / 64 / 128 rows: 24 / 24 / 27 / 33 / 51 us, [4096, 14336]
-// 15 / 15 / 16 / 16 / 23 us; 28 / 28 / 30 / 39 / 62 and 16 / 17 / 17 / 19 / 28 us when operands were moved to uniform registers for each
-// MMA (tc_common.cuh), 203 / 199 / 199 / 199 / 201 and 361 / 354 / 353 / 353 / 356 us when 128 x 128 output tiles left most SMs idle and four
+// 15 / 15 / 16 / 16 / 23 us; 28 / 28 / 30 / 39 / 62 and 16 / 17 / 17 / 19 / 28 us when MMAs were issued behind `lane == 0`
+// (tc_common.cuh), 203 / 199 / 199 / 199 / 201 and 361 / 354 / 353 / 353 / 356 us when 128 x 128 output tiles left most SMs idle and four
 // converter warps wrote scaled bf16 tiles to shared memory. The floor (packed weights at copy bandwidth) is 9 and 4.5 us. K of 128 or 256 with
 // more than one wave of tiles: gemm_dq_short.cu.
 // The reference has quantise / dequantise kernels only (kernel/quantization/quantize_cuda.cu), no GEMM on them.
@@ -79,15 +79,6 @@ __device__ __forceinline__ float4 dq_ld_peer(uint32_t local_addr, uint32_t rank)
                : "r"(ra)
                : "memory");
   return v;
-}
-
-__device__ __forceinline__ void dq_tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-      "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
-      "r"(r[14]), "r"(r[15])
-      : "memory");
 }
 
 template <int BT, bool INT4>
@@ -236,13 +227,13 @@ __global__ void __launch_bounds__(DqCfg<BT>::THREADS, DqCfg<BT>::CTAS) gemm_dq_k
             int4x8_to_bf16(w[c].y, o + 4);
             int4x8_to_bf16(w[c].z, o + 8);
             int4x8_to_bf16(w[c].w, o + 12);
-            dq_tmem_st16(tA + c * 16, o);
+            tmem_st16(tA + c * 16, o);
           } else {
             e4m3x4_to_bf16(w[c].x, o + (c & 1) * 8);
             e4m3x4_to_bf16(w[c].y, o + (c & 1) * 8 + 2);
             e4m3x4_to_bf16(w[c].z, o + (c & 1) * 8 + 4);
             e4m3x4_to_bf16(w[c].w, o + (c & 1) * 8 + 6);
-            if (c & 1) dq_tmem_st16(tA + h * 32 + (c >> 1) * 16, o);
+            if (c & 1) tmem_st16(tA + h * 32 + (c >> 1) * 16, o);
           }
         }
       }

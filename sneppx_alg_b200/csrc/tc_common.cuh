@@ -38,10 +38,9 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// Warp index and one lane of a warp, in the forms that the compiler knows to be uniform / a single thread: operands of the tcgen05 and TMA
-// instructions behind them are then computed in uniform registers. Behind `lane == 0` each operand is moved there first: an issuing thread takes
-// 58 cycles for a 128 x 16 x 16 tcgen05.mma, 16 so (64 cycles of work in one of 128 x 128 x 16 just hide it, with nothing else to issue).
-// Reading int4 [28672, 4096] for 16 rows 27.8 -> 24.0 us, bf16 [2560, 5120] for one row 8.7 -> 7.9 us.
+// Warp index from a shuffle, and one elected lane of a warp. An issuing thread takes 58 cycles for a
+// 128 x 16 x 16 tcgen05.mma behind `lane == 0`, 16 behind these (64 cycles of work in one of 128 x 128 x 16 just hide the former, with nothing else
+// to issue). Reading int4 [28672, 4096] for 16 rows 27.8 -> 24.0 us, bf16 [2560, 5120] for one row 8.7 -> 7.9 us.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
@@ -72,28 +71,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
   return ok != 0;
-}
-
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {   // does not suspend the thread
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bound of a thread that polls several barriers, asked now and then: `t0` is 0 when the wait begins. False: given up.
-__device__ __forceinline__ bool mbar_poll_time(uint64_t& t0, volatile int* s_abort, int* g_status, int code) {
-  if (*s_abort) return false;
-  const uint64_t now = globaltimer_ns();
-  if (t0 == 0) t0 = now;
-  else if (now - t0 > SX_WAIT_TIMEOUT_NS) {
-    *s_abort = 1;
-    if (g_status) atomicCAS(g_status, 0, code);
-    return false;
-  }
-  return true;
 }
 
 // Bounded wait on an mbarrier phase. `s_abort` is a CTA-shared flag; `g_status` the kernel's

@@ -174,7 +174,7 @@ class SxWinAttnArgs(C.Structure):
 _lock = threading.Lock()
 _lib = None
 _status = {}
-launch_count = 0  # number of kernel-library entry points called (bench.py reports it)
+launch_count = 0  # number of kernel-library entry points called, each of which launches one or more kernels (bench.py reports it)
 
 
 def lib() -> C.CDLL:

@@ -220,7 +220,6 @@ def decode_step(model, states, seq_ids, last_tokens):
             a.conv_w, a.conv_b = own["conv_weight"].data_ptr(), own["conv_bias"].data_ptr()
             a.dt_bias, a.a_log, a.D = own["dt_bias"].data_ptr(), own["A_log"].data_ptr(), own["D"].data_ptr()
             _lib.call("sx_mamba2_step", C.byref(a), stream)
-        _lib.launch_count += 4 * L      # five kernels a call
         last = x if L == 1 else res[1 - ((L - 1) & 1)]
         _lib.call("sx_rmsnorm_fwd", _lib.ptr(out), _lib.ptr(last), _lib.ptr(model.norm.weight), _lib.ptr(hn), _lib.ptr(None), _lib.ptr(None),
                   _lib.c_ll(B), _lib.c_int(d), _lib.c_float(model.norm.eps), stream)
